@@ -120,6 +120,11 @@ int plan_layout(int64_t n, int bits, int num_digits, Layout* L, bool allow_split
   *L = Layout();
   L->api_bits = bits;
   L->sub = 1;
+  // A whole sort's result is the stable order of the 64-bit keys whatever the
+  // digit width, so it need not go digit by digit, unless a pass kernel of
+  // another family or shape is asked for by name (LSB_WIDE_DIGITS, LSB_ONESWEEP_VARIANT).
+  const bool whole_sort = allow_split && !compact && num_digits == lsb_num_passes(bits) &&
+                          wide_mode() == WideMode::kSplit && onesweep_variant() == 0;
   if (bits == 16 && !compact && wide_mode() == WideMode::kWide) {
     // one pass per 16-bit digit (lsb_wide.cu)
     L->family = Family::kWide;
@@ -175,13 +180,20 @@ int plan_layout(int64_t n, int bits, int num_digits, Layout* L, bool allow_split
     L->off_dstart = off;
     off = align_up(off + nbins * 4u, 256);
   }
-  L->total = off;
+  L->total = off;  // the pass kernels' need, so that a workspace serves every route
+  if (whole_sort && (uint64_t)n <= top_small_limit()) {
+    // one CTA sorts the whole array: the control block is all it uses
+    L->family = Family::kTop;
+    L->stat_bits = bits;
+    L->stat_digits = num_digits;
+  }
   return 0;
 }
 
 int run_passes(Elem* X, Elem* Y, int first_digit, int target_parity, void* ws, const Layout& L,
                cudaStream_t st) {
   unsigned char* w = static_cast<unsigned char*>(ws);
+  if (L.family == Family::kTop) return top_run(X, Y, w, L, st) ? LSB_ERR_CUDA : LSB_OK;
   if (cudaMemsetAsync(w, 0, kCtrlBytes, st) != cudaSuccess) return LSB_ERR_CUDA;
   first_digit *= L.sub;  // split wide digits: sub-digits 2d and 2d+1
   int rc = (L.family == Family::kOnesweep) ? onesweep_run(X, Y, first_digit, target_parity, w, L, st)

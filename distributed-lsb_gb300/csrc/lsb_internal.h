@@ -9,6 +9,8 @@
 //    16-bit digit and one HBM round trip per pass; tiles are sorted by the
 //    digit's high byte into an L2-resident chunk buffer, then each high-byte
 //    bucket of a chunk is gathered and placed by its low byte (lsb_wide.cu).
+//  * "top" family (whole sorts): one CTA sorts an array that fits in its shared
+//    memory in one launch (lsb_top.cu).
 //  * "task" family (digit_bits >= 12, the reference's 16-bit digits): per pass
 //    a count kernel over contiguous tasks, a digit-major scan of the
 //    [digit][task] count table and a stable scatter -- the reference's own
@@ -32,7 +34,7 @@ struct DeviceInfo {
 // Properties of the current device (cached per device id).
 int current_device_info(DeviceInfo* info);
 
-enum class Family { kOnesweep = 0, kTask = 1, kWide = 2 };
+enum class Family { kOnesweep = 0, kTask = 1, kWide = 2, kTop = 3 };
 
 // Byte offsets inside the caller's workspace (all 256-byte aligned).
 struct Layout {
@@ -60,6 +62,10 @@ struct Layout {
   // region of lsb_wide.cu (scheduler, bucket sizes, running prefixes, chunk
   // buffers, piece tables, status ring)
   size_t off_wide = 0;
+  // top family: digits of the plan that lsb_query reports (the kernels' own
+  // digits are the onesweep family's, see plan_layout)
+  int stat_bits = 0;
+  int stat_digits = 0;
 };
 
 // allow_split: digits of 12, 14 or 16 bits may run as two half-width
@@ -81,6 +87,11 @@ int task_run(Elem* X, Elem* Y, int first_digit, int target_parity, unsigned char
              const Layout& L, cudaStream_t st);
 int wide_run(Elem* X, Elem* Y, int first_digit, int target_parity, unsigned char* ws,
              const Layout& L, cudaStream_t st);
+// Whole sort by the top family; the result is in X. The control block is
+// cleared by the kernels.
+int top_run(Elem* X, Elem* Y, unsigned char* ws, const Layout& L, cudaStream_t st);
+// Largest array of the one-CTA sort.
+uint32_t top_small_limit();
 // One wide digit as two half-width onesweep passes src -> mid -> dst (L: a
 // split layout of two sub-digits starting at first_digit); src is not written.
 int onesweep_pass_via(const Elem* src, Elem* mid, Elem* dst, int first_digit, unsigned char* ws,
@@ -99,6 +110,8 @@ int hist16(const Elem* data, uint32_t n, int first_digit, int num_digits, uint32
 // constant digits (skipped), buffer parity of every pass (lsb_onesweep.cu).
 __global__ void __launch_bounds__(1024) k_plan(const uint32_t* __restrict__ ghist, uint32_t* __restrict__ gstart, uint32_t n,
                        int bits, int num_digits, int target_parity, int api_bits, int sub, Ctrl* ctrl);
+// LSB_ONESWEEP_VARIANT, 0 when unset: another value selects a shape of the pass kernel.
+int onesweep_variant();
 uint32_t onesweep_tile_elems(int bits);
 // the look-back wait of the sort kernels on a predecessor that never publishes
 // (failure-detection self-test); ws: kCtrlBytes + 32 bytes, zeroed by the caller

@@ -1333,7 +1333,7 @@ struct OnesweepChoice {
   size_t smem;
 };
 
-static int onesweep_variant() {
+int onesweep_variant() {
   const char* e = std::getenv("LSB_ONESWEEP_VARIANT");
   const int v = e ? std::atoi(e) : 0;
   return (v >= 0 && v <= 4) ? v : 0;

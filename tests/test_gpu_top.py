@@ -1,0 +1,58 @@
+"""The sort of whole arrays without going through every digit: arrays of one
+shared-memory tile in one launch. Sizes at the edges of the tile shapes, key
+sets that are even, clustered, duplicated, ordered and constant; bit-exact
+against the oracle's stable sort, and the plan lsb_query reports."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from conftest import to_dev, to_np
+
+pytestmark = pytest.mark.gpu
+
+
+def _elems(keys):
+    a = np.empty((len(keys), 2), dtype=np.uint64)
+    a[:, 0] = keys
+    a[:, 1] = np.arange(len(keys), dtype=np.uint64)
+    return a
+
+
+def key_sets(n, seed):
+    """Named key arrays (uint64) of n elements: what a tile's bins meet."""
+    r = np.random.default_rng(seed)
+    full = r.integers(0, 1 << 64, n, dtype=np.uint64)
+    yield "uniform", full
+    yield "reverse", np.sort(full)[::-1].copy()
+    yield "few", r.integers(0, 3, n).astype(np.uint64)
+    yield "dups", full[r.integers(0, max(1, n // 30), n)]
+    # an even spread and one cluster whose keys agree in all but their lowest bits
+    c = full.copy()
+    c[: n // 2] = np.uint64(1 << 60) + r.integers(0, 1000, n // 2).astype(np.uint64)
+    yield "cluster", r.permutation(c)
+    yield "extremes", np.where(r.random(n) < 0.5, np.uint64(0), np.uint64(2**64 - 1))
+    yield "low_bits", (full & np.uint64(0xFFF)) | np.uint64(0xABCDEF << 40)
+    # neighbours in the last bits of a wide range: the slots' key bits tie
+    yield "close", np.repeat(full[: n // 2 + 1], 2)[:n] ^ r.integers(0, 2, n).astype(np.uint64)
+
+
+def _run(lsb, cuda, a, bits):
+    A = to_dev(a, cuda)
+    B = cuda.empty_like(A)
+    ws = lsb.alloc_workspace(a.shape[0], bits)
+    lsb.sort_pairs(A, B, bits, workspace=ws)
+    return to_np(A), lsb.query(ws)
+
+
+@pytest.mark.parametrize("n", [2, 31, 33, 511, 513, 1000, 4607, 4608, 4609, 9215, 9216, 9217])
+def test_one_tile(lsb, cuda, oracle, n):
+    for name, keys in key_sets(n, n):
+        a = _elems(keys)
+        got, st = _run(lsb, cuda, a, 8)
+        assert np.array_equal(got, oracle.stable_sort_by_key(a)), (n, name)
+        diff = int(np.bitwise_or.reduce(keys ^ keys[0]))
+        skipped = sum(1 << d for d in range(8) if not (diff >> (8 * d)) & 0xFF)
+        runs = 8 - bin(skipped).count("1")
+        assert (st.device_status, st.passes_planned, st.skipped_mask, st.passes_run, st.final_copy, st.n) == (
+            0, 8, skipped, runs, runs & 1, n), (n, name)
