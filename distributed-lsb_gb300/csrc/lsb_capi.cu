@@ -181,11 +181,22 @@ int plan_layout(int64_t n, int bits, int num_digits, Layout* L, bool allow_split
     off = align_up(off + nbins * 4u, 256);
   }
   L->total = off;  // the pass kernels' need, so that a workspace serves every route
-  if (whole_sort && (uint64_t)n <= top_small_limit()) {
-    // one CTA sorts the whole array: the control block is all it uses
+  if (whole_sort && top_serves((uint32_t)n)) {
     L->family = Family::kTop;
     L->stat_bits = bits;
     L->stat_digits = num_digits;
+    L->bits = 8;
+    L->num_digits = 8;
+    off = kCtrlBytes;
+    L->off_hist = off;
+    off = align_up(off + 8u * 256u * 4u, 256);
+    L->off_gstart = off;
+    off = align_up(off + 8u * 256u * 4u, 256);
+    L->tile_elems = onesweep_top_tile();
+    L->ring_tiles = std::max<uint32_t>(1u, (uint32_t)((n + L->tile_elems - 1) / L->tile_elems));
+    L->off_ring = off;
+    off = align_up(off + (size_t)L->ring_tiles * 256u * 8u, 256);
+    L->total = std::max(L->total, off);
   }
   return 0;
 }

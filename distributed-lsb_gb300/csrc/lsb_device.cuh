@@ -28,11 +28,33 @@ constexpr uint32_t kWhereLookback = 1;
 constexpr uint32_t kWhereRingReuse = 2;
 constexpr uint32_t kWhereScatter = 3;
 constexpr uint32_t kWhereBulkCopy = 6;   // a bulk copy's completion barrier
+constexpr uint32_t kWhereGridBarrier = 8;  // the grid barrier of the run merges
 
 // Spin limit for every device-side wait: after this many polls (with a
 // nanosleep back-off of up to 256 ns each) the kernel records
 // kStatusTimeout, skips its stores and returns, so no wait can hang the GPU.
 constexpr uint32_t kSpinLimit = 1u << 22;
+
+// Device-side plan of a sort by top digits (lsb_top.cu), chosen from a sample
+// of the keys. With the key shifted left until bit `hb1` is out, the digits
+// are its `passes` highest bytes, lowest first. Keys outside the block
+// [lo, hi] of 2^hb1 keys count as all zeros (below) or all ones (above), which
+// keeps the digits in key order whatever the sample missed.
+struct TopPlan {
+  uint64_t lo, hi;
+  uint32_t hb1;            // 64: the block is the whole key range
+  uint32_t passes;
+  uint32_t run_mask;       // bit p: pass p runs (its digit is not constant)
+  uint32_t par_mask;       // bit p: pass p reads Y, writes X
+  uint32_t src_parity;     // 1: the passes leave the data in Y
+  uint32_t complete;       // the digits cover every bit in which keys differ
+  uint32_t diff[2];        // bits in which some key differs from the first one
+  uint32_t hist_done;      // CTAs of the histogram that have finished
+  uint32_t num_chunks;     // chunks of runs too long for a tile
+  uint32_t num_runs;
+  uint32_t max_rounds;     // merge rounds of the longest run
+  uint32_t barrier;        // arrivals at the merge kernel's grid barrier
+};
 
 // Control block at the start of every workspace. Zeroed by
 // the host before each sort or pass; written only by the kernels after that.
@@ -51,9 +73,12 @@ struct Ctrl {
   uint32_t lookback_polls;         // diagnostics: windows that found a predecessor unpublished
   uint32_t parity[kMaxPasses + 1]; // parity[p]: 0 = pass p reads X, writes Y; 1 = reads Y, writes X
   uint32_t ticket[kMaxPasses];     // tile dispenser per pass (in-order tile dispatch)
-  // diagnostics of the 16-bit pass when LSB_WIDE_PROFILE is set: SM cycles
-  // and counts per phase, summed over CTAs, for its first four passes
-  unsigned long long wide_prof[4][12];
+  union {
+    // diagnostics of the 16-bit pass when LSB_WIDE_PROFILE is set: SM cycles
+    // and counts per phase, summed over CTAs, for its first four passes
+    unsigned long long wide_prof[4][12];
+    TopPlan top;
+  };
 };
 static_assert(sizeof(Ctrl) <= 1024, "control block must fit its 1 KiB slot");
 constexpr size_t kCtrlBytes = 1024;
@@ -63,6 +88,30 @@ constexpr size_t kCtrlBytes = 1024;
 __device__ __forceinline__ bool pass_skipped(const Ctrl* ctrl, int pass) {
   const uint32_t m = pass < 32 ? ctrl->skip_mask_lo : ctrl->skip_mask_hi;
   return (m >> (pass & 31)) & 1u;
+}
+
+// Digit of pass p of a sort by top digits: ((key >> right) << left) & 255, and
+// 0 or 255 for keys outside the block when there are any (clamp).
+struct TopWindow {
+  uint64_t lo, hi;
+  uint32_t right, left;
+  bool clamp;
+};
+__device__ __forceinline__ TopWindow top_window(const TopPlan& p, int pass) {
+  TopWindow w;
+  w.lo = p.lo;
+  w.hi = p.hi;
+  w.clamp = p.hb1 < 64u;
+  const int s = (int)p.hb1 - 8 * ((int)p.passes - pass);
+  w.right = s > 0 ? (uint32_t)s : 0u;
+  w.left = s < 0 ? (uint32_t)-s : 0u;
+  return w;
+}
+__device__ __forceinline__ uint32_t top_digit(const TopWindow& w, uint64_t key) {
+  return ((uint32_t)(key >> w.right) << w.left) & 255u;
+}
+__device__ __forceinline__ uint32_t top_digit_clamped(const TopWindow& w, uint64_t key) {
+  return key < w.lo ? 0u : key > w.hi ? 255u : top_digit(w, key);
 }
 
 // A batch of independent arrays sorted together (null tile_seg: one array).

@@ -9,8 +9,10 @@
 //    16-bit digit and one HBM round trip per pass; tiles are sorted by the
 //    digit's high byte into an L2-resident chunk buffer, then each high-byte
 //    bucket of a chunk is gathered and placed by its low byte (lsb_wide.cu).
-//  * "top" family (whole sorts): one CTA sorts an array that fits in its shared
-//    memory in one launch (lsb_top.cu).
+//  * "top" family (whole sorts): an array that fits in one CTA's shared memory
+//    is sorted there in one launch; a larger one by its top digits only, as
+//    many passes as it takes until the runs of equal windows fit, and then run
+//    by run in shared memory (lsb_top.cu).
 //  * "task" family (digit_bits >= 12, the reference's 16-bit digits): per pass
 //    a count kernel over contiguous tasks, a digit-major scan of the
 //    [digit][task] count table and a stable scatter -- the reference's own
@@ -90,8 +92,13 @@ int wide_run(Elem* X, Elem* Y, int first_digit, int target_parity, unsigned char
 // Whole sort by the top family; the result is in X. The control block is
 // cleared by the kernels.
 int top_run(Elem* X, Elem* Y, unsigned char* ws, const Layout& L, cudaStream_t st);
-// Largest array of the one-CTA sort.
-uint32_t top_small_limit();
+// Sizes the top family sorts.
+bool top_serves(uint32_t n);
+// Tile of its passes (its look-back ring has a slot for each).
+uint32_t onesweep_top_tile();
+// Pass `pass` of the plan in ctrl->top; gstart: that pass's digit starts.
+int onesweep_top_pass(Elem* X, Elem* Y, uint32_t n, int pass, const uint32_t* gstart, uint64_t* ring,
+                      uint32_t tiles, Ctrl* ctrl, const DeviceInfo& dev, cudaStream_t st);
 // One wide digit as two half-width onesweep passes src -> mid -> dst (L: a
 // split layout of two sub-digits starting at first_digit); src is not written.
 int onesweep_pass_via(const Elem* src, Elem* mid, Elem* dst, int first_digit, unsigned char* ws,

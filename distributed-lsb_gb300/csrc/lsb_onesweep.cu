@@ -409,8 +409,9 @@ __device__ __forceinline__ void lookback_adjacent(const uint64_t* __restrict__ r
 // clears its own counter column after staging, so no barrier separates a
 // tile's stores from the next tile's ranking.
 // BITS > 0 fixes the digit width at compile time (8 and 11: the common widths);
-// BITS == 0 takes it from `bits_rt`.
-template <int THREADS, int K, int MINB, typename CNT, int BITS>
+// BITS == 0 takes it from `bits_rt`. TOP: the digit's bits, whether the pass
+// runs and the buffers' parity come from ctrl->top (sorts by top digits).
+template <int THREADS, int K, int MINB, typename CNT, int BITS, bool TOP = false>
 __global__ void __launch_bounds__(THREADS, MINB)
     k_onesweep(Elem* __restrict__ X, Elem* __restrict__ Y, uint32_t n, int bits_rt, int pass,
                int digit, const uint32_t* __restrict__ gstart, uint64_t* __restrict__ ring,
@@ -425,10 +426,12 @@ __global__ void __launch_bounds__(THREADS, MINB)
   __shared__ uint32_t s_err[2];
   __shared__ uint32_t s_wt[W];
 
-  if (pass_skipped(ctrl, pass)) return;
+  if (TOP ? !((ctrl->top.run_mask >> pass) & 1u) : pass_skipped(ctrl, pass)) return;
   const int bits = BITS > 0 ? BITS : bits_rt;
   const uint32_t nbins = 1u << bits, mask = nbins - 1u;
   const int shift = bits * digit;  // `pass` indexes this call's passes, `digit` the key
+  __shared__ TopWindow s_win;  // not in registers: used once per tile
+  if (TOP && threadIdx.x == 0) s_win = top_window(ctrl->top, pass);
   const uint32_t cnt_words = (uint32_t)(onesweep_counter_bytes(nbins, WP, sizeof(CNT)) / 16u);
   const bool column_clear = nbins <= 256u;
   Elem* stage = reinterpret_cast<Elem*>(smem);                         // [E] tile in digit order
@@ -437,11 +440,11 @@ __global__ void __launch_bounds__(THREADS, MINB)
   uint32_t* gbase = tstart + nbins;   // [nbins] destination of the bin's first element
   uint32_t* tcount = gbase + nbins;   // [nbins] this tile's count of each bin
 
-  const uint32_t par = ctrl->parity[pass];
+  const uint32_t par = TOP ? (ctrl->top.par_mask >> pass) & 1u : ctrl->parity[pass];
   const Elem* __restrict__ src = par ? Y : X;
   Elem* __restrict__ dst = par ? X : Y;
   const bool segmented = seg.tile_seg != nullptr;
-  const uint32_t num_tiles = segmented ? *seg.num_tiles : (n + E - 1) / E;
+  const uint32_t num_tiles = segmented ? *seg.num_tiles : (n - 1u) / E + 1u;
   // statuses with reach when every tile of the pass has its own ring slot and
   // each bin has its own walking thread; tile-tagged statuses otherwise
   const bool reach = ring_tiles >= num_tiles && nbins <= (uint32_t)THREADS;
@@ -531,10 +534,26 @@ __global__ void __launch_bounds__(THREADS, MINB)
 
     // 1. digits
     uint32_t d[K];
+    if (TOP) {
+      const TopWindow win = s_win;
+      if (win.clamp) {
 #pragma unroll
-    for (int k = 0; k < K; k++)
-      d[k] = (full || warp * 32u * K + (uint32_t)k * 32u + lane < tile_len)
-                 ? digit_of(v[k].key, shift, mask) : kSentinel;
+        for (int k = 0; k < K; k++) d[k] = top_digit_clamped(win, v[k].key);
+      } else {
+#pragma unroll
+        for (int k = 0; k < K; k++) d[k] = top_digit(win, v[k].key);
+      }
+      if (!full) {
+#pragma unroll
+        for (int k = 0; k < K; k++)
+          if (warp * 32u * K + (uint32_t)k * 32u + lane >= tile_len) d[k] = kSentinel;
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < K; k++)
+        d[k] = (full || warp * 32u * K + (uint32_t)k * 32u + lane < tile_len)
+                   ? digit_of(v[k].key, shift, mask) : kSentinel;
+    }
 
     // 2. stable rank inside each warp: peers with the same digit, in item order
     uint32_t r[K];
@@ -1409,6 +1428,22 @@ int onesweep_launch_v(int bits, int variant, uint32_t grid, Elem* X, Elem* Y, ui
   ProfScope prof("onesweep_scatter", st);
   c.kern<<<grid, c.threads, c.smem, st>>>(X, Y, n, bits, pass, digit, gstart, ring, done, ring_tiles,
                                           ctrl, seg);
+  return cudaPeekAtLastError() == cudaSuccess ? 0 : 5;
+}
+
+// The default shape's 8-bit pass with digits, order and buffers from ctrl->top.
+constexpr int kTopThreads = 512, kTopItems = 16;
+uint32_t onesweep_top_tile() { return (uint32_t)kTopThreads * kTopItems; }
+
+int onesweep_top_pass(Elem* X, Elem* Y, uint32_t n, int pass, const uint32_t* gstart, uint64_t* ring,
+                      uint32_t tiles, Ctrl* ctrl, const DeviceInfo& dev, cudaStream_t st) {
+  auto kern = k_onesweep<kTopThreads, kTopItems, 1, uint32_t, 8, true>;
+  const size_t smem = reg_kernel_smem(8, kTopThreads, kTopItems);
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 5;
+  const uint32_t grid = std::max<uint32_t>(1u, std::min<uint32_t>(tiles, (uint32_t)dev.sm_count));
+  ProfScope prof("onesweep_scatter", st);
+  // one ring slot per tile: no slot is reused, so there are no completion tags
+  kern<<<grid, kTopThreads, smem, st>>>(X, Y, n, 8, pass, 0, gstart, ring, nullptr, tiles, ctrl, SegDesc{});
   return cudaPeekAtLastError() == cudaSuccess ? 0 : 5;
 }
 

@@ -3,27 +3,49 @@
 //
 // A tile of m elements is sorted through an array of 32-bit slots, so that
 // the 16-byte elements themselves are read once, at the end, in sorted order:
-//   1. smallest and largest key; a tile that is in order already is done;
-//   2. each key's bin: the range [min, max] is cut into NB equal bins, 1.8
-//      or more per element, and one shared atomic per element counts them and
-//      gives the element a place among its bin's (in any order);
-//   3. an exclusive scan of the bins' counts; each element's slot is written:
+//   1. each key's bin: a range that holds the tile's keys is cut into NB equal
+//      bins, 1.8 or more per element, and one shared atomic per element counts
+//      them and gives the element a place among its bin's (in any order);
+//   2. an exclusive scan of the bins' counts; each element's slot is written:
 //      (the key's next 18 or 19 bits below the bin, the element's position in the tile);
-//   4. an element's rank in its bin is the number of its bin's slots below
+//   3. an element's rank in its bin is the number of its bin's slots below
 //      its own: positions break ties, which makes the sort stable although the
 //      atomics are not. Slots that agree in the key bits compare whole keys.
 // So a tile costs one atomic per element whatever the key width, where ranking
 // by 8-bit digits (ballots and per-warp counters) costs one round per digit.
-// Evenly spread keys put 0.56 elements in a bin at most on average. A tile
-// with a bin above kMaxBin elements (duplicates, clusters) is sorted by merging
-// instead: K consecutive elements per thread by a sorting network, then
-// log2(threads) rounds of merge-path merges of position lists. That costs the
-// same for any keys: about six times the even case.
+// Evenly spread keys put 0.56 elements in a bin at most on average. When a bin
+// has more than kMaxBin elements (duplicates, clusters), the bins are laid over
+// the range from the smallest to the largest key instead; when that does not
+// help either, a tile that is not in order already is sorted by the bits in
+// which its keys differ, eight at a time from the lowest (stable ranks by
+// ballots and per-warp counters). A round costs about as much as a quarter of
+// the sort by bins, and duplicates or clusters leave few bits.
 #pragma once
 
 #include "lsb_device.cuh"
 
 namespace lsb {
+
+// Shared-memory accesses under a predicate: no branch around them, so that the
+// K independent accesses of a thread are all in flight together.
+__device__ __forceinline__ uint32_t atom_add_if(bool on, uint32_t* p, uint32_t v) {
+  uint32_t old = 0;
+  asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %3, 0;\n @p atom.shared.add.u32 %0, [%1], %2;\n}\n"
+               : "+r"(old)
+               : "r"(smem_u32(p)), "r"(v), "r"((uint32_t)on)
+               : "memory");
+  return old;
+}
+__device__ __forceinline__ void st_shared_if(bool on, uint32_t* p, uint32_t v) {
+  asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %2, 0;\n @p st.shared.u32 [%0], %1;\n}\n" ::"r"(smem_u32(p)), "r"(v),
+               "r"((uint32_t)on)
+               : "memory");
+}
+__device__ __forceinline__ void store_elem_if(bool on, Elem* p, const Elem& e) {
+  asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %3, 0;\n @p st.global.v2.u64 [%0], {%1, %2};\n}\n" ::"l"(p), "l"(e.key),
+               "l"(e.val), "r"((uint32_t)on)
+               : "memory");
+}
 
 template <int THREADS, int K>
 struct TileSort {
@@ -35,18 +57,17 @@ struct TileSort {
   static constexpr uint32_t kBins = (uint32_t)THREADS * kBinsPerThread;
   static constexpr uint32_t kPosBits = kCap <= 8192 ? 13 : 14;  // bits of a position in a slot
   static constexpr uint32_t kPosMask = (1u << kPosBits) - 1u;
-  static constexpr uint32_t kMaxBin = 40;
+  static constexpr uint32_t kMaxBin = 64;
   static_assert(kCap <= (1u << kPosBits) && K <= 16 && kWarps <= 32, "position bits, network, warp totals");
 
   // shared memory: elements, slots (or two position lists), bin counts (16 bits each)
   static constexpr size_t kElemBytes = (size_t)kCap * sizeof(Elem);
-  static constexpr size_t kSlotBytes = (size_t)kCap * 4u;
-  static constexpr size_t kBinBytes = (size_t)kBins * 2u;
+  static constexpr size_t kSlotBytes = (size_t)kCap * 4u + 16u;  // two position lists; what is read past the last slot
+  static constexpr size_t kBinBytes = (size_t)kBins * 2u + 16u;  // and the end of the last bin
   static constexpr size_t kSmem = kElemBytes + kSlotBytes + kBinBytes;
 
   struct Shared {
-    uint64_t wmin[kWarps], wmax[kWarps];
-    uint32_t wdiff[2][kWarps];
+    uint64_t wmin[kWarps], wmax[kWarps], wdiff[kWarps];
     uint32_t wtot[kWarps];
   };
 
@@ -61,201 +82,208 @@ struct TileSort {
     return (uint64_t)hi << 32 | lo;
   }
 
-  // Bin and, below it, 32 bits of fraction of a key: monotone in the key.
-  // x = (key - min) >> sh fits 32 bits; with f = 0 there are fewer distinct x
-  // than bins (then sh is 0 and a bin holds one key value), else the bin is
-  // floor(x * f / 2^32).
+  // Bin and, below it, 32 bits of fraction of a key: monotone in the key. The
+  // distance from base, shifted up until range's highest bit is the 64th, has
+  // its upper 32 bits scaled to bins: floor(x * f / 2^32).
   struct Scale {
     uint64_t base;
-    uint32_t sh, f;
+    uint32_t up, f;
   };
-  static __device__ __forceinline__ Scale make_scale(uint64_t mn, uint64_t mx) {
+  static __device__ __forceinline__ Scale make_scale(uint64_t base, uint64_t range) {  // range > 0
     Scale s;
-    const uint64_t range = mx - mn;
-    s.base = mn;
-    const int lz = __clzll((long long)range);
-    s.sh = lz < 32 ? (uint32_t)(32 - lz) : 0u;
-    const uint32_t xr = (uint32_t)(range >> s.sh);
-    s.f = xr < kBins ? 0u : (uint32_t)(((uint64_t)kBins << 32) / ((uint64_t)xr + 1u));
+    s.base = base;
+    s.up = (uint32_t)__clzll((long long)range);
+    const uint32_t xr = (uint32_t)((range << s.up) >> 32);
+    // kBins 2^32 / (xr + 1), a little less: xr's bin must stay below kBins. In
+    // 32-bit floats (relative errors below 2^-21 in all), taken down by 2^-19.
+    s.f = (uint32_t)(__fdividef((float)kBins * 4294967296.0f, (float)xr + 1.0f) * (1.0f - 1.0f / 524288.0f));
     return s;
   }
   static __device__ __forceinline__ uint32_t bin_of(const Scale& s, uint64_t key, uint32_t* frac) {
-    const uint32_t x = (uint32_t)((key - s.base) >> s.sh);
-    const uint64_t p = (uint64_t)x * s.f;
-    *frac = s.f ? (uint32_t)p : 0u;
-    return s.f ? (uint32_t)(p >> 32) : x;
+    const uint64_t d = key - s.base;
+    const uint32_t hi = s.up < 32u ? (uint32_t)(d >> 32) : (uint32_t)d, lo = s.up < 32u ? (uint32_t)d : 0u;
+    const uint64_t p = (uint64_t)__funnelshift_l(lo, hi, s.up) * s.f;  // the shift counts modulo 32
+    *frac = (uint32_t)p;
+    return (uint32_t)(p >> 32);
   }
 
-  // Sorts the m <= kCap elements in[0..m) (shared memory, not changed) and
-  // calls emit(rank, element) once for each from the thread that holds it;
-  // neighbouring threads get neighbouring ranks but for a bin's few elements.
-  // If the tile is in order already: nothing is emitted when `in_place`.
+  // Sorts the elements in[lo, hi) (shared memory, not changed; hi <= kCap) and
+  // calls emit(on, rank, element) for each, from the thread that holds it, and
+  // possibly more often with on = false; neighbouring threads get neighbouring
+  // ranks but for a bin's few elements. Every key is in [base, base + range];
+  // with range = 0 that is not known yet. A tile that turns out to be in order
+  // need not be emitted when `in_place`.
   // `slot` and `bins` are the tile's shared arrays; every thread of the CTA
-  // calls this together, after a barrier that makes in[] visible. On return
+  // calls this together, with in[] visible and bins[] not in use. On return
   // threads may still be reading in[], slot[] and bins[]: a barrier is due
-  // before they are written again. With diff_out, thread 0 gets there the bits
-  // in which any two keys differ.
+  // before they are written again.
   template <typename Emit>
-  static __device__ __forceinline__ void sort(const Elem* in, uint32_t m, uint32_t* slot, uint32_t* bins,
-                                              Shared& sh, bool in_place, Emit emit,
-                                              uint64_t* diff_out = nullptr) {
-    const uint32_t tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
-    // 1. zero the bins; smallest and largest key, order
-    {
-      uint4* z = reinterpret_cast<uint4*>(bins) + tid * 2u;
-      z[0] = make_uint4(0, 0, 0, 0);
-      z[1] = make_uint4(0, 0, 0, 0);
-    }
-    uint64_t mn = ~0ull, mx = 0ull;
+  static __device__ __forceinline__ void sort(const Elem* in, uint32_t lo, uint32_t hi, uint64_t base, uint64_t range,
+                                              uint32_t* slot, uint32_t* bins, Shared& sh, bool in_place, Emit emit) {
+    if (range == 0 || !sort_even(in, lo, hi, make_scale(base, range), slot, bins, sh, emit))
+      sort_any(in, lo, hi, slot, bins, sh, in_place, emit);
+  }
+
+  // Bins over the tile's own range of keys; bit by bit when that is uneven too.
+  template <typename Emit>
+  static __device__ __noinline__ void sort_any(const Elem* in, uint32_t lo, uint32_t hi, uint32_t* slot,
+                                               uint32_t* bins, Shared& sh, bool in_place, Emit emit) {
+    const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
+    const uint64_t k0 = in[lo].key;
+    uint64_t mn = ~0ull, mx = 0ull, diff = 0ull;
     bool inversion = false;
-#pragma unroll
-    for (int k = 0; k < K; k++) {
-      const uint32_t p = tid + (uint32_t)k * THREADS;
-      if (p < m) {
-        const uint64_t key = in[p].key;
-        mn = key < mn ? key : mn;
-        mx = key > mx ? key : mx;
-        if (p) inversion |= in[p - 1u].key > key;
-      }
+    for (uint32_t p = lo + threadIdx.x; p < hi; p += THREADS) {
+      const uint64_t key = in[p].key;
+      mn = key < mn ? key : mn;
+      mx = key > mx ? key : mx;
+      diff |= key ^ k0;
+      if (p + 1u < hi) inversion |= key > in[p + 1u].key;
     }
     mn = warp_min(mn);
     mx = warp_max(mx);
+    diff = (uint64_t)__reduce_or_sync(0xffffffffu, (uint32_t)(diff >> 32)) << 32 |
+           __reduce_or_sync(0xffffffffu, (uint32_t)diff);
+    __syncthreads();  // sh and the arrays are no longer read
     if (lane == 0) {
       sh.wmin[warp] = mn;
       sh.wmax[warp] = mx;
+      sh.wdiff[warp] = diff;
     }
-    if (diff_out) {
-      uint64_t x = 0;
-      const uint64_t k0 = in[0].key;
-#pragma unroll
-      for (int k = 0; k < K; k++) {
-        const uint32_t p = tid + (uint32_t)k * THREADS;
-        if (p < m) x |= in[p].key ^ k0;
-      }
-      const uint32_t lo = __reduce_or_sync(0xffffffffu, (uint32_t)x);
-      const uint32_t hi = __reduce_or_sync(0xffffffffu, (uint32_t)(x >> 32));
-      if (lane == 0) {
-        sh.wdiff[0][warp] = lo;
-        sh.wdiff[1][warp] = hi;
-      }
-    }
-    const bool unsorted = __syncthreads_or(inversion);
-    if (diff_out && tid == 0) {
-      uint64_t x = 0;
-      for (int w = 0; w < kWarps; w++) x |= (uint64_t)sh.wdiff[1][w] << 32 | sh.wdiff[0][w];
-      *diff_out = x;
-    }
-    if (!unsorted) {
-      if (!in_place) {
-#pragma unroll
-        for (int k = 0; k < K; k++) {
-          const uint32_t p = tid + (uint32_t)k * THREADS;
-          if (p < m) emit(p, in[p]);
-        }
-      }
+    if (!__syncthreads_or(inversion)) {
+      if (!in_place)
+        for (uint32_t p = lo + threadIdx.x; p < hi; p += THREADS) emit(true, p - lo, in[p]);
       return;
     }
     mn = warp_min(lane < (uint32_t)kWarps ? sh.wmin[lane] : ~0ull);
     mx = warp_max(lane < (uint32_t)kWarps ? sh.wmax[lane] : 0ull);
-    const Scale sc = make_scale(mn, mx);
+    if (sort_even(in, lo, hi, make_scale(mn, mx - mn), slot, bins, sh, emit)) return;
+    diff = lane < (uint32_t)kWarps ? sh.wdiff[lane] : 0ull;
+    diff = (uint64_t)__reduce_or_sync(0xffffffffu, (uint32_t)(diff >> 32)) << 32 |
+           __reduce_or_sync(0xffffffffu, (uint32_t)diff);
+    sort_bits(in + lo, hi - lo, diff, slot, bins, sh, emit);
+  }
 
-    // 2. count: bin, place among the bin's elements and fraction of each element
+  // The sort by bins; false, with nothing emitted, when a bin has too many elements.
+  template <typename Emit>
+  static __device__ __forceinline__ bool sort_even(const Elem* in, uint32_t lo, uint32_t hi, const Scale sc,
+                                                   uint32_t* slot, uint32_t* bins, Shared& sh, Emit emit) {
+    const uint32_t tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
+    const uint32_t m = hi - lo;
+    uint16_t* start = reinterpret_cast<uint16_t*>(bins);
+    // keys within 2^31 of each other: next keys are at least 2 f >= 2 (kBins - 1)
+    // >= 2^kPosBits apart on the scale, so slots that agree in the key bits hold one key
+    static_assert(2u * (kBins - 1u) >= (1u << kPosBits), "exact slots");
+    const bool whole = sc.up >= 33u;
+    {
+      uint4* z = reinterpret_cast<uint4*>(bins) + tid * 2u;
+      z[0] = make_uint4(0, 0, 0, 0);
+      z[1] = make_uint4(0, 0, 0, 0);
+      if (tid == 0) start[kBins] = (uint16_t)m;
+    }
+    __syncthreads();
+    // 1. bin, place among the bin's elements and fraction of each element
     uint32_t place[K], frac[K];
 #pragma unroll
     for (int k = 0; k < K; k++) {
       const uint32_t p = tid + (uint32_t)k * THREADS;
-      if (p < m) {
-        const uint32_t b = bin_of(sc, in[p].key, &frac[k]);
-        const uint32_t s16 = (b & 1u) << 4;
-        const uint32_t old = atomicAdd(&bins[b >> 1], 1u << s16);
-        place[k] = b << 16 | ((old >> s16) & 0xffffu);
-      }
+      const bool on = p - lo < m;
+      const uint32_t b = bin_of(sc, in[on ? p : lo].key, &frac[k]);
+      const uint32_t s16 = (b & 1u) << 4;
+      const uint32_t old = atom_add_if(on, bins + (b >> 1), 1u << s16);
+      place[k] = b << 16 | ((old >> s16) & 0xffffu);
     }
     __syncthreads();
-    // 3. exclusive scan of the counts; thread t owns bins [16 t, 16 t + 16)
-    uint32_t w8[8], maxc = 0, sum = 0;
+    // 2. exclusive scan of the counts; thread t owns bins [16 t, 16 t + 16)
     {
-      const uint4* q = reinterpret_cast<const uint4*>(bins) + tid * 2u;
-      const uint4 a = q[0], b = q[1];
-      w8[0] = a.x, w8[1] = a.y, w8[2] = a.z, w8[3] = a.w;
-      w8[4] = b.x, w8[5] = b.y, w8[6] = b.z, w8[7] = b.w;
-    }
+      uint32_t w8[8], maxc = 0, sum = 0;
+      uint4* q = reinterpret_cast<uint4*>(bins) + tid * 2u;
+      {
+        const uint4 a = q[0], b = q[1];
+        w8[0] = a.x, w8[1] = a.y, w8[2] = a.z, w8[3] = a.w;
+        w8[4] = b.x, w8[5] = b.y, w8[6] = b.z, w8[7] = b.w;
+      }
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
-      const uint32_t lo = w8[i] & 0xffffu, hi = w8[i] >> 16;
-      maxc = max(maxc, max(lo, hi));
-      w8[i] = sum | (sum + lo) << 16;
-      sum += lo + hi;
-    }
-    uint32_t inc = sum;
+      for (int i = 0; i < 8; i++) {
+        maxc = __vmaxu2(maxc, w8[i]);
+        const uint32_t c0 = w8[i] & 0xffffu, c1 = w8[i] >> 16;
+        w8[i] = sum | (sum + c0) << 16;
+        sum += c0 + c1;
+      }
+      uint32_t inc = sum;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
-      if (lane >= (uint32_t)o) inc += y;
-    }
-    if (lane == 31) sh.wtot[warp] = inc;
-    const bool uneven = __syncthreads_or(maxc > kMaxBin);
-    if (uneven) {
-      merge_sorted(in, m, slot, emit);
-      return;
-    }
-    {
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= (uint32_t)o) inc += y;
+      }
+      if (lane == 31) sh.wtot[warp] = inc;
+      if (__syncthreads_or(max(maxc & 0xffffu, maxc >> 16) > kMaxBin)) return false;
       uint32_t off = inc - sum;
       const uint32_t wt = lane < (uint32_t)kWarps ? sh.wtot[lane] : 0u;
       off += __reduce_add_sync(0xffffffffu, lane < warp ? wt : 0u);
       const uint32_t both = off | off << 16;
-      uint4* q = reinterpret_cast<uint4*>(bins) + tid * 2u;
       q[0] = make_uint4(w8[0] + both, w8[1] + both, w8[2] + both, w8[3] + both);
       q[1] = make_uint4(w8[4] + both, w8[5] + both, w8[6] + both, w8[7] + both);
     }
     __syncthreads();
-    const uint16_t* start = reinterpret_cast<const uint16_t*>(bins);
 #pragma unroll
     for (int k = 0; k < K; k++) {
       const uint32_t p = tid + (uint32_t)k * THREADS;
-      if (p < m) slot[start[place[k] >> 16] + (place[k] & 0xffffu)] = (frac[k] & ~kPosMask) | p;
+      const uint32_t q = start[place[k] >> 16] + (place[k] & 0xffffu);
+      st_shared_if(p - lo < m, slot + q, (frac[k] & ~kPosMask) | p);
     }
     __syncthreads();
-    // 4. rank inside the bin, elements out
-#pragma unroll 3
-    for (int k = 0; k < K; k++) {
-      const uint32_t p = tid + (uint32_t)k * THREADS;
-      if (p < m) {
-        const uint32_t v = slot[p];
-        const Elem e = in[v & kPosMask];
+    // 3. rank inside the bin, elements out: three rows of the tile at a time,
+    // their loads in flight together; the first four slots of the bin without
+    // a branch (slots past the tile's last are read but not counted)
+    static_assert(K % 3 == 0 || K % 2 == 0, "rows per step");
+    constexpr int R = K % 3 == 0 ? 3 : 2;
+#pragma unroll 1
+    for (uint32_t row = tid; row - tid < m; row += R * THREADS) {
+      uint32_t v[R], r[R];
+      Elem e[R];
+#pragma unroll
+      for (int i = 0; i < R; i++) v[i] = slot[min(row + (uint32_t)i * THREADS, m - 1u)];
+#pragma unroll
+      for (int i = 0; i < R; i++) e[i] = in[v[i] & kPosMask];
+#pragma unroll
+      for (int i = 0; i < R; i++) {
         uint32_t f;
-        const uint32_t b = bin_of(sc, e.key, &f);
-        const uint32_t s = start[b], t = b + 1u < kBins ? start[b + 1u] : m;
-        uint32_t r = s, close = 0;
-        for (uint32_t q = s; q < t; q++) {
-          const uint32_t u = slot[q];
-          r += u < v ? 1u : 0u;
-          close += (u ^ v) <= kPosMask ? 1u : 0u;
-        }
-        if (close > 1u) {  // key bits of the slots agree: whole keys, then positions
-          r = s;
-          for (uint32_t q = s; q < t; q++) {
-            const uint32_t j = slot[q] & kPosMask;
-            const uint64_t kj = in[j].key;
-            r += (kj < e.key || (kj == e.key && j < (v & kPosMask))) ? 1u : 0u;
+        const uint32_t b = bin_of(sc, e[i].key, &f);
+        const uint32_t s = start[b], cnt = start[b + 1u] - s;
+        const uint32_t* q = slot + s;
+        bool close = cnt > 4u;
+        r[i] = s;
+#pragma unroll
+        for (uint32_t j = 0; j < 4u; j++) {
+          const uint32_t u = q[j];
+          if (j < cnt) {
+            r[i] += u < v[i] ? 1u : 0u;
+            close |= ((u ^ v[i]) - 1u) < kPosMask;
           }
         }
-        emit(r, e);
+        if (close && (cnt > 4u || !whole)) {  // more slots, or key bits that agree: whole keys, then positions
+          r[i] = s;
+          for (uint32_t j = 0; j < cnt; j++) {
+            const uint32_t u = q[j];
+            bool before = u < v[i];
+            if (!whole && (u ^ v[i]) <= kPosMask) {
+              const uint64_t ku = in[u & kPosMask].key;
+              before = ku < e[i].key || (ku == e[i].key && u < v[i]);
+            }
+            r[i] += before ? 1u : 0u;
+          }
+        }
       }
+#pragma unroll
+      for (int i = 0; i < R; i++) emit(row + (uint32_t)i * THREADS < m, r[i], e[i]);
     }
+    return true;
   }
 
-  // One thread's K outputs of the stable merge of neighbouring sorted position
-  // lists of length len (src, m positions in all) into dst.
-  static __device__ __forceinline__ void merge_round(const Elem* in, const uint16_t* src, uint16_t* dst,
-                                                     uint32_t m, uint32_t len) {
-    const uint32_t d0 = threadIdx.x * (uint32_t)K;
-    if (d0 >= m) return;
-    const uint32_t base = d0 / (2u * len) * (2u * len);
-    const uint32_t la = min(len, m - base), lb = min(len, m - base - la);
-    const uint16_t* a = src + base;
-    const uint16_t* b = a + la;
-    const uint32_t d = d0 - base;
+  // Outputs [d, d + cnt) of the stable merge of the sorted position lists a
+  // (la of them, the earlier run) and b into dst, by one thread.
+  static __device__ __forceinline__ void merge_span(const Elem* in, const uint16_t* a, uint32_t la, const uint16_t* b,
+                                                    uint32_t lb, uint32_t d, uint32_t cnt, uint16_t* dst) {
     uint32_t lo = d > lb ? d - lb : 0u, hi = min(d, la);
     while (lo < hi) {
       const uint32_t mid = (lo + hi) >> 1;
@@ -263,62 +291,94 @@ struct TileSort {
       else hi = mid;
     }
     uint32_t i = lo, j = d - lo;
-    const uint32_t cnt = min((uint32_t)K, m - d0);
     uint32_t pa = i < la ? a[i] : 0u, pb = j < lb ? b[j] : 0u;
     uint64_t ka = in[pa].key, kb = in[pb].key;
     for (uint32_t q = 0; q < cnt; q++) {
       if (j >= lb || (i < la && ka <= kb)) {
-        dst[d0 + q] = (uint16_t)pa;
+        dst[q] = (uint16_t)pa;
         if (++i < la) ka = in[pa = a[i]].key;
       } else {
-        dst[d0 + q] = (uint16_t)pb;
+        dst[q] = (uint16_t)pb;
         if (++j < lb) kb = in[pb = b[j]].key;
       }
     }
   }
 
-  // The same result for any keys, by merging (see the head of this file).
+  // The merge of in[0..la) and in[la..la + lb), as positions in dst; id[i] = i.
+  static __device__ __forceinline__ void merge_parts(const Elem* in, const uint16_t* id, uint16_t* dst, uint32_t la,
+                                                     uint32_t lb) {
+    const uint32_t d0 = threadIdx.x * (uint32_t)K;
+    if (d0 < la + lb) merge_span(in, id, la, id + la, lb, d0, min((uint32_t)K, la + lb - d0), dst + d0);
+  }
+
+  // Stable order of in[0, m) by the bits of `diff` (those in which keys differ).
   template <typename Emit>
-  static __device__ __noinline__ void merge_sorted(const Elem* in, uint32_t m, uint32_t* slot, Emit emit) {
+  static __device__ __noinline__ void sort_bits(const Elem* in, uint32_t m, uint64_t diff, uint32_t* slot,
+                                                uint32_t* bins, Shared& sh, Emit emit) {
+    constexpr uint32_t WP = kWarps + 1;  // padded row of a digit's per-warp counters
+    constexpr uint32_t kParts = kWarps / 8;
+    static_assert(kWarps % 8 == 0 && 256u * WP * 2u <= kBinBytes, "eight counters per thread in the scan");
+    const uint32_t tid = threadIdx.x, lane = lane_id(), warp = tid >> 5, lt = lanemask_lt();
     uint16_t* cur = reinterpret_cast<uint16_t*>(slot);
     uint16_t* nxt = cur + kCap;
-    const uint32_t d0 = threadIdx.x * (uint32_t)K;
-    {
-      // K neighbours per thread: odd-even transposition, which keeps equal keys in place
-      uint64_t key[K];
-      uint32_t pos[K];
+    uint16_t* cnt = reinterpret_cast<uint16_t*>(bins);
+    const uint32_t i0 = warp * 32u * K + lane;  // this thread's places: i0 + 32 k
+    for (bool first = true; diff; first = false) {
+      const int s = __ffsll((long long)diff) - 1;
+      diff &= ~(255ull << s);
+      for (uint32_t i = tid; i < 256u * WP / 2u; i += THREADS) bins[i] = 0u;
+      __syncthreads();
+      uint32_t pd[K], r[K];  // position | digit << 16, rank among the warp's equal digits
 #pragma unroll
       for (int k = 0; k < K; k++) {
-        pos[k] = d0 + (uint32_t)k;
-        key[k] = pos[k] < m ? in[pos[k]].key : ~0ull;
+        const uint32_t i = i0 + 32u * (uint32_t)k;
+        const uint32_t p = i < m ? (first ? i : (uint32_t)cur[i]) : 0u;
+        pd[k] = p | ((uint32_t)(in[p].key >> s) & 255u) << 16;
       }
 #pragma unroll
-      for (int r = 0; r < K; r++) {
+      for (int k = 0; k < K; k++) {
+        const bool valid = i0 + 32u * (uint32_t)k < m;
+        const uint32_t d = pd[k] >> 16;
+        const uint32_t peers = warp_peers(d, 8, valid);
+        uint16_t* c = &cnt[d * WP + warp];
+        const uint32_t before = *c;
+        r[k] = before + __popc(peers & lt);
+        __syncwarp();
+        if (valid) *c = (uint16_t)(before + __popc(peers));
+        __syncwarp();
+      }
+      __syncthreads();
+      {
+        uint16_t* c = &cnt[tid / kParts * WP + tid % kParts * 8u];
+        uint32_t v[8], sum = 0;
 #pragma unroll
-        for (int k = r & 1; k + 1 < K; k += 2) {
-          if (key[k] > key[k + 1]) {
-            const uint64_t t = key[k];
-            key[k] = key[k + 1];
-            key[k + 1] = t;
-            const uint32_t u = pos[k];
-            pos[k] = pos[k + 1];
-            pos[k + 1] = u;
-          }
+        for (int j = 0; j < 8; j++) {
+          v[j] = sum;
+          sum += c[j];
         }
+        uint32_t inc = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+          if (lane >= (uint32_t)o) inc += y;
+        }
+        if (lane == 31) sh.wtot[warp] = inc;
+        __syncthreads();
+        const uint32_t wt = lane < (uint32_t)kWarps ? sh.wtot[lane] : 0u;
+        const uint32_t off = inc - sum + __reduce_add_sync(0xffffffffu, lane < warp ? wt : 0u);
+#pragma unroll
+        for (int j = 0; j < 8; j++) c[j] = (uint16_t)(off + v[j]);
       }
+      __syncthreads();
 #pragma unroll
       for (int k = 0; k < K; k++)
-        if (d0 + (uint32_t)k < m) cur[d0 + k] = (uint16_t)pos[k];
-    }
-    __syncthreads();
-    for (uint32_t len = K; len < m; len *= 2u) {
-      merge_round(in, cur, nxt, m, len);
+        if (i0 + 32u * (uint32_t)k < m) nxt[cnt[(pd[k] >> 16) * WP + warp] + r[k]] = (uint16_t)pd[k];
       __syncthreads();
       uint16_t* t = cur;
       cur = nxt;
       nxt = t;
     }
-    for (uint32_t p = threadIdx.x; p < m; p += THREADS) emit(p, in[cur[p]]);
+    for (uint32_t p = tid; p < m; p += THREADS) emit(true, p, in[cur[p]]);
   }
 };
 

@@ -56,3 +56,47 @@ def test_one_tile(lsb, cuda, oracle, n):
         runs = 8 - bin(skipped).count("1")
         assert (st.device_status, st.passes_planned, st.skipped_mask, st.passes_run, st.final_copy, st.n) == (
             0, 8, skipped, runs, runs & 1, n), (n, name)
+
+
+def large_key_sets(n, seed):
+    """Keys that leave short runs, long runs in order, long runs that must be merged, and none."""
+    r = np.random.default_rng(seed)
+    full = r.integers(0, 1 << 64, n, dtype=np.uint64)
+    yield "uniform", full
+    yield "sorted", np.sort(full)
+    yield "reverse", np.sort(full)[::-1].copy()
+    yield "equal", np.full(n, 0x0123456789ABCDEF, dtype=np.uint64)
+    yield "low_20_bits", full & np.uint64(0xFFFFF)
+    yield "offset_range", (full & np.uint64(0x3FFFFFFF)) + np.uint64(0x7FFFFFFFF0000000)
+    # one key for half of the elements: its run is in order, or mixed with its neighbours
+    yield "half_zero", np.where(r.random(n) < 0.5, np.uint64(0), full)
+    h = np.where(r.random(n) < 0.5, np.uint64(1 << 63), full)
+    h[r.integers(0, n, 50)] = np.uint64((1 << 63) + 1)
+    yield "half_one_key_and_close_ones", h
+    # three top halves: runs of a third of the array, all different below
+    yield "three_prefixes", (r.integers(0, 3, n).astype(np.uint64) << np.uint64(61)) | (full >> np.uint64(32))
+    # a narrow cluster that a sample sees little of, and keys far outside the others' block
+    c = full.copy()
+    k = max(n // 100, 20)
+    c[r.permutation(n)[:k]] = np.uint64(0x5555000000000000) + r.integers(0, 1 << 30, k).astype(np.uint64)
+    yield "cluster", c
+    o = full & np.uint64(0xFFFFFFFF)
+    o[r.integers(0, n, 3)] = np.uint64(2**64 - 1)
+    o |= np.uint64(1 << 40)
+    o[r.integers(0, n, 3)] = np.uint64(7)
+    yield "outliers", o
+    yield "equal_but_few", np.where(r.random(n) < 3e-4, full, np.uint64(0xFFFFFFFF00000000))
+    yield "dups", full[r.integers(0, max(1, n // 3000), n)]
+
+
+@pytest.mark.parametrize("n", [9217, 300007, (5 << 18) - 1, (5 << 18) + 1, (1 << 22) + 3])
+def test_top_digits(lsb, cuda, oracle, n):
+    """Runs of every kind, below and above the size from which arrays are passed
+    over by their top digits only."""
+    for name, keys in large_key_sets(n, n):
+        a = _elems(keys)
+        got, st = _run(lsb, cuda, a, 16)
+        assert np.array_equal(got, oracle.stable_sort_by_key(a)), (n, name)
+        diff = int(np.bitwise_or.reduce(keys ^ keys[0]))
+        skipped = sum(1 << d for d in range(4) if not (diff >> (16 * d)) & 0xFFFF)
+        assert (st.device_status, st.passes_planned, st.skipped_mask, st.n) == (0, 4, skipped, n), (n, name)
