@@ -47,6 +47,7 @@ struct TopPlan {
   uint32_t run_mask;       // bit p: pass p runs (its digit is not constant)
   uint32_t par_mask;       // bit p: pass p reads Y, writes X
   uint32_t src_parity;     // 1: the passes leave the data in Y
+  uint32_t skewed;         // heavy keys: tiles of runs are mostly in order
   uint32_t complete;       // the digits cover every bit in which keys differ
   uint32_t diff[2];        // bits in which some key differs from the first one
   uint32_t hist_done;      // CTAs of the histogram that have finished

@@ -10,9 +10,10 @@
 //    digit's high byte into an L2-resident chunk buffer, then each high-byte
 //    bucket of a chunk is gathered and placed by its low byte (lsb_wide.cu).
 //  * "top" family (whole sorts): an array that fits in one CTA's shared memory
-//    is sorted there in one launch; a larger one by its top digits only, as
-//    many passes as it takes until the runs of equal windows fit, and then run
-//    by run in shared memory (lsb_top.cu).
+//    is sorted there in one launch (lsb_top.cu); a larger one by its top digits
+//    only, as many passes as it takes until the runs of equal windows fit, and
+//    then run by run in shared memory: in one cooperative launch while every
+//    tile has a CTA of its own (lsb_mid.cu), else pass by pass (lsb_top.cu).
 //  * "task" family (digit_bits >= 12, the reference's 16-bit digits): per pass
 //    a count kernel over contiguous tasks, a digit-major scan of the
 //    [digit][task] count table and a stable scatter -- the reference's own
@@ -92,8 +93,10 @@ int wide_run(Elem* X, Elem* Y, int first_digit, int target_parity, unsigned char
 // Whole sort by the top family; the result is in X. The control block is
 // cleared by the kernels.
 int top_run(Elem* X, Elem* Y, unsigned char* ws, const Layout& L, cudaStream_t st);
-// Sizes the top family sorts.
-bool top_serves(uint32_t n);
+// Its one-launch form (lsb_mid.cu): largest array, workspace, launch.
+uint32_t mid_limit(const DeviceInfo& dev);
+size_t mid_workspace_bytes(uint32_t n, const DeviceInfo& dev);
+int mid_run(Elem* X, Elem* Y, unsigned char* ws, const Layout& L, const DeviceInfo& dev, cudaStream_t st);
 // Tile of its passes (its look-back ring has a slot for each).
 uint32_t onesweep_top_tile();
 // Pass `pass` of the plan in ctrl->top; gstart: that pass's digit starts.

@@ -14,12 +14,13 @@
 // So a tile costs one atomic per element whatever the key width, where ranking
 // by 8-bit digits (ballots and per-warp counters) costs one round per digit.
 // Evenly spread keys put 0.56 elements in a bin at most on average. When a bin
-// has more than kMaxBin elements (duplicates, clusters), the bins are laid over
-// the range from the smallest to the largest key instead; when that does not
-// help either, a tile that is not in order already is sorted by the bits in
-// which its keys differ, eight at a time from the lowest (stable ranks by
-// ballots and per-warp counters). A round costs about as much as a quarter of
-// the sort by bins, and duplicates or clusters leave few bits.
+// has more than kMaxBin elements, the bins are laid over the range from the
+// smallest to the largest key instead. What is heavy then are mostly
+// duplicates: a warp takes such a bin key by key, and a bitmap of the key's
+// positions gives the ranks (heavy_bins). A tile with many different keys in a
+// bin even so (clusters) is sorted by the bits in which its keys differ, eight
+// at a time from the lowest (stable ranks by ballots and per-warp counters).
+// 10^4 Zipf keys: 52 us bit by bit.
 #pragma once
 
 #include "lsb_device.cuh"
@@ -57,7 +58,11 @@ struct TileSort {
   static constexpr uint32_t kBins = (uint32_t)THREADS * kBinsPerThread;
   static constexpr uint32_t kPosBits = kCap <= 8192 ? 13 : 14;  // bits of a position in a slot
   static constexpr uint32_t kPosMask = (1u << kPosBits) - 1u;
-  static constexpr uint32_t kMaxBin = 64;
+  static constexpr uint32_t kMaxBin = 24;
+  static constexpr uint32_t kMaxHeavy = kCap / (kMaxBin + 1u);  // bins above it
+  static constexpr uint32_t kFewRounds = 4;  // of eight bits: no dearer than another try with bins
+  static constexpr uint32_t kFewKeys = 12;   // of 32 in a heavy bin: taken key by key
+  static constexpr uint32_t kManyKeys = 64;  // largest heavy bin of many keys compared pair by pair
   static_assert(kCap <= (1u << kPosBits) && K <= 16 && kWarps <= 32, "position bits, network, warp totals");
 
   // shared memory: elements, slots (or two position lists), bin counts (16 bits each)
@@ -69,6 +74,7 @@ struct TileSort {
   struct Shared {
     uint64_t wmin[kWarps], wmax[kWarps], wdiff[kWarps];
     uint32_t wtot[kWarps];
+    uint32_t heavy_n, heavy[kMaxHeavy];  // first slot << 16 | elements
   };
 
   static __device__ __forceinline__ uint64_t warp_min(uint64_t v) {
@@ -120,14 +126,15 @@ struct TileSort {
   template <typename Emit>
   static __device__ __forceinline__ void sort(const Elem* in, uint32_t lo, uint32_t hi, uint64_t base, uint64_t range,
                                               uint32_t* slot, uint32_t* bins, Shared& sh, bool in_place, Emit emit) {
-    if (range == 0 || !sort_even(in, lo, hi, make_scale(base, range), slot, bins, sh, emit))
-      sort_any(in, lo, hi, slot, bins, sh, in_place, emit);
+    if (range == 0 || !sort_even<false>(in, lo, hi, make_scale(base, range), slot, bins, sh, emit))
+      sort_any(in, lo, hi, slot, bins, sh, range == 0, in_place, emit);
   }
 
-  // Bins over the tile's own range of keys; bit by bit when that is uneven too.
+  // Bins over the tile's own range of keys (unless other bins were tried and a
+  // few rounds of bits will do); bit by bit when that is uneven too.
   template <typename Emit>
   static __device__ __noinline__ void sort_any(const Elem* in, uint32_t lo, uint32_t hi, uint32_t* slot,
-                                               uint32_t* bins, Shared& sh, bool in_place, Emit emit) {
+                                               uint32_t* bins, Shared& sh, bool first_try, bool in_place, Emit emit) {
     const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
     const uint64_t k0 = in[lo].key;
     uint64_t mn = ~0ull, mx = 0ull, diff = 0ull;
@@ -156,15 +163,21 @@ struct TileSort {
     }
     mn = warp_min(lane < (uint32_t)kWarps ? sh.wmin[lane] : ~0ull);
     mx = warp_max(lane < (uint32_t)kWarps ? sh.wmax[lane] : 0ull);
-    if (sort_even(in, lo, hi, make_scale(mn, mx - mn), slot, bins, sh, emit)) return;
     diff = lane < (uint32_t)kWarps ? sh.wdiff[lane] : 0ull;
     diff = (uint64_t)__reduce_or_sync(0xffffffffu, (uint32_t)(diff >> 32)) << 32 |
            __reduce_or_sync(0xffffffffu, (uint32_t)diff);
+    uint32_t rounds = 0;
+    for (uint64_t d = diff; d; d &= ~(255ull << (__ffsll((long long)d) - 1))) rounds++;
+    if ((first_try || rounds > kFewRounds) &&
+        sort_even<true>(in, lo, hi, make_scale(mn, mx - mn), slot, bins, sh, emit))
+      return;
+    __syncthreads();
     sort_bits(in + lo, hi - lo, diff, slot, bins, sh, emit);
   }
 
-  // The sort by bins; false, with nothing emitted, when a bin has too many elements.
-  template <typename Emit>
+  // The sort by bins; false when a bin has too many elements (HEAVY: too many
+  // different keys; then some may have been emitted).
+  template <bool HEAVY, typename Emit>
   static __device__ __forceinline__ bool sort_even(const Elem* in, uint32_t lo, uint32_t hi, const Scale sc,
                                                    uint32_t* slot, uint32_t* bins, Shared& sh, Emit emit) {
     const uint32_t tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
@@ -178,7 +191,7 @@ struct TileSort {
       uint4* z = reinterpret_cast<uint4*>(bins) + tid * 2u;
       z[0] = make_uint4(0, 0, 0, 0);
       z[1] = make_uint4(0, 0, 0, 0);
-      if (tid == 0) start[kBins] = (uint16_t)m;
+      if (tid == 0) start[kBins] = (uint16_t)m, sh.heavy_n = 0u;
     }
     __syncthreads();
     // 1. bin, place among the bin's elements and fraction of each element
@@ -216,13 +229,22 @@ struct TileSort {
         if (lane >= (uint32_t)o) inc += y;
       }
       if (lane == 31) sh.wtot[warp] = inc;
-      if (__syncthreads_or(max(maxc & 0xffffu, maxc >> 16) > kMaxBin)) return false;
+      maxc = max(maxc & 0xffffu, maxc >> 16);
+      if (__syncthreads_or(maxc > kMaxBin) && !HEAVY) return false;
       uint32_t off = inc - sum;
       const uint32_t wt = lane < (uint32_t)kWarps ? sh.wtot[lane] : 0u;
       off += __reduce_add_sync(0xffffffffu, lane < warp ? wt : 0u);
       const uint32_t both = off | off << 16;
       q[0] = make_uint4(w8[0] + both, w8[1] + both, w8[2] + both, w8[3] + both);
       q[1] = make_uint4(w8[4] + both, w8[5] + both, w8[6] + both, w8[7] + both);
+      if (HEAVY && maxc > kMaxBin) {
+#pragma unroll
+        for (int i = 0; i < 16; i++) {
+          const uint32_t s0 = (w8[i >> 1] >> (16 * (i & 1))) & 0xffffu;
+          const uint32_t s1 = i < 15 ? (w8[(i + 1) >> 1] >> (16 * ((i + 1) & 1))) & 0xffffu : sum;
+          if (s1 - s0 > kMaxBin) sh.heavy[atomicAdd(&sh.heavy_n, 1u)] = (off + s0) << 16 | (s1 - s0);
+        }
+      }
     }
     __syncthreads();
 #pragma unroll
@@ -232,11 +254,19 @@ struct TileSort {
       st_shared_if(p - lo < m, slot + q, (frac[k] & ~kPosMask) | p);
     }
     __syncthreads();
+    if (HEAVY) {  // a large bin of many keys: nothing here helps
+      const uint32_t count = sh.heavy_n;
+      bool lost = false;
+      for (uint32_t h = warp; h < count; h += kWarps) {
+        const uint32_t c = sh.heavy[h] & 0xffffu;
+        lost |= c > kManyKeys && probe_keys(in, slot, sh.heavy[h] >> 16, c) > kFewKeys;
+      }
+      if (__syncthreads_or(lost)) return false;
+    }
     // 3. rank inside the bin, elements out: three rows of the tile at a time,
     // their loads in flight together; the first four slots of the bin without
     // a branch (slots past the tile's last are read but not counted)
-    static_assert(K % 3 == 0 || K % 2 == 0, "rows per step");
-    constexpr int R = K % 3 == 0 ? 3 : 2;
+    constexpr int R = K % 3 == 0 ? 3 : K % 2 == 0 ? 2 : 1;
 #pragma unroll 1
     for (uint32_t row = tid; row - tid < m; row += R * THREADS) {
       uint32_t v[R], r[R];
@@ -261,23 +291,173 @@ struct TileSort {
             close |= ((u ^ v[i]) - 1u) < kPosMask;
           }
         }
-        if (close && (cnt > 4u || !whole)) {  // more slots, or key bits that agree: whole keys, then positions
+        if (HEAVY && cnt > kMaxBin) {
+          r[i] = kCap;  // heavy_bins emits it
+        } else if (close && (cnt > 4u || !whole)) {  // more slots, or key bits that agree: whole keys, then positions
           r[i] = s;
-          for (uint32_t j = 0; j < cnt; j++) {
-            const uint32_t u = q[j];
-            bool before = u < v[i];
-            if (!whole && (u ^ v[i]) <= kPosMask) {
-              const uint64_t ku = in[u & kPosMask].key;
-              before = ku < e[i].key || (ku == e[i].key && u < v[i]);
+          for (uint32_t j = 0; j < cnt; j += 4u) {
+            uint32_t u[4];
+            uint64_t ku[4];
+#pragma unroll
+            for (uint32_t x = 0; x < 4u; x++) u[x] = q[min(j + x, cnt - 1u)];
+#pragma unroll
+            for (uint32_t x = 0; x < 4u; x++) ku[x] = in[u[x] & kPosMask].key;
+#pragma unroll
+            for (uint32_t x = 0; x < 4u; x++) {
+              const bool tie = (u[x] ^ v[i]) <= kPosMask && ku[x] != e[i].key;
+              r[i] += j + x < cnt && (tie ? ku[x] < e[i].key : u[x] < v[i]) ? 1u : 0u;
             }
-            r[i] += before ? 1u : 0u;
           }
         }
       }
 #pragma unroll
-      for (int i = 0; i < R; i++) emit(row + (uint32_t)i * THREADS < m, r[i], e[i]);
+      for (int i = 0; i < R; i++) emit(row + (uint32_t)i * THREADS < m && (!HEAVY || r[i] < kCap), r[i], e[i]);
     }
-    return true;
+    return !HEAVY || sh.heavy_n == 0u || heavy_bins(in, slot, bins, sh, emit);
+  }
+
+  // The heavy bins' elements, one warp per bin and the whole CTA for the largest:
+  // for each key of the bin from the smallest, a bitmap of its elements'
+  // positions in the tile, whose prefix counts are the ranks. A bin of many
+  // different keys is ranked pair by pair, or, above kManyKeys elements, left
+  // (false).
+  static constexpr uint32_t kWords = (kCap + 31u) / 32u, kPerLane = (kWords + 31u) / 32u;
+  static constexpr uint32_t kMapWords = kWords + kWords / 2u + 1u;  // the bitmap and 16-bit prefix counts
+  static constexpr uint32_t kFit = (uint32_t)(kBinBytes / 4u) / kMapWords;
+  static constexpr uint32_t kTakers = kFit < (uint32_t)kWarps ? kFit : (uint32_t)kWarps;
+  static constexpr uint32_t kLargeBin = 512;  // elements from which the whole CTA takes a bin
+
+  // One warp: before[w] = bits in the words below w of the bitmap; all bits in it.
+  static __device__ __forceinline__ uint32_t count_map(const uint32_t* map, uint16_t* before) {
+    const uint32_t lane = lane_id();
+    uint32_t sum = 0, part[kPerLane];
+#pragma unroll
+    for (uint32_t i = 0; i < kPerLane; i++) {
+      part[i] = sum;
+      const uint32_t x = lane * kPerLane + i;
+      sum += x < kWords ? (uint32_t)__popc(map[x]) : 0u;
+    }
+    uint32_t inc = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= (uint32_t)o) inc += y;
+    }
+#pragma unroll
+    for (uint32_t i = 0; i < kPerLane; i++)
+      if (lane * kPerLane + i < kWords) before[lane * kPerLane + i] = (uint16_t)(inc - sum + part[i]);
+    return __shfl_sync(0xffffffffu, inc, 31);
+  }
+  static __device__ __forceinline__ uint32_t map_rank(const uint32_t* map, const uint16_t* before, uint32_t p) {
+    return before[p >> 5] + (uint32_t)__popc(map[p >> 5] & ((1u << (p & 31u)) - 1u));
+  }
+  // One warp: different keys among 32 of the bin's.
+  static __device__ __forceinline__ uint32_t probe_keys(const Elem* in, const uint32_t* slot, uint32_t s, uint32_t c) {
+    const uint64_t key = in[slot[s + lane_id() * c / 32u] & kPosMask].key;
+    const uint32_t same = __match_any_sync(0xffffffffu, (unsigned long long)key);
+    return (uint32_t)__popc(__ballot_sync(0xffffffffu, __ffs((int)same) - 1 == (int)lane_id()));
+  }
+
+  template <typename Emit>
+  static __device__ __noinline__ bool heavy_bins(const Elem* in, const uint32_t* slot, uint32_t* bins, Shared& sh,
+                                                 Emit emit) {
+    const uint32_t tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
+    bool ok = true;
+    __syncthreads();  // the bins' starts are no longer read
+    const uint32_t count = sh.heavy_n;
+    for (uint32_t h = 0; h < count; h++) {
+      const uint32_t s = sh.heavy[h] >> 16, c = sh.heavy[h] & 0xffffu;
+      if (c < kLargeBin) continue;
+      if (probe_keys(in, slot, s, c) > kFewKeys) {  // the same answer in every warp
+        ok = false;
+        continue;
+      }
+      uint32_t* map = bins;
+      uint16_t* before = reinterpret_cast<uint16_t*>(map + kWords);
+      uint32_t done = 0;
+      uint64_t last = 0;
+      for (uint32_t it = 0; it < 2u * kFewKeys && done < c; it++) {
+        uint64_t mn = ~0ull;
+        for (uint32_t j = tid; j < c; j += THREADS) {
+          const uint64_t key = in[slot[s + j] & kPosMask].key;
+          if ((done == 0 || key > last) && key < mn) mn = key;
+        }
+        mn = warp_min(mn);
+        if (lane == 0) sh.wmin[warp] = mn;
+        for (uint32_t i = tid; i < kWords; i += THREADS) map[i] = 0u;
+        __syncthreads();
+        mn = warp_min(lane < (uint32_t)kWarps ? sh.wmin[lane] : ~0ull);
+        for (uint32_t j = tid; j < c; j += THREADS) {
+          const uint32_t p = slot[s + j] & kPosMask;
+          if (in[p].key == mn) atomicOr(&map[p >> 5], 1u << (p & 31u));
+        }
+        __syncthreads();
+        if (warp == 0) {
+          const uint32_t all = count_map(map, before);
+          if (lane == 0) sh.wtot[0] = all;
+        }
+        __syncthreads();
+        for (uint32_t j = tid; j < c; j += THREADS) {
+          const uint32_t p = slot[s + j] & kPosMask;
+          const Elem e = in[p];
+          if (e.key == mn) emit(true, s + done + map_rank(map, before, p), e);
+        }
+        done += sh.wtot[0];
+        last = mn;
+        __syncthreads();
+      }
+      ok = ok && done >= c;
+    }
+    uint32_t* map = bins + warp * kMapWords;
+    uint16_t* before = reinterpret_cast<uint16_t*>(map + kWords);
+    for (uint32_t h = warp; warp < kTakers && h < count; h += kTakers) {
+      const uint32_t s = sh.heavy[h] >> 16, c = sh.heavy[h] & 0xffffu;
+      if (c >= kLargeBin) continue;
+      uint32_t done = 0;
+      if (probe_keys(in, slot, s, c) <= kFewKeys) {
+        uint64_t last = 0;
+        for (uint32_t it = 0; it < 2u * kFewKeys && done < c; it++) {
+          uint64_t mn = ~0ull;
+          for (uint32_t j = lane; j < c; j += 32u) {
+            const uint64_t key = in[slot[s + j] & kPosMask].key;
+            if ((done == 0 || key > last) && key < mn) mn = key;
+          }
+          mn = warp_min(mn);
+          for (uint32_t i = lane; i < kWords; i += 32u) map[i] = 0u;
+          __syncwarp();
+          for (uint32_t j = lane; j < c; j += 32u) {
+            const uint32_t p = slot[s + j] & kPosMask;
+            if (in[p].key == mn) atomicOr(&map[p >> 5], 1u << (p & 31u));
+          }
+          __syncwarp();
+          const uint32_t all = count_map(map, before);
+          __syncwarp();
+          for (uint32_t j = lane; j < c; j += 32u) {
+            const uint32_t p = slot[s + j] & kPosMask;
+            const Elem e = in[p];
+            if (e.key == mn) emit(true, s + done + map_rank(map, before, p), e);
+          }
+          done += all;
+          last = mn;
+          __syncwarp();
+        }
+      } else if (c <= kManyKeys) {
+        for (uint32_t j = lane; j < c; j += 32u) {
+          const uint32_t p = slot[s + j] & kPosMask;
+          const Elem e = in[p];
+          uint32_t r = s;
+          for (uint32_t q = 0; q < c; q++) {
+            const uint32_t o = slot[s + q] & kPosMask;
+            const uint64_t ko = in[o].key;
+            r += (ko < e.key || (ko == e.key && o < p)) ? 1u : 0u;
+          }
+          emit(true, r, e);
+        }
+        done = c;
+      }
+      ok = ok && done >= c;
+    }
+    return !__syncthreads_or(!ok);
   }
 
   // Outputs [d, d + cnt) of the stable merge of the sorted position lists a

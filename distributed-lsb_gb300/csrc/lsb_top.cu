@@ -10,31 +10,9 @@
 #include <algorithm>
 #include <cmath>
 
-#include "lsb_internal.h"
-#include "lsb_tile.cuh"
+#include "lsb_top.cuh"
 
 namespace lsb {
-
-// The pass plan lsb_query reports, from the bits in which the keys differ: a
-// digit in which no key differs counts as skipped (thread 0 of one CTA).
-__device__ __forceinline__ void write_plan(Ctrl* ctrl, uint64_t diff, uint32_t n, int bits, int num_digits,
-                                           int api_bits, int sub) {
-  uint32_t lo = 0, hi = 0, runs = 0;
-  const uint64_t mask = (1ull << bits) - 1ull;
-  for (int p = 0; p < num_digits; p++) {
-    if ((diff >> (bits * p)) & mask) runs++;
-    else if (p < 32) lo |= 1u << p;
-    else hi |= 1u << (p - 32);
-  }
-  ctrl->skip_mask_lo = lo;
-  ctrl->skip_mask_hi = hi;
-  ctrl->passes_run = runs;
-  ctrl->final_copy = runs & 1u;
-  ctrl->num_passes = (uint32_t)num_digits;
-  ctrl->api_bits = (uint32_t)api_bits;
-  ctrl->sub = (uint32_t)sub;
-  ctrl->n = n;
-}
 
 // ---------------------------------------------------------------------------
 // one CTA, one launch
@@ -94,12 +72,6 @@ __global__ void __launch_bounds__(THREADS, 1)
 using SmallHalf = TileSort<512, 9>;
 using SmallFull = TileSort<1024, 9>;
 
-// Between the two the launches and their latency set the time, and eight passes
-// of one tile per SM were no worse than one or two with a sample before them
-// when keys are skewed (10^6 Zipf keys: 153 us against 234; uniform 153 against 62).
-constexpr uint32_t kTopFrom = 5u << 18;
-bool top_serves(uint32_t n) { return n <= SmallFull::kCap || n >= kTopFrom; }
-
 template <int THREADS>
 static int small_sort(Elem* X, const Layout& L, Ctrl* ctrl, cudaStream_t st) {
   auto kern = k_small_sort<THREADS, 9>;
@@ -131,49 +103,29 @@ using Tile = TileSort<512, 9>;  // 106 KB: two CTAs per SM, one's loads and stor
 constexpr uint32_t kCap = Tile::kCap;
 // Mean run length up to which a pass is saved: six standard deviations below a tile.
 constexpr uint32_t kMeanRun = 4220;
-constexpr int kSampleThreads = 1024;
-using SampleTile = TileSort<kSampleThreads, 4>;
-constexpr uint32_t kSample = SampleTile::kCap;
-constexpr size_t kSampleSmem = SampleTile::kSmem + (size_t)kSample * 8u;
+constexpr int kTopSample = 4;  // keys per thread of the sample: 4096
 constexpr int kTopHistThreads = 512;
 constexpr int kTopHistUnroll = 4;
 
-// What the sample's statistics are held against (host-side, from n alone).
-struct SampleRule {
-  uint32_t tmin, tmax;  // fewest passes that shorten even runs to a tile, most passes launched
-  uint32_t tall;        // passes that leave a heavy key alone in its run
-  uint32_t far;         // this many sample keys apart in one window: a run longer than a tile
-  uint32_t near_limit;  // neighbours that may share a window before the mean run is too long
-  uint32_t far_limit;   // keys in runs longer than a tile that are left to the merges
-};
-
-static SampleRule sample_rule(uint32_t n) {
+SampleRule sample_rule(uint32_t n, uint32_t sample, uint32_t mean_run, uint32_t often, double spread) {
   SampleRule r;
   auto passes_for = [&](double per_run) {
     uint32_t t = 1;
     while (t < 8 && (double)n > per_run * std::pow(256.0, (double)t)) t++;
     return t;
   };
-  r.tmin = passes_for(kMeanRun);
-  // Unused launches cost about 2 us each: below 2^26 elements only two passes
-  // more than even keys need are kept ready, and the merges, whose rounds then
-  // stay nearly in L2, take what those leave.
-  r.tmax = n >= (1u << 26) ? 8u : std::min(8u, r.tmin + 2u);
-  r.tall = passes_for(1.0 / 16.0);
-  const double lam = (double)kMeanRun * kSample / n;
+  r.tmin = passes_for(mean_run);
+  r.tmax = 8u;
+  r.tall = passes_for(1.0 / spread);
+  const double lam = (double)mean_run * sample / n, lom = (double)often * sample / n;
   r.far = (uint32_t)(lam + 4.0 * std::sqrt(lam) + 4.0);
+  r.heavy = (uint32_t)(lom + 4.0 * std::sqrt(lom) + 4.0);
   const double l = 1.25 * lam, f = 1.0 - (1.0 - std::exp(-l)) / l;
-  r.near_limit = (uint32_t)(kSample * f + 3.0 * std::sqrt(kSample * f)) + 1u;
-  r.far_limit = kSample / 64u;
+  r.near_limit = (uint32_t)(sample * f + 3.0 * std::sqrt(sample * f)) + 1u;
+  r.far_limit = sample / 64u;
+  // sampled twice by chance: sample^2 / (2 n) pairs; every key k times in the array: k times that
+  r.dups = std::max<uint32_t>(3u, (uint32_t)(4.0 * sample * sample / n));
   return r;
-}
-
-__device__ __forceinline__ uint32_t mix32(uint32_t x) {
-  x ^= x >> 16;
-  x *= 0x85EBCA6Bu;
-  x ^= x >> 13;
-  x *= 0xC2B2AE35u;
-  return x ^ x >> 16;
 }
 
 // Bound by latency (one CTA: 4096 scattered reads, a tile sort, two counts);
@@ -181,73 +133,22 @@ __device__ __forceinline__ uint32_t mix32(uint32_t x) {
 __global__ void __launch_bounds__(kSampleThreads, 1)
     k_top_sample(const Elem* __restrict__ data, uint32_t n, SampleRule rule, uint32_t* __restrict__ hist, Ctrl* ctrl) {
   extern __shared__ __align__(128) unsigned char smem[];
-  __shared__ typename SampleTile::Shared sh;
-  __shared__ uint32_t s_near[8], s_far[8];
-  Elem* in = reinterpret_cast<Elem*>(smem);
-  uint32_t* slot = reinterpret_cast<uint32_t*>(smem + SampleTile::kElemBytes);
-  uint32_t* bins = reinterpret_cast<uint32_t*>(smem + SampleTile::kElemBytes + SampleTile::kSlotBytes);
-  uint64_t* s = reinterpret_cast<uint64_t*>(smem + SampleTile::kSmem);
+  __shared__ typename SampleTile<kTopSample>::Shared sh;
+  __shared__ uint32_t s_near[8], s_far[9];
   const uint32_t tid = threadIdx.x;
-  uint64_t key[4];
-#pragma unroll
-  for (int k = 0; k < 4; k++) {
-    const uint32_t i = tid + (uint32_t)k * kSampleThreads;
-    // places drawn independently of each other (not one per stretch: of an
-    // array nearly in order that would be the most even sample there is)
-    key[k] = data[((uint64_t)mix32(i + 1u) * n) >> 32].key;
-  }
   for (uint32_t i = tid; i < kCtrlBytes / 4u; i += kSampleThreads) reinterpret_cast<uint32_t*>(ctrl)[i] = 0u;
   for (uint32_t i = tid; i < 8u * 256u; i += kSampleThreads) hist[i] = 0u;
-  if (tid < 8) s_near[tid] = s_far[tid] = 0u;
-#pragma unroll
-  for (int k = 0; k < 4; k++) in[tid + (uint32_t)k * kSampleThreads] = Elem{key[k], 0};
-  __syncthreads();
-  SampleTile::sort(in, 0, kSample, 0, 0, slot, bins, sh, false, [&](bool on, uint32_t r, const Elem& e) {
-    if (on) s[r] = e.key;
-  });
-  __syncthreads();
-  const uint64_t first = s[0], span = first ^ s[kSample - 1u];
+  if (tid < 8) s_near[tid] = 0u;
+  if (tid < 9) s_far[tid] = 0u;
+  const uint64_t* s = sample_keys<kTopSample>(data, n, smem, sh);
+  const uint64_t first = s[0], span = first ^ s[SampleTile<kTopSample>::kCap - 1u];
   const uint32_t hb1 = span ? 64u - (uint32_t)__clzll((long long)span) : 64u;
-  // nibble T-1 of near / far: this thread's keys that share T windows (but
-  // not all 64 bits) with the next key / with the key `far` places on
-  uint32_t near = 0, farm = 0;
-  bool heavy = false;
-#pragma unroll
-  for (int k = 0; k < 4; k++) {
-    const uint32_t i = tid + (uint32_t)k * kSampleThreads;
-    const uint64_t ki = s[i];
-    auto shared_windows = [&](uint32_t j) {
-      const uint32_t bits = hb1 - min(hb1, 64u - (uint32_t)__clzll((long long)(ki ^ s[j])));
-      return 0x11111111u & ((1u << (4u * (bits >> 3))) - 1u);  // bits < 64: the keys differ
-    };
-    if (i + 1u < kSample && s[i + 1u] != ki) near += shared_windows(i + 1u);
-    if (i + rule.far - 1u < kSample) {
-      if (s[i + rule.far - 1u] == ki) heavy = true;
-      else farm += shared_windows(i + rule.far - 1u);
-    }
-  }
-  {
-    const uint32_t n0 = __reduce_add_sync(0xffffffffu, near & 0x0F0F0F0Fu);
-    const uint32_t n1 = __reduce_add_sync(0xffffffffu, (near >> 4) & 0x0F0F0F0Fu);
-    const uint32_t f0 = __reduce_add_sync(0xffffffffu, farm & 0x0F0F0F0Fu);
-    const uint32_t f1 = __reduce_add_sync(0xffffffffu, (farm >> 4) & 0x0F0F0F0Fu);
-    const uint32_t l = lane_id();
-    if (l < 8) {
-      atomicAdd(&s_near[l], ((l & 1u ? n1 : n0) >> (8u * (l >> 1))) & 0xFFu);
-      atomicAdd(&s_far[l], ((l & 1u ? f1 : f0) >> (8u * (l >> 1))) & 0xFFu);
-    }
-  }
-  heavy = __syncthreads_or(heavy);
+  bool skewed;
+  const uint32_t t = sample_passes<kTopSample>(s, hb1, rule, s_near, s_far, &skewed);
   if (tid == 0) {
     TopPlan& p = ctrl->top;
-    const uint32_t full = (hb1 + 7u) / 8u, most = min(rule.tmax, full);
-    uint32_t t = min(rule.tmin, full);
-    while (t < most && !(s_near[t - 1u] <= rule.near_limit && s_far[t - 1u] <= rule.far_limit &&
-                         (!heavy || t >= rule.tall)))
-      t++;
-    // one pass more that leaves nothing to sort costs no more than sorting the runs
-    if (t + 1u == full && t < rule.tmax) t = full;
     p.passes = t;
+    p.skewed = skewed ? 1u : 0u;
     p.hb1 = hb1;
     p.lo = hb1 < 64u ? first >> hb1 << hb1 : 0ull;
     p.hi = hb1 < 64u ? p.lo | ((1ull << hb1) - 1ull) : ~0ull;
@@ -430,58 +331,7 @@ __global__ void __launch_bounds__(kTopHistThreads, 4)
 }
 
 // ---------------------------------------------------------------------------
-// runs of equal windows
-
-// The window a key falls in: equal for the keys of one run.
-struct RunKey {
-  uint64_t lo, hi;  // smallest and largest key of the block
-  uint32_t shift;
-};
-__device__ __forceinline__ uint64_t run_of(const RunKey& w, uint64_t key) {
-  const uint64_t k = key < w.lo ? w.lo : key > w.hi ? w.hi : key;
-  return k >> w.shift;
-}
-__device__ __forceinline__ RunKey run_key(const TopPlan& p) {
-  RunKey w;
-  w.lo = p.lo;
-  w.hi = p.hi;
-  w.shift = p.hb1 > 8u * p.passes ? p.hb1 - 8u * p.passes : 0u;
-  return w;
-}
-
-// One warp: first index in [from, to) whose key is in another run than r
-// (every key before it in r), else `to`. In global memory by relaxed loads: a
-// neighbouring CTA may be sorting the run, which keeps its keys inside it.
-template <bool GLOBAL>
-__device__ __forceinline__ uint32_t run_end(const Elem* a, const RunKey& w, uint64_t r, uint32_t from, uint32_t to) {
-  uint32_t lo = from, hi = to;
-  while (lo < hi) {
-    const uint32_t step = (hi - lo - 1u) / 32u + 1u;
-    const uint64_t i = (uint64_t)lo + (uint64_t)lane_id() * step;
-    const bool same = i < hi && run_of(w, GLOBAL ? ld_relaxed_u64(&a[i].key) : a[i].key) == r;
-    const uint32_t t = (uint32_t)__popc(__ballot_sync(0xffffffffu, same));
-    if (t == 0) return lo;
-    const uint64_t nhi = (uint64_t)lo + (uint64_t)t * step;
-    hi = nhi < hi ? (uint32_t)nhi : hi;
-    lo += (t - 1u) * step + 1u;
-  }
-  return lo;
-}
-
-// One warp: first index in [0, to] of the run r that a[to] (shared memory) is in.
-__device__ __forceinline__ uint32_t run_start(const Elem* a, const RunKey& w, uint64_t r, uint32_t to) {
-  uint32_t lo = 0, hi = to;  // a[i] for i < lo is in earlier runs, a[hi] in r
-  while (lo < hi) {
-    const uint32_t step = (hi - lo - 1u) / 32u + 1u;
-    const uint32_t i = lo + lane_id() * step;
-    const bool earlier = i < hi && run_of(w, a[i].key) != r;
-    const uint32_t t = (uint32_t)__popc(__ballot_sync(0xffffffffu, earlier));
-    if (t == 0) return lo;
-    hi = min(hi, lo + t * step);
-    lo += (t - 1u) * step + 1u;
-  }
-  return lo;
-}
+// the runs
 
 // A chunk of a run too long for a tile: elements [b + k kCap, ...) of the run [b, e).
 struct RunChunk {
@@ -514,10 +364,7 @@ __device__ __forceinline__ void push_run(Ctrl* ctrl, RunChunk* chunks, uint32_t*
 // Sorts the runs in place (data in X) or from Y into X. The array is cut every
 // `stride` elements; a CTA takes the runs that start in its part, as many whole
 // runs at a time as fit in a tile: it brings in a tile's worth from where it
-// stands (one bulk copy; the piece of a run at the end comes again with the
-// next tile), finds the last run start in it and sorts up to there.
-// In place a CTA may read elements of a run that its neighbour is rewriting,
-// but only to see which run they are in, which does not change.
+// stands by one bulk copy, and sorts the whole runs in it (sort_runs).
 // 2^30 elements after three passes: 7.4 ms, 4.6 TB/s of the 32 bytes per
 // element, bound by the sort's instructions (about 150 per 32 elements) and
 // shared-memory accesses (45 wavefronts per 32) at 32 resident warps per SM.
@@ -525,11 +372,10 @@ __global__ void __launch_bounds__(Tile::kThreads, 2)
     k_top_finish(Elem* __restrict__ X, Elem* __restrict__ Y, uint32_t n, uint32_t stride,
                  RunChunk* __restrict__ chunks, uint32_t* __restrict__ unsorted, Ctrl* ctrl) {
   constexpr int THREADS = Tile::kThreads;
-  constexpr uint32_t kNone = 0xffffffffu;
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ typename Tile::Shared sh;
   __shared__ __align__(8) uint64_t s_bar;
-  __shared__ uint32_t s_first, s_beyond, s_last, s_end;
+  __shared__ RunMarks s_marks;
   __shared__ RunKey s_w;
   Elem* in = reinterpret_cast<Elem*>(smem);
   uint32_t* slot = reinterpret_cast<uint32_t*>(smem + Tile::kElemBytes);
@@ -537,138 +383,48 @@ __global__ void __launch_bounds__(Tile::kThreads, 2)
   const TopPlan& plan = ctrl->top;
   const uint32_t par = plan.src_parity;
   const Elem* src = par ? Y : X;
-  const bool in_place = par == 0;
   if (plan.complete) {  // in order: at most to be copied
-    if (!in_place)
+    if (par)
       for (uint64_t i = (uint64_t)blockIdx.x * THREADS + threadIdx.x; i < n; i += (uint64_t)gridDim.x * THREADS)
         store_elem(X + i, load_elem_stream(Y + i));
     return;
   }
   if (error_raised(ctrl)) return;
-  const uint32_t tid = threadIdx.x, warp = tid >> 5;
   const uint32_t bar = smem_u32(&s_bar);
-  if (tid == 0) {
+  if (threadIdx.x == 0) {
     s_w = run_key(plan);
     mbar_init(bar, 1);
     fence_mbar_init();
   }
-  const bool clamped = plan.hb1 < 64u;
+  const bool clamped = plan.hb1 < 64u, skewed = plan.skewed != 0u;
   const uint32_t shift = run_key(plan).shift;
   const uint32_t parts = (uint32_t)(((uint64_t)n + stride - 1u) / stride);
   uint32_t phase = 0;
-  for (uint32_t part = blockIdx.x; part < parts; part += gridDim.x) {
-    uint32_t g = (uint32_t)((uint64_t)part * stride);
-    const uint32_t limit = (uint32_t)min((uint64_t)g + stride, (uint64_t)n);
-    bool known = part == 0;  // g is known to be a run's start
-    while (g < limit) {
-      const uint32_t w0 = known ? g : g - 1u;
-      const uint32_t cnt = min(kCap, n - w0);
-      // src[w0, w0 + cnt) into in[]
-      __syncthreads();  // in[] is no longer read
-      if (tid == 0) {
-        fence_proxy_async_smem();
-        mbar_arrive_expect_tx(bar, cnt * (uint32_t)sizeof(Elem));
-        for (uint32_t o = 0; o < cnt; o += 2048u)
-          bulk_g2s(smem_u32(in + o), src + w0 + o, min(2048u, cnt - o) * (uint32_t)sizeof(Elem), bar);
-      }
-      const bool ok = mbar_wait_bounded(bar, phase);
-      phase ^= 1u;
-      if (!ok) record_error(ctrl, kStatusTimeout, kWhereBulkCopy);
-      if (__syncthreads_or(!ok)) return;
-      // first run start, first one at or after `limit`, last one (tile
-      // positions; kNone, cnt and 0 when there is none), by one warp each
-      if (warp == 0) {
-        const uint32_t e = run_start(in, s_w, run_of(s_w, in[cnt - 1u].key), cnt - 1u);
-        if (lane_id() == 0) s_last = e;
-      } else if (warp == 1) {
-        const uint32_t l = limit - w0;
-        const uint32_t e = l < cnt ? run_end<false>(in, s_w, run_of(s_w, in[l - 1u].key), l, cnt) : cnt;
-        if (lane_id() == 0) s_beyond = e;
-      } else if (warp == 2) {
-        const uint32_t e = known ? 0u : run_end<false>(in, s_w, run_of(s_w, in[0].key), 1u, cnt);
-        if (lane_id() == 0) s_first = e < cnt ? e : kNone;
-      }
-      __syncthreads();
-      const uint32_t first = s_first, beyond = s_beyond, last = s_last;
-      const bool at_end = w0 + cnt == n;
-      if (first == kNone) {  // inside a run that an earlier part has
-        if (at_end || w0 + cnt >= limit) break;
-        if (warp == 0) {
-          const uint32_t e = run_end<true>(src, s_w, run_of(s_w, in[0].key), w0 + cnt, limit);
-          if (lane_id() == 0) s_end = e;
-        }
-        __syncthreads();
-        g = s_end;
-        known = true;
-        continue;
-      }
-      if (w0 + first >= limit) break;
-      const uint32_t end = beyond < cnt ? beyond : at_end ? cnt : last;
-      known = true;
-      if (end > first) {
-        g = w0 + end;
-        if (end - first == 1u && in_place) continue;
-        // whole runs: bins over their range of keys (clamped keys can lie
-        // outside it: then over the tile's own range)
-        uint64_t base = 0, range = 0;
-        if (!clamped) {
-          base = in[first].key >> shift << shift;
-          range = (in[end - 1u].key | ((1ull << shift) - 1ull)) - base;
-        }
-        Elem* out = X + w0 + first;
-        Tile::sort(in, first, end, base, range, slot, bins, sh, in_place,
-                   [&](bool on, uint32_t r, const Elem& e) { store_elem_if(on, out + r, e); });
-      } else if (first > 0u) {  // one run from `first`, not whole in the tile yet
-        g = w0 + first;
-      } else {  // a run longer than a tile
-        if (warp == 0) {
-          const uint32_t e = run_end<true>(src, s_w, run_of(s_w, in[0].key), w0 + cnt, n);
-          push_run(ctrl, chunks, unsorted, n, w0, e);
-          if (lane_id() == 0) s_end = e;
-        }
-        __syncthreads();
-        g = s_end;
-      }
+  auto load = [&](uint32_t from, uint32_t cnt) {
+    __syncthreads();  // in[] is no longer read
+    if (threadIdx.x == 0) {
+      fence_proxy_async_smem();
+      mbar_arrive_expect_tx(bar, cnt * (uint32_t)sizeof(Elem));
+      for (uint32_t o = 0; o < cnt; o += 2048u)
+        bulk_g2s(smem_u32(in + o), src + from + o, min(2048u, cnt - o) * (uint32_t)sizeof(Elem), bar);
     }
+    const bool ok = mbar_wait_bounded(bar, phase);
+    phase ^= 1u;
+    if (!ok) record_error(ctrl, kStatusTimeout, kWhereBulkCopy);
+    return !__syncthreads_or(!ok);
+  };
+  auto long_run = [&](uint32_t b, uint32_t e) { push_run(ctrl, chunks, unsorted, n, b, e); };
+  for (uint32_t part = blockIdx.x; part < parts; part += gridDim.x) {
+    const uint32_t g = (uint32_t)((uint64_t)part * stride);
+    const uint32_t limit = (uint32_t)min((uint64_t)g + stride, (uint64_t)n);
+    if (!sort_runs<Tile>(src, X, n, g, limit, part == 0, s_w, clamped, skewed, shift, in, slot, bins, sh, s_marks, load,
+                         long_run))
+      return;
   }
 }
 
 // ---------------------------------------------------------------------------
 // runs longer than a tile
-
-// Every CTA of the (co-resident) grid arrives; false when the wait ran out or
-// an error was raised.
-__device__ __forceinline__ bool grid_barrier(Ctrl* ctrl, uint32_t* round) {
-  __shared__ bool s_ok;
-  *round += 1u;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    atomicAdd(&ctrl->top.barrier, 1u);
-    const uint32_t want = *round * gridDim.x;
-    uint32_t it = 0, ns = 32;
-    bool ok = true;
-    while (ld_acquire_u32(&ctrl->top.barrier) < want) {
-      if (++it >= kSpinLimit || ((it & 63u) == 0u && error_raised(ctrl))) {
-        record_error(ctrl, kStatusTimeout, kWhereGridBarrier);
-        ok = false;
-        break;
-      }
-      __nanosleep(ns);
-      if (ns < 256) ns <<= 1;
-    }
-    __threadfence();
-    s_ok = ok;
-  }
-  __syncthreads();
-  return s_ok;
-}
-
-__device__ __forceinline__ Elem load_elem_l2(const Elem* p) {
-  Elem e;  // L2 only: another CTA has written it since this kernel began
-  asm volatile("ld.global.cg.v2.u64 {%0, %1}, [%2];" : "=l"(e.key), "=l"(e.val) : "l"(p) : "memory");
-  return e;
-}
 
 // One warp: elements of a among the first d of the stable merge of a and b.
 __device__ __forceinline__ uint32_t merge_split(const Elem* a, uint32_t la, const Elem* b, uint32_t lb, uint32_t d) {
@@ -805,11 +561,16 @@ int top_run(Elem* X, Elem* Y, unsigned char* ws, const Layout& L, cudaStream_t s
   if (n <= SmallFull::kCap) return small_sort<1024>(X, L, ctrl, st);
   DeviceInfo dev;
   if (int rc = current_device_info(&dev)) return rc;
+  if (n <= mid_limit(dev)) return mid_run(X, Y, ws, L, dev, st);
   uint32_t* hist = reinterpret_cast<uint32_t*>(ws + L.off_hist);
   uint32_t* gstart = reinterpret_cast<uint32_t*>(ws + L.off_gstart);
   uint64_t* ring = reinterpret_cast<uint64_t*>(ws + L.off_ring);
-  const SampleRule rule = sample_rule(n);
-  if (cudaFuncSetAttribute(k_top_sample, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSampleSmem) !=
+  SampleRule rule = sample_rule(n, SampleTile<kTopSample>::kCap, kMeanRun, kMeanRun, 16.0);
+  // Unused launches cost about 2 us each: below 2^26 elements only two passes
+  // more than even keys need are kept ready, and the merges, whose rounds then
+  // stay nearly in L2, take what those leave.
+  if (n < (1u << 26)) rule.tmax = std::min(8u, rule.tmin + 2u);
+  if (cudaFuncSetAttribute(k_top_sample, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSampleSmem<kTopSample>) !=
           cudaSuccess ||
       cudaFuncSetAttribute(k_top_finish, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Tile::kSmem) !=
           cudaSuccess ||
@@ -817,7 +578,7 @@ int top_run(Elem* X, Elem* Y, unsigned char* ws, const Layout& L, cudaStream_t s
     return 5;
   {
     ProfScope prof("top_sample", st);
-    k_top_sample<<<1, kSampleThreads, kSampleSmem, st>>>(X, n, rule, hist, ctrl);
+    k_top_sample<<<1, kSampleThreads, kSampleSmem<kTopSample>, st>>>(X, n, rule, hist, ctrl);
   }
   {
     // four CTAs per SM, fewer when they would have under four rounds of reads each
