@@ -192,7 +192,7 @@ int plan_layout(int64_t n, int bits, int num_digits, Layout* L, bool allow_split
     off = align_up(off + 8u * 256u * 4u, 256);
     L->off_gstart = off;
     off = align_up(off + 8u * 256u * 4u, 256);
-    L->tile_elems = onesweep_top_tile();
+    L->tile_elems = onesweep_top_tile(0);
     L->ring_tiles = std::max<uint32_t>(1u, (uint32_t)((n + L->tile_elems - 1) / L->tile_elems));
     L->off_ring = off;
     off = align_up(off + (size_t)L->ring_tiles * 256u * 8u, 256);

@@ -98,7 +98,8 @@ struct TopWindow {
   uint32_t right, left;
   bool clamp;
 };
-__device__ __forceinline__ TopWindow top_window(const TopPlan& p, int pass) {
+template <class Plan>  // TopPlan or SegPlan
+__device__ __forceinline__ TopWindow top_window(const Plan& p, int pass) {
   TopWindow w;
   w.lo = p.lo;
   w.hi = p.hi;
@@ -115,14 +116,26 @@ __device__ __forceinline__ uint32_t top_digit_clamped(const TopWindow& w, uint64
   return key < w.lo ? 0u : key > w.hi ? 255u : top_digit(w, key);
 }
 
+// Plan of one array of a batch of independent arrays, as TopPlan; its passes
+// all run, so every array's data is in Y after an odd number of them. passes =
+// 0: the array fits in a tile.
+struct SegPlan {
+  uint64_t lo, hi;
+  uint32_t hb1, passes, skewed, complete;
+  uint32_t diff[2];
+  uint32_t pad[2];
+};
+
 // A batch of independent arrays sorted together (null tile_seg: one array).
+// Arrays with more passes come first in the tiles' order, so that a pass's
+// tiles are the first num_tiles[pass].
 struct SegDesc {
   const uint32_t* tile_seg = nullptr;   // [tiles] segment of each tile
   const uint32_t* seg_tile0 = nullptr;  // [nseg] first tile of each segment
   const int64_t* seg_off = nullptr;     // [nseg + 1] element offsets of the segments
-  const uint32_t* seg_gstart = nullptr; // [nseg][passes][2^b] exclusive digit starts
-  const uint32_t* num_tiles = nullptr;  // tiles in the batch (device word)
-  int num_passes = 0;
+  const uint32_t* seg_gstart = nullptr; // [nseg][8][256] exclusive digit starts
+  const uint32_t* num_tiles = nullptr;  // [8] tiles of each pass
+  const SegPlan* plan = nullptr;        // [nseg]
 };
 
 // Bytes of the onesweep kernel's per-warp counters ([bins][wp] entries of

@@ -97,11 +97,20 @@ int top_run(Elem* X, Elem* Y, unsigned char* ws, const Layout& L, cudaStream_t s
 uint32_t mid_limit(const DeviceInfo& dev);
 size_t mid_workspace_bytes(uint32_t n, const DeviceInfo& dev);
 int mid_run(Elem* X, Elem* Y, unsigned char* ws, const Layout& L, const DeviceInfo& dev, cudaStream_t st);
-// Tile of its passes (its look-back ring has a slot for each).
-uint32_t onesweep_top_tile();
-// Pass `pass` of the plan in ctrl->top; gstart: that pass's digit starts.
+// Tile of its passes (their look-back ring has a slot for each) in the shapes
+// 0: 512 threads x 16, 1 CTA/SM; 2: 256 x 16, 2 CTAs/SM.
+uint32_t onesweep_top_tile(int variant);
+// Pass `pass` of the plan in ctrl->top, or of a batch's plans; gstart: that
+// pass's digit starts (one array); ctas: persistent CTAs, 0 = every resident slot.
 int onesweep_top_pass(Elem* X, Elem* Y, uint32_t n, int pass, const uint32_t* gstart, uint64_t* ring,
-                      uint32_t tiles, Ctrl* ctrl, const DeviceInfo& dev, cudaStream_t st);
+                      uint32_t tiles, Ctrl* ctrl, const SegDesc& seg, int variant, uint32_t ctas,
+                      const DeviceInfo& dev, cudaStream_t st);
+// The merges of runs longer than a tile (lsb_top.cu): list of chunks and marks
+// of their runs, at most top_list_bytes(n) together.
+struct RunChunk;
+size_t top_list_bytes(uint32_t n);
+int top_merge(Elem* X, Elem* Y, uint32_t n, RunChunk* chunks, uint32_t* unsorted, Ctrl* ctrl, const DeviceInfo& dev,
+              cudaStream_t st);
 // One wide digit as two half-width onesweep passes src -> mid -> dst (L: a
 // split layout of two sub-digits starting at first_digit); src is not written.
 int onesweep_pass_via(const Elem* src, Elem* mid, Elem* dst, int first_digit, unsigned char* ws,
@@ -134,12 +143,6 @@ int selftest_ring_slot(unsigned char* ws, cudaStream_t st);
 int selftest_bulk_copy(unsigned char* ws, cudaStream_t st);
 size_t selftest_wide_bytes();
 int selftest_wide_wait(int which, unsigned char* ws, cudaStream_t st);
-// explicit kernel shape (variant 0: 512 threads x 16, 1 CTA/SM; 2: 256 x 16, 2 CTAs/SM)
-uint32_t onesweep_tile_elems_v(int bits, int variant);
-uint32_t onesweep_grid_v(int bits, int variant, const DeviceInfo& dev, uint32_t tiles);
-int onesweep_launch_v(int bits, int variant, uint32_t grid, Elem* X, Elem* Y, uint32_t n, int pass,
-                      int digit, const uint32_t* gstart, uint64_t* ring, uint32_t* done,
-                      uint32_t ring_tiles, Ctrl* ctrl, const SegDesc& seg, cudaStream_t st);
 uint32_t onesweep_grid(int bits, const DeviceInfo& dev, uint32_t n);
 uint32_t task_count(const DeviceInfo& dev, uint32_t n);
 

@@ -393,7 +393,7 @@ int mid_run(Elem* X, Elem* Y, unsigned char* ws, const Layout& L, const DeviceIn
   uint32_t max_runs = mid_max_runs(n);
   // A key that overfills its bins makes a tile uneven, unless the tile is in
   // order: 2048 windows per element leave a tile without a mixed run.
-  SampleRule rule = sample_rule(n, SampleTile<kMidSample>::kCap, MidTile::kCap - 576u, MidTile::kMaxBin, 2048.0);
+  SampleRule rule = sample_rule(n, SampleTile<kMidSample>::kCap, MidTile::kCap - 576u, MidTile::kMaxBin, 2048.0f);
   const void* kern = items == 2u   ? (const void*)k_mid_sort<2>
                      : items == 4u ? (const void*)k_mid_sort<4>
                                    : (const void*)k_mid_sort<8>;

@@ -426,12 +426,13 @@ __global__ void __launch_bounds__(THREADS, MINB)
   __shared__ uint32_t s_err[2];
   __shared__ uint32_t s_wt[W];
 
-  if (TOP ? !((ctrl->top.run_mask >> pass) & 1u) : pass_skipped(ctrl, pass)) return;
+  const bool segmented = TOP && seg.tile_seg != nullptr;
+  if (TOP ? !segmented && !((ctrl->top.run_mask >> pass) & 1u) : pass_skipped(ctrl, pass)) return;
   const int bits = BITS > 0 ? BITS : bits_rt;
   const uint32_t nbins = 1u << bits, mask = nbins - 1u;
   const int shift = bits * digit;  // `pass` indexes this call's passes, `digit` the key
-  __shared__ TopWindow s_win;  // not in registers: used once per tile
-  if (TOP && threadIdx.x == 0) s_win = top_window(ctrl->top, pass);
+  __shared__ TopWindow s_win[2];  // not in registers: used once per tile
+  if (TOP && !segmented && threadIdx.x < 2) s_win[threadIdx.x] = top_window(ctrl->top, pass);
   const uint32_t cnt_words = (uint32_t)(onesweep_counter_bytes(nbins, WP, sizeof(CNT)) / 16u);
   const bool column_clear = nbins <= 256u;
   Elem* stage = reinterpret_cast<Elem*>(smem);                         // [E] tile in digit order
@@ -440,11 +441,10 @@ __global__ void __launch_bounds__(THREADS, MINB)
   uint32_t* gbase = tstart + nbins;   // [nbins] destination of the bin's first element
   uint32_t* tcount = gbase + nbins;   // [nbins] this tile's count of each bin
 
-  const uint32_t par = TOP ? (ctrl->top.par_mask >> pass) & 1u : ctrl->parity[pass];
+  const uint32_t par = segmented ? (uint32_t)pass & 1u : TOP ? (ctrl->top.par_mask >> pass) & 1u : ctrl->parity[pass];
   const Elem* __restrict__ src = par ? Y : X;
   Elem* __restrict__ dst = par ? X : Y;
-  const bool segmented = seg.tile_seg != nullptr;
-  const uint32_t num_tiles = segmented ? *seg.num_tiles : (n - 1u) / E + 1u;
+  const uint32_t num_tiles = segmented ? seg.num_tiles[pass] : (n - 1u) / E + 1u;
   // statuses with reach when every tile of the pass has its own ring slot and
   // each bin has its own walking thread; tile-tagged statuses otherwise
   const bool reach = ring_tiles >= num_tiles && nbins <= (uint32_t)THREADS;
@@ -476,7 +476,7 @@ __global__ void __launch_bounds__(THREADS, MINB)
       ti.len = min(E, se - ti.begin);
       ti.seg_base = sb;
       ti.first = j == 0;
-      ti.gs = seg.seg_gstart + ((size_t)sg * seg.num_passes + pass) * nbins;
+      ti.gs = seg.seg_gstart + ((size_t)sg * 8u + (uint32_t)pass) * 256u;
     }
     return ti;
   };
@@ -503,7 +503,10 @@ __global__ void __launch_bounds__(THREADS, MINB)
   };
 
   clear_counters();
-  if (threadIdx.x == 0) s_tile = atomicAdd(&ctrl->ticket[pass], 1u);
+  if (threadIdx.x == 0) {
+    s_tile = atomicAdd(&ctrl->ticket[pass], 1u);
+    if (segmented && s_tile < num_tiles) s_win[0] = top_window(seg.plan[seg.tile_seg[s_tile]], pass);
+  }
   __syncthreads();
   uint32_t t = s_tile;
   if (t < num_tiles) load_tile(t);
@@ -535,7 +538,7 @@ __global__ void __launch_bounds__(THREADS, MINB)
     // 1. digits
     uint32_t d[K];
     if (TOP) {
-      const TopWindow win = s_win;
+      const TopWindow win = s_win[iter & 1u];
       if (win.clamp) {
 #pragma unroll
         for (int k = 0; k < K; k++) d[k] = top_digit_clamped(win, v[k].key);
@@ -607,6 +610,8 @@ __global__ void __launch_bounds__(THREADS, MINB)
 
     uint64_t* my = ring + (size_t)slot * nbins;
     const uint32_t t_next = s_next;
+    if (segmented && threadIdx.x == THREADS - 1 && t_next < num_tiles)
+      s_win[(iter + 1u) & 1u] = top_window(seg.plan[seg.tile_seg[t_next]], pass);
     // 3. per-bin totals of the tile (published at once), scan of the totals,
     //    per-(bin, warp) starts in the digit-sorted tile written back into
     //    the counters, the tile-local start of each bin into tstart[]
@@ -799,7 +804,7 @@ template <int BITS>
 __global__ void __launch_bounds__(512, 1)
     k_onesweep2r(Elem* __restrict__ X, Elem* __restrict__ Y, uint32_t n, int, int pass, int digit,
                  const uint32_t* __restrict__ gstart, uint64_t* __restrict__ ring,
-                 uint32_t* __restrict__ done, uint32_t ring_tiles, Ctrl* ctrl, SegDesc seg) {
+                 uint32_t* __restrict__ done, uint32_t ring_tiles, Ctrl* ctrl, SegDesc) {
   constexpr int THREADS = 512, K = 16, W = THREADS / 32, WP = W + 1;
   constexpr uint32_t E = THREADS * K;
   constexpr int LB = (BITS + 1) / 2, HB = BITS - LB;
@@ -829,8 +834,7 @@ __global__ void __launch_bounds__(512, 1)
   const uint32_t par = ctrl->parity[pass];
   const Elem* __restrict__ src = par ? Y : X;
   Elem* __restrict__ dst = par ? X : Y;
-  const bool segmented = seg.tile_seg != nullptr;
-  const uint32_t num_tiles = segmented ? *seg.num_tiles : (n + E - 1) / E;
+  const uint32_t num_tiles = (n - 1u) / E + 1u;
   const uint32_t warp = threadIdx.x >> 5, lane = lane_id();
   const uint32_t lt = lanemask_lt();
   const uint32_t b0 = threadIdx.x * BPT;  // this thread's bins [b0, b0 + BPT)
@@ -842,22 +846,11 @@ __global__ void __launch_bounds__(512, 1)
   };
   auto tile_info = [&](uint32_t t) {
     TileInfo ti;
-    if (!segmented) {
-      ti.begin = t * E;
-      ti.len = min(E, n - ti.begin);
-      ti.seg_base = 0;
-      ti.first = t == 0;
-      ti.gs = gstart;
-    } else {
-      const uint32_t sg = seg.tile_seg[t];
-      const uint32_t j = t - seg.seg_tile0[sg];
-      const uint32_t sb = (uint32_t)seg.seg_off[sg], se = (uint32_t)seg.seg_off[sg + 1];
-      ti.begin = sb + j * E;
-      ti.len = min(E, se - ti.begin);
-      ti.seg_base = sb;
-      ti.first = j == 0;
-      ti.gs = seg.seg_gstart + ((size_t)sg * seg.num_passes + pass) * NB;
-    }
+    ti.begin = t * E;
+    ti.len = min(E, n - ti.begin);
+    ti.seg_base = 0;
+    ti.first = t == 0;
+    ti.gs = gstart;
     return ti;
   };
 
@@ -1408,42 +1401,23 @@ static OnesweepChoice onesweep_choice(int bits) { return onesweep_choice(bits, o
 
 uint32_t onesweep_tile_elems(int bits) { return onesweep_choice(bits).tile; }
 
-uint32_t onesweep_tile_elems_v(int bits, int variant) {
-  return onesweep_choice(bits, variant).tile;
-}
-
-uint32_t onesweep_grid_v(int bits, int variant, const DeviceInfo& dev, uint32_t tiles) {
-  const OnesweepChoice c = onesweep_choice(bits, variant);
-  cudaFuncSetAttribute(c.kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.smem);
-  int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, c.kern, c.threads, c.smem);
-  per_sm = std::max(per_sm, 1);
-  return std::max<uint32_t>(1, std::min<uint32_t>(tiles, (uint32_t)(dev.sm_count * per_sm)));
-}
-
-int onesweep_launch_v(int bits, int variant, uint32_t grid, Elem* X, Elem* Y, uint32_t n, int pass,
-                      int digit, const uint32_t* gstart, uint64_t* ring, uint32_t* done,
-                      uint32_t ring_tiles, Ctrl* ctrl, const SegDesc& seg, cudaStream_t st) {
-  const OnesweepChoice c = onesweep_choice(bits, variant);
-  ProfScope prof("onesweep_scatter", st);
-  c.kern<<<grid, c.threads, c.smem, st>>>(X, Y, n, bits, pass, digit, gstart, ring, done, ring_tiles,
-                                          ctrl, seg);
-  return cudaPeekAtLastError() == cudaSuccess ? 0 : 5;
-}
-
-// The default shape's 8-bit pass with digits, order and buffers from ctrl->top.
-constexpr int kTopThreads = 512, kTopItems = 16;
-uint32_t onesweep_top_tile() { return (uint32_t)kTopThreads * kTopItems; }
+// The 8-bit pass with its digits, and whether it runs, from ctrl->top or the
+// batch's plans, in the shapes 0 and 2.
+uint32_t onesweep_top_tile(int variant) { return variant == 2 ? 4096u : 8192u; }
 
 int onesweep_top_pass(Elem* X, Elem* Y, uint32_t n, int pass, const uint32_t* gstart, uint64_t* ring,
-                      uint32_t tiles, Ctrl* ctrl, const DeviceInfo& dev, cudaStream_t st) {
-  auto kern = k_onesweep<kTopThreads, kTopItems, 1, uint32_t, 8, true>;
-  const size_t smem = reg_kernel_smem(8, kTopThreads, kTopItems);
+                      uint32_t tiles, Ctrl* ctrl, const SegDesc& seg, int variant, uint32_t ctas,
+                      const DeviceInfo& dev, cudaStream_t st) {
+  const int threads = variant == 2 ? 256 : 512;
+  auto kern = variant == 2 ? k_onesweep<256, 16, 2, uint32_t, 8, true> : k_onesweep<512, 16, 1, uint32_t, 8, true>;
+  const size_t smem = reg_kernel_smem(8, threads, 16);
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 5;
-  const uint32_t grid = std::max<uint32_t>(1u, std::min<uint32_t>(tiles, (uint32_t)dev.sm_count));
+  uint32_t grid = (uint32_t)dev.sm_count * (variant == 2 ? 2u : 1u);
+  if (ctas > 0) grid = std::min(grid, ctas);
+  grid = std::max<uint32_t>(1u, std::min(grid, tiles));
   ProfScope prof("onesweep_scatter", st);
   // one ring slot per tile: no slot is reused, so there are no completion tags
-  kern<<<grid, kTopThreads, smem, st>>>(X, Y, n, 8, pass, 0, gstart, ring, nullptr, tiles, ctrl, SegDesc{});
+  kern<<<grid, threads, smem, st>>>(X, Y, n, 8, pass, 0, gstart, ring, nullptr, tiles, ctrl, seg);
   return cudaPeekAtLastError() == cudaSuccess ? 0 : 5;
 }
 

@@ -99,34 +99,9 @@ static int small_sort(Elem* X, const Layout& L, Ctrl* ctrl, cudaStream_t st) {
 // 0.48 ms, 2^28 15.0 -> 6.4 ms, 2^30 58.6 -> 30.8 ms (three passes), 2^28 Zipf
 // 16.0 -> 9.8 ms (four passes; heavy keys stay in order), against eight passes.
 
-using Tile = TileSort<512, 9>;  // 106 KB: two CTAs per SM, one's loads and stores beside the other's sort
-constexpr uint32_t kCap = Tile::kCap;
-// Mean run length up to which a pass is saved: six standard deviations below a tile.
-constexpr uint32_t kMeanRun = 4220;
 constexpr int kTopSample = 4;  // keys per thread of the sample: 4096
 constexpr int kTopHistThreads = 512;
 constexpr int kTopHistUnroll = 4;
-
-SampleRule sample_rule(uint32_t n, uint32_t sample, uint32_t mean_run, uint32_t often, double spread) {
-  SampleRule r;
-  auto passes_for = [&](double per_run) {
-    uint32_t t = 1;
-    while (t < 8 && (double)n > per_run * std::pow(256.0, (double)t)) t++;
-    return t;
-  };
-  r.tmin = passes_for(mean_run);
-  r.tmax = 8u;
-  r.tall = passes_for(1.0 / spread);
-  const double lam = (double)mean_run * sample / n, lom = (double)often * sample / n;
-  r.far = (uint32_t)(lam + 4.0 * std::sqrt(lam) + 4.0);
-  r.heavy = (uint32_t)(lom + 4.0 * std::sqrt(lom) + 4.0);
-  const double l = 1.25 * lam, f = 1.0 - (1.0 - std::exp(-l)) / l;
-  r.near_limit = (uint32_t)(sample * f + 3.0 * std::sqrt(sample * f)) + 1u;
-  r.far_limit = sample / 64u;
-  // sampled twice by chance: sample^2 / (2 n) pairs; every key k times in the array: k times that
-  r.dups = std::max<uint32_t>(3u, (uint32_t)(4.0 * sample * sample / n));
-  return r;
-}
 
 // Bound by latency (one CTA: 4096 scattered reads, a tile sort, two counts);
 // it also clears what the later kernels count in, in place of three memsets.
@@ -333,34 +308,6 @@ __global__ void __launch_bounds__(kTopHistThreads, 4)
 // ---------------------------------------------------------------------------
 // the runs
 
-// A chunk of a run too long for a tile: elements [b + k kCap, ...) of the run [b, e).
-struct RunChunk {
-  uint32_t b, e, k, run;
-};
-__host__ __device__ __forceinline__ uint32_t max_chunks(uint32_t n) { return 2u * (n / kCap) + 2u; }
-
-// One warp: the run [b, e) goes to the merge kernel's list (in the ring, which
-// the passes are done with): at most n / kCap runs of at least kCap elements.
-__device__ __forceinline__ void push_run(Ctrl* ctrl, RunChunk* chunks, uint32_t* unsorted, uint32_t n, uint32_t b,
-                                         uint32_t e) {
-  const uint32_t lane = lane_id();
-  const uint32_t m = (e - b - 1u) / kCap + 1u;
-  uint32_t at = 0, run = 0;
-  if (lane == 0) {
-    at = atomicAdd(&ctrl->top.num_chunks, m);
-    run = atomicAdd(&ctrl->top.num_runs, 1u);
-    atomicMax(&ctrl->top.max_rounds, 32u - (uint32_t)__clz((int)(m - 1u)));
-  }
-  at = __shfl_sync(0xffffffffu, at, 0);
-  run = __shfl_sync(0xffffffffu, run, 0);
-  if ((uint64_t)at + m > max_chunks(n)) {  // the keys changed while they were sorted
-    if (lane == 0) record_error(ctrl, kStatusInconsistent, kWhereScatter);
-    return;
-  }
-  if (lane == 0) unsorted[run] = 0u;
-  for (uint32_t k = lane; k < m; k += 32u) chunks[at + k] = RunChunk{b, e, k, run};
-}
-
 // Sorts the runs in place (data in X) or from Y into X. The array is cut every
 // `stride` elements; a CTA takes the runs that start in its part, as many whole
 // runs at a time as fit in a tile: it brings in a tile's worth from where it
@@ -400,20 +347,8 @@ __global__ void __launch_bounds__(Tile::kThreads, 2)
   const uint32_t shift = run_key(plan).shift;
   const uint32_t parts = (uint32_t)(((uint64_t)n + stride - 1u) / stride);
   uint32_t phase = 0;
-  auto load = [&](uint32_t from, uint32_t cnt) {
-    __syncthreads();  // in[] is no longer read
-    if (threadIdx.x == 0) {
-      fence_proxy_async_smem();
-      mbar_arrive_expect_tx(bar, cnt * (uint32_t)sizeof(Elem));
-      for (uint32_t o = 0; o < cnt; o += 2048u)
-        bulk_g2s(smem_u32(in + o), src + from + o, min(2048u, cnt - o) * (uint32_t)sizeof(Elem), bar);
-    }
-    const bool ok = mbar_wait_bounded(bar, phase);
-    phase ^= 1u;
-    if (!ok) record_error(ctrl, kStatusTimeout, kWhereBulkCopy);
-    return !__syncthreads_or(!ok);
-  };
-  auto long_run = [&](uint32_t b, uint32_t e) { push_run(ctrl, chunks, unsorted, n, b, e); };
+  auto load = [&](uint32_t from, uint32_t cnt) { return load_tile_bulk(in, src + from, cnt, bar, &phase, ctrl); };
+  auto long_run = [&](uint32_t b, uint32_t e) { push_run(ctrl, chunks, unsorted, n, b, e, par); };
   for (uint32_t part = blockIdx.x; part < parts; part += gridDim.x) {
     const uint32_t g = (uint32_t)((uint64_t)part * stride);
     const uint32_t limit = (uint32_t)min((uint64_t)g + stride, (uint64_t)n);
@@ -459,15 +394,13 @@ __global__ void __launch_bounds__(Tile::kThreads, 2)
   uint32_t* slot = reinterpret_cast<uint32_t*>(smem + Tile::kElemBytes);
   uint32_t* bins = reinterpret_cast<uint32_t*>(smem + Tile::kElemBytes + Tile::kSlotBytes);
   const uint32_t tid = threadIdx.x, warp = tid >> 5;
-  const uint32_t par = ctrl->top.src_parity;
-  const Elem* src = par ? Y : X;
   const uint32_t rounds = ctrl->top.max_rounds;
   uint32_t barriers = 0;
   // runs in order stay (or are copied); the others are marked. Each warp reads
   // its part of a chunk and the element after it, nine loads at a time.
   for (uint32_t c = blockIdx.x; c < total; c += gridDim.x) {
     const RunChunk t = chunks[c];
-    const Elem* run = src + t.b;
+    const Elem* run = (t.par ? Y : X) + t.b;
     const uint32_t len = t.e - t.b, at = t.k * kCap + warp * 32u * K;
     const uint32_t m = min(len - t.k * kCap, kCap);  // the chunk's
     Elem e[K];
@@ -482,7 +415,7 @@ __global__ void __launch_bounds__(Tile::kThreads, 2)
       if (lane_id() == 31) next = head;
       inversion |= e[k].key > next;
       const uint32_t i = warp * 32u * K + (uint32_t)k * 32u + lane_id();
-      if (par && i < m) store_elem(X + t.b + t.k * kCap + i, e[k]);
+      if (t.par && i < m) store_elem(X + t.b + t.k * kCap + i, e[k]);
     }
     if (__any_sync(0xffffffffu, inversion) && lane_id() == 0) unsorted[t.run] = 1u;
   }
@@ -495,6 +428,7 @@ __global__ void __launch_bounds__(Tile::kThreads, 2)
     if (!ld_relaxed_u32(unsorted + t.run)) continue;
     any = true;
     const uint32_t lo = t.b + t.k * kCap, m = min(t.e - lo, kCap);
+    const Elem* src = t.par ? Y : X;
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < K; k++) {
@@ -551,6 +485,21 @@ __global__ void __launch_bounds__(Tile::kThreads, 2)
   }
 }
 
+size_t top_list_bytes(uint32_t n) { return (size_t)max_chunks(n) * (sizeof(RunChunk) + 4u); }
+
+int top_merge(Elem* X, Elem* Y, uint32_t n, RunChunk* chunks, uint32_t* unsorted, Ctrl* ctrl, const DeviceInfo& dev,
+              cudaStream_t st) {
+  if (cudaFuncSetAttribute(k_top_merge, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Tile::kSmem) != cudaSuccess)
+    return 5;
+  const RunChunk* list = chunks;
+  void* args[] = {&X, &Y, &n, &list, &unsorted, &ctrl};
+  ProfScope prof("top_merge", st);
+  return cudaLaunchCooperativeKernel((const void*)k_top_merge, dim3((uint32_t)dev.sm_count * 2u), dim3(Tile::kThreads),
+                                     args, Tile::kSmem, st) == cudaSuccess
+             ? 0
+             : 5;
+}
+
 // ---------------------------------------------------------------------------
 // driver
 
@@ -565,7 +514,7 @@ int top_run(Elem* X, Elem* Y, unsigned char* ws, const Layout& L, cudaStream_t s
   uint32_t* hist = reinterpret_cast<uint32_t*>(ws + L.off_hist);
   uint32_t* gstart = reinterpret_cast<uint32_t*>(ws + L.off_gstart);
   uint64_t* ring = reinterpret_cast<uint64_t*>(ws + L.off_ring);
-  SampleRule rule = sample_rule(n, SampleTile<kTopSample>::kCap, kMeanRun, kMeanRun, 16.0);
+  SampleRule rule = sample_rule(n, SampleTile<kTopSample>::kCap, kMeanRun, kMeanRun, 16.0f);
   // Unused launches cost about 2 us each: below 2^26 elements only two passes
   // more than even keys need are kept ready, and the merges, whose rounds then
   // stay nearly in L2, take what those leave.
@@ -573,8 +522,7 @@ int top_run(Elem* X, Elem* Y, unsigned char* ws, const Layout& L, cudaStream_t s
   if (cudaFuncSetAttribute(k_top_sample, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSampleSmem<kTopSample>) !=
           cudaSuccess ||
       cudaFuncSetAttribute(k_top_finish, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Tile::kSmem) !=
-          cudaSuccess ||
-      cudaFuncSetAttribute(k_top_merge, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Tile::kSmem) != cudaSuccess)
+          cudaSuccess)
     return 5;
   {
     ProfScope prof("top_sample", st);
@@ -591,7 +539,7 @@ int top_run(Elem* X, Elem* Y, unsigned char* ws, const Layout& L, cudaStream_t s
   }
   if (cudaPeekAtLastError() != cudaSuccess) return 5;
   for (uint32_t p = 0; p < rule.tmax; p++)
-    if (int rc = onesweep_top_pass(X, Y, n, (int)p, gstart + p * 256u, ring, L.ring_tiles, ctrl, dev, st)) return rc;
+    if (int rc = onesweep_top_pass(X, Y, n, (int)p, gstart + p * 256u, ring, L.ring_tiles, ctrl, SegDesc{}, 0, 0u, dev, st)) return rc;
   RunChunk* chunks = reinterpret_cast<RunChunk*>(ring);
   uint32_t* unsorted = reinterpret_cast<uint32_t*>(chunks + max_chunks(n));
   {
@@ -609,16 +557,7 @@ int top_run(Elem* X, Elem* Y, unsigned char* ws, const Layout& L, cudaStream_t s
     k_top_finish<<<grid, Tile::kThreads, Tile::kSmem, st>>>(X, Y, n, stride, chunks, unsorted, ctrl);
   }
   if (cudaPeekAtLastError() != cudaSuccess) return 5;
-  {
-    uint32_t nn = n;
-    const RunChunk* cc = chunks;
-    void* args[] = {&X, &Y, &nn, &cc, &unsorted, &ctrl};
-    ProfScope prof("top_merge", st);
-    if (cudaLaunchCooperativeKernel((const void*)k_top_merge, dim3((uint32_t)dev.sm_count * 2u), dim3(Tile::kThreads), args,
-                                    Tile::kSmem, st) != cudaSuccess)
-      return 5;
-  }
-  return 0;
+  return top_merge(X, Y, n, chunks, unsorted, ctrl, dev, st);
 }
 
 }  // namespace lsb

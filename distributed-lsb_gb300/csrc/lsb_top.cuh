@@ -52,7 +52,29 @@ struct SampleRule {
 // mean_run: the mean run length up to which a pass is saved. Keys that occur
 // more than `often` times are heavy, and the passes then have `spread` windows
 // or more per element. sample: keys in the sample.
-SampleRule sample_rule(uint32_t n, uint32_t sample, uint32_t mean_run, uint32_t often, double spread);
+__host__ __device__ inline uint32_t passes_for(float n, float per_run) {
+  uint32_t t = 1;
+  for (float most = per_run * 256.0f; t < 8u && n > most; most *= 256.0f) t++;
+  return t;
+}
+__host__ __device__ inline SampleRule sample_rule(uint32_t n, uint32_t sample, uint32_t mean_run, uint32_t often,
+                                                  float spread) {
+  SampleRule r;
+  const float per = (float)sample / (float)n;
+  r.tmin = passes_for((float)n, (float)mean_run);
+  r.tmax = 8u;
+  r.tall = passes_for((float)n, 1.0f / spread);
+  const float lam = (float)mean_run * per, lom = (float)often * per;
+  r.far = (uint32_t)(lam + 4.0f * sqrtf(lam) + 4.0f);
+  r.heavy = (uint32_t)(lom + 4.0f * sqrtf(lom) + 4.0f);
+  const float l = 1.25f * lam, f = 1.0f - (1.0f - expf(-l)) / l;
+  r.near_limit = (uint32_t)((float)sample * f + 3.0f * sqrtf((float)sample * f)) + 1u;
+  r.far_limit = sample / 64u;
+  // sampled twice by chance: sample^2 / (2 n) pairs; every key k times in the array: k times that
+  const float pairs = 4.0f * (float)sample * per;
+  r.dups = pairs > 3.0f ? (uint32_t)pairs : 3u;
+  return r;
+}
 
 __device__ __forceinline__ uint32_t mix32(uint32_t x) {
   x ^= x >> 16;
@@ -152,7 +174,8 @@ __device__ __forceinline__ uint64_t run_of(const RunKey& w, uint64_t key) {
   const uint64_t k = key < w.lo ? w.lo : key > w.hi ? w.hi : key;
   return k >> w.shift;
 }
-__device__ __forceinline__ RunKey run_key(const TopPlan& p) {
+template <class Plan>
+__device__ __forceinline__ RunKey run_key(const Plan& p) {
   RunKey w;
   w.lo = p.lo;
   w.hi = p.hi;
@@ -325,6 +348,58 @@ __device__ __forceinline__ bool sort_runs(const Elem* src, Elem* X, uint32_t n, 
     }
   }
   return true;
+}
+
+// ---------------------------------------------------------------------------
+// tiles of runs and runs longer than a tile
+
+using Tile = TileSort<512, 9>;  // 106 KB: two CTAs per SM, one's loads and stores beside the other's sort
+constexpr uint32_t kCap = Tile::kCap;
+// Mean run length up to which a pass is saved: six standard deviations below a tile.
+constexpr uint32_t kMeanRun = 4220;
+// A chunk of a run too long for a tile: elements [b + k kCap, ...) of the run [b, e).
+struct RunChunk {
+  uint32_t b, e, k, run : 31, par : 1;  // par: the run lies in Y
+};
+__host__ __device__ __forceinline__ uint32_t max_chunks(uint32_t n) { return 2u * (n / kCap) + 2u; }
+
+// One warp: the run [b, e) goes to the merge kernel's list (in the ring, which
+// the passes are done with): at most n / kCap runs of at least kCap elements.
+__device__ __forceinline__ void push_run(Ctrl* ctrl, RunChunk* chunks, uint32_t* unsorted, uint32_t n, uint32_t b,
+                                         uint32_t e, uint32_t par) {
+  const uint32_t lane = lane_id();
+  const uint32_t m = (e - b - 1u) / kCap + 1u;
+  uint32_t at = 0, run = 0;
+  if (lane == 0) {
+    at = atomicAdd(&ctrl->top.num_chunks, m);
+    run = atomicAdd(&ctrl->top.num_runs, 1u);
+    atomicMax(&ctrl->top.max_rounds, 32u - (uint32_t)__clz((int)(m - 1u)));
+  }
+  at = __shfl_sync(0xffffffffu, at, 0);
+  run = __shfl_sync(0xffffffffu, run, 0);
+  if ((uint64_t)at + m > max_chunks(n)) {  // the keys changed while they were sorted
+    if (lane == 0) record_error(ctrl, kStatusInconsistent, kWhereScatter);
+    return;
+  }
+  if (lane == 0) unsorted[run] = 0u;
+  for (uint32_t k = lane; k < m; k += 32u) chunks[at + k] = RunChunk{b, e, k, run, par};
+}
+
+// src[0, cnt) into in[] by bulk copies that complete on the barrier `bar` (of one
+// arrival), for the whole CTA; false when the wait ran out.
+__device__ __forceinline__ bool load_tile_bulk(Elem* in, const Elem* src, uint32_t cnt, uint32_t bar, uint32_t* phase,
+                                               Ctrl* ctrl) {
+  __syncthreads();  // in[] is no longer read
+  if (threadIdx.x == 0) {
+    fence_proxy_async_smem();
+    mbar_arrive_expect_tx(bar, cnt * (uint32_t)sizeof(Elem));
+    for (uint32_t o = 0; o < cnt; o += 2048u)
+      bulk_g2s(smem_u32(in + o), src + o, min(2048u, cnt - o) * (uint32_t)sizeof(Elem), bar);
+  }
+  const bool ok = mbar_wait_bounded(bar, *phase);
+  *phase ^= 1u;
+  if (!ok) record_error(ctrl, kStatusTimeout, kWhereBulkCopy);
+  return !__syncthreads_or(!ok);
 }
 
 // ---------------------------------------------------------------------------

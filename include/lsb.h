@@ -73,8 +73,8 @@ typedef struct lsb_stats {
   int32_t device_status;  /* LSB_OK or LSB_ERR_DEVICE_TIMEOUT                      */
   int32_t passes_planned; /* ceil(64 / digit_bits)                                  */
   int32_t passes_run;     /* passes whose digit was not constant                    */
-  uint32_t skipped_mask;  /* bit p set: digit p was constant and its pass skipped   */
-  int32_t final_copy;     /* 1 if an odd pass count required a copy back into A     */
+  uint32_t skipped_mask;  /* bit p set: digit p was constant (nothing to sort by)   */
+  int32_t final_copy;     /* 1 if that many kernel passes would end in d_b          */
   int32_t digit_bits;
   int64_t n;
 } lsb_stats_t;
@@ -98,7 +98,10 @@ int lsb_workspace_bytes(int64_t n, int digit_bits, size_t* bytes);
 
 /* Stably sort d_a[0..n) by key; d_b[0..n) is scratch. Result in d_a.
  * Replaces mySort(A, B) (mpi/mpi_lsbsort.cpp:592-597), whose result is also
- * left in A with B as scratch (:591).
+ * left in A with B as scratch (:591). The result does not depend on digit_bits:
+ * the sort passes over the top digits only, as many as leave runs that fit in
+ * shared memory, and sorts those there; lsb_query reports by digit_bits which
+ * digits are constant.
  * d_workspace: a device buffer of at least lsb_workspace_bytes(n, b) bytes,
  * 256-byte aligned, or NULL. With a workspace the call is asynchronous on
  * `stream`; lsb_query() reports device-side failures. With NULL the library
@@ -175,11 +178,13 @@ int lsb_verify(const lsb_elem_t* d_in, const lsb_elem_t* d_out, int64_t n, uint6
  * buffer in the same launches. Segment s is d_a[off[s] .. off[s+1]) with
  * off[0] = 0 and off[nseg] = n_total (device array of nseg + 1 int64). Each
  * segment ends up sorted exactly as lsb_sort_pairs would sort it alone.
- * Digit widths 1..11, 12, 14 and 16 (wide even widths run as two half-width
- * sub-passes per digit). */
+ * Digit widths 1..11, 12, 14 and 16 are accepted. Arrays that fit in a CTA's
+ * shared memory are sorted there; larger ones are passed over by as many of
+ * their top digits as leave runs that fit. */
 typedef struct lsb_tuning {
-  int32_t digit_bits; /* digit width of the passes (result identical for all)  */
-  int32_t variant;    /* kernel shape: 0 = 8192-element tiles, 1 CTA per SM;
+  int32_t digit_bits; /* digit width that lsb_query reports by (result identical
+                         for all; the passes choose their own digits)          */
+  int32_t variant;    /* shape of the passes: 0 = 8192-element tiles, 1 CTA per SM;
                          2 = 4096-element tiles, 2 CTAs per SM                 */
   int32_t ctas;       /* persistent CTAs of the passes (0 = every resident slot) */
   int32_t reserved;
@@ -196,8 +201,8 @@ int lsb_sort_segmented(lsb_elem_t* d_a, lsb_elem_t* d_b, int64_t n_total,
                        const int64_t* d_seg_offsets, int64_t nseg, const lsb_tuning_t* opt_tuning,
                        void* d_workspace, size_t workspace_bytes, void* stream);
 
-/* Autotuner: times every candidate configuration (digit width 8, 11 or 16,
- * kernel shape 0 or 2, all resident CTAs or one per SM or half the SMs) on a
+/* Autotuner: times every candidate configuration (kernel shape 0 or 2, all
+ * resident CTAs or one per SM or half the SMs; digit width 8) on a
  * sample batch with the same segment sizes as
  * h_seg_offsets (host array, nseg + 1 entries; random keys, at most ~2^26
  * elements) and returns the fastest. Results are cached per size class (log2

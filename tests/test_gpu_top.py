@@ -100,3 +100,26 @@ def test_top_digits(lsb, cuda, oracle, n):
         diff = int(np.bitwise_or.reduce(keys ^ keys[0]))
         skipped = sum(1 << d for d in range(4) if not (diff >> (16 * d)) & 0xFFFF)
         assert (st.device_status, st.passes_planned, st.skipped_mask, st.n) == (0, 4, skipped, n), (n, name)
+
+
+@pytest.mark.parametrize("variant", [0, 2])
+def test_segments_of_every_kind(lsb, cuda, oracle, variant):
+    """A batch whose arrays take each route: empty, one element, at the edges of
+    the on-chip tile, one and two passes, and every kind of keys above."""
+    parts = []
+    for i, n in enumerate((0, 1, 2, 1000, 4607, 4608, 4609, 9217, 40000, 1100001)):
+        sets = dict(large_key_sets(n, n)) if n > 9000 else dict(key_sets(n, n)) if n > 1 else {"one": np.arange(n, dtype=np.uint64)}
+        for keys in sets.values() if n < 1000000 else [sets["uniform"], sets["dups"], sets["half_one_key_and_close_ones"]]:
+            parts.append(_elems(keys))
+    order = np.random.default_rng(variant).permutation(len(parts))
+    parts = [parts[i] for i in order]
+    off = np.zeros(len(parts) + 1, dtype=np.int64)
+    off[1:] = np.cumsum([len(x) for x in parts])
+    A = to_dev(np.concatenate(parts), cuda)
+    B = cuda.empty_like(A)
+    ws = lsb.alloc_segmented_workspace(A.shape[0], len(parts), 16)
+    lsb.sort_segmented(A, B, cuda.from_numpy(off).cuda(), tuning=lsb.Tuning(digit_bits=16, variant=variant), workspace=ws)
+    assert lsb.query(ws).device_status == 0
+    got = to_np(A)
+    for s, a in enumerate(parts):
+        assert np.array_equal(got[off[s]:off[s + 1]], oracle.stable_sort_by_key(a)), (s, len(a))
