@@ -75,6 +75,16 @@ int current_device_info(DeviceInfo* info) {
   return 0;
 }
 
+bool allow_smem(const void* kern, size_t bytes, std::atomic<uint64_t>* done) {
+  int dev = -1;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0) return false;
+  const uint64_t bit = dev < 64 ? 1ull << dev : 0ull;
+  if (done->load(std::memory_order_acquire) & bit) return true;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) return false;
+  done->fetch_or(bit, std::memory_order_release);
+  return true;
+}
+
 int pool_alloc(void** ptr, size_t bytes, cudaStream_t st) {
   cudaMemPool_t pool = device_pool();
   if (!pool) return LSB_ERR_NO_DEVICE;
@@ -159,8 +169,10 @@ int plan_layout(int64_t n, int bits, int num_digits, Layout* L, bool allow_split
   if (bits <= kMaxOnesweepBits) {
     L->family = Family::kOnesweep;
     L->tile_elems = onesweep_tile_elems(bits);
-    L->grid = onesweep_grid(bits, dev, L->n);
     const uint32_t tiles = (uint32_t)((n + L->tile_elems - 1) / L->tile_elems);
+    // (a whole sort launches its own shapes: only the ring's size is asked for)
+    if (!whole_sort || (uint64_t)tiles * ((uint64_t)8u << bits) > std::max<uint64_t>(64ull << 20, (uint64_t)n * 2u))
+      L->grid = onesweep_grid(bits, dev, L->n);
     L->ring_tiles = ring_slots((uint64_t)n, tiles, bits, L->grid, compact);
     L->off_hist = off;
     off = align_up(off + (size_t)num_digits * nbins * 4u, 256);

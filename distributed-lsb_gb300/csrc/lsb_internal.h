@@ -21,6 +21,7 @@
 //    scan, shuffle) with MPI ranks replaced by CTAs.
 #pragma once
 
+#include <atomic>
 #include <cstddef>
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -165,6 +166,12 @@ inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 // Stream-ordered allocation from the library's per-device pool (freed blocks
 // stay in the pool for later calls). Returns an LSB_ERR_* code.
 int pool_alloc(void** ptr, size_t bytes, cudaStream_t st);
+
+// Allows kernel `kern` `bytes` of dynamic shared memory on the current device.
+// `done`: the call site's own word, a bit for each device where that has been
+// done (devices from 64 on ask every time); the attribute stays set, and asking
+// for it costs a microsecond of each call.
+bool allow_smem(const void* kern, size_t bytes, std::atomic<uint64_t>* done);
 
 // Host-buffer sort (lsb_host.cu): the number of chunks whose copies overlap
 // the sorts of earlier chunks (1 = copy in, sort, copy out), and the chunked

@@ -397,8 +397,8 @@ int mid_run(Elem* X, Elem* Y, unsigned char* ws, const Layout& L, const DeviceIn
   const void* kern = items == 2u   ? (const void*)k_mid_sort<2>
                      : items == 4u ? (const void*)k_mid_sort<4>
                                    : (const void*)k_mid_sort<8>;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMidSmem) != cudaSuccess ||
-      cudaMemsetAsync(ws, 0, kCtrlBytes, st) != cudaSuccess)
+  static std::atomic<uint64_t> allowed[3];
+  if (!allow_smem(kern, kMidSmem, &allowed[items >> 2]) || cudaMemsetAsync(ws, 0, kCtrlBytes, st) != cudaSuccess)
     return 5;
   // CTAs beyond the tiles take a share of the runs
   const uint32_t grid = std::min<uint32_t>((uint32_t)dev.sm_count, std::max(tiles, (n - 1u) / 2048u + 1u));

@@ -1411,7 +1411,8 @@ int onesweep_top_pass(Elem* X, Elem* Y, uint32_t n, int pass, const uint32_t* gs
   const int threads = variant == 2 ? 256 : 512;
   auto kern = variant == 2 ? k_onesweep<256, 16, 2, uint32_t, 8, true> : k_onesweep<512, 16, 1, uint32_t, 8, true>;
   const size_t smem = reg_kernel_smem(8, threads, 16);
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 5;
+  static std::atomic<uint64_t> allowed[2];
+  if (!allow_smem((const void*)kern, smem, &allowed[variant == 2 ? 1 : 0])) return 5;
   uint32_t grid = (uint32_t)dev.sm_count * (variant == 2 ? 2u : 1u);
   if (ctas > 0) grid = std::min(grid, ctas);
   grid = std::max<uint32_t>(1u, std::min(grid, tiles));

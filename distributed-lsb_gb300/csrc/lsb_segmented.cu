@@ -396,8 +396,9 @@ static int seg_run(Elem* A, Elem* B, const int64_t* seg_off, void* ws, const Seg
   DeviceInfo dev;
   if (int rc = current_device_info(&dev)) return rc;
   const size_t sample_smem = kSampleSmem<kSegSample>;
-  if (cudaFuncSetAttribute(k_seg_sample, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sample_smem) != cudaSuccess ||
-      cudaFuncSetAttribute(k_seg_finish, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Tile::kSmem) != cudaSuccess)
+  static std::atomic<uint64_t> allowed[2];
+  if (!allow_smem((const void*)k_seg_sample, sample_smem, &allowed[0]) ||
+      !allow_smem((const void*)k_seg_finish, Tile::kSmem, &allowed[1]))
     return LSB_ERR_CUDA;
   // passes that the largest array there can be might need and two more, the
   // four of heavy keys, or all eight when empty launches (2 us each) do not count

@@ -7,7 +7,7 @@
 //      bins, 1.8 or more per element, and one shared atomic per element counts
 //      them and gives the element a place among its bin's (in any order);
 //   2. an exclusive scan of the bins' counts; each element's slot is written:
-//      (the key's next 18 or 19 bits below the bin, the element's position in the tile);
+//      (the key's next 18 to 22 bits below the bin, the element's position in the tile);
 //   3. an element's rank in its bin is the number of its bin's slots below
 //      its own: positions break ties, which makes the sort stable although the
 //      atomics are not. Slots that agree in the key bits compare whole keys.
@@ -56,7 +56,8 @@ struct TileSort {
   static constexpr uint32_t kCap = (uint32_t)THREADS * K;     // largest tile
   static constexpr int kBinsPerThread = 16;
   static constexpr uint32_t kBins = (uint32_t)THREADS * kBinsPerThread;
-  static constexpr uint32_t kPosBits = kCap <= 8192 ? 13 : 14;  // bits of a position in a slot
+  // bits of a position in a slot
+  static constexpr uint32_t kPosBits = kCap <= 1024 ? 10 : kCap <= 2048 ? 11 : kCap <= 4096 ? 12 : kCap <= 8192 ? 13 : 14;
   static constexpr uint32_t kPosMask = (1u << kPosBits) - 1u;
   static constexpr uint32_t kMaxBin = 24;
   static constexpr uint32_t kMaxHeavy = kCap / (kMaxBin + 1u);  // bins above it

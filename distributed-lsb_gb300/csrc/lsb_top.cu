@@ -76,7 +76,8 @@ template <int THREADS>
 static int small_sort(Elem* X, const Layout& L, Ctrl* ctrl, cudaStream_t st) {
   auto kern = k_small_sort<THREADS, 9>;
   const size_t smem = TileSort<THREADS, 9>::kSmem;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 5;
+  static std::atomic<uint64_t> allowed;  // of this instance
+  if (!allow_smem((const void*)kern, smem, &allowed)) return 5;
   ProfScope prof("small_sort", st);
   kern<<<1, THREADS, smem, st>>>(X, L.n, L.stat_bits, L.stat_digits, L.api_bits, L.sub, ctrl);
   return cudaPeekAtLastError() == cudaSuccess ? 0 : 5;
@@ -489,8 +490,8 @@ size_t top_list_bytes(uint32_t n) { return (size_t)max_chunks(n) * (sizeof(RunCh
 
 int top_merge(Elem* X, Elem* Y, uint32_t n, RunChunk* chunks, uint32_t* unsorted, Ctrl* ctrl, const DeviceInfo& dev,
               cudaStream_t st) {
-  if (cudaFuncSetAttribute(k_top_merge, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Tile::kSmem) != cudaSuccess)
-    return 5;
+  static std::atomic<uint64_t> allowed;
+  if (!allow_smem((const void*)k_top_merge, Tile::kSmem, &allowed)) return 5;
   const RunChunk* list = chunks;
   void* args[] = {&X, &Y, &n, &list, &unsorted, &ctrl};
   ProfScope prof("top_merge", st);
@@ -519,10 +520,9 @@ int top_run(Elem* X, Elem* Y, unsigned char* ws, const Layout& L, cudaStream_t s
   // more than even keys need are kept ready, and the merges, whose rounds then
   // stay nearly in L2, take what those leave.
   if (n < (1u << 26)) rule.tmax = std::min(8u, rule.tmin + 2u);
-  if (cudaFuncSetAttribute(k_top_sample, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSampleSmem<kTopSample>) !=
-          cudaSuccess ||
-      cudaFuncSetAttribute(k_top_finish, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Tile::kSmem) !=
-          cudaSuccess)
+  static std::atomic<uint64_t> allowed[2];
+  if (!allow_smem((const void*)k_top_sample, kSampleSmem<kTopSample>, &allowed[0]) ||
+      !allow_smem((const void*)k_top_finish, Tile::kSmem, &allowed[1]))
     return 5;
   {
     ProfScope prof("top_sample", st);

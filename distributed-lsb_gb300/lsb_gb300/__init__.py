@@ -167,16 +167,25 @@ def _check(rc: int, what: str) -> None:
         raise LsbError(rc, what)
 
 
+_raw_stream = None
+
+
 def _stream_ptr(stream):
-    if stream is None:
+    """cudaStream_t of `stream`, or of the current device's current stream."""
+    global _raw_stream
+    if stream is not None:
+        return stream.cuda_stream
+    if _raw_stream is None:
         import torch
 
-        stream = torch.cuda.current_stream()
-    return ctypes.c_void_p(stream.cuda_stream)
+        torch.cuda.init()
+        get, device = torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice
+        _raw_stream = lambda: get(device())  # noqa: E731 - a Stream object per call costs 3 us
+    return _raw_stream()
 
 
-def _ptr(t) -> ctypes.c_void_p:
-    return ctypes.c_void_p(t.data_ptr()) if t is not None and t.numel() else ctypes.c_void_p(0)
+def _ptr(t) -> int:
+    return t.data_ptr() if t is not None and t.numel() else 0
 
 
 def num_passes(digit_bits: int) -> int:
@@ -200,11 +209,11 @@ def sort_pairs(a, b, digit_bits: int = 16, workspace=None, stream=None) -> None:
     """mySort(A, B): sorts ``a`` (int64 (n, 2) CUDA tensor) in place by key,
     stably; ``b`` is scratch of the same shape. Asynchronous when a workspace
     tensor is given, blocking (and status-checked) otherwise."""
-    n = a.shape[0]
-    ws = _ptr(workspace) if workspace is not None else ctypes.c_void_p(0)
     wsb = workspace.numel() if workspace is not None else 0
-    _check(load().lsb_sort_pairs(_ptr(a), _ptr(b), n, digit_bits, ws, wsb, _stream_ptr(stream)),
-           "lsb_sort_pairs")
+    rc = (_lib or load()).lsb_sort_pairs(a.data_ptr(), 0 if b is None else b.data_ptr(), a.size(0), digit_bits,
+                                         workspace.data_ptr() if wsb else 0, wsb, _stream_ptr(stream))
+    if rc:
+        _check(rc, "lsb_sort_pairs")
 
 
 def pass_workspace_bytes(n: int, digit_bits: int) -> int:
@@ -217,7 +226,7 @@ def pass_workspace_bytes(n: int, digit_bits: int) -> int:
 def global_shuffle(src, dst, digit: int, digit_bits: int = 16, workspace=None, stream=None) -> None:
     """One pass: ``dst`` = ``src`` stably sorted by ``digit``."""
     n = src.shape[0]
-    ws = _ptr(workspace) if workspace is not None else ctypes.c_void_p(0)
+    ws = _ptr(workspace)
     wsb = workspace.numel() if workspace is not None else 0
     _check(load().lsb_pass(_ptr(src), _ptr(dst), n, digit_bits, digit, ws, wsb, _stream_ptr(stream)),
            "lsb_pass")
@@ -323,7 +332,7 @@ def tune_segmented(offsets_host, stream=None) -> Tuning:
 def sort_segmented(a, b, offsets, tuning: Tuning | None = None, workspace=None, stream=None) -> None:
     """Sorts every segment a[offsets[s]:offsets[s+1]] in place (offsets: int64
     CUDA tensor of nseg + 1 entries)."""
-    ws = _ptr(workspace) if workspace is not None else ctypes.c_void_p(0)
+    ws = _ptr(workspace)
     wsb = workspace.numel() if workspace is not None else 0
     tp = ctypes.byref(tuning) if tuning is not None else None
     _check(load().lsb_sort_segmented(_ptr(a), _ptr(b), a.shape[0], _ptr(offsets), offsets.shape[0] - 1, tp,
