@@ -47,6 +47,7 @@
 #include <cstring>
 
 #include "lsb_internal.h"
+#include "lsb_tile.cuh"
 
 namespace lsb {
 
@@ -208,7 +209,7 @@ __device__ __forceinline__ void byte_flush(const uint32_t* words, uint32_t* g) {
 // ---------------------------------------------------------------------------
 // histogram of ND 16-bit digits, one read of the keys
 
-constexpr int kH16Threads = 512;
+constexpr int kH16Threads = 1024;
 constexpr int kH16Unroll = 8;
 
 // group == 1: the CTAs share the whole array (grid-stride) and count digits
@@ -217,12 +218,19 @@ constexpr int kH16Unroll = 8;
 // counting the ND digits from first_digit + r*ND, so that L2 serves every
 // read of a key after the first: G*ND digits in one HBM read without the
 // shared memory for all of them in one CTA.
+// All of a round's counter additions are issued before any of their returned
+// words is looked at, so that their shared-memory round trips overlap, and one
+// test covers them: the rare carries are repaired afterwards. dump: the CTA's
+// counters are stored there as they are, ND x 64 KiB, and k_hist16_sum adds
+// them up; without it they go to the counts by one global atomic for each bin
+// that is not empty, which for 2^26 even keys took a third of the time.
 template <int ND>
-__global__ void __launch_bounds__(kH16Threads, ND == 1 ? 3 : 1)
+__global__ void __launch_bounds__(kH16Threads, ND == 1 ? 2 : 1)
     k_hist16(const Elem* __restrict__ data, uint32_t n, int first_digit,
-             uint32_t* __restrict__ ghist, uint32_t group) {
-  extern __shared__ uint32_t cw[];  // [ND][16384]
-  for (uint32_t i = threadIdx.x; i < ND * 16384u; i += blockDim.x) cw[i] = 0u;
+             uint32_t* __restrict__ ghist, uint32_t group, uint32_t* __restrict__ dump) {
+  extern __shared__ __align__(16) uint32_t cw[];  // [ND][16384]
+  for (uint32_t i = threadIdx.x; i < ND * 4096u; i += blockDim.x)
+    reinterpret_cast<uint4*>(cw)[i] = make_uint4(0, 0, 0, 0);
   __syncthreads();
   const uint32_t lane = lane_id();
   const uint64_t chunk = 32u * kH16Unroll;
@@ -244,49 +252,77 @@ __global__ void __launch_bounds__(kH16Threads, ND == 1 ? 3 : 1)
     threads_total = (uint64_t)gridDim.x * blockDim.x;
     gt = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   }
+  const int shift = 16 * first_digit;
+  uint32_t held[ND] = {}, held_n[ND] = {};
   const uint64_t full_end = lo + (hi - lo) / chunk * chunk;
   for (uint64_t base = lo + gw * chunk; base < full_end; base += warps_total * chunk) {
-    uint64_t key[kH16Unroll];
+    uint64_t key[kH16Unroll];  // the counted digits, lowest first
 #pragma unroll
-    for (int u = 0; u < kH16Unroll; u++)
-      key[u] = load_elem_stream(data + base + (uint64_t)u * 32u + lane).key;
-    // All the round's counter additions are issued before any of their
-    // returned words is looked at, so that their shared-memory round trips
-    // overlap; the rare carries are repaired afterwards.
+    for (int u = 0; u < kH16Unroll; u++) {
+      const Elem e = load_elem_stream(data + base + (uint64_t)u * 32u + lane);
+      key[u] = ND <= 2 ? (uint64_t)(uint32_t)(e.key >> shift) : e.key >> shift;
+    }
     constexpr int kHalf = kH16Unroll / 2;
 #pragma unroll
     for (int h0 = 0; h0 < kH16Unroll; h0 += kHalf) {
-      uint32_t old[kHalf][ND], inc[kHalf][ND], dig[kHalf][ND];
+      uint32_t old[kHalf][ND];
+      bool carry = false;
+      uint32_t same = 0;
 #pragma unroll
-      for (int uu = 0; uu < kHalf; uu++) {
-        const int u = h0 + uu;
+      for (int u = 0; u < kHalf; u++) {
         // bits in which some lane's key differs from lane 0's: a digit whose
         // bits are all clear there is the same in the whole warp (skewed
-        // inputs), and lane 0 counts all 32 at once
-        const uint64_t x = key[u] ^ __shfl_sync(0xffffffffu, key[u], 0);
-        const uint64_t diff = ((uint64_t)__reduce_or_sync(0xffffffffu, (uint32_t)(x >> 32)) << 32) |
-                              __reduce_or_sync(0xffffffffu, (uint32_t)x);
+        // inputs); the warp counts such a digit in a register while it lasts
+        const uint64_t k = key[h0 + u];
+        const uint32_t xl = __reduce_or_sync(0xffffffffu, (uint32_t)k ^ __shfl_sync(0xffffffffu, (uint32_t)k, 0));
+        const uint32_t xh =
+            ND <= 2 ? 0u
+                    : __reduce_or_sync(0xffffffffu, (uint32_t)(k >> 32) ^ __shfl_sync(0xffffffffu, (uint32_t)(k >> 32), 0));
 #pragma unroll
         for (int dd = 0; dd < ND; dd++) {
-          const int shift = 16 * (first_digit + dd);
-          const uint32_t d = digit_of(key[u], shift, 0xFFFFu);
-          const uint32_t v = digit_of(diff, shift, 0xFFFFu) == 0u ? (lane == 0 ? 32u : 0u) : 1u;
-          dig[uu][dd] = d;
-          inc[uu][dd] = v;
-          old[uu][dd] = v ? atomicAdd(&cw[dd * 16384 + (d >> 2)], v << ((d & 3u) * 8u)) : 0u;
+          const uint32_t d = (uint32_t)(k >> (16 * dd)) & 0xFFFFu;
+          const bool mixed = ((dd < 2 ? xl : xh) >> (16 * (dd & 1)) & 0xFFFFu) != 0u;
+          old[u][dd] = atom_add_if(mixed, &cw[dd * 16384 + (d >> 2)], 1u << ((d & 3u) * 8u));  // 0 if not
+          if (!mixed) same |= 1u << (u * ND + dd);
         }
       }
 #pragma unroll
-      for (int uu = 0; uu < kHalf; uu++) {
+      for (int u = 0; u < kHalf; u++)
 #pragma unroll
         for (int dd = 0; dd < ND; dd++) {
-          const uint32_t d = dig[uu][dd], v = inc[uu][dd];
-          if (((old[uu][dd] >> ((d & 3u) * 8u)) & 0xFFu) + v >= 256u)
-            byte_carry_fix(old[uu][dd], d, ghist + (size_t)dd * 65536u);
+          const uint32_t q = (uint32_t)(key[h0 + u] >> (16 * dd)) & 3u;
+          carry |= ((old[u][dd] >> (8u * q)) & 0xFFu) == 0xFFu;
         }
+      if (same) {
+#pragma unroll
+        for (int u = 0; u < kHalf; u++)
+#pragma unroll
+          for (int dd = 0; dd < ND; dd++) {
+            if (!(same >> (u * ND + dd) & 1u)) continue;
+            const uint32_t d = (uint32_t)(key[h0 + u] >> (16 * dd)) & 0xFFFFu;
+            if (d != held[dd]) {
+              if (lane == 0 && held_n[dd]) atomicAdd(&ghist[(size_t)dd * 65536u + held[dd]], held_n[dd]);
+              held[dd] = d;
+              held_n[dd] = 0u;
+            }
+            held_n[dd] += 32u;
+          }
+      }
+      if (carry) {
+#pragma unroll
+        for (int u = 0; u < kHalf; u++)
+#pragma unroll
+          for (int dd = 0; dd < ND; dd++) {
+            const uint32_t d = (uint32_t)(key[h0 + u] >> (16 * dd)) & 0xFFFFu;
+            if (((old[u][dd] >> (8u * (d & 3u))) & 0xFFu) == 0xFFu)
+              byte_carry_fix(old[u][dd], d, ghist + (size_t)dd * 65536u);
+          }
       }
     }
   }
+#pragma unroll
+  for (int dd = 0; dd < ND; dd++)
+    if (lane == 0 && held_n[dd]) atomicAdd(&ghist[(size_t)dd * 65536u + held[dd]], held_n[dd]);
   for (uint64_t i = full_end + gt; i < hi; i += threads_total) {
     const uint64_t k = load_elem_stream(data + i).key;
 #pragma unroll
@@ -295,69 +331,104 @@ __global__ void __launch_bounds__(kH16Threads, ND == 1 ? 3 : 1)
                  ghist + (size_t)dd * 65536u);
   }
   __syncthreads();
+  if (dump) {
+    uint4* to = reinterpret_cast<uint4*>(dump + (size_t)blockIdx.x * ND * 16384u);
+    for (uint32_t i = threadIdx.x; i < ND * 4096u; i += blockDim.x) to[i] = reinterpret_cast<const uint4*>(cw)[i];
+  } else {
 #pragma unroll
-  for (int dd = 0; dd < ND; dd++) byte_flush(cw + dd * 16384, ghist + (size_t)dd * 65536u);
+    for (int dd = 0; dd < ND; dd++) byte_flush(cw + dd * 16384, ghist + (size_t)dd * 65536u);
+  }
+}
+
+// Adds the counters that the CTAs of k_hist16<nd> stored to the counts of their
+// digits. One thread per word (four bins), blockIdx.y a share of the groups;
+// byte pairs are added up in 16 bits, 255 groups at most at a time.
+constexpr uint32_t kH16Shares = 8;
+__global__ void __launch_bounds__(256)
+    k_hist16_sum(const uint32_t* __restrict__ dump, uint32_t nd, uint32_t group, uint32_t groups,
+                 uint32_t* __restrict__ counts) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;  // digit * 16384 + word
+  const uint32_t digit = i >> 14, word = i & 16383u, role = digit / nd, dd = digit % nd;
+  if (role >= group) return;
+  const uint32_t g0 = (uint32_t)((uint64_t)groups * blockIdx.y / gridDim.y);
+  const uint32_t g1 = (uint32_t)((uint64_t)groups * (blockIdx.y + 1u) / gridDim.y);
+  uint32_t sum[4] = {};
+  for (uint32_t g = g0; g < g1; g += 255u) {
+    uint32_t even = 0, odd = 0;
+    const uint32_t e = min(g1, g + 255u);
+#pragma unroll 8
+    for (uint32_t q = g; q < e; q++) {
+      const uint32_t w = dump[((size_t)(q * group + role) * nd + dd) * 16384u + word];
+      even += w & 0x00FF00FFu;
+      odd += (w >> 8) & 0x00FF00FFu;
+    }
+    sum[0] += even & 0xFFFFu;
+    sum[1] += odd & 0xFFFFu;
+    sum[2] += even >> 16;
+    sum[3] += odd >> 16;
+  }
+#pragma unroll
+  for (int b = 0; b < 4; b++)
+    if (sum[b]) atomicAdd(&counts[(size_t)digit * 65536u + 4u * word + (uint32_t)b], sum[b]);
 }
 
 // Counts of 16-bit digits [first_digit, first_digit + num_digits) into
-// d_counts[num_digits][65536] (uint32; zeroed here). The default reads the
-// keys once per three digits; with four digits, LSB_HIST16 selects one HBM
-// read by groups of CTAs over the same range (L2 serves the group's other
-// reads): "pairs" (two digits per CTA, 128 KiB, one CTA per SM) or "quads"
-// (one digit per CTA, 64 KiB, three CTAs per SM). All give the same counts.
-static int hist16_group() {
+// d_counts[num_digits][65536] (uint32; zeroed here). Four digits: one HBM read
+// by groups of CTAs over the same range (L2 serves the group's other reads),
+// "pairs" of CTAs with two digits each (128 KiB, one CTA per SM) by default;
+// LSB_HIST16 selects "quads" (one digit each, 64 KiB, two CTAs per SM) or
+// "split" (a read per three digits). All give the same counts. Where a CTA
+// counts 2^17 keys or more its counters are stored and summed up by a second
+// kernel (scratch: they may come from the library's pool).
+// 2^26 uniform keys, four digits (GB300): two reads with the flush by atomics
+// 637 us, of which the counting was 32 instructions per digit; this form, 12.
+static uint32_t hist16_group() {
   const char* e = std::getenv("LSB_HIST16");
-  if (e && std::strcmp(e, "pairs") == 0) return 2;
-  if (e && std::strcmp(e, "quads") == 0) return 4;
-  return 0;
+  if (e && std::strcmp(e, "split") == 0) return 1u;
+  if (e && std::strcmp(e, "quads") == 0) return 4u;
+  return 2u;
 }
 
 template <int ND>
-static int hist16_grouped(const Elem* data, uint32_t n, int first_digit, uint32_t* d_counts,
-                          uint32_t group, const DeviceInfo& dev, cudaStream_t st) {
+static int hist16_launch(const Elem* data, uint32_t n, int first_digit, uint32_t* d_counts,
+                         uint32_t group, bool scratch, const DeviceInfo& dev, cudaStream_t st) {
   const size_t smem = (size_t)ND * 65536u;
-  if (cudaFuncSetAttribute(k_hist16<ND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-      cudaSuccess)
-    return 5;
-  int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_hist16<ND>, kH16Threads, smem);
-  per_sm = std::max(per_sm, 1);
+  static std::atomic<uint64_t> allowed;  // of this instance
+  if (!allow_smem((const void*)k_hist16<ND>, smem, &allowed)) return 5;
   // enough groups to fill every resident slot, none with less than a few rounds of work
-  const uint64_t want = ((uint64_t)n + 8u * kH16Threads * kH16Unroll - 1) / (8u * kH16Threads * kH16Unroll);
-  const uint64_t slots = std::max<uint64_t>(1, (uint64_t)dev.sm_count * per_sm / group);
+  const uint64_t least = 4u * kH16Threads * kH16Unroll;
+  const uint64_t want = ((uint64_t)n + least - 1) / least;
+  const uint64_t slots = std::max<uint64_t>(1, (uint64_t)dev.sm_count * (ND == 1 ? 2u : 1u) / group);
   const uint32_t groups = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(want, slots));
-  ProfScope prof("hist16", st);
-  k_hist16<ND><<<group * groups, kH16Threads, smem, st>>>(data, n, first_digit, d_counts, group);
+  void* dump = nullptr;
+  if (scratch && n / groups >= (1u << 17) && pool_alloc(&dump, (size_t)group * groups * smem, st) != 0) dump = nullptr;
+  {
+    ProfScope prof("hist16", st);
+    k_hist16<ND><<<group * groups, kH16Threads, smem, st>>>(data, n, first_digit, d_counts, group,
+                                                            static_cast<uint32_t*>(dump));
+  }
+  if (dump) {
+    ProfScope prof("hist16_sum", st);
+    k_hist16_sum<<<dim3(group * ND * 64u, kH16Shares), 256, 0, st>>>(static_cast<const uint32_t*>(dump), ND, group,
+                                                                     groups, d_counts);
+    cudaFreeAsync(dump, st);
+  }
   return cudaPeekAtLastError() == cudaSuccess ? 0 : 5;
 }
 
 int hist16(const Elem* data, uint32_t n, int first_digit, int num_digits, uint32_t* d_counts,
-           cudaStream_t st) {
+           bool scratch, cudaStream_t st) {
   DeviceInfo dev;
   if (int rc = current_device_info(&dev)) return rc;
   if (cudaMemsetAsync(d_counts, 0, (size_t)num_digits * 65536u * 4u, st) != cudaSuccess) return 5;
   if (n == 0) return 0;
-  const int group = hist16_group();
-  if (num_digits == 4 && group == 2) return hist16_grouped<2>(data, n, first_digit, d_counts, 2u, dev, st);
-  if (num_digits == 4 && group == 4) return hist16_grouped<1>(data, n, first_digit, d_counts, 4u, dev, st);
+  const uint32_t group = hist16_group();
+  if (num_digits == 4 && group == 2u) return hist16_launch<2>(data, n, first_digit, d_counts, 2u, scratch, dev, st);
+  if (num_digits == 4 && group == 4u) return hist16_launch<1>(data, n, first_digit, d_counts, 4u, scratch, dev, st);
   for (int d0 = 0; d0 < num_digits; d0 += 3) {
     const int nd = std::min(3, num_digits - d0);
-    auto kern = nd == 3 ? k_hist16<3> : nd == 2 ? k_hist16<2> : k_hist16<1>;
-    const size_t smem = (size_t)nd * 65536u;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-        cudaSuccess)
-      return 5;
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kH16Threads, smem);
-    per_sm = std::max(per_sm, 1);
-    const uint64_t per_cta = (uint64_t)kH16Threads * kH16Unroll * 8u;
-    const uint64_t want = (n + per_cta - 1) / per_cta;
-    const uint32_t grid = (uint32_t)std::max<uint64_t>(
-        1, std::min<uint64_t>(want, (uint64_t)dev.sm_count * per_sm));
-    ProfScope prof("hist16", st);
-    kern<<<grid, kH16Threads, smem, st>>>(data, n, first_digit + d0,
-                                          d_counts + (size_t)d0 * 65536u, 0u);
-    if (cudaPeekAtLastError() != cudaSuccess) return 5;
+    auto launch = nd == 3 ? hist16_launch<3> : nd == 2 ? hist16_launch<2> : hist16_launch<1>;
+    if (int rc = launch(data, n, first_digit + d0, d_counts + (size_t)d0 * 65536u, 1u, scratch, dev, st)) return rc;
   }
   return 0;
 }
@@ -968,7 +1039,7 @@ int wide_run(Elem* X, Elem* Y, int first_digit, int target_parity, unsigned char
   unsigned char* wbase = ws + L.off_wide;
   DeviceInfo dev;
   if (int rc = current_device_info(&dev)) return rc;
-  if (int rc = hist16(X, L.n, first_digit, L.num_digits, hist, st)) return rc;
+  if (int rc = hist16(X, L.n, first_digit, L.num_digits, hist, false, st)) return rc;
   {
     ProfScope prof("plan", st);
     k_plan16_scan<<<L.num_digits, kPlan16Threads, 0, st>>>(hist, gstart, L.n, ctrl);
