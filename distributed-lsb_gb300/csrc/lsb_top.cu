@@ -100,6 +100,7 @@ static int small_sort(Elem* X, const Layout& L, Ctrl* ctrl, cudaStream_t st) {
 // 0.48 ms, 2^28 15.0 -> 6.4 ms, 2^30 58.6 -> 30.8 ms (three passes), 2^28 Zipf
 // 16.0 -> 9.8 ms (four passes; heavy keys stay in order), against eight passes.
 
+constexpr uint32_t kSmallRun = 1700;  // the same of the small tile, with room for one and a half
 constexpr int kTopSample = 4;  // keys per thread of the sample: 4096
 constexpr int kTopHistThreads = 512;
 constexpr int kTopHistUnroll = 4;
@@ -313,21 +314,26 @@ __global__ void __launch_bounds__(kTopHistThreads, 4)
 // `stride` elements; a CTA takes the runs that start in its part, as many whole
 // runs at a time as fit in a tile: it brings in a tile's worth from where it
 // stands by one bulk copy, and sorts the whole runs in it (sort_runs).
-// 2^30 elements after three passes: 7.4 ms, 4.6 TB/s of the 32 bytes per
-// element, bound by the sort's instructions (about 150 per 32 elements) and
-// shared-memory accesses (45 wavefronts per 32) at 32 resident warps per SM.
-__global__ void __launch_bounds__(Tile::kThreads, 2)
+// 2^30 elements after three passes (runs of 64): 7.7 ms with tiles of 4608 in
+// two CTAs per SM, 7.1 ms (4.8 TB/s of the 32 bytes per element) with 2304 in
+// four, whose phases overlap better; three of 3072 take 7.4, one of 9216 9.2.
+// Bound by the shared-memory pipe (70 % busy: 50 wavefronts and 180
+// instructions per 32 elements) at 32 resident warps per SM. (Digits of 7 bits
+// make a pass 4 % faster and the runs eight times as long, which costs the
+// small tiles as much: 27.7 ms for passes and runs either way.)
+template <class TS, int CTAS>
+__global__ void __launch_bounds__(TS::kThreads, CTAS)
     k_top_finish(Elem* __restrict__ X, Elem* __restrict__ Y, uint32_t n, uint32_t stride,
                  RunChunk* __restrict__ chunks, uint32_t* __restrict__ unsorted, Ctrl* ctrl) {
-  constexpr int THREADS = Tile::kThreads;
+  constexpr int THREADS = TS::kThreads;
   extern __shared__ __align__(128) unsigned char smem[];
-  __shared__ typename Tile::Shared sh;
+  __shared__ typename TS::Shared sh;
   __shared__ __align__(8) uint64_t s_bar;
   __shared__ RunMarks s_marks;
   __shared__ RunKey s_w;
   Elem* in = reinterpret_cast<Elem*>(smem);
-  uint32_t* slot = reinterpret_cast<uint32_t*>(smem + Tile::kElemBytes);
-  uint32_t* bins = reinterpret_cast<uint32_t*>(smem + Tile::kElemBytes + Tile::kSlotBytes);
+  uint32_t* slot = reinterpret_cast<uint32_t*>(smem + TS::kElemBytes);
+  uint32_t* bins = reinterpret_cast<uint32_t*>(smem + TS::kElemBytes + TS::kSlotBytes);
   const TopPlan& plan = ctrl->top;
   const uint32_t par = plan.src_parity;
   const Elem* src = par ? Y : X;
@@ -353,7 +359,7 @@ __global__ void __launch_bounds__(Tile::kThreads, 2)
   for (uint32_t part = blockIdx.x; part < parts; part += gridDim.x) {
     const uint32_t g = (uint32_t)((uint64_t)part * stride);
     const uint32_t limit = (uint32_t)min((uint64_t)g + stride, (uint64_t)n);
-    if (!sort_runs<Tile>(src, X, n, g, limit, part == 0, s_w, clamped, skewed, shift, in, slot, bins, sh, s_marks, load,
+    if (!sort_runs<TS>(src, X, n, g, limit, part == 0, s_w, clamped, skewed, shift, in, slot, bins, sh, s_marks, load,
                          long_run))
       return;
   }
@@ -515,14 +521,23 @@ int top_run(Elem* X, Elem* Y, unsigned char* ws, const Layout& L, cudaStream_t s
   uint32_t* hist = reinterpret_cast<uint32_t*>(ws + L.off_hist);
   uint32_t* gstart = reinterpret_cast<uint32_t*>(ws + L.off_gstart);
   uint64_t* ring = reinterpret_cast<uint64_t*>(ws + L.off_ring);
-  SampleRule rule = sample_rule(n, SampleTile<kTopSample>::kCap, kMeanRun, kMeanRun, 16.0f);
+  // Even runs up to kSmallRun leave the small tile half full or better, and six
+  // standard deviations of room
+  const uint32_t least = passes_for((float)n, (float)kMeanRun);
+  const double even_run = (double)n / std::pow(256.0, (double)least);
+  const bool small_tile = even_run <= (double)kSmallRun;
+  SampleRule rule = sample_rule(n, SampleTile<kTopSample>::kCap, small_tile ? kSmallRun : kMeanRun, kMeanRun, 16.0f);
   // Unused launches cost about 2 us each: below 2^26 elements only two passes
   // more than even keys need are kept ready, and the merges, whose rounds then
   // stay nearly in L2, take what those leave.
   if (n < (1u << 26)) rule.tmax = std::min(8u, rule.tmin + 2u);
-  static std::atomic<uint64_t> allowed[2];
+  static std::atomic<uint64_t> allowed[3];
+  const auto finish = small_tile ? k_top_finish<SmallTile, 4> : k_top_finish<Tile, 2>;
+  const uint32_t cap = small_tile ? SmallTile::kCap : Tile::kCap;
+  const int threads = small_tile ? SmallTile::kThreads : Tile::kThreads;
+  const size_t smem = small_tile ? SmallTile::kSmem : Tile::kSmem;
   if (!allow_smem((const void*)k_top_sample, kSampleSmem<kTopSample>, &allowed[0]) ||
-      !allow_smem((const void*)k_top_finish, Tile::kSmem, &allowed[1]))
+      !allow_smem((const void*)finish, smem, &allowed[small_tile ? 1 : 2]))
     return 5;
   {
     ProfScope prof("top_sample", st);
@@ -546,15 +561,16 @@ int top_run(Elem* X, Elem* Y, unsigned char* ws, const Layout& L, cudaStream_t s
     // A tile is left a run short on average (its last run is not whole), so a
     // part of `per` tiles is as long as its runs fill `per` tiles, or, with runs
     // that fill a tile by themselves, as `per` runs. Parts of 1 to 16 tiles:
-    // enough of them for six rounds of two CTAs per SM, and else few, since the
-    // run across a part's start is read twice.
-    const uint32_t run = (uint32_t)((double)n / std::pow(256.0, (double)rule.tmin));
-    const uint32_t fill = std::max(run, kCap - std::min(kCap, run + run / 2u));
-    const uint32_t per = std::max<uint32_t>(1u, std::min<uint32_t>(16u, n / fill / ((uint32_t)dev.sm_count * 12u)));
+    // enough of them for six rounds of every resident CTA, and else few, since
+    // the run across a part's start is read twice.
+    const uint32_t run = (uint32_t)even_run;
+    const uint32_t fill = std::max(run, cap - std::min(cap, run + run / 2u));
+    const uint32_t resident = (uint32_t)dev.sm_count * (small_tile ? 4u : 2u);
+    const uint32_t per = std::max<uint32_t>(1u, std::min<uint32_t>(16u, n / fill / (resident * 6u)));
     const uint32_t stride = per * fill;
     const uint32_t grid = (uint32_t)(((uint64_t)n + stride - 1u) / stride);
     ProfScope prof("top_finish", st);
-    k_top_finish<<<grid, Tile::kThreads, Tile::kSmem, st>>>(X, Y, n, stride, chunks, unsorted, ctrl);
+    finish<<<grid, threads, smem, st>>>(X, Y, n, stride, chunks, unsorted, ctrl);
   }
   if (cudaPeekAtLastError() != cudaSuccess) return 5;
   return top_merge(X, Y, n, chunks, unsorted, ctrl, dev, st);

@@ -355,16 +355,18 @@ __device__ __forceinline__ bool sort_runs(const Elem* src, Elem* X, uint32_t n, 
 
 using Tile = TileSort<512, 9>;  // 106 KB: two CTAs per SM, one's loads and stores beside the other's sort
 constexpr uint32_t kCap = Tile::kCap;
+using SmallTile = TileSort<256, 9>;  // 54 KB: four CTAs per SM
 // Mean run length up to which a pass is saved: six standard deviations below a tile.
 constexpr uint32_t kMeanRun = 4220;
 // A chunk of a run too long for a tile: elements [b + k kCap, ...) of the run [b, e).
 struct RunChunk {
   uint32_t b, e, k, run : 31, par : 1;  // par: the run lies in Y
 };
-__host__ __device__ __forceinline__ uint32_t max_chunks(uint32_t n) { return 2u * (n / kCap) + 2u; }
+__host__ __device__ __forceinline__ uint32_t max_chunks(uint32_t n) { return 3u * (n / kCap) + 2u; }
 
 // One warp: the run [b, e) goes to the merge kernel's list (in the ring, which
-// the passes are done with): at most n / kCap runs of at least kCap elements.
+// the passes are done with): runs of at least kCap / 2 elements, so at most
+// 2 n / kCap of them.
 __device__ __forceinline__ void push_run(Ctrl* ctrl, RunChunk* chunks, uint32_t* unsorted, uint32_t n, uint32_t b,
                                          uint32_t e, uint32_t par) {
   const uint32_t lane = lane_id();
