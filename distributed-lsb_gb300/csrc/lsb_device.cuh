@@ -43,6 +43,7 @@ constexpr uint32_t kSpinLimit = 1u << 22;
 struct TopPlan {
   uint64_t lo, hi;
   uint32_t hb1;            // 64: the block is the whole key range
+  uint32_t clamp;          // some key may lie outside the block (after the histogram: one does)
   uint32_t passes;
   uint32_t run_mask;       // bit p: pass p runs (its digit is not constant)
   uint32_t par_mask;       // bit p: pass p reads Y, writes X
@@ -103,7 +104,7 @@ __device__ __forceinline__ TopWindow top_window(const Plan& p, int pass) {
   TopWindow w;
   w.lo = p.lo;
   w.hi = p.hi;
-  w.clamp = p.hb1 < 64u;
+  w.clamp = p.clamp != 0u;
   const int s = (int)p.hb1 - 8 * ((int)p.passes - pass);
   w.right = s > 0 ? (uint32_t)s : 0u;
   w.left = s < 0 ? (uint32_t)-s : 0u;
@@ -121,9 +122,9 @@ __device__ __forceinline__ uint32_t top_digit_clamped(const TopWindow& w, uint64
 // 0: the array fits in a tile.
 struct SegPlan {
   uint64_t lo, hi;
-  uint32_t hb1, passes, skewed, complete;
+  uint32_t hb1, clamp, passes, skewed, complete;
   uint32_t diff[2];
-  uint32_t pad[2];
+  uint32_t pad;
 };
 
 // A batch of independent arrays sorted together (null tile_seg: one array).

@@ -62,6 +62,7 @@ __global__ void __launch_bounds__(kSampleThreads, 2)
       p.passes = sample_passes<kSegSample>(k, p.hb1, rule, s_near, s_far, &skewed);
       p.skewed = skewed ? 1u : 0u;
       if (p.hb1 < 64u) {
+        p.clamp = 1u;
         p.lo = first >> p.hb1 << p.hb1;
         p.hi = p.lo | ((1ull << p.hb1) - 1ull);
       }
@@ -246,6 +247,7 @@ __global__ void __launch_bounds__(256)
       SegPlan& p = plans[sg];
       const uint64_t d = (uint64_t)p.diff[1] << 32 | p.diff[0];
       const bool inside = p.hb1 >= 64u || ((d | (data[seg_off[sg]].key ^ p.lo)) >> p.hb1) == 0;
+      p.clamp = inside ? 0u : 1u;
       p.complete = (d == 0 || (p.hb1 <= 8u * passes && inside)) ? 1u : 0u;
     }
   }
@@ -311,7 +313,7 @@ __global__ void __launch_bounds__(Tile::kThreads, 2)
     __syncthreads();
     if (threadIdx.x == 0) s_w = run_key(plan);
     auto long_run = [&](uint32_t b, uint32_t e) { push_run(ctrl, chunks, unsorted, n, at + b, at + e, par); };
-    if (!sort_runs<Tile>(src, dst, len, g, limit, g == 0, s_w, plan.hb1 < 64u, plan.skewed != 0u, run_key(plan).shift,
+    if (!sort_runs<Tile>(src, dst, len, g, limit, g == 0, s_w, plan.clamp != 0u, plan.skewed != 0u, run_key(plan).shift,
                          in, slot, bins, sh, s_marks, load, long_run))
       return;
   }

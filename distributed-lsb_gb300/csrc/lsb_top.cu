@@ -127,6 +127,7 @@ __global__ void __launch_bounds__(kSampleThreads, 1)
     p.passes = t;
     p.skewed = skewed ? 1u : 0u;
     p.hb1 = hb1;
+    p.clamp = hb1 < 64u ? 1u : 0u;
     p.lo = hb1 < 64u ? first >> hb1 << hb1 : 0ull;
     p.hi = hb1 < 64u ? p.lo | ((1ull << hb1) - 1ull) : ~0ull;
   }
@@ -301,7 +302,9 @@ __global__ void __launch_bounds__(kTopHistThreads, 4)
     q.run_mask = run;
     q.par_mask = pars;
     q.src_parity = par;
+    // keys in the block, as usual: no pass need look
     const bool inside = q.hb1 >= 64u || ((d | (first ^ q.lo)) >> q.hb1) == 0;
+    q.clamp = inside ? 0u : 1u;
     q.complete = (d == 0 || (q.hb1 <= 8u * T && inside)) ? 1u : 0u;
     write_plan(ctrl, d, n, bits, num_digits, api_bits, sub);
   }
@@ -350,7 +353,7 @@ __global__ void __launch_bounds__(TS::kThreads, CTAS)
     mbar_init(bar, 1);
     fence_mbar_init();
   }
-  const bool clamped = plan.hb1 < 64u, skewed = plan.skewed != 0u;
+  const bool clamped = plan.clamp != 0u, skewed = plan.skewed != 0u;
   const uint32_t shift = run_key(plan).shift;
   const uint32_t parts = (uint32_t)(((uint64_t)n + stride - 1u) / stride);
   uint32_t phase = 0;
@@ -526,7 +529,8 @@ int top_run(Elem* X, Elem* Y, unsigned char* ws, const Layout& L, cudaStream_t s
   const uint32_t least = passes_for((float)n, (float)kMeanRun);
   const double even_run = (double)n / std::pow(256.0, (double)least);
   const bool small_tile = even_run <= (double)kSmallRun;
-  SampleRule rule = sample_rule(n, SampleTile<kTopSample>::kCap, small_tile ? kSmallRun : kMeanRun, kMeanRun, 16.0f);
+  SampleRule rule = sample_rule(n, SampleTile<kTopSample>::kCap, small_tile ? kSmallRun : kMeanRun, kMeanRun,
+                                n <= (1u << 28) ? 16.0f : 4.0f);  // four passes for heavy keys up to 2^30 elements
   // Unused launches cost about 2 us each: below 2^26 elements only two passes
   // more than even keys need are kept ready, and the merges, whose rounds then
   // stay nearly in L2, take what those leave.

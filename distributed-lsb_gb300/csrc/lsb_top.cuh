@@ -177,8 +177,8 @@ __device__ __forceinline__ uint64_t run_of(const RunKey& w, uint64_t key) {
 template <class Plan>
 __device__ __forceinline__ RunKey run_key(const Plan& p) {
   RunKey w;
-  w.lo = p.lo;
-  w.hi = p.hi;
+  w.lo = p.clamp ? p.lo : 0ull;
+  w.hi = p.clamp ? p.hi : ~0ull;
   w.shift = p.hb1 > 8u * p.passes ? p.hb1 - 8u * p.passes : 0u;
   return w;
 }
