@@ -101,27 +101,29 @@ static int small_sort(Elem* X, const Layout& L, Ctrl* ctrl, cudaStream_t st) {
 // 16.0 -> 9.8 ms (four passes; heavy keys stay in order), against eight passes.
 
 constexpr uint32_t kSmallRun = 1700;  // the same of the small tile, with room for one and a half
+constexpr uint32_t kBigRun = 8640;    // and of the big one
 constexpr int kTopSample = 4;  // keys per thread of the sample: 4096
 constexpr int kTopHistThreads = 512;
 constexpr int kTopHistUnroll = 4;
 
 // Bound by latency (one CTA: 4096 scattered reads, a tile sort, two counts);
 // it also clears what the later kernels count in, in place of three memsets.
+template <int S>
 __global__ void __launch_bounds__(kSampleThreads, 1)
     k_top_sample(const Elem* __restrict__ data, uint32_t n, SampleRule rule, uint32_t* __restrict__ hist, Ctrl* ctrl) {
   extern __shared__ __align__(128) unsigned char smem[];
-  __shared__ typename SampleTile<kTopSample>::Shared sh;
+  __shared__ typename SampleTile<S>::Shared sh;
   __shared__ uint32_t s_near[8], s_far[9];
   const uint32_t tid = threadIdx.x;
   for (uint32_t i = tid; i < kCtrlBytes / 4u; i += kSampleThreads) reinterpret_cast<uint32_t*>(ctrl)[i] = 0u;
   for (uint32_t i = tid; i < 8u * 256u; i += kSampleThreads) hist[i] = 0u;
   if (tid < 8) s_near[tid] = 0u;
   if (tid < 9) s_far[tid] = 0u;
-  const uint64_t* s = sample_keys<kTopSample>(data, n, smem, sh);
-  const uint64_t first = s[0], span = first ^ s[SampleTile<kTopSample>::kCap - 1u];
+  const uint64_t* s = sample_keys<S>(data, n, smem, sh);
+  const uint64_t first = s[0], span = first ^ s[SampleTile<S>::kCap - 1u];
   const uint32_t hb1 = span ? 64u - (uint32_t)__clzll((long long)span) : 64u;
   bool skewed;
-  const uint32_t t = sample_passes<kTopSample>(s, hb1, rule, s_near, s_far, &skewed);
+  const uint32_t t = sample_passes<S>(s, hb1, rule, s_near, s_far, &skewed);
   if (tid == 0) {
     TopPlan& p = ctrl->top;
     p.passes = t;
@@ -524,28 +526,42 @@ int top_run(Elem* X, Elem* Y, unsigned char* ws, const Layout& L, cudaStream_t s
   uint32_t* hist = reinterpret_cast<uint32_t*>(ws + L.off_hist);
   uint32_t* gstart = reinterpret_cast<uint32_t*>(ws + L.off_gstart);
   uint64_t* ring = reinterpret_cast<uint64_t*>(ws + L.off_ring);
-  // Even runs up to kSmallRun leave the small tile half full or better, and six
-  // standard deviations of room
+  // The tile of the last step. The big one is slower (one CTA per SM) but holds
+  // runs twice as long: it is taken where one pass is then enough (1.5M elements
+  // 89 against 104 us). Above 2^28 elements it would save the third pass (2^29:
+  // 13.6 against 15.5 ms), but costs more than that when keys occur some thirty
+  // times (33.7 against 28.8 ms), which a sample does not show. Else even runs up
+  // to kSmallRun leave the small one half full or better, with six standard
+  // deviations of room.
   const uint32_t least = passes_for((float)n, (float)kMeanRun);
-  const double even_run = (double)n / std::pow(256.0, (double)least);
+  const bool big = least == 2u && n <= 256u * kBigRun;
+  const double even_run = (double)n / std::pow(256.0, (double)(big ? 1u : least));
   const bool small_tile = even_run <= (double)kSmallRun;
-  SampleRule rule = sample_rule(n, SampleTile<kTopSample>::kCap, small_tile ? kSmallRun : kMeanRun, kMeanRun,
+  // a smaller sample decides as well for fewer elements, and 5 us sooner
+  const bool short_sample = n < (1u << 26);
+  const uint32_t mean_run = big ? kBigRun : small_tile ? kSmallRun : kMeanRun;
+  SampleRule rule = sample_rule(n, short_sample ? SampleTile<1>::kCap : SampleTile<kTopSample>::kCap, mean_run, mean_run,
                                 n <= (1u << 28) ? 16.0f : 4.0f);  // four passes for heavy keys up to 2^30 elements
-  // Unused launches cost about 2 us each: below 2^26 elements only two passes
-  // more than even keys need are kept ready, and the merges, whose rounds then
-  // stay nearly in L2, take what those leave.
-  if (n < (1u << 26)) rule.tmax = std::min(8u, rule.tmin + 2u);
-  static std::atomic<uint64_t> allowed[3];
-  const auto finish = small_tile ? k_top_finish<SmallTile, 4> : k_top_finish<Tile, 2>;
-  const uint32_t cap = small_tile ? SmallTile::kCap : Tile::kCap;
-  const int threads = small_tile ? SmallTile::kThreads : Tile::kThreads;
-  const size_t smem = small_tile ? SmallTile::kSmem : Tile::kSmem;
-  if (!allow_smem((const void*)k_top_sample, kSampleSmem<kTopSample>, &allowed[0]) ||
-      !allow_smem((const void*)finish, smem, &allowed[small_tile ? 1 : 2]))
+  // Unused launches cost about 2 us each: below 2^26 elements only the four
+  // passes of heavy keys, or two more than even keys need, are kept ready, and
+  // the merges, whose rounds then stay nearly in L2, take what those leave.
+  if (n < (1u << 26)) rule.tmax = std::max(4u, std::min(8u, rule.tmin + 2u));
+  static std::atomic<uint64_t> allowed[5];
+  const auto finish = big          ? k_top_finish<BigTile, 1>
+                      : small_tile ? k_top_finish<SmallTile, 4>
+                                   : k_top_finish<Tile, 2>;
+  const uint32_t cap = big ? BigTile::kCap : small_tile ? SmallTile::kCap : Tile::kCap;
+  const int threads = big ? BigTile::kThreads : small_tile ? SmallTile::kThreads : Tile::kThreads;
+  const size_t smem = big ? BigTile::kSmem : small_tile ? SmallTile::kSmem : Tile::kSmem;
+  const uint32_t ctas = big ? 1u : small_tile ? 4u : 2u;
+  const auto sample = short_sample ? k_top_sample<1> : k_top_sample<kTopSample>;
+  const size_t sample_smem = short_sample ? kSampleSmem<1> : kSampleSmem<kTopSample>;
+  if (!allow_smem((const void*)sample, sample_smem, &allowed[short_sample ? 3 : 4]) ||
+      !allow_smem((const void*)finish, smem, &allowed[big ? 2 : small_tile ? 1 : 0]))
     return 5;
   {
     ProfScope prof("top_sample", st);
-    k_top_sample<<<1, kSampleThreads, kSampleSmem<kTopSample>, st>>>(X, n, rule, hist, ctrl);
+    sample<<<1, kSampleThreads, sample_smem, st>>>(X, n, rule, hist, ctrl);
   }
   {
     // four CTAs per SM, fewer when they would have under four rounds of reads each
@@ -569,7 +585,7 @@ int top_run(Elem* X, Elem* Y, unsigned char* ws, const Layout& L, cudaStream_t s
     // the run across a part's start is read twice.
     const uint32_t run = (uint32_t)even_run;
     const uint32_t fill = std::max(run, cap - std::min(cap, run + run / 2u));
-    const uint32_t resident = (uint32_t)dev.sm_count * (small_tile ? 4u : 2u);
+    const uint32_t resident = (uint32_t)dev.sm_count * ctas;
     const uint32_t per = std::max<uint32_t>(1u, std::min<uint32_t>(16u, n / fill / (resident * 6u)));
     const uint32_t stride = per * fill;
     const uint32_t grid = (uint32_t)(((uint64_t)n + stride - 1u) / stride);

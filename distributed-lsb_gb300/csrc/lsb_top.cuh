@@ -356,6 +356,7 @@ __device__ __forceinline__ bool sort_runs(const Elem* src, Elem* X, uint32_t n, 
 using Tile = TileSort<512, 9>;  // 106 KB: two CTAs per SM, one's loads and stores beside the other's sort
 constexpr uint32_t kCap = Tile::kCap;
 using SmallTile = TileSort<256, 9>;  // 54 KB: four CTAs per SM
+using BigTile = TileSort<1024, 9>;   // 212 KB: one CTA per SM
 // Mean run length up to which a pass is saved: six standard deviations below a tile.
 constexpr uint32_t kMeanRun = 4220;
 // A chunk of a run too long for a tile: elements [b + k kCap, ...) of the run [b, e).
