@@ -15,11 +15,14 @@
 // by 8-bit digits (ballots and per-warp counters) costs one round per digit.
 // Evenly spread keys put 0.56 elements in a bin at most on average. When a bin
 // has more than kMaxBin elements, the bins are laid over the range from the
-// smallest to the largest key instead. What is heavy then are mostly
-// duplicates: a warp takes such a bin key by key, and a bitmap of the key's
-// positions gives the ranks (heavy_bins). A tile with many different keys in a
-// bin even so (clusters) is sorted by the bits in which its keys differ, eight
-// at a time from the lowest (stable ranks by ballots and per-warp counters).
+// smallest to the largest key instead. What shares a bin then are mostly
+// duplicates: bins of up to kSlotsBin elements are ranked by slots alone, which
+// is checked before any element goes out (2^28 elements, every key thirty times:
+// 12.1 ms; 14.7 ms when every pair's whole keys are compared); a warp takes a
+// larger one key by key, and a bitmap of the key's positions gives the ranks
+// (heavy_bins). A tile with many different keys in a large bin (clusters) is
+// sorted by the bits in which its keys differ, eight at a time from the lowest
+// (stable ranks by ballots and per-warp counters).
 // 10^4 Zipf keys: 52 us bit by bit.
 #pragma once
 
@@ -59,11 +62,11 @@ struct TileSort {
   // bits of a position in a slot
   static constexpr uint32_t kPosBits = kCap <= 1024 ? 10 : kCap <= 2048 ? 11 : kCap <= 4096 ? 12 : kCap <= 8192 ? 13 : 14;
   static constexpr uint32_t kPosMask = (1u << kPosBits) - 1u;
-  static constexpr uint32_t kMaxBin = 24;
-  static constexpr uint32_t kMaxHeavy = kCap / (kMaxBin + 1u);  // bins above it
+  static constexpr uint32_t kMaxBin = 24;    // elements of a bin compared by whole keys
+  static constexpr uint32_t kSlotsBin = 64;  // and, in a tile with bins above that, by slots
+  static constexpr uint32_t kMaxHeavy = kCap / (kSlotsBin + 1u);  // bins above it
   static constexpr uint32_t kFewRounds = 4;  // of eight bits: no dearer than another try with bins
   static constexpr uint32_t kFewKeys = 12;   // of 32 in a heavy bin: taken key by key
-  static constexpr uint32_t kManyKeys = 64;  // largest heavy bin of many keys compared pair by pair
   static_assert(kCap <= (1u << kPosBits) && K <= 16 && kWarps <= 32, "position bits, network, warp totals");
 
   // shared memory: elements, slots (or two position lists), bin counts (16 bits each)
@@ -238,12 +241,12 @@ struct TileSort {
       const uint32_t both = off | off << 16;
       q[0] = make_uint4(w8[0] + both, w8[1] + both, w8[2] + both, w8[3] + both);
       q[1] = make_uint4(w8[4] + both, w8[5] + both, w8[6] + both, w8[7] + both);
-      if (HEAVY && maxc > kMaxBin) {
+      if (HEAVY && maxc > kSlotsBin) {
 #pragma unroll
         for (int i = 0; i < 16; i++) {
           const uint32_t s0 = (w8[i >> 1] >> (16 * (i & 1))) & 0xffffu;
           const uint32_t s1 = i < 15 ? (w8[(i + 1) >> 1] >> (16 * ((i + 1) & 1))) & 0xffffu : sum;
-          if (s1 - s0 > kMaxBin) sh.heavy[atomicAdd(&sh.heavy_n, 1u)] = (off + s0) << 16 | (s1 - s0);
+          if (s1 - s0 > kSlotsBin) sh.heavy[atomicAdd(&sh.heavy_n, 1u)] = (off + s0) << 16 | (s1 - s0);
         }
       }
     }
@@ -260,7 +263,7 @@ struct TileSort {
       bool lost = false;
       for (uint32_t h = warp; h < count; h += kWarps) {
         const uint32_t c = sh.heavy[h] & 0xffffu;
-        lost |= c > kManyKeys && probe_keys(in, slot, sh.heavy[h] >> 16, c) > kFewKeys;
+        lost |= probe_keys(in, slot, sh.heavy[h] >> 16, c) > kFewKeys;
       }
       if (__syncthreads_or(lost)) return false;
     }
@@ -268,14 +271,32 @@ struct TileSort {
     // their loads in flight together; the first four slots of the bin without
     // a branch (slots past the tile's last are read but not counted)
     constexpr int R = K % 3 == 0 ? 3 : K % 2 == 0 ? 2 : 1;
-#pragma unroll 1
-    for (uint32_t row = tid; row - tid < m; row += R * THREADS) {
-      uint32_t v[R], r[R];
-      Elem e[R];
+    // the rank of (v, key) among the slots q[0, cnt): whole keys where key bits agree, then positions
+    auto exact = [&](const uint32_t* q, uint32_t cnt, uint32_t v, uint64_t key) {
+      uint32_t r = 0;
+      for (uint32_t j = 0; j < cnt; j += 4u) {
+        uint32_t u[4];
+        uint64_t ku[4];
+#pragma unroll
+        for (uint32_t x = 0; x < 4u; x++) u[x] = q[min(j + x, cnt - 1u)];
+#pragma unroll
+        for (uint32_t x = 0; x < 4u; x++) ku[x] = in[u[x] & kPosMask].key;
+#pragma unroll
+        for (uint32_t x = 0; x < 4u; x++) {
+          const bool tie = (u[x] ^ v) <= kPosMask && ku[x] != key;
+          r += j + x < cnt && (tie ? ku[x] < key : u[x] < v) ? 1u : 0u;
+        }
+      }
+      return r;
+    };
+    bool lost = false;
+    auto load_rows = [&](uint32_t row, uint32_t (&v)[R], Elem (&e)[R]) {
 #pragma unroll
       for (int i = 0; i < R; i++) v[i] = slot[min(row + (uint32_t)i * THREADS, m - 1u)];
 #pragma unroll
       for (int i = 0; i < R; i++) e[i] = in[v[i] & kPosMask];
+    };
+    auto rank_rows = [&](const uint32_t (&v)[R], const Elem (&e)[R], uint32_t* r) {
 #pragma unroll
       for (int i = 0; i < R; i++) {
         uint32_t f;
@@ -292,36 +313,70 @@ struct TileSort {
             close |= ((u ^ v[i]) - 1u) < kPosMask;
           }
         }
-        if (HEAVY && cnt > kMaxBin) {
+        if (HEAVY && cnt > kSlotsBin) {
           r[i] = kCap;  // heavy_bins emits it
-        } else if (close && (cnt > 4u || !whole)) {  // more slots, or key bits that agree: whole keys, then positions
-          r[i] = s;
-          for (uint32_t j = 0; j < cnt; j += 4u) {
+        } else if (HEAVY && cnt > 4u) {
+          // slots alone: right when all that agree in the key bits hold the same
+          // key, and so when each holds the key of the lowest of them
+          uint32_t low = v[i];
+          for (uint32_t j = 4u; j < cnt; j += 4u) {
             uint32_t u[4];
-            uint64_t ku[4];
 #pragma unroll
             for (uint32_t x = 0; x < 4u; x++) u[x] = q[min(j + x, cnt - 1u)];
 #pragma unroll
-            for (uint32_t x = 0; x < 4u; x++) ku[x] = in[u[x] & kPosMask].key;
+            for (uint32_t x = 0; x < 4u; x++) r[i] += j + x < cnt && u[x] < v[i] ? 1u : 0u;
 #pragma unroll
-            for (uint32_t x = 0; x < 4u; x++) {
-              const bool tie = (u[x] ^ v[i]) <= kPosMask && ku[x] != e[i].key;
-              r[i] += j + x < cnt && (tie ? ku[x] < e[i].key : u[x] < v[i]) ? 1u : 0u;
-            }
+            for (uint32_t x = 0; x < 4u; x++) low = min(low, u[x] >= (v[i] & ~kPosMask) ? u[x] : low);
           }
+#pragma unroll
+          for (uint32_t x = 0; x < 4u; x++) low = min(low, q[x] >= (v[i] & ~kPosMask) ? q[x] : low);
+          lost |= !whole && in[low & kPosMask].key != e[i].key;
+        } else if (close && (cnt > 4u || !whole)) {  // more slots, or key bits that agree
+          r[i] = s + exact(q, cnt, v[i], e[i].key);
         }
       }
+    };
+    uint32_t v[R], r[K];
+    Elem e[R];
+    if (!HEAVY) {
+#pragma unroll 1
+      for (uint32_t row = tid; row - tid < m; row += R * THREADS) {
+        load_rows(row, v, e);
+        rank_rows(v, e, r);
 #pragma unroll
-      for (int i = 0; i < R; i++) emit(row + (uint32_t)i * THREADS < m && (!HEAVY || r[i] < kCap), r[i], e[i]);
+        for (int i = 0; i < R; i++) emit(row + (uint32_t)i * THREADS < m, r[i], e[i]);
+      }
+      return true;
     }
-    return !HEAVY || sh.heavy_n == 0u || heavy_bins(in, slot, bins, sh, emit);
+    // All ranks before the first element goes out, since some may be wrong: then
+    // bins of five and more are ranked again, by whole keys.
+#pragma unroll
+    for (int k = 0; k < K; k += R) {
+      load_rows(tid + (uint32_t)k * THREADS, v, e);
+      rank_rows(v, e, r + k);
+    }
+    lost = __syncthreads_or(lost);
+#pragma unroll
+    for (int k = 0; k < K; k += R) {
+      load_rows(tid + (uint32_t)k * THREADS, v, e);
+#pragma unroll
+      for (int i = 0; i < R; i++) {
+        if (lost && r[k + i] < kCap) {
+          uint32_t f;
+          const uint32_t b = bin_of(sc, e[i].key, &f);
+          const uint32_t s = start[b], cnt = start[b + 1u] - s;
+          if (cnt > 4u) r[k + i] = s + exact(slot + s, cnt, v[i], e[i].key);
+        }
+        emit(tid + (uint32_t)(k + i) * THREADS < m && r[k + i] < kCap, r[k + i], e[i]);
+      }
+    }
+    return sh.heavy_n == 0u || heavy_bins(in, slot, bins, sh, emit);
   }
 
   // The heavy bins' elements, one warp per bin and the whole CTA for the largest:
   // for each key of the bin from the smallest, a bitmap of its elements'
   // positions in the tile, whose prefix counts are the ranks. A bin of many
-  // different keys is ranked pair by pair, or, above kManyKeys elements, left
-  // (false).
+  // different keys is left (false).
   static constexpr uint32_t kWords = (kCap + 31u) / 32u, kPerLane = (kWords + 31u) / 32u;
   static constexpr uint32_t kMapWords = kWords + kWords / 2u + 1u;  // the bitmap and 16-bit prefix counts
   static constexpr uint32_t kFit = (uint32_t)(kBinBytes / 4u) / kMapWords;
@@ -442,19 +497,6 @@ struct TileSort {
           last = mn;
           __syncwarp();
         }
-      } else if (c <= kManyKeys) {
-        for (uint32_t j = lane; j < c; j += 32u) {
-          const uint32_t p = slot[s + j] & kPosMask;
-          const Elem e = in[p];
-          uint32_t r = s;
-          for (uint32_t q = 0; q < c; q++) {
-            const uint32_t o = slot[s + q] & kPosMask;
-            const uint64_t ko = in[o].key;
-            r += (ko < e.key || (ko == e.key && o < p)) ? 1u : 0u;
-          }
-          emit(true, r, e);
-        }
-        done = c;
       }
       ok = ok && done >= c;
     }

@@ -34,6 +34,8 @@ def key_sets(n, seed):
     yield "extremes", np.where(r.random(n) < 0.5, np.uint64(0), np.uint64(2**64 - 1))
     yield "low_bits", (full & np.uint64(0xFFF)) | np.uint64(0xABCDEF << 40)
     # neighbours in the last bits of a wide range: the slots' key bits tie
+    c = full[r.integers(0, max(1, n // 30), n)]
+    yield "close_dups", c ^ r.integers(0, 2, n).astype(np.uint64)
     yield "close", np.repeat(full[: n // 2 + 1], 2)[:n] ^ r.integers(0, 2, n).astype(np.uint64)
 
 
