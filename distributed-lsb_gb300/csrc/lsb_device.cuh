@@ -43,6 +43,7 @@ constexpr uint32_t kSpinLimit = 1u << 22;
 struct TopPlan {
   uint64_t lo, hi;
   uint32_t hb1;            // 64: the block is the whole key range
+  uint32_t big;            // runs for the last step with the big tile
   uint32_t clamp;          // some key may lie outside the block (after the histogram: one does)
   uint32_t passes;
   uint32_t run_mask;       // bit p: pass p runs (its digit is not constant)

@@ -113,21 +113,22 @@ __global__ void __launch_bounds__(kSampleThreads, 1)
     k_top_sample(const Elem* __restrict__ data, uint32_t n, SampleRule rule, uint32_t* __restrict__ hist, Ctrl* ctrl) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ typename SampleTile<S>::Shared sh;
-  __shared__ uint32_t s_near[8], s_far[9];
+  __shared__ uint32_t s_near[8], s_far[11];
   const uint32_t tid = threadIdx.x;
   for (uint32_t i = tid; i < kCtrlBytes / 4u; i += kSampleThreads) reinterpret_cast<uint32_t*>(ctrl)[i] = 0u;
   for (uint32_t i = tid; i < 8u * 256u; i += kSampleThreads) hist[i] = 0u;
   if (tid < 8) s_near[tid] = 0u;
-  if (tid < 9) s_far[tid] = 0u;
+  if (tid < 11) s_far[tid] = 0u;
   const uint64_t* s = sample_keys<S>(data, n, smem, sh);
   const uint64_t first = s[0], span = first ^ s[SampleTile<S>::kCap - 1u];
   const uint32_t hb1 = span ? 64u - (uint32_t)__clzll((long long)span) : 64u;
-  bool skewed;
-  const uint32_t t = sample_passes<S>(s, hb1, rule, s_near, s_far, &skewed);
+  bool skewed, big;
+  const uint32_t t = sample_passes<S>(s, hb1, rule, s_near, s_far, &skewed, &big);
   if (tid == 0) {
     TopPlan& p = ctrl->top;
     p.passes = t;
     p.skewed = skewed ? 1u : 0u;
+    p.big = big ? 1u : 0u;
     p.hb1 = hb1;
     p.clamp = hb1 < 64u ? 1u : 0u;
     p.lo = hb1 < 64u ? first >> hb1 << hb1 : 0ull;
@@ -329,7 +330,7 @@ __global__ void __launch_bounds__(kTopHistThreads, 4)
 template <class TS, int CTAS>
 __global__ void __launch_bounds__(TS::kThreads, CTAS)
     k_top_finish(Elem* __restrict__ X, Elem* __restrict__ Y, uint32_t n, uint32_t stride,
-                 RunChunk* __restrict__ chunks, uint32_t* __restrict__ unsorted, Ctrl* ctrl) {
+                 RunChunk* __restrict__ chunks, uint32_t* __restrict__ unsorted, uint32_t big, Ctrl* ctrl) {
   constexpr int THREADS = TS::kThreads;
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ typename TS::Shared sh;
@@ -340,6 +341,7 @@ __global__ void __launch_bounds__(TS::kThreads, CTAS)
   uint32_t* slot = reinterpret_cast<uint32_t*>(smem + TS::kElemBytes);
   uint32_t* bins = reinterpret_cast<uint32_t*>(smem + TS::kElemBytes + TS::kSlotBytes);
   const TopPlan& plan = ctrl->top;
+  if (plan.big != big) return;
   const uint32_t par = plan.src_parity;
   const Elem* src = par ? Y : X;
   if (plan.complete) {  // in order: at most to be copied
@@ -527,38 +529,35 @@ int top_run(Elem* X, Elem* Y, unsigned char* ws, const Layout& L, cudaStream_t s
   uint32_t* gstart = reinterpret_cast<uint32_t*>(ws + L.off_gstart);
   uint64_t* ring = reinterpret_cast<uint64_t*>(ws + L.off_ring);
   // The tile of the last step. The big one is slower (one CTA per SM) but holds
-  // runs twice as long: it is taken where one pass is then enough (1.5M elements
-  // 89 against 104 us). Above 2^28 elements it would save the third pass (2^29:
-  // 13.6 against 15.5 ms), but costs more than that when keys occur some thirty
-  // times (33.7 against 28.8 ms), which a sample does not show. Else even runs up
-  // to kSmallRun leave the small one half full or better, with six standard
-  // deviations of room.
+  // runs twice as long. It is the only one where it leaves one pass (1.5M
+  // elements: 89 against 104 us). Where it can save the third, it is launched
+  // beside the other one and the sample decides, which may find keys denser than
+  // even ones: 2^29 uniform keys 15.5 -> 13.7 ms, 2^28 of a 29-bit range 8.2 -> 6.7
+  // ms. Else even runs up to kSmallRun leave the small one half full or better,
+  // with six standard deviations of room.
   const uint32_t least = passes_for((float)n, (float)kMeanRun);
-  const bool big = least == 2u && n <= 256u * kBigRun;
-  const double even_run = (double)n / std::pow(256.0, (double)(big ? 1u : least));
+  const bool only_big = least == 2u && n <= 256u * kBigRun;
+  const bool may_big = n > (1u << 27) && n <= 65536u * kBigRun;
+  const double even_run = (double)n / std::pow(256.0, (double)(only_big ? 1u : least));
   const bool small_tile = even_run <= (double)kSmallRun;
   // a smaller sample decides as well for fewer elements, and 5 us sooner
   const bool short_sample = n < (1u << 26);
-  const uint32_t mean_run = big ? kBigRun : small_tile ? kSmallRun : kMeanRun;
+  const uint32_t mean_run = only_big ? kBigRun : small_tile ? kSmallRun : kMeanRun;
   SampleRule rule = sample_rule(n, short_sample ? SampleTile<1>::kCap : SampleTile<kTopSample>::kCap, mean_run, mean_run,
                                 n <= (1u << 28) ? 16.0f : 4.0f);  // four passes for heavy keys up to 2^30 elements
   // Unused launches cost about 2 us each: below 2^26 elements only the four
   // passes of heavy keys, or two more than even keys need, are kept ready, and
   // the merges, whose rounds then stay nearly in L2, take what those leave.
   if (n < (1u << 26)) rule.tmax = std::max(4u, std::min(8u, rule.tmin + 2u));
+  if (may_big) {
+    const SampleRule wide = sample_rule(n, SampleTile<kTopSample>::kCap, kBigRun / 1.25f, kBigRun, 16.0f);
+    rule.big_tmin = 2u;
+    rule.big_near = wide.near_limit;
+  }
   static std::atomic<uint64_t> allowed[5];
-  const auto finish = big          ? k_top_finish<BigTile, 1>
-                      : small_tile ? k_top_finish<SmallTile, 4>
-                                   : k_top_finish<Tile, 2>;
-  const uint32_t cap = big ? BigTile::kCap : small_tile ? SmallTile::kCap : Tile::kCap;
-  const int threads = big ? BigTile::kThreads : small_tile ? SmallTile::kThreads : Tile::kThreads;
-  const size_t smem = big ? BigTile::kSmem : small_tile ? SmallTile::kSmem : Tile::kSmem;
-  const uint32_t ctas = big ? 1u : small_tile ? 4u : 2u;
   const auto sample = short_sample ? k_top_sample<1> : k_top_sample<kTopSample>;
   const size_t sample_smem = short_sample ? kSampleSmem<1> : kSampleSmem<kTopSample>;
-  if (!allow_smem((const void*)sample, sample_smem, &allowed[short_sample ? 3 : 4]) ||
-      !allow_smem((const void*)finish, smem, &allowed[big ? 2 : small_tile ? 1 : 0]))
-    return 5;
+  if (!allow_smem((const void*)sample, sample_smem, &allowed[short_sample ? 3 : 4])) return 5;
   {
     ProfScope prof("top_sample", st);
     sample<<<1, kSampleThreads, sample_smem, st>>>(X, n, rule, hist, ctrl);
@@ -577,21 +576,30 @@ int top_run(Elem* X, Elem* Y, unsigned char* ws, const Layout& L, cudaStream_t s
     if (int rc = onesweep_top_pass(X, Y, n, (int)p, gstart + p * 256u, ring, L.ring_tiles, ctrl, SegDesc{}, 0, 0u, dev, st)) return rc;
   RunChunk* chunks = reinterpret_cast<RunChunk*>(ring);
   uint32_t* unsorted = reinterpret_cast<uint32_t*>(chunks + max_chunks(n));
-  {
-    // A tile is left a run short on average (its last run is not whole), so a
-    // part of `per` tiles is as long as its runs fill `per` tiles, or, with runs
-    // that fill a tile by themselves, as `per` runs. Parts of 1 to 16 tiles:
-    // enough of them for six rounds of every resident CTA, and else few, since
-    // the run across a part's start is read twice.
-    const uint32_t run = (uint32_t)even_run;
-    const uint32_t fill = std::max(run, cap - std::min(cap, run + run / 2u));
+  // A tile is left a run short on average (its last run is not whole), so a
+  // part of `per` tiles is as long as its runs fill `per` tiles, or, with runs
+  // that fill a tile by themselves, as `per` runs. Parts of 1 to 16 tiles:
+  // enough of them for six rounds of every resident CTA, and else few, since
+  // the run across a part's start is read twice.
+  auto finish = [&](auto kernel, auto tile, uint32_t ctas, double run_length, uint32_t big, std::atomic<uint64_t>* ok) {
+    using TS = decltype(tile);
+    if (!allow_smem((const void*)kernel, TS::kSmem, ok)) return false;
+    const uint32_t run = (uint32_t)run_length;
+    const uint32_t fill = std::max(run, TS::kCap - std::min(TS::kCap, run + run / 2u));
     const uint32_t resident = (uint32_t)dev.sm_count * ctas;
     const uint32_t per = std::max<uint32_t>(1u, std::min<uint32_t>(16u, n / fill / (resident * 6u)));
     const uint32_t stride = per * fill;
     const uint32_t grid = (uint32_t)(((uint64_t)n + stride - 1u) / stride);
     ProfScope prof("top_finish", st);
-    finish<<<grid, threads, smem, st>>>(X, Y, n, stride, chunks, unsorted, ctrl);
-  }
+    kernel<<<grid, TS::kThreads, TS::kSmem, st>>>(X, Y, n, stride, chunks, unsorted, big, ctrl);
+    return cudaPeekAtLastError() == cudaSuccess;
+  };
+  const auto big_kernel = k_top_finish<BigTile, 1>;
+  if (!(only_big     ? finish(big_kernel, BigTile{}, 1u, even_run, 0u, &allowed[2])
+        : small_tile ? finish(k_top_finish<SmallTile, 4>, SmallTile{}, 4u, even_run, 0u, &allowed[1])
+                     : finish(k_top_finish<Tile, 2>, Tile{}, 2u, even_run, 0u, &allowed[0])) ||
+      (may_big && !finish(big_kernel, BigTile{}, 1u, (double)n / 65536.0, 1u, &allowed[2])))
+    return 5;
   if (cudaPeekAtLastError() != cudaSuccess) return 5;
   return top_merge(X, Y, n, chunks, unsorted, ctrl, dev, st);
 }

@@ -48,6 +48,7 @@ struct SampleRule {
   uint32_t near_limit;  // neighbours that may share a window before the mean run is too long
   uint32_t dups;        // equal neighbours from which most keys occur eight times or more
   uint32_t far_limit;   // keys in runs longer than a tile that are put up with
+  uint32_t big_tmin, big_near;  // tmin and near_limit for the big tile; tmax and more: it is not to be had
 };
 // mean_run: the mean run length up to which a pass is saved. Keys that occur
 // more than `often` times are heavy, and the passes then have `spread` windows
@@ -63,6 +64,8 @@ __host__ __device__ inline SampleRule sample_rule(uint32_t n, uint32_t sample, u
   const float per = (float)sample / (float)n;
   r.tmin = passes_for((float)n, (float)mean_run);
   r.tmax = 8u;
+  r.big_tmin = 9u;
+  r.big_near = 0u;
   r.tall = passes_for((float)n, 1.0f / spread);
   const float lam = (float)mean_run * per, lom = (float)often * per;
   r.far = (uint32_t)(lam + 4.0f * sqrtf(lam) + 4.0f);
@@ -114,19 +117,23 @@ __device__ __forceinline__ const uint64_t* sample_keys(const Elem* data, uint32_
 
 // Passes over the highest bytes below bit hb1 after which the sample s lets
 // expect runs of at most a tile, the same answer in every thread. near, far: 8
-// and 9 shared words, zeroed before the sample was sorted. *skewed: a key is heavy.
+// and 9 shared words, 11 with `big`, zeroed before the sample was sorted. *skewed:
+// a key is heavy. *big: the runs are for the big tile (null: not to be had).
 template <int S>
 __device__ __forceinline__ uint32_t sample_passes(const uint64_t* s, uint32_t hb1, const SampleRule& rule,
-                                                  uint32_t* s_near, uint32_t* s_far, bool* skewed) {
+                                                  uint32_t* s_near, uint32_t* s_far, bool* skewed,
+                                                  bool* big = nullptr) {
   // nibble T-1 of near / far: this thread's keys that share T windows (but
   // not all 64 bits) with the next key / with the key `far` places on
   constexpr uint32_t kSample = SampleTile<S>::kCap;
   uint32_t near = 0, farm = 0, equal = 0;
+  uint64_t diff = 0;
   bool heavy = false;
 #pragma unroll
   for (int k = 0; k < S; k++) {
     const uint32_t i = threadIdx.x + (uint32_t)k * kSampleThreads;
     const uint64_t ki = s[i];
+    diff |= ki ^ s[0];
     auto shared_windows = [&](uint32_t j) {
       const uint32_t bits = hb1 - min(hb1, 64u - (uint32_t)__clzll((long long)(ki ^ s[j])));
       return 0x11111111u & ((1u << (4u * (bits >> 3))) - 1u);  // bits < 64: the keys differ
@@ -149,15 +156,29 @@ __device__ __forceinline__ uint32_t sample_passes(const uint64_t* s, uint32_t hb
       atomicAdd(&s_far[l], ((l & 1u ? f1 : f0) >> (8u * (l >> 1))) & 0xFFu);
     }
   }
+  if (big) {  // bits in which keys differ
+    const uint32_t d0 = __reduce_or_sync(0xffffffffu, (uint32_t)diff), d1 = __reduce_or_sync(0xffffffffu, (uint32_t)(diff >> 32));
+    if (lane_id() == 0) {
+      atomicOr(&s_far[9], d0);
+      atomicOr(&s_far[10], d1);
+    }
+  }
   equal = __reduce_add_sync(0xffffffffu, equal);
   if (lane_id() == 0 && equal) atomicAdd(&s_far[8], equal);
   heavy = __syncthreads_or(heavy);
   *skewed = heavy;
+  auto enough = [&](uint32_t t, uint32_t near_limit) {
+    return s_near[t - 1u] <= near_limit && s_far[t - 1u] <= rule.far_limit && (!heavy || t >= rule.tall);
+  };
   const uint32_t full = (hb1 + 7u) / 8u, most = min(rule.tmax, full);
   uint32_t t = min(rule.tmin, full);
-  while (t < most && !(s_near[t - 1u] <= rule.near_limit && s_far[t - 1u] <= rule.far_limit &&
-                       (!heavy || t >= rule.tall)))
-    t++;
+  while (t < most && !enough(t, rule.near_limit)) t++;
+  if (big) {  // a pass less, if the big tile's bins will be even: no bit of the keys constant
+    const uint64_t varies = (uint64_t)s_far[10] << 32 | s_far[9];
+    *big = t > 1u && t - 1u >= rule.big_tmin && t < full && enough(t - 1u, rule.big_near) && s_far[8] < rule.dups &&
+           varies == ~0ull >> (64u - hb1);
+    if (*big) return t - 1u;
+  }
   // one pass more that leaves nothing to sort costs less than sorting runs of duplicates
   return t + 1u == full && t < rule.tmax && s_far[8] >= rule.dups ? full : t;
 }

@@ -125,3 +125,30 @@ def test_segments_of_every_kind(lsb, cuda, oracle, variant):
     got = to_np(A)
     for s, a in enumerate(parts):
         assert np.array_equal(got[off[s]:off[s + 1]], oracle.stable_sort_by_key(a)), (s, len(a))
+
+
+@pytest.mark.parametrize("n,kind", [(280000001, "uniform"), (280000001, "cluster"), (1 << 28, "dense"), (566231040, "uniform")])
+def test_runs_of_the_big_tile(lsb, cuda, n, kind):
+    """Two passes where the usual tile would need three: runs of 4272 to 8640
+    elements, and a run longer than any tile among them. Checked on the GPU: each
+    value is the index of its key, and (key, value) rises strictly."""
+    torch = cuda
+    src = torch.randint(-2**63, 2**63 - 1, (n,), dtype=torch.int64, device="cuda", generator=torch.Generator("cuda").manual_seed(n))
+    if kind == "cluster":
+        src[::1000] = (src[::1000] & 0xFFFFFFFF) + (77 << 48)
+    if kind == "dense":  # 28 bits of keys in a block of 29
+        i = torch.arange(777777, 777777 + n, dtype=torch.int64, device="cuda")
+        src = i ^ (i >> 3)
+    A = torch.empty((n, 2), dtype=torch.int64, device="cuda")
+    A[:, 0] = src
+    A[:, 1] = torch.arange(n, dtype=torch.int64, device="cuda")
+    B = torch.empty_like(A)
+    ws = lsb.alloc_workspace(n, 16)
+    lsb.sort_pairs(A, B, 16, workspace=ws)
+    assert lsb.query(ws).device_status == 0
+    del B
+    for lo in range(0, n, 1 << 26):
+        a = A[lo:min(n, lo + (1 << 26) + 1)]
+        assert torch.equal(src[a[:, 1]], a[:, 0])
+        k = a[:, 0] ^ (-2**63)
+        assert bool(((k[1:] > k[:-1]) | ((k[1:] == k[:-1]) & (a[1:, 1] > a[:-1, 1]))).all())
