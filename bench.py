@@ -5,7 +5,8 @@ Workload (the headline configuration): one step = one full LSD sort
 (lsb_sort_pairs, the reference's mySort, mpi/mpi_lsbsort.cpp:592-597) of
 2^30 16-byte {uint64 key, uint64 value} elements, keys uniform from the seeded
 splitmix64 stream, value = index, 16-bit digits (the reference's RADIX, 4
-digits, each run as two stable 8-bit sub-passes). The input is restored from
+digits: the same bytes whatever passes the library chooses, here three over the
+keys' top bytes and one on-chip sort of the runs they leave). The input is restored from
 a resident copy before every step (not timed), so every step sorts the same
 unsorted 16 GiB array; arrays are far larger than L2, and the restore copy
 itself sweeps L2.
@@ -31,8 +32,8 @@ Prints ONE JSON line (rank 0):
                the same sort through the other digit widths and kernel
                families (all give the same bytes)
   histogram_b16
-               lsb_histogram at 16-bit digits: one read per three digits
-               (default) against one HBM read by CTA pairs or quads
+               lsb_histogram at 16-bit digits: one HBM read by CTA pairs
+               (default) or quads, against one read per three digits
   sharded      the sharded sort (block distribution, count all-gather and
                element all-to-all per pass) over NCCL, 2^28 elements per rank
 
@@ -291,7 +292,8 @@ def configs_leg(args, lsb, torch, peaks: dict) -> dict:
     (input restored from a resident copy before every step, CUDA events,
     checked with the O(n) device verifier): the reference's CPU-runnable size
     2^24, and 2^28 in the four skewed key distributions, with the sort's
-    roofline on the passes it actually ran (8 B + 32 B per executed pass)."""
+    roofline on one read of the keys and a round trip per digit in which they
+    differ (8 B + 32 B per such digit)."""
     bits = 16
     cases = [("small_2p24_uniform", 1 << 24, "uniform"),
              ("skew_2p28_low32", 1 << 28, "low32"), ("skew_2p28_zipf", 1 << 28, "zipf"),
@@ -401,7 +403,8 @@ def gpu_arm(args, ranks: Ranks):
     dom_ms = prof[dom][1] / prof[dom][0]
     # algorithmic bytes per launch of the dominant kernel (per element, x n)
     per_elem = {"task_scatter": 32, "onesweep_scatter": 32, "wide_pass": 32, "task_count": 8,
-                "hist_digits": 8, "hist16": 8, "final_copy": 32}.get(dom, 0)
+                "hist_digits": 8, "top_hist": 8, "top_finish": 32, "mid_sort": 32, "small_sort": 32, "hist16": 8,
+                "final_copy": 32}.get(dom, 0)
     peaks = measured_peaks()
     achieved = per_elem * n / (dom_ms / 1e3) / 1e9
     traffic, traffic_src = committed_traffic(dom, n, bits)
@@ -545,8 +548,8 @@ def gpu_arm(args, ranks: Ranks):
 
 def histogram_b16_leg(lsb, torch, data, reps: int = 3) -> dict:
     """lsb_histogram at 16-bit digits (four digits of every key) in its three
-    forms: one read of the keys per three digits (default), and one HBM read by
-    CTA pairs (two digits each) or CTA quads (one digit each). Kernel time from
+    forms: one HBM read by CTA pairs (two digits each, the default) or CTA quads
+    (one digit each), and one read of the keys per three digits. Kernel time from
     the library's own launch events; the counts of all forms must agree."""
     res, counts = {}, {}
     for form in ("pairs", "quads", "split"):
@@ -567,7 +570,7 @@ def histogram_b16_leg(lsb, torch, data, reps: int = 3) -> dict:
                 os.environ.pop("LSB_HIST16", None)
             else:
                 os.environ["LSB_HIST16"] = old
-        launches, total = prof.get("hist16", (0, 0.0))
+        launches, total = (sum(prof.get(k, (0, 0.0))[i] for k in ("hist16", "hist16_sum")) for i in (0, 1))
         counts[form] = h
         res[form] = {"ms": round(total / reps, 4), "launches": launches // reps,
                      "hbm_reads_of_keys": 2 if form == "split" else 1}

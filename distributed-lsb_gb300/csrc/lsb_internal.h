@@ -102,9 +102,10 @@ int mid_run(Elem* X, Elem* Y, unsigned char* ws, const Layout& L, const DeviceIn
 // 0: 512 threads x 16, 1 CTA/SM; 2: 256 x 16, 2 CTAs/SM.
 uint32_t onesweep_top_tile(int variant);
 // Pass `pass` of the plan in ctrl->top, or of a batch's plans; gstart: that
-// pass's digit starts (one array); ctas: persistent CTAs, 0 = every resident slot.
+// pass's digit starts (one array); ctas: persistent CTAs, 0 = every resident slot. spare: one that even
+// keys do not need, under its own name in the launch times.
 int onesweep_top_pass(Elem* X, Elem* Y, uint32_t n, int pass, const uint32_t* gstart, uint64_t* ring,
-                      uint32_t tiles, Ctrl* ctrl, const SegDesc& seg, int variant, uint32_t ctas,
+                      uint32_t tiles, Ctrl* ctrl, const SegDesc& seg, int variant, uint32_t ctas, bool spare,
                       const DeviceInfo& dev, cudaStream_t st);
 // The merges of runs longer than a tile (lsb_top.cu): list of chunks and marks
 // of their runs, at most top_list_bytes(n) together.

@@ -1406,7 +1406,7 @@ uint32_t onesweep_tile_elems(int bits) { return onesweep_choice(bits).tile; }
 uint32_t onesweep_top_tile(int variant) { return variant == 2 ? 4096u : 8192u; }
 
 int onesweep_top_pass(Elem* X, Elem* Y, uint32_t n, int pass, const uint32_t* gstart, uint64_t* ring,
-                      uint32_t tiles, Ctrl* ctrl, const SegDesc& seg, int variant, uint32_t ctas,
+                      uint32_t tiles, Ctrl* ctrl, const SegDesc& seg, int variant, uint32_t ctas, bool spare,
                       const DeviceInfo& dev, cudaStream_t st) {
   const int threads = variant == 2 ? 256 : 512;
   auto kern = variant == 2 ? k_onesweep<256, 16, 2, uint32_t, 8, true> : k_onesweep<512, 16, 1, uint32_t, 8, true>;
@@ -1416,7 +1416,7 @@ int onesweep_top_pass(Elem* X, Elem* Y, uint32_t n, int pass, const uint32_t* gs
   uint32_t grid = (uint32_t)dev.sm_count * (variant == 2 ? 2u : 1u);
   if (ctas > 0) grid = std::min(grid, ctas);
   grid = std::max<uint32_t>(1u, std::min(grid, tiles));
-  ProfScope prof("onesweep_scatter", st);
+  ProfScope prof(spare ? "onesweep_spare" : "onesweep_scatter", st);
   // one ring slot per tile: no slot is reused, so there are no completion tags
   kern<<<grid, threads, smem, st>>>(X, Y, n, 8, pass, 0, gstart, ring, nullptr, tiles, ctrl, seg);
   return cudaPeekAtLastError() == cudaSuccess ? 0 : 5;

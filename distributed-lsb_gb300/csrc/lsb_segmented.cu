@@ -436,7 +436,7 @@ static int seg_run(Elem* A, Elem* B, const int64_t* seg_off, void* ws, const Seg
   seg.num_tiles = ntiles;
   seg.plan = plans;
   for (uint32_t p = 0; p < passes; p++)
-    if (onesweep_top_pass(A, B, L.n, (int)p, nullptr, ring, L.max_tiles, ctrl, seg, L.variant, L.ctas, dev, st))
+    if (onesweep_top_pass(A, B, L.n, (int)p, nullptr, ring, L.max_tiles, ctrl, seg, L.variant, L.ctas, false, dev, st))
       return LSB_ERR_CUDA;
   RunChunk* chunks = reinterpret_cast<RunChunk*>(ring);
   uint32_t* unsorted = reinterpret_cast<uint32_t*>(chunks + max_chunks(L.n));

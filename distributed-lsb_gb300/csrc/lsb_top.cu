@@ -572,8 +572,11 @@ int top_run(Elem* X, Elem* Y, unsigned char* ws, const Layout& L, cudaStream_t s
                                                  L.api_bits, L.sub, ctrl);
   }
   if (cudaPeekAtLastError() != cudaSuccess) return 5;
-  for (uint32_t p = 0; p < rule.tmax; p++)
-    if (int rc = onesweep_top_pass(X, Y, n, (int)p, gstart + p * 256u, ring, L.ring_tiles, ctrl, SegDesc{}, 0, 0u, dev, st)) return rc;
+  for (uint32_t p = 0; p < rule.tmax; p++) {
+    const bool spare = p >= rule.tmin - (may_big ? 1u : 0u);  // one that even keys do not need: most return at once
+    if (int rc = onesweep_top_pass(X, Y, n, (int)p, gstart + p * 256u, ring, L.ring_tiles, ctrl, SegDesc{}, 0, 0u, spare, dev, st))
+      return rc;
+  }
   RunChunk* chunks = reinterpret_cast<RunChunk*>(ring);
   uint32_t* unsorted = reinterpret_cast<uint32_t*>(chunks + max_chunks(n));
   // A tile is left a run short on average (its last run is not whole), so a
