@@ -211,6 +211,7 @@ struct TileSort {
     }
     __syncthreads();
     // 2. exclusive scan of the counts; thread t owns bins [16 t, 16 t + 16)
+    bool over;
     {
       uint32_t w8[8], maxc = 0, sum = 0;
       uint4* q = reinterpret_cast<uint4*>(bins) + tid * 2u;
@@ -234,7 +235,8 @@ struct TileSort {
       }
       if (lane == 31) sh.wtot[warp] = inc;
       maxc = max(maxc & 0xffffu, maxc >> 16);
-      if (__syncthreads_or(maxc > kMaxBin) && !HEAVY) return false;
+      over = __syncthreads_or(maxc > kMaxBin) != 0;
+      if (over && !HEAVY) return false;
       uint32_t off = inc - sum;
       const uint32_t wt = lane < (uint32_t)kWarps ? sh.wtot[lane] : 0u;
       off += __reduce_add_sync(0xffffffffu, lane < warp ? wt : 0u);
@@ -296,7 +298,7 @@ struct TileSort {
 #pragma unroll
       for (int i = 0; i < R; i++) e[i] = in[v[i] & kPosMask];
     };
-    auto rank_rows = [&](const uint32_t (&v)[R], const Elem (&e)[R], uint32_t* r) {
+    auto rank_rows = [&](const bool by_slots, const uint32_t (&v)[R], const Elem (&e)[R], uint32_t* r) {
 #pragma unroll
       for (int i = 0; i < R; i++) {
         uint32_t f;
@@ -313,9 +315,9 @@ struct TileSort {
             close |= ((u ^ v[i]) - 1u) < kPosMask;
           }
         }
-        if (HEAVY && cnt > kSlotsBin) {
+        if (HEAVY && by_slots && cnt > kSlotsBin) {
           r[i] = kCap;  // heavy_bins emits it
-        } else if (HEAVY && cnt > 4u) {
+        } else if (HEAVY && by_slots && cnt > 4u) {
           // slots alone: right when all that agree in the key bits hold the same
           // key, and so when each holds the key of the lowest of them
           uint32_t low = v[i];
@@ -338,11 +340,11 @@ struct TileSort {
     };
     uint32_t v[R], r[K];
     Elem e[R];
-    if (!HEAVY) {
+    if (!HEAVY || !over) {
 #pragma unroll 1
       for (uint32_t row = tid; row - tid < m; row += R * THREADS) {
         load_rows(row, v, e);
-        rank_rows(v, e, r);
+        rank_rows(false, v, e, r);
 #pragma unroll
         for (int i = 0; i < R; i++) emit(row + (uint32_t)i * THREADS < m, r[i], e[i]);
       }
@@ -353,7 +355,7 @@ struct TileSort {
 #pragma unroll
     for (int k = 0; k < K; k += R) {
       load_rows(tid + (uint32_t)k * THREADS, v, e);
-      rank_rows(v, e, r + k);
+      rank_rows(HEAVY, v, e, r + k);
     }
     lost = __syncthreads_or(lost);
 #pragma unroll

@@ -19,7 +19,7 @@ namespace lsb {
 
 // Bound by latency: one read of the tile, seven barriers, one write. Twelve
 // launches (clears, the histogram, the plan, eight passes and the copy back)
-// took 112 us for 1000 elements with the array's own copy; this takes 20.5 us.
+// took 112 us for 1000 elements with the array's own copy; this takes 11.3 us.
 template <int THREADS, int K>
 __global__ void __launch_bounds__(THREADS, 1)
     k_small_sort(Elem* __restrict__ a, uint32_t n, int bits, int num_digits, int api_bits, int sub, Ctrl* ctrl) {
@@ -97,17 +97,20 @@ static int small_sort(Elem* X, const Layout& L, Ctrl* ctrl, cudaStream_t st) {
 //                 and sorted by chunks and merges unless they are in order
 // The result does not depend on the sample: it only decides how short the
 // runs are, and so the time. Measured (GB300, sort alone): 2^24 uniform 1.10 ->
-// 0.48 ms, 2^28 15.0 -> 6.4 ms, 2^30 58.6 -> 30.8 ms (three passes), 2^28 Zipf
-// 16.0 -> 9.8 ms (four passes; heavy keys stay in order), against eight passes.
+// 0.47 ms, 2^28 15.0 -> 6.5 ms, 2^29 29.4 -> 13.7 ms (two passes), 2^30 58.6 ->
+// 30.9 ms (three), 2^28 Zipf 16.0 -> 9.4 ms (four; heavy keys stay in order),
+// against eight passes.
 
-constexpr uint32_t kSmallRun = 1700;  // the same of the small tile, with room for one and a half
-constexpr uint32_t kBigRun = 8640;    // and of the big one
+// Longest even runs for the small tile (one and a half of them fit) and for the
+// big one (six standard deviations below it); for the usual one: kMeanRun.
+constexpr uint32_t kSmallRun = 1700, kBigRun = 8640;
 constexpr int kTopSample = 4;  // keys per thread of the sample: 4096
 constexpr int kTopHistThreads = 512;
 constexpr int kTopHistUnroll = 4;
 
-// Bound by latency (one CTA: 4096 scattered reads, a tile sort, two counts);
-// it also clears what the later kernels count in, in place of three memsets.
+// Bound by latency (one CTA: scattered reads, a tile sort, two counts: 11 us with
+// 1024 keys, 17 to 20 with 4096); it also clears what the later kernels count in,
+// in place of three memsets.
 template <int S>
 __global__ void __launch_bounds__(kSampleThreads, 1)
     k_top_sample(const Elem* __restrict__ data, uint32_t n, SampleRule rule, uint32_t* __restrict__ hist, Ctrl* ctrl) {
