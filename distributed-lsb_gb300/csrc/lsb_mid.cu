@@ -1,5 +1,5 @@
 // lsb_mid.cu -- whole sorts of arrays too large for one CTA but small enough
-// for every CTA to hold a tile of them: one cooperative launch.
+// for every CTA to hold a tile of them: one launch, cooperative or of one cluster.
 //
 // At these sizes (9217 elements to 8192 per SM) memory traffic is nothing and
 // launches are everything: the histogram, the plan and each pass cost a launch
@@ -19,7 +19,7 @@
 //      missed them) have the array passed over by every digit that differs.
 // Bound by latency: about four grid barriers and as many trips to L2. Measured
 // (GB300, sort alone, eight launched passes -> this): 10^4 uniform keys 131 ->
-// 32 us, 10^5 153 -> 28, 10^6 153 -> 42; Zipf keys (four digits) 10^5 153 -> 79,
+// 25 us, 10^5 153 -> 28, 10^6 153 -> 42; Zipf keys (four digits) 10^5 153 -> 79,
 // 10^6 155 -> 139. The tile
 // stays in shared memory, not in registers: with 1024 threads its elements
 // spill, and beside 217 KB of shared memory there is no L1 to spill to (a
@@ -60,8 +60,9 @@ struct MidWindow {
   }
 };
 
-// K elements per thread: tiles of 1024 K.
-template <int K>
+// K elements per thread: tiles of 1024 K. CLUSTER: the grid is one cluster, whose
+// barriers are in hardware, and clears the control block itself.
+template <int K, bool CLUSTER>
 __global__ void __launch_bounds__(kMidThreads, 1)
     k_mid_sort(Elem* X, Elem* Y, uint32_t n, SampleRule rule, uint16_t* table, MidRun* runs, uint32_t max_runs,
                int bits, int num_digits, int api_bits, int sub, Ctrl* ctrl) {
@@ -89,6 +90,12 @@ __global__ void __launch_bounds__(kMidThreads, 1)
   uint32_t barriers = 0, buf = 0;
   MidWindow win;
 
+  auto all_arrived = [&]() {
+    if (!CLUSTER) return grid_barrier(ctrl, &barriers);
+    cluster_arrive();
+    cluster_wait();
+    return true;
+  };
   auto load_tile = [&](const Elem* src) {
     __syncthreads();
     Elem v[K];
@@ -228,6 +235,11 @@ __global__ void __launch_bounds__(kMidThreads, 1)
   if (tid < 8) s_near[tid] = 0u;
   if (tid < 9) s_far[tid] = 0u;
   const uint64_t first_key = ld_relaxed_u64(&X[0].key);
+  if (CLUSTER) {
+    if (t == 0)
+      for (uint32_t i = tid; i < kCtrlBytes / 4u; i += kMidThreads) reinterpret_cast<uint32_t*>(ctrl)[i] = 0u;
+    cluster_arrive();
+  }
   load_tile(X);
   {
     uint64_t x = 0;
@@ -244,8 +256,9 @@ __global__ void __launch_bounds__(kMidThreads, 1)
     }
   }
   __syncthreads();
+  if (CLUSTER) cluster_wait();
   if (tid < 2 && s_diff[tid]) atomicOr(&ctrl->top.diff[tid], s_diff[tid]);
-  if (!grid_barrier(ctrl, &barriers)) return;
+  if (!all_arrived()) return;
   const uint64_t diff = (uint64_t)__ldcg(&ctrl->top.diff[1]) << 32 | __ldcg(&ctrl->top.diff[0]);
   if (t == 0 && tid == 0) write_plan(ctrl, diff, n, bits, num_digits, api_bits, sub);
   if (diff == 0) return;
@@ -256,7 +269,7 @@ __global__ void __launch_bounds__(kMidThreads, 1)
   win.hb1 = hb1, win.passes = 1u;
   win.set_pass(0);
   count_tile();
-  if (!grid_barrier(ctrl, &barriers)) return;
+  if (!all_arrived()) return;
   add_up();
   const bool exact = full == 1u || s_max <= MidTile::kCap;
   bool skewed = false;
@@ -282,13 +295,13 @@ __global__ void __launch_bounds__(kMidThreads, 1)
         load_tile(par ? Y : X);
         buf ^= 1u;
         count_tile();
-        if (!grid_barrier(ctrl, &barriers)) return;
+        if (!all_arrived()) return;
         add_up();
       }
       if (s_one) continue;  // the digit is the same everywhere
       scatter(par ? X : Y);
       par ^= 1u;
-      if (!grid_barrier(ctrl, &barriers)) return;
+      if (!all_arrived()) return;
     }
     const Elem* src = par ? Y : X;
     if (win.passes == full && !win.clamp) {  // in order
@@ -342,7 +355,7 @@ __global__ void __launch_bounds__(kMidThreads, 1)
                        load, long_run);
     if (exact) return;
     // 4. runs longer than a tile: copied into X, and whether they are in order
-    if (!grid_barrier(ctrl, &barriers)) return;
+    if (!all_arrived()) return;
     const uint32_t count = min(ld_relaxed_u32(&ctrl->top.num_runs), max_runs);
     if (count == 0) return;
     MidRun* list = reinterpret_cast<MidRun*>(smem);
@@ -359,7 +372,7 @@ __global__ void __launch_bounds__(kMidThreads, 1)
       }
     }
     if (__any_sync(0xffffffffu, inversion) && lane == 0) atomicOr(&ctrl->top.num_chunks, 1u);
-    if (!grid_barrier(ctrl, &barriers)) return;
+    if (!all_arrived()) return;
     if (ld_relaxed_u32(&ctrl->top.num_chunks) == 0u) return;
     win.lo = 0ull, win.hi = ~0ull, win.clamp = false;
     win.hb1 = hb1, win.passes = full;
@@ -384,6 +397,45 @@ size_t mid_workspace_bytes(uint32_t n, const DeviceInfo& dev) {
   return kCtrlBytes + (size_t)mid_tiles(n, mid_items(n, dev)) * 256u * 2u * 2u + (size_t)mid_max_runs(n) * sizeof(MidRun);
 }
 
+// Up to 16 tiles of 2048 elements the grid is one cluster of 16 CTAs: no clear
+// before it, no cooperative launch, barriers in hardware. 32768 uniform elements
+// 26 -> 23 us, Zipf keys 49 -> 45. Larger tiles in the cluster lose that again
+// against more CTAs (50000: 27 us either way, 65537: 31 against 26).
+constexpr uint32_t kMidCluster = 16, kMidClusterItems = 2;
+
+static cudaLaunchConfig_t mid_cluster_config(cudaLaunchAttribute* attr, cudaStream_t st) {
+  attr->id = cudaLaunchAttributeClusterDimension;
+  attr->val.clusterDim.x = kMidCluster;
+  attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3(kMidCluster);
+  c.blockDim = dim3(kMidThreads);
+  c.dynamicSmemBytes = kMidSmem;
+  c.stream = st;
+  c.attrs = attr;
+  c.numAttrs = 1;
+  return c;
+}
+
+// Whether the current device has room for such a cluster; asked once per device.
+static bool mid_cluster_fits(const void* kern) {
+  static std::atomic<uint64_t> yes, no;
+  int dev = -1;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+  const uint64_t bit = 1ull << dev;
+  if (yes.load(std::memory_order_acquire) & bit) return true;
+  if (no.load(std::memory_order_acquire) & bit) return false;
+  cudaLaunchAttribute attr;
+  const cudaLaunchConfig_t config = mid_cluster_config(&attr, nullptr);
+  int clusters = 0;
+  const bool fits = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMidSmem) == cudaSuccess &&
+                    cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                    cudaOccupancyMaxActiveClusters(&clusters, kern, &config) == cudaSuccess && clusters > 0;
+  if (!fits) cudaGetLastError();
+  (fits ? yes : no).fetch_or(bit, std::memory_order_release);
+  return fits;
+}
+
 int mid_run(Elem* X, Elem* Y, unsigned char* ws, const Layout& L, const DeviceInfo& dev, cudaStream_t st) {
   Ctrl* ctrl = reinterpret_cast<Ctrl*>(ws);
   uint32_t n = L.n;
@@ -394,16 +446,25 @@ int mid_run(Elem* X, Elem* Y, unsigned char* ws, const Layout& L, const DeviceIn
   // A key that overfills its bins makes a tile uneven, unless the tile is in
   // order: 2048 windows per element leave a tile without a mixed run.
   SampleRule rule = sample_rule(n, SampleTile<kMidSample>::kCap, MidTile::kCap - 576u, MidTile::kMaxBin, 2048.0f);
-  const void* kern = items == 2u   ? (const void*)k_mid_sort<2>
-                     : items == 4u ? (const void*)k_mid_sort<4>
-                                   : (const void*)k_mid_sort<8>;
+  int bits = L.stat_bits, digits = L.stat_digits, api_bits = L.api_bits, sub = L.sub;
+  void* args[] = {&X, &Y, &n, &rule, &table, &runs, &max_runs, &bits, &digits, &api_bits, &sub, &ctrl};
+  if (n <= kMidCluster * kMidClusterItems * (uint32_t)kMidThreads) {
+    const void* kern = (const void*)k_mid_sort<(int)kMidClusterItems, true>;
+    if (mid_cluster_fits(kern)) {
+      cudaLaunchAttribute attr;
+      const cudaLaunchConfig_t config = mid_cluster_config(&attr, st);
+      ProfScope prof("mid_sort", st);
+      return cudaLaunchKernelExC(&config, kern, args) == cudaSuccess ? 0 : 5;
+    }
+  }
+  const void* kern = items == 2u   ? (const void*)k_mid_sort<2, false>
+                     : items == 4u ? (const void*)k_mid_sort<4, false>
+                                   : (const void*)k_mid_sort<8, false>;
   static std::atomic<uint64_t> allowed[3];
   if (!allow_smem(kern, kMidSmem, &allowed[items >> 2]) || cudaMemsetAsync(ws, 0, kCtrlBytes, st) != cudaSuccess)
     return 5;
   // CTAs beyond the tiles take a share of the runs
   const uint32_t grid = std::min<uint32_t>((uint32_t)dev.sm_count, std::max(tiles, (n - 1u) / 2048u + 1u));
-  int bits = L.stat_bits, digits = L.stat_digits, api_bits = L.api_bits, sub = L.sub;
-  void* args[] = {&X, &Y, &n, &rule, &table, &runs, &max_runs, &bits, &digits, &api_bits, &sub, &ctrl};
   ProfScope prof("mid_sort", st);
   return cudaLaunchCooperativeKernel(kern, dim3(grid), dim3(kMidThreads), args, kMidSmem, st) == cudaSuccess ? 0 : 5;
 }

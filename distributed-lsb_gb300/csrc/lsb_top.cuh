@@ -456,4 +456,8 @@ __device__ __forceinline__ bool grid_barrier(Ctrl* ctrl, uint32_t* round) {
   return s_ok;
 }
 
+// The same of one cluster of CTAs, in hardware; global memory is ordered by it too.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+
 }  // namespace lsb

@@ -91,7 +91,7 @@ def large_key_sets(n, seed):
     yield "dups", full[r.integers(0, max(1, n // 3000), n)]
 
 
-@pytest.mark.parametrize("n", [9217, 65537, 300007, 311296, 311297, 622593, 1245184, 1245185, (1 << 22) + 3])
+@pytest.mark.parametrize("n", [9217, 32768, 32769, 65537, 300007, 311296, 311297, 622593, 1245184, 1245185, (1 << 22) + 3])
 def test_top_digits(lsb, cuda, oracle, n):
     """Runs of every kind, in one launch up to 8192 elements per SM (at the edges
     of its tile sizes on 152 SMs) and pass by pass above."""
