@@ -218,7 +218,7 @@ int run_passes(Elem* X, Elem* Y, int first_digit, int target_parity, void* ws, c
                cudaStream_t st) {
   unsigned char* w = static_cast<unsigned char*>(ws);
   if (L.family == Family::kTop) return top_run(X, Y, w, L, st) ? LSB_ERR_CUDA : LSB_OK;
-  if (cudaMemsetAsync(w, 0, kCtrlBytes, st) != cudaSuccess) return LSB_ERR_CUDA;
+  if (L.family != Family::kOnesweep && cudaMemsetAsync(w, 0, kCtrlBytes, st) != cudaSuccess) return LSB_ERR_CUDA;
   first_digit *= L.sub;  // split wide digits: sub-digits 2d and 2d+1
   int rc = (L.family == Family::kOnesweep) ? onesweep_run(X, Y, first_digit, target_parity, w, L, st)
            : (L.family == Family::kWide)    ? wide_run(X, Y, first_digit, target_parity, w, L, st)
@@ -501,12 +501,9 @@ int lsb_pass(const lsb_elem_t* d_src, lsb_elem_t* d_dst, int64_t n, int digit_bi
     unsigned char* wb = static_cast<unsigned char*>(w);
     Elem* mid = reinterpret_cast<Elem*>(wb + align_up(Ls.total, 256));
     int rc = LSB_OK;
-    if (cudaMemsetAsync(wb, 0, kCtrlBytes, st) != cudaSuccess) rc = LSB_ERR_CUDA;
-    if (rc == LSB_OK) {
-      const int r = onesweep_pass_via(reinterpret_cast<const Elem*>(d_src), mid,
-                                      reinterpret_cast<Elem*>(d_dst), digit * 2, wb, Ls, st);
-      if (r) rc = r == 1 ? LSB_ERR_INVALID_ARG : LSB_ERR_CUDA;
-    }
+    const int r = onesweep_pass_via(reinterpret_cast<const Elem*>(d_src), mid,
+                                    reinterpret_cast<Elem*>(d_dst), digit * 2, wb, Ls, st);
+    if (r) rc = r == 1 ? LSB_ERR_INVALID_ARG : LSB_ERR_CUDA;
     if (d_workspace) return rc;
     uint32_t dev_err = 0;
     if (rc == LSB_OK &&

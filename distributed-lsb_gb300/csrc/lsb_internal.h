@@ -94,6 +94,10 @@ int wide_run(Elem* X, Elem* Y, int first_digit, int target_parity, unsigned char
 // Whole sort by the top family; the result is in X. The control block is
 // cleared by the kernels.
 int top_run(Elem* X, Elem* Y, unsigned char* ws, const Layout& L, cudaStream_t st);
+// One pass over the 8-bit digits [first_digit, first_digit + L.num_digits), one or
+// two, from src into dst; where the layout has a look-back slot for every tile.
+bool top_pass_fits(const Layout& L);
+int top_pass_run(const Elem* src, Elem* mid, Elem* dst, int first_digit, unsigned char* ws, const Layout& L, cudaStream_t st);
 // Its one-launch form (lsb_mid.cu): largest array, workspace, launch.
 uint32_t mid_limit(const DeviceInfo& dev);
 size_t mid_workspace_bytes(uint32_t n, const DeviceInfo& dev);

@@ -1523,6 +1523,8 @@ int onesweep_run(Elem* X, Elem* Y, int first_digit, int target_parity, unsigned 
   const uint32_t nbins = 1u << L.bits;
   const uint32_t tiles = (L.n + L.tile_elems - 1) / L.tile_elems;
   const uint32_t used_slots = std::min(tiles, L.ring_tiles);
+  if (L.num_digits == 1 && target_parity == 1 && top_pass_fits(L)) return top_pass_run(X, nullptr, Y, first_digit, ws, L, st);
+  if (cudaMemsetAsync(ws, 0, kCtrlBytes, st) != cudaSuccess) return 5;
   if (cudaMemsetAsync(ring, 0, (size_t)used_slots * nbins * 8u, st) != cudaSuccess) return 5;
   if (cudaMemsetAsync(done, 0, (size_t)L.ring_tiles * 4u, st) != cudaSuccess) return 5;
   if (int rc = histogram_u32(X, L.n, L.bits, first_digit, L.num_digits, hist, st)) return rc;
@@ -1571,6 +1573,8 @@ int onesweep_pass_via(const Elem* src, Elem* mid, Elem* dst, int first_digit, un
   const uint32_t tiles = (L.n + L.tile_elems - 1) / L.tile_elems;
   const uint32_t used_slots = std::min(tiles, L.ring_tiles);
   if (L.num_digits != 2) return 1;
+  if (top_pass_fits(L)) return top_pass_run(src, mid, dst, first_digit, ws, L, st);
+  if (cudaMemsetAsync(ws, 0, kCtrlBytes, st) != cudaSuccess) return 5;
   if (cudaMemsetAsync(ring, 0, (size_t)used_slots * nbins * 8u, st) != cudaSuccess) return 5;
   if (cudaMemsetAsync(done, 0, (size_t)L.ring_tiles * 4u, st) != cudaSuccess) return 5;
   if (int rc = histogram_u32(src, L.n, L.bits, first_digit, 2, hist, st)) return rc;

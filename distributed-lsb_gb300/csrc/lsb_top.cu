@@ -215,7 +215,7 @@ __device__ __noinline__ void count_many_windows(const Elem* __restrict__ data, u
 __global__ void __launch_bounds__(kTopHistThreads, 4)
     k_top_hist(const Elem* __restrict__ data, uint32_t n, uint32_t* __restrict__ hist, uint32_t* __restrict__ gstart,
                uint4* __restrict__ ring, uint64_t ring_words, int bits, int num_digits, int api_bits, int sub,
-               Ctrl* ctrl) {
+               uint32_t single, Ctrl* ctrl) {
   __shared__ uint32_t h[8 * 256];
   __shared__ uint32_t s_diff[2];
   __shared__ uint32_t s_const;
@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(kTopHistThreads, 4)
   __syncthreads();
   const uint64_t first = data[0].key;
   uint64_t diff = 0;
-  if (p.hb1 < 64u) {
+  if (p.clamp) {
     switch (T) {
       case 1: count_windows<1, true>(data, n, p, h, first, &diff); break;
       case 2: count_windows<2, true>(data, n, p, h, first, &diff); break;
@@ -304,6 +304,19 @@ __global__ void __launch_bounds__(kTopHistThreads, 4)
         run |= 1u << t;
         par ^= 1u;
       }
+    }
+    if (single) {  // every pass runs, so that the result lands in its place whatever the digits
+      const uint32_t constant = single == 1u ? s_const & 1u : 0u;
+      q.run_mask = (1u << T) - 1u;
+      q.par_mask = 2u;
+      ctrl->skip_mask_lo = constant;
+      ctrl->passes_run = single - constant;
+      ctrl->final_copy = constant;
+      ctrl->num_passes = single;
+      ctrl->api_bits = (uint32_t)api_bits;
+      ctrl->sub = (uint32_t)sub;
+      ctrl->n = n;
+      return;
     }
     q.run_mask = run;
     q.par_mask = pars;
@@ -518,6 +531,60 @@ int top_merge(Elem* X, Elem* Y, uint32_t n, RunChunk* chunks, uint32_t* unsorted
 }
 
 // ---------------------------------------------------------------------------
+// one digit
+
+// Plan of a single pass over the `passes` bytes below bit hb1; it also clears
+// what the later kernels count in.
+__global__ void __launch_bounds__(kSampleThreads) k_pass_plan(uint32_t* __restrict__ hist, uint32_t hb1, uint32_t passes, Ctrl* ctrl) {
+  for (uint32_t i = threadIdx.x; i < kCtrlBytes / 4u; i += kSampleThreads) reinterpret_cast<uint32_t*>(ctrl)[i] = 0u;
+  for (uint32_t i = threadIdx.x; i < passes * 256u; i += kSampleThreads) hist[i] = 0u;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    ctrl->top.passes = passes;
+    ctrl->top.hb1 = hb1;
+  }
+}
+
+static int top_hist(const Elem* X, unsigned char* ws, const Layout& L, uint32_t single, const DeviceInfo& dev, cudaStream_t st) {
+  // four CTAs per SM, fewer when they would have under four rounds of reads each
+  const uint32_t per_cta = (uint32_t)kTopHistThreads * kTopHistUnroll * 4u;
+  const uint32_t grid = std::max<uint32_t>(1u, std::min<uint32_t>((L.n - 1u) / per_cta + 1u, (uint32_t)dev.sm_count * 4u));
+  ProfScope prof("top_hist", st);
+  k_top_hist<<<grid, kTopHistThreads, 0, st>>>(
+      X, L.n, reinterpret_cast<uint32_t*>(ws + L.off_hist), reinterpret_cast<uint32_t*>(ws + L.off_gstart),
+      reinterpret_cast<uint4*>(ws + L.off_ring), ((uint64_t)(L.n - 1u) / onesweep_top_tile(0) + 1u) * 256u * 8u / 16u, L.stat_bits, L.stat_digits,
+      L.api_bits, L.sub, single, reinterpret_cast<Ctrl*>(ws));
+  return cudaPeekAtLastError() == cudaSuccess ? 0 : 5;
+}
+
+// globalShuffle of an 8-bit digit (mpi/mpi_lsbsort.cpp:493-589), or of two in
+// turn through mid. Clears, histogram and plan take two launches, not seven: with
+// the count of its digits, a 16-bit digit of 65537 elements 122 -> 75 us, of 2^26
+// 1409 -> 1352.
+bool top_pass_fits(const Layout& L) {
+  return L.bits == 8 && L.tile_elems == onesweep_top_tile(0) && L.ring_tiles >= (L.n - 1u) / L.tile_elems + 1u;
+}
+int top_pass_run(const Elem* src, Elem* mid, Elem* dst, int first_digit, unsigned char* ws, const Layout& L, cudaStream_t st) {
+  Ctrl* ctrl = reinterpret_cast<Ctrl*>(ws);
+  DeviceInfo dev;
+  if (int rc = current_device_info(&dev)) return rc;
+  const uint32_t passes = (uint32_t)L.num_digits;
+  const uint32_t* gstart = reinterpret_cast<const uint32_t*>(ws + L.off_gstart);
+  uint64_t* ring = reinterpret_cast<uint64_t*>(ws + L.off_ring);
+  {
+    ProfScope prof("plan", st);
+    k_pass_plan<<<1, kSampleThreads, 0, st>>>(reinterpret_cast<uint32_t*>(ws + L.off_hist),
+                                              8u * ((uint32_t)first_digit + passes), passes, ctrl);
+  }
+  if (int rc = top_hist(src, ws, L, passes, dev, st)) return rc;
+  Elem* in = const_cast<Elem*>(src);  // read only: pass 0 reads X
+  if (int rc = onesweep_top_pass(in, passes == 1u ? dst : mid, L.n, 0, gstart, ring, L.ring_tiles, ctrl, SegDesc{}, 0, 0u, false, dev, st))
+    return rc;
+  if (passes == 1u) return 0;
+  return onesweep_top_pass(dst, mid, L.n, 1, gstart + 256u, ring, L.ring_tiles, ctrl, SegDesc{}, 0, 0u, false, dev, st);
+}
+
+// ---------------------------------------------------------------------------
 // driver
 
 int top_run(Elem* X, Elem* Y, unsigned char* ws, const Layout& L, cudaStream_t st) {
@@ -565,16 +632,7 @@ int top_run(Elem* X, Elem* Y, unsigned char* ws, const Layout& L, cudaStream_t s
     ProfScope prof("top_sample", st);
     sample<<<1, kSampleThreads, sample_smem, st>>>(X, n, rule, hist, ctrl);
   }
-  {
-    // four CTAs per SM, fewer when they would have under four rounds of reads each
-    const uint32_t per_cta = (uint32_t)kTopHistThreads * kTopHistUnroll * 4u;
-    const uint32_t grid = std::max<uint32_t>(1u, std::min<uint32_t>((n - 1u) / per_cta + 1u, (uint32_t)dev.sm_count * 4u));
-    ProfScope prof("top_hist", st);
-    k_top_hist<<<grid, kTopHistThreads, 0, st>>>(X, n, hist, gstart, reinterpret_cast<uint4*>(ring),
-                                                 (uint64_t)L.ring_tiles * 256u * 8u / 16u, L.stat_bits, L.stat_digits,
-                                                 L.api_bits, L.sub, ctrl);
-  }
-  if (cudaPeekAtLastError() != cudaSuccess) return 5;
+  if (int rc = top_hist(X, ws, L, 0u, dev, st)) return rc;
   for (uint32_t p = 0; p < rule.tmax; p++) {
     const bool spare = p >= rule.tmin - (may_big ? 1u : 0u);  // one that even keys do not need: most return at once
     if (int rc = onesweep_top_pass(X, Y, n, (int)p, gstart + p * 256u, ring, L.ring_tiles, ctrl, SegDesc{}, 0, 0u, spare, dev, st))

@@ -152,3 +152,25 @@ def test_runs_of_the_big_tile(lsb, cuda, n, kind):
         assert torch.equal(src[a[:, 1]], a[:, 0])
         k = a[:, 0] ^ (-2**63)
         assert bool(((k[1:] > k[:-1]) | ((k[1:] == k[:-1]) & (a[1:, 1] > a[:-1, 1]))).all())
+
+
+@pytest.mark.parametrize("n", [1, 2, 8191, 8192, 8193, 70001])
+@pytest.mark.parametrize("bits", [8, 16])
+def test_one_digit(lsb, cuda, n, bits):
+    """Single passes over the lowest, a constant and the highest digit, in one
+    sub-pass or two, at the edges of the pass's tile; the source stays as it was."""
+    r = np.random.default_rng(n)
+    keys = r.integers(0, 1 << 64, n, dtype=np.uint64) & ~np.uint64(0xFFFF0000) | np.uint64(0x5A5A0000)
+    a = _elems(keys)
+    last = 64 // bits - 1
+    for digit in (0, 16 // bits, last):
+        src = to_dev(a, cuda)
+        dst = cuda.empty_like(src)
+        ws = cuda.empty(lsb.pass_workspace_bytes(n, bits), dtype=cuda.uint8, device="cuda")
+        lsb.global_shuffle(src, dst, digit, bits, workspace=ws)
+        d = (keys >> np.uint64(bits * digit)) & np.uint64((1 << bits) - 1)
+        assert np.array_equal(to_np(dst), a[np.argsort(d, kind="stable")]), (n, bits, digit)
+        assert np.array_equal(to_np(src), a)
+        constant = int(len(np.unique(d)) == 1) if bits == 8 else 0
+        st = lsb.query(ws)
+        assert (st.device_status, st.skipped_mask, st.passes_run, st.n) == (0, constant, 1 - constant, n), (n, bits, digit)
