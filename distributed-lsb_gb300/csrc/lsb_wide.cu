@@ -378,8 +378,9 @@ __global__ void __launch_bounds__(256)
 // "pairs" of CTAs with two digits each (128 KiB, one CTA per SM) by default;
 // LSB_HIST16 selects "quads" (one digit each, 64 KiB, two CTAs per SM) or
 // "split" (a read per three digits). All give the same counts. Where a CTA
-// counts 2^17 keys or more its counters are stored and summed up by a second
-// kernel (scratch: they may come from the library's pool).
+// counts 2^14 keys or more its counters are stored and summed up by a second
+// kernel (scratch: they may come from the library's pool): 4 10^6 keys 74 -> 41
+// us; at 13000 keys per CTA both take 31.
 // 2^26 uniform keys, four digits (GB300): two reads with the flush by atomics
 // 628 us at 32 instructions per digit; this form 231 us at 20.
 static uint32_t hist16_group() {
@@ -395,13 +396,14 @@ static int hist16_launch(const Elem* data, uint32_t n, int first_digit, uint32_t
   const size_t smem = (size_t)ND * 65536u;
   static std::atomic<uint64_t> allowed;  // of this instance
   if (!allow_smem((const void*)k_hist16<ND>, smem, &allowed)) return 5;
-  // enough groups to fill every resident slot, none with less than a few rounds of work
-  const uint64_t least = 4u * kH16Threads * kH16Unroll;
+  // enough groups to fill every resident slot, none with less than a round of
+  // work (65537 keys 29 -> 19 us against groups of four rounds)
+  const uint64_t least = (uint64_t)kH16Threads * kH16Unroll;
   const uint64_t want = ((uint64_t)n + least - 1) / least;
   const uint64_t slots = std::max<uint64_t>(1, (uint64_t)dev.sm_count * (ND == 1 ? 2u : 1u) / group);
   const uint32_t groups = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(want, slots));
   void* dump = nullptr;
-  if (scratch && n / groups >= (1u << 17) && pool_alloc(&dump, (size_t)group * groups * smem, st) != 0) dump = nullptr;
+  if (scratch && n / groups >= (1u << 14) && pool_alloc(&dump, (size_t)group * groups * smem, st) != 0) dump = nullptr;
   {
     ProfScope prof("hist16", st);
     k_hist16<ND><<<group * groups, kH16Threads, smem, st>>>(data, n, first_digit, d_counts, group,

@@ -174,3 +174,15 @@ def test_one_digit(lsb, cuda, n, bits):
         constant = int(len(np.unique(d)) == 1) if bits == 8 else 0
         st = lsb.query(ws)
         assert (st.device_status, st.skipped_mask, st.passes_run, st.n) == (0, constant, 1 - constant, n), (n, bits, digit)
+
+
+@pytest.mark.parametrize("n", [8193, 16384 * 76 - 1, 16384 * 76, 3000001])
+def test_histogram_of_16_bits(lsb, cuda, n):
+    """Counters that go to the counts by atomics, and stored ones (from 2^14 keys
+    per pair of CTAs, at the edge on 152 SMs); one digit is constant, one heavy."""
+    r = np.random.default_rng(n)
+    keys = r.integers(0, 1 << 64, n, dtype=np.uint64) & ~np.uint64(0xFFFF0000) | np.uint64(0x12340000)
+    keys[r.random(n) < 0.5] &= np.uint64(0x0000FFFFFFFFFFFF)
+    h = lsb.histogram(to_dev(_elems(keys), cuda), 16).cpu().numpy().reshape(4, 65536)
+    for d in range(4):
+        assert np.array_equal(h[d], np.bincount((keys >> np.uint64(16 * d)) & np.uint64(0xFFFF), minlength=65536)), (n, d)
