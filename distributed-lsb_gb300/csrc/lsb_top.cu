@@ -606,7 +606,7 @@ int top_run(Elem* X, Elem* Y, unsigned char* ws, const Layout& L, cudaStream_t s
   // ms. Else even runs up to kSmallRun leave the small one half full or better,
   // with six standard deviations of room.
   const uint32_t least = passes_for((float)n, (float)kMeanRun);
-  const bool only_big = least == 2u && n <= 256u * kBigRun;
+  const bool only_big = least == 2u && n <= 256u * 7600u;  // runs of repeated keys vary more
   const bool may_big = n > (1u << 27) && n <= 65536u * kBigRun;
   const double even_run = (double)n / std::pow(256.0, (double)(only_big ? 1u : least));
   const bool small_tile = even_run <= (double)kSmallRun;
@@ -615,12 +615,19 @@ int top_run(Elem* X, Elem* Y, unsigned char* ws, const Layout& L, cudaStream_t s
   const uint32_t mean_run = only_big ? kBigRun : small_tile ? kSmallRun : kMeanRun;
   SampleRule rule = sample_rule(n, short_sample ? SampleTile<1>::kCap : SampleTile<kTopSample>::kCap, mean_run, mean_run,
                                 n <= (1u << 28) ? 16.0f : 4.0f);  // four passes for heavy keys up to 2^30 elements
+  // With so few windows most neighbours share one, and hardly more do when runs
+  // are twice as long, all for the merges (1.6 10^6 nearly sorted keys: 167 us, with
+  // a pass more 115): the limit is that of even runs, and three standard deviations.
+  if (only_big) {
+    const double lam = (double)kBigRun * SampleTile<1>::kCap / n, f = 1.0 - (1.0 - std::exp(-lam)) / lam;
+    rule.near_limit = (uint32_t)(SampleTile<1>::kCap * f + 3.0 * std::sqrt(SampleTile<1>::kCap * f * (1.0 - f)));
+  }
   // Unused launches cost about 2 us each: below 2^26 elements only the four
   // passes of heavy keys, or two more than even keys need, are kept ready, and
   // the merges, whose rounds then stay nearly in L2, take what those leave.
   if (n < (1u << 26)) rule.tmax = std::max(4u, std::min(8u, rule.tmin + 2u));
   if (may_big) {
-    const SampleRule wide = sample_rule(n, SampleTile<kTopSample>::kCap, kBigRun / 1.25f, kBigRun, 16.0f);
+    const SampleRule wide = sample_rule(n, SampleTile<kTopSample>::kCap, (uint32_t)(kBigRun / 1.25f), kBigRun, 16.0f);
     rule.big_tmin = 2u;
     rule.big_near = wide.near_limit;
   }
