@@ -192,7 +192,7 @@ int plan_layout(int64_t n, int bits, int num_digits, Layout* L, bool allow_split
     L->off_dstart = off;
     off = align_up(off + nbins * 4u, 256);
   }
-  L->total = off;  // the pass kernels' need, so that a workspace serves every route
+  L->total = off;  // the pass kernels' need, so that a workspace serves every route of this size
   if (whole_sort) {
     L->family = Family::kTop;
     L->stat_bits = bits;
@@ -208,7 +208,7 @@ int plan_layout(int64_t n, int bits, int num_digits, Layout* L, bool allow_split
     L->ring_tiles = std::max<uint32_t>(1u, (uint32_t)((n + L->tile_elems - 1) / L->tile_elems));
     L->off_ring = off;
     off = align_up(off + (size_t)L->ring_tiles * 256u * 8u, 256);
-    if ((uint64_t)n > 1u && (uint64_t)n <= mid_limit(dev)) off = std::max(off, mid_workspace_bytes((uint32_t)n, dev));
+    if (n > 1) off = std::max(off, mid_workspace_bytes((uint32_t)n, dev));
     L->total = std::max(L->total, off);
   }
   return 0;

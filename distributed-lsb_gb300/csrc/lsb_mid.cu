@@ -392,9 +392,13 @@ static uint32_t mid_items(uint32_t n, const DeviceInfo& dev) {
 static uint32_t mid_tiles(uint32_t n, uint32_t items) { return (n - 1u) / (items * (uint32_t)kMidThreads) + 1u; }
 static uint32_t mid_max_runs(uint32_t n) { return n / MidTile::kCap + 1u; }
 
-// Two count tables and the list of long runs, after the control block.
+// Two count tables and the list of long runs, after the control block: what any
+// size up to n needs, so that a workspace of the largest array serves the smaller
+// ones (the tiles double where they outnumber the SMs, and are then half as many).
 size_t mid_workspace_bytes(uint32_t n, const DeviceInfo& dev) {
-  return kCtrlBytes + (size_t)mid_tiles(n, mid_items(n, dev)) * 256u * 2u * 2u + (size_t)mid_max_runs(n) * sizeof(MidRun);
+  n = std::min(n, mid_limit(dev));
+  const uint32_t tiles = std::min(mid_tiles(n, 2u), (uint32_t)dev.sm_count);
+  return kCtrlBytes + (size_t)tiles * 256u * 2u * 2u + (size_t)mid_max_runs(n) * sizeof(MidRun);
 }
 
 // Up to 16 tiles of 2048 elements the grid is one cluster of 16 CTAs: no clear

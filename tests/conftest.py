@@ -67,3 +67,24 @@ def to_np(t) -> np.ndarray:
 
 def to_dev(a: np.ndarray, torch):
     return torch.from_numpy(np.ascontiguousarray(a).view(np.int64).copy()).cuda()
+
+
+@pytest.fixture(scope="session")
+def faked(lsb, tmp_path_factory):
+    """faked(code, **environment): runs Python code in a process of its own whose
+    CUDA runtime calls go through fake_cudart.c; returns what it printed."""
+    import subprocess
+
+    from lsb_gb300 import _build
+
+    so = str(tmp_path_factory.mktemp("fake") / "libfake_cudart.so")
+    subprocess.run(["gcc", "-shared", "-fPIC", "-O1", "-I" + os.path.join(_build._cuda_home(), "include"),
+                    os.path.join(ROOT, "tests", "fake_cudart.c"), "-o", so, "-ldl"], check=True)
+
+    def run(code, **env):
+        r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300, cwd=ROOT,
+                           env={**os.environ, "PYTHONPATH": PKG + os.pathsep + ROOT, "LD_PRELOAD": so, **env})
+        assert r.returncode == 0, r.stdout + r.stderr
+        return r.stdout
+
+    return run
