@@ -10,6 +10,8 @@
 #include <mutex>
 #include <vector>
 
+#include <cuda.h>
+
 #include "../../include/lsb.h"
 #include "lsb_internal.h"
 
@@ -83,6 +85,42 @@ bool allow_smem(const void* kern, size_t bytes, std::atomic<uint64_t>* done) {
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) return false;
   done->fetch_or(bit, std::memory_order_release);
   return true;
+}
+
+// A function of the driver, null where the driver has none of that name.
+static void* driver_function(const char* name, unsigned version) {
+  void* f = nullptr;
+  cudaDriverEntryPointQueryResult found = cudaDriverEntryPointSymbolNotFound;
+  if (cudaGetDriverEntryPointByVersion(name, &f, version, cudaEnableDefault, &found) != cudaSuccess) cudaGetLastError();
+  return found == cudaDriverEntryPointSuccess ? f : nullptr;
+}
+
+// The current context's number, which no later context gets again; 0: not known.
+static uint64_t context_id() {
+  static const auto id_of = reinterpret_cast<decltype(&cuCtxGetId)>(driver_function("cuCtxGetId", 12000));
+  unsigned long long id = 0;
+  return id_of && id_of(nullptr, &id) == CUDA_SUCCESS ? (uint64_t)id : 0u;
+}
+
+uint32_t stream_sms(cudaStream_t st, const DeviceInfo& dev) {
+  static const auto stream_green = reinterpret_cast<decltype(&cuStreamGetGreenCtx)>(driver_function("cuStreamGetGreenCtx", 12040));
+  static const auto green_resource = reinterpret_cast<decltype(&cuGreenCtxGetDevResource)>(driver_function("cuGreenCtxGetDevResource", 12040));
+  static const auto current = reinterpret_cast<decltype(&cuCtxGetCurrent)>(driver_function("cuCtxGetCurrent", 4000));
+  static const auto resource = reinterpret_cast<decltype(&cuCtxGetDevResource)>(driver_function("cuCtxGetDevResource", 12040));
+  CUdevResource r = {};
+  CUgreenCtx green = nullptr;
+  if (st && stream_green && green_resource && stream_green(st, &green) == CUDA_SUCCESS && green)
+    return green_resource(green, &r, CU_DEV_RESOURCE_TYPE_SM) == CUDA_SUCCESS ? r.sm.smCount : 0u;
+  // a context keeps its SMs; asking for them takes 0.3 us
+  static std::atomic<uint64_t> known;  // context number << 16 | SMs
+  const uint64_t id = context_id(), k = known.load(std::memory_order_relaxed);
+  if (id && k >> 16 == id) return (uint32_t)(k & 0xffffu);
+  CUcontext ctx = nullptr;
+  if (!current || !resource || current(&ctx) != CUDA_SUCCESS || !ctx ||
+      resource(ctx, &r, CU_DEV_RESOURCE_TYPE_SM) != CUDA_SUCCESS)
+    return (uint32_t)dev.sm_count;
+  if (id) known.store(id << 16 | r.sm.smCount, std::memory_order_relaxed);
+  return r.sm.smCount;
 }
 
 int pool_alloc(void** ptr, size_t bytes, cudaStream_t st) {

@@ -28,7 +28,7 @@ constexpr uint32_t kWhereLookback = 1;
 constexpr uint32_t kWhereRingReuse = 2;
 constexpr uint32_t kWhereScatter = 3;
 constexpr uint32_t kWhereBulkCopy = 6;   // a bulk copy's completion barrier
-constexpr uint32_t kWhereGridBarrier = 8;  // the grid barrier of the run merges
+constexpr uint32_t kWhereGridBarrier = 8;  // arrivals of other CTAs: a grid barrier, work items of a step before
 
 // Spin limit for every device-side wait: after this many polls (with a
 // nanosleep back-off of up to 256 ns each) the kernel records
@@ -56,7 +56,10 @@ struct TopPlan {
   uint32_t num_chunks;     // chunks of runs too long for a tile
   uint32_t num_runs;
   uint32_t max_rounds;     // merge rounds of the longest run
-  uint32_t barrier;        // arrivals at the merge kernel's grid barrier
+  uint32_t barrier;        // arrivals at a grid barrier
+  uint32_t merge_ticket;   // the run merges' work items: handed out,
+  uint32_t merge_done;     // and finished
+  uint32_t merge_any;      // a run is not in order
 };
 
 // Control block at the start of every workspace. Zeroed by
@@ -278,6 +281,19 @@ __device__ __forceinline__ bool wait_done_tag(const uint32_t* word, uint32_t wan
     got = acquire ? ld_acquire_u32(word) : ld_relaxed_u32(word);
   }
   return false;
+}
+
+// One thread: bounded wait until the count at `word` has reached `want`; false,
+// after recording kStatusTimeout, when it does not or an error is raised elsewhere.
+__device__ __forceinline__ bool wait_arrivals(const uint32_t* word, uint32_t want, Ctrl* ctrl) {
+  for (uint32_t it = 1; ld_acquire_u32(word) < want; it++) {
+    if (it >= kSpinLimit || ((it & 63u) == 0u && error_raised(ctrl))) {
+      record_error(ctrl, kStatusTimeout, kWhereGridBarrier);
+      return false;
+    }
+    if (it > 64u) __nanosleep(128);  // the first polls, some tens of microseconds, without a pause
+  }
+  return true;
 }
 
 // Bounded wait for phase `phase` of the barrier: false after kSpinLimit tries.

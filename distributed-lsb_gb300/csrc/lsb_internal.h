@@ -98,7 +98,10 @@ int top_run(Elem* X, Elem* Y, unsigned char* ws, const Layout& L, cudaStream_t s
 // two, from src into dst; where the layout has a look-back slot for every tile.
 bool top_pass_fits(const Layout& L);
 int top_pass_run(const Elem* src, Elem* mid, Elem* dst, int first_digit, unsigned char* ws, const Layout& L, cudaStream_t st);
-// Its one-launch form (lsb_mid.cu): largest array, workspace, launch.
+// Its one-launch form (lsb_mid.cu): largest array, workspace, launch. It needs
+// every CTA resident: kMidRefused, with nothing done, where the stream has not the
+// SMs for that or the launch is refused.
+constexpr int kMidRefused = -1;
 uint32_t mid_limit(const DeviceInfo& dev);
 size_t mid_workspace_bytes(uint32_t n, const DeviceInfo& dev);
 int mid_run(Elem* X, Elem* Y, unsigned char* ws, const Layout& L, const DeviceInfo& dev, cudaStream_t st);
@@ -178,6 +181,10 @@ int pool_alloc(void** ptr, size_t bytes, cudaStream_t st);
 // done (devices from 64 on ask every time); the attribute stays set, and asking
 // for it costs a microsecond of each call.
 bool allow_smem(const void* kern, size_t bytes, std::atomic<uint64_t>* done);
+
+// SMs that kernels on `st` can use: fewer than the device has on a stream of a
+// green context or in a context with a share of the SMs.
+uint32_t stream_sms(cudaStream_t st, const DeviceInfo& dev);
 
 // Host-buffer sort (lsb_host.cu): the number of chunks whose copies overlap
 // the sorts of earlier chunks (1 = copy in, sort, copy out), and the chunked

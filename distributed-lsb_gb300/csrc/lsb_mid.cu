@@ -452,13 +452,16 @@ int mid_run(Elem* X, Elem* Y, unsigned char* ws, const Layout& L, const DeviceIn
   SampleRule rule = sample_rule(n, SampleTile<kMidSample>::kCap, MidTile::kCap - 576u, MidTile::kMaxBin, 2048.0f);
   int bits = L.stat_bits, digits = L.stat_digits, api_bits = L.api_bits, sub = L.sub;
   void* args[] = {&X, &Y, &n, &rule, &table, &runs, &max_runs, &bits, &digits, &api_bits, &sub, &ctrl};
-  if (n <= kMidCluster * kMidClusterItems * (uint32_t)kMidThreads) {
+  const uint32_t sms = stream_sms(st, dev);
+  if (tiles > sms) return kMidRefused;
+  if (n <= kMidCluster * kMidClusterItems * (uint32_t)kMidThreads && sms == (uint32_t)dev.sm_count) {
     const void* kern = (const void*)k_mid_sort<(int)kMidClusterItems, true>;
     if (mid_cluster_fits(kern)) {
       cudaLaunchAttribute attr;
       const cudaLaunchConfig_t config = mid_cluster_config(&attr, st);
       ProfScope prof("mid_sort", st);
-      return cudaLaunchKernelExC(&config, kern, args) == cudaSuccess ? 0 : 5;
+      if (cudaLaunchKernelExC(&config, kern, args) == cudaSuccess) return 0;
+      cudaGetLastError();
     }
   }
   const void* kern = items == 2u   ? (const void*)k_mid_sort<2, false>
@@ -468,9 +471,11 @@ int mid_run(Elem* X, Elem* Y, unsigned char* ws, const Layout& L, const DeviceIn
   if (!allow_smem(kern, kMidSmem, &allowed[items >> 2]) || cudaMemsetAsync(ws, 0, kCtrlBytes, st) != cudaSuccess)
     return 5;
   // CTAs beyond the tiles take a share of the runs
-  const uint32_t grid = std::min<uint32_t>((uint32_t)dev.sm_count, std::max(tiles, (n - 1u) / 2048u + 1u));
+  const uint32_t grid = std::min<uint32_t>(sms, std::max(tiles, (n - 1u) / 2048u + 1u));
   ProfScope prof("mid_sort", st);
-  return cudaLaunchCooperativeKernel(kern, dim3(grid), dim3(kMidThreads), args, kMidSmem, st) == cudaSuccess ? 0 : 5;
+  if (cudaLaunchCooperativeKernel(kern, dim3(grid), dim3(kMidThreads), args, kMidSmem, st) == cudaSuccess) return 0;
+  cudaGetLastError();
+  return kMidRefused;
 }
 
 }  // namespace lsb

@@ -410,8 +410,12 @@ __device__ __forceinline__ uint32_t merge_split(const Elem* a, uint32_t la, cons
 // Runs that do not fit in a tile. Usual keys leave none and the kernel returns
 // at once. Heavy keys do: one key fills the run, it is in order and only read
 // (or copied into X). The rest is sorted by chunks of a tile and pairwise
-// stable merges, all CTAs on one round at a time. A cooperative launch: the
-// grid barrier needs every CTA resident.
+// stable merges. Step 0 checks, step 1 sorts the chunks, step 2 + r is round r of
+// the merges; an item of work is a few chunks' share of a step, and the items of all
+// steps are handed out in order by one ticket. An item waits until the steps before its own
+// are finished. Whoever has those items is running and waits for earlier ones
+// only, so no CTA needs another one to be resident, and the stream may own fewer
+// SMs than the device has.
 __global__ void __launch_bounds__(Tile::kThreads, 2)
     k_top_merge(Elem* X, Elem* Y, uint32_t n, const RunChunk* __restrict__ chunks, uint32_t* unsorted, Ctrl* ctrl) {
   constexpr int K = Tile::kItems, THREADS = Tile::kThreads;
@@ -419,99 +423,115 @@ __global__ void __launch_bounds__(Tile::kThreads, 2)
   if (total == 0u || error_raised(ctrl)) return;
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ typename Tile::Shared sh;
-  __shared__ uint32_t s_split[2];
+  __shared__ uint32_t s_split[2], s_item;
+  __shared__ bool s_go;
   Elem* in = reinterpret_cast<Elem*>(smem);
   uint32_t* slot = reinterpret_cast<uint32_t*>(smem + Tile::kElemBytes);
   uint32_t* bins = reinterpret_cast<uint32_t*>(smem + Tile::kElemBytes + Tile::kSlotBytes);
   const uint32_t tid = threadIdx.x, warp = tid >> 5;
-  const uint32_t rounds = ctrl->top.max_rounds;
-  uint32_t barriers = 0;
-  // runs in order stay (or are copied); the others are marked. Each warp reads
-  // its part of a chunk and the element after it, nine loads at a time.
-  for (uint32_t c = blockIdx.x; c < total; c += gridDim.x) {
-    const RunChunk t = chunks[c];
-    const Elem* run = (t.par ? Y : X) + t.b;
-    const uint32_t len = t.e - t.b, at = t.k * kCap + warp * 32u * K;
-    const uint32_t m = min(len - t.k * kCap, kCap);  // the chunk's
-    Elem e[K];
-#pragma unroll
-    for (int k = 0; k < K; k++) e[k] = load_elem_stream(run + min(at + (uint32_t)k * 32u + lane_id(), len - 1u));
-    const uint64_t after = at + 32u * K < len ? run[at + 32u * K].key : ~0ull;
-    bool inversion = false;
-#pragma unroll
-    for (int k = 0; k < K; k++) {
-      uint64_t next = __shfl_down_sync(0xffffffffu, e[k].key, 1);
-      const uint64_t head = k + 1 < K ? __shfl_sync(0xffffffffu, e[k + 1 < K ? k + 1 : k].key, 0) : after;
-      if (lane_id() == 31) next = head;
-      inversion |= e[k].key > next;
-      const uint32_t i = warp * 32u * K + (uint32_t)k * 32u + lane_id();
-      if (t.par && i < m) store_elem(X + t.b + t.k * kCap + i, e[k]);
-    }
-    if (__any_sync(0xffffffffu, inversion) && lane_id() == 0) unsorted[t.run] = 1u;
-  }
-  if (!grid_barrier(ctrl, &barriers)) return;
+  const uint32_t steps = 2u + ctrl->top.max_rounds;
+  // eight items for each CTA: an item costs a trip to the ticket and two barriers
+  // (2^28 Zipf keys, 58000 chunks in order: 11.2 ms the sort with an item per chunk, 10.0 so)
+  const uint32_t per = total / (gridDim.x * 8u) + 1u, items = (total - 1u) / per + 1u;
   auto rounds_of = [](const RunChunk& t) { return 32u - (uint32_t)__clz((int)((t.e - t.b - 1u) / kCap)); };
-  // chunks, each into the buffer from which the merges end in X
-  bool any = false;
-  for (uint32_t c = blockIdx.x; c < total; c += gridDim.x) {
-    const RunChunk t = chunks[c];
-    if (!ld_relaxed_u32(unsorted + t.run)) continue;
-    any = true;
-    const uint32_t lo = t.b + t.k * kCap, m = min(t.e - lo, kCap);
-    const Elem* src = t.par ? Y : X;
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < K; k++) {
-      const uint32_t i = tid + (uint32_t)k * THREADS;
-      if (i < m) in[i] = load_elem_l2(src + lo + i);
+  uint32_t step_now = 0;
+  if (tid == 0) s_item = atomicAdd(&ctrl->top.merge_ticket, 1u);
+  __syncthreads();
+  for (;;) {
+    const uint32_t item = s_item, step = item / items;
+    if (step >= steps) return;
+    if (step != step_now) {
+      if (tid == 0) {
+        // when the check has found nothing to merge, every later step is left out
+        bool go = step_now != 0u || (wait_arrivals(&ctrl->top.merge_done, items, ctrl) &&
+                                     ld_relaxed_u32(&ctrl->top.merge_any) != 0u);
+        go = go && wait_arrivals(&ctrl->top.merge_done, step * items, ctrl);
+        __threadfence();
+        s_go = go;
+      }
+      __syncthreads();
+      if (!s_go) return;
+      step_now = step;
     }
-    __syncthreads();
-    Elem* out = ((rounds_of(t) & 1u) ? Y : X) + lo;
-    Tile::sort(in, 0, m, 0, 0, slot, bins, sh, out == src + lo,
-               [&](bool on, uint32_t r, const Elem& e) { store_elem_if(on, out + r, e); });
-  }
-  // no run to merge anywhere: the marks are the same for every CTA
-  if (!any) {
-    for (uint32_t c = tid; c < total; c += THREADS) any |= ld_relaxed_u32(unsorted + chunks[c].run) != 0u;
-  }
-  if (!__syncthreads_or(any)) return;
-  if (!grid_barrier(ctrl, &barriers)) return;
-  for (uint32_t r = 0; r < rounds; r++) {
-    for (uint32_t c = blockIdx.x; c < total; c += gridDim.x) {
+    for (uint32_t c = item % items * per; c < min(total, (item % items + 1u) * per); c++) {
       const RunChunk t = chunks[c];
-      const uint32_t mine = rounds_of(t);
-      if (r >= mine || !ld_relaxed_u32(unsorted + t.run)) continue;
-      const Elem* from = (((mine - r) & 1u) ? Y : X) + t.b;
-      Elem* to = (((mine - r) & 1u) ? X : Y) + t.b;
       const uint32_t len = t.e - t.b, pos = t.k * kCap, cnt = min(kCap, len - pos);
-      const uint64_t half = (uint64_t)kCap << r;
-      const uint32_t base = (uint32_t)(pos / (2u * half) * (2u * half));
-      const uint32_t la = (uint32_t)min(half, (uint64_t)(len - base));
-      const uint32_t lb = (uint32_t)min(half, (uint64_t)(len - base - la));
-      const Elem* a = from + base;
-      const Elem* b = a + la;
-      const uint32_t d0 = pos - base, d1 = d0 + cnt;
-      __syncthreads();
-      if (warp < 2) {
-        const uint32_t i = merge_split(a, la, b, lb, warp ? d1 : d0);
-        if (lane_id() == 0) s_split[warp] = i;
-      }
-      __syncthreads();
-      const uint32_t i0 = s_split[0], na = s_split[1] - i0, j0 = d0 - i0;
+      if (step == 0u) {
+        // runs in order stay (or are copied); the others are marked. Each warp reads
+        // its part of a chunk and the element after it, nine loads at a time.
+        const Elem* run = (t.par ? Y : X) + t.b;
+        const uint32_t at = pos + warp * 32u * K;
+        Elem e[K];
 #pragma unroll
-      for (int k = 0; k < K; k++) {
-        const uint32_t i = tid + (uint32_t)k * THREADS;
-        if (i < cnt) in[i] = load_elem_l2(i < na ? a + i0 + i : b + j0 + (i - na));
+        for (int k = 0; k < K; k++) e[k] = load_elem_stream(run + min(at + (uint32_t)k * 32u + lane_id(), len - 1u));
+        const uint64_t after = at + 32u * K < len ? run[at + 32u * K].key : ~0ull;
+        bool inversion = false;
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+          uint64_t next = __shfl_down_sync(0xffffffffu, e[k].key, 1);
+          const uint64_t head = k + 1 < K ? __shfl_sync(0xffffffffu, e[k + 1 < K ? k + 1 : k].key, 0) : after;
+          if (lane_id() == 31) next = head;
+          inversion |= e[k].key > next;
+          const uint32_t i = warp * 32u * K + (uint32_t)k * 32u + lane_id();
+          if (t.par && i < cnt) store_elem(X + t.b + pos + i, e[k]);
+        }
+        if (__any_sync(0xffffffffu, inversion) && lane_id() == 0) {
+          unsorted[t.run] = 1u;
+          ctrl->top.merge_any = 1u;
+        }
+      } else if (ld_relaxed_u32(unsorted + t.run)) {
+        if (step == 1u) {  // a chunk, into the buffer from which the merges end in X
+          const Elem* src = (t.par ? Y : X) + t.b + pos;
+          __syncthreads();
+#pragma unroll
+          for (int k = 0; k < K; k++) {
+            const uint32_t i = tid + (uint32_t)k * THREADS;
+            if (i < cnt) in[i] = load_elem_l2(src + i);
+          }
+          __syncthreads();
+          Elem* out = ((rounds_of(t) & 1u) ? Y : X) + t.b + pos;
+          Tile::sort(in, 0, cnt, 0, 0, slot, bins, sh, out == src,
+                     [&](bool on, uint32_t r, const Elem& e) { store_elem_if(on, out + r, e); });
+        } else if (const uint32_t r = step - 2u, mine = rounds_of(t); r < mine) {
+          const Elem* from = (((mine - r) & 1u) ? Y : X) + t.b;
+          Elem* to = (((mine - r) & 1u) ? X : Y) + t.b;
+          const uint64_t half = (uint64_t)kCap << r;
+          const uint32_t base = (uint32_t)(pos / (2u * half) * (2u * half));
+          const uint32_t la = (uint32_t)min(half, (uint64_t)(len - base));
+          const uint32_t lb = (uint32_t)min(half, (uint64_t)(len - base - la));
+          const Elem* a = from + base;
+          const Elem* b = a + la;
+          const uint32_t d0 = pos - base, d1 = d0 + cnt;
+          __syncthreads();
+          if (warp < 2) {
+            const uint32_t i = merge_split(a, la, b, lb, warp ? d1 : d0);
+            if (lane_id() == 0) s_split[warp] = i;
+          }
+          __syncthreads();
+          const uint32_t i0 = s_split[0], na = s_split[1] - i0, j0 = d0 - i0;
+#pragma unroll
+          for (int k = 0; k < K; k++) {
+            const uint32_t i = tid + (uint32_t)k * THREADS;
+            if (i < cnt) in[i] = load_elem_l2(i < na ? a + i0 + i : b + j0 + (i - na));
+          }
+          uint16_t* id = reinterpret_cast<uint16_t*>(slot);
+          uint16_t* order = id + kCap;
+          for (uint32_t i = tid; i < cnt; i += THREADS) id[i] = (uint16_t)i;
+          __syncthreads();
+          Tile::merge_parts(in, id, order, na, cnt - na);
+          __syncthreads();
+          for (uint32_t i = tid; i < cnt; i += THREADS) store_elem(to + pos + i, in[order[i]]);
+        }
       }
-      uint16_t* id = reinterpret_cast<uint16_t*>(slot);
-      uint16_t* order = id + kCap;
-      for (uint32_t i = tid; i < cnt; i += THREADS) id[i] = (uint16_t)i;
-      __syncthreads();
-      Tile::merge_parts(in, id, order, na, cnt - na);
-      __syncthreads();
-      for (uint32_t i = tid; i < cnt; i += THREADS) store_elem(to + pos + i, in[order[i]]);
     }
-    if (!grid_barrier(ctrl, &barriers)) return;
+    __syncthreads();
+    if (tid == 0) {
+      __threadfence();
+      atomicAdd(&ctrl->top.merge_done, 1u);
+      // not sooner: a CTA would hold two items of a step while others have none
+      s_item = atomicAdd(&ctrl->top.merge_ticket, 1u);
+    }
+    __syncthreads();
   }
 }
 
@@ -521,13 +541,9 @@ int top_merge(Elem* X, Elem* Y, uint32_t n, RunChunk* chunks, uint32_t* unsorted
               cudaStream_t st) {
   static std::atomic<uint64_t> allowed;
   if (!allow_smem((const void*)k_top_merge, Tile::kSmem, &allowed)) return 5;
-  const RunChunk* list = chunks;
-  void* args[] = {&X, &Y, &n, &list, &unsorted, &ctrl};
   ProfScope prof("top_merge", st);
-  return cudaLaunchCooperativeKernel((const void*)k_top_merge, dim3((uint32_t)dev.sm_count * 2u), dim3(Tile::kThreads),
-                                     args, Tile::kSmem, st) == cudaSuccess
-             ? 0
-             : 5;
+  k_top_merge<<<(uint32_t)dev.sm_count * 2u, Tile::kThreads, Tile::kSmem, st>>>(X, Y, n, chunks, unsorted, ctrl);
+  return cudaPeekAtLastError() == cudaSuccess ? 0 : 5;
 }
 
 // ---------------------------------------------------------------------------
@@ -594,7 +610,10 @@ int top_run(Elem* X, Elem* Y, unsigned char* ws, const Layout& L, cudaStream_t s
   if (n <= SmallFull::kCap) return small_sort<1024>(X, L, ctrl, st);
   DeviceInfo dev;
   if (int rc = current_device_info(&dev)) return rc;
-  if (n <= mid_limit(dev)) return mid_run(X, Y, ws, L, dev, st);
+  if (n <= mid_limit(dev)) {
+    const int rc = mid_run(X, Y, ws, L, dev, st);
+    if (rc != kMidRefused) return rc;
+  }
   uint32_t* hist = reinterpret_cast<uint32_t*>(ws + L.off_hist);
   uint32_t* gstart = reinterpret_cast<uint32_t*>(ws + L.off_gstart);
   uint64_t* ring = reinterpret_cast<uint64_t*>(ws + L.off_ring);

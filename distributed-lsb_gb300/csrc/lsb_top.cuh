@@ -438,19 +438,8 @@ __device__ __forceinline__ bool grid_barrier(Ctrl* ctrl, uint32_t* round) {
   if (threadIdx.x == 0) {
     __threadfence();
     atomicAdd(&ctrl->top.barrier, 1u);
-    const uint32_t want = *round * gridDim.x;
-    uint32_t it = 0;
-    bool ok = true;
-    while (ld_acquire_u32(&ctrl->top.barrier) < want) {
-      if (++it >= kSpinLimit || ((it & 63u) == 0u && error_raised(ctrl))) {
-        record_error(ctrl, kStatusTimeout, kWhereGridBarrier);
-        ok = false;
-        break;
-      }
-      if (it > 64u) __nanosleep(128);  // the first polls, some tens of microseconds, without a pause
-    }
+    s_ok = wait_arrivals(&ctrl->top.barrier, *round * gridDim.x, ctrl);
     __threadfence();
-    s_ok = ok;
   }
   __syncthreads();
   return s_ok;

@@ -10,7 +10,13 @@
 
 static int refuse(void) { return getenv("FAKE_REFUSE") != NULL; }
 static int sms(void) { return getenv("FAKE_SMS") ? atoi(getenv("FAKE_SMS")) : 0; }
-#define REAL(name) ((__typeof__(&name))dlsym(RTLD_NEXT, #name))
+/* the runtime that the library has loaded, which is not in the global scope */
+static void* real(const char* name) {
+  static void* rt;
+  if (!rt) rt = dlopen("libcudart.so.13", RTLD_LAZY);
+  return dlsym(rt, name);
+}
+#define REAL(name) ((__typeof__(&name))real(#name))
 
 cudaError_t cudaLaunchCooperativeKernel(const void* f, dim3 g, dim3 b, void** a, size_t s, cudaStream_t st) {
   return refuse() ? cudaErrorCooperativeLaunchTooLarge : REAL(cudaLaunchCooperativeKernel)(f, g, b, a, s, st);
