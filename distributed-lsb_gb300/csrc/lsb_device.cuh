@@ -302,6 +302,15 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t phase) 
     if (mbar_try_wait(bar, phase)) return true;
   return false;
 }
+// The same for bulk copies that complete on the barrier: false, with kStatusTimeout
+// recorded, when the wait ran out. Copies still in flight are then waited for a
+// second time, so that none lands in the CTA's shared memory after it has left.
+__device__ __forceinline__ bool wait_copies(uint32_t bar, uint32_t phase, Ctrl* ctrl) {
+  if (mbar_wait_bounded(bar, phase)) return true;
+  record_error(ctrl, kStatusTimeout, kWhereBulkCopy);
+  mbar_wait_bounded(bar, phase);
+  return false;
+}
 __device__ __forceinline__ Elem lds_elem(const Elem* p) {
   Elem e;
   asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];" : "=l"(e.key), "=l"(e.val) : "r"(smem_u32(p)));

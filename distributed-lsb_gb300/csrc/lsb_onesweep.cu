@@ -1454,16 +1454,26 @@ __global__ void k_selftest_ring_slot(Ctrl* ctrl, uint32_t* done) {
   (void)wait_done_tag(done, ring_tag(0, 1u), ld_relaxed_u32(done), false, ctrl);
 }
 
-// a bulk copy's completion barrier: 16 bytes are expected that no copy
-// delivers, so the barrier's phase never completes
+// a bulk copy's completion barrier: the copy of its 16 bytes is started only when
+// the wait for it has run out, and must still have landed when the waiter leaves
 __global__ void k_selftest_bulk_copy(Ctrl* ctrl) {
   __shared__ __align__(8) uint64_t s_bar;
-  if (threadIdx.x != 0) return;
+  __shared__ __align__(16) Elem s_elem;
   const uint32_t bar = smem_u32(&s_bar);
-  mbar_init(bar, 1);
-  fence_mbar_init();
-  mbar_arrive_expect_tx(bar, 16u);
-  if (!mbar_wait_bounded(bar, 0u)) record_error(ctrl, kStatusTimeout, kWhereBulkCopy);
+  if (threadIdx.x == 0) {
+    mbar_init(bar, 1);
+    fence_mbar_init();
+    mbar_arrive_expect_tx(bar, (uint32_t)sizeof(Elem));
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    if (wait_copies(bar, 0u, ctrl) || !mbar_try_wait(bar, 0u)) ctrl->error = kStatusInconsistent;
+  } else if (threadIdx.x == 32) {
+    for (uint32_t it = 0; it < 16u * kSpinLimit && !error_raised(ctrl); it++) __nanosleep(256);
+    bulk_g2s(smem_u32(&s_elem), ctrl, (uint32_t)sizeof(Elem), bar);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) mbar_wait_bounded(bar, 0u);
 }
 
 int selftest_ring_slot(unsigned char* ws, cudaStream_t st) {
@@ -1473,7 +1483,7 @@ int selftest_ring_slot(unsigned char* ws, cudaStream_t st) {
 }
 
 int selftest_bulk_copy(unsigned char* ws, cudaStream_t st) {
-  k_selftest_bulk_copy<<<1, 32, 0, st>>>(reinterpret_cast<Ctrl*>(ws));
+  k_selftest_bulk_copy<<<1, 64, 0, st>>>(reinterpret_cast<Ctrl*>(ws));
   return cudaPeekAtLastError() == cudaSuccess ? 0 : 5;
 }
 

@@ -420,9 +420,8 @@ __device__ __forceinline__ bool load_tile_bulk(Elem* in, const Elem* src, uint32
     for (uint32_t o = 0; o < cnt; o += 2048u)
       bulk_g2s(smem_u32(in + o), src + o, min(2048u, cnt - o) * (uint32_t)sizeof(Elem), bar);
   }
-  const bool ok = mbar_wait_bounded(bar, *phase);
+  const bool ok = wait_copies(bar, *phase, ctrl);
   *phase ^= 1u;
-  if (!ok) record_error(ctrl, kStatusTimeout, kWhereBulkCopy);
   return !__syncthreads_or(!ok);
 }
 
