@@ -736,10 +736,10 @@ int lsb_profile_enable(int on) {
 }
 
 int lsb_selftest_wait(int which, void* stream, int* device_status) {
-  if (!device_status || which < LSB_WAIT_LOOKBACK || which > LSB_WAIT_SCHEDULER)
+  if (!device_status || which < LSB_WAIT_LOOKBACK || which > LSB_WAIT_ARRIVALS)
     return LSB_ERR_INVALID_ARG;
   cudaStream_t st = (cudaStream_t)stream;
-  const bool wide = which >= LSB_WAIT_BUCKET_PREFIX;
+  const bool wide = which >= LSB_WAIT_BUCKET_PREFIX && which <= LSB_WAIT_SCHEDULER;
   const size_t bytes = wide ? lsb::selftest_wide_bytes() : kCtrlBytes + 32u;
   void* ws = nullptr;
   if (int rc = pool_alloc(&ws, bytes, st)) return rc;
@@ -753,6 +753,7 @@ int lsb_selftest_wait(int which, void* stream, int* device_status) {
       case LSB_WAIT_LOOKBACK: r = lsb::selftest_lookback_timeout(w, st); break;
       case LSB_WAIT_RING_SLOT: r = lsb::selftest_ring_slot(w, st); break;
       case LSB_WAIT_BULK_COPY: r = lsb::selftest_bulk_copy(w, st); break;
+      case LSB_WAIT_ARRIVALS: r = lsb::selftest_arrivals(w, st); break;
       default: r = lsb::selftest_wide_wait(which - LSB_WAIT_BUCKET_PREFIX, w, st); break;
     }
     if (r != 0 || cudaMemcpyAsync(&c, ws, sizeof c, cudaMemcpyDeviceToHost, st) != cudaSuccess)

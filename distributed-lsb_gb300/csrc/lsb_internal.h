@@ -145,12 +145,13 @@ uint32_t onesweep_tile_elems(int bits);
 // the look-back wait of the sort kernels on a predecessor that never publishes
 // (failure-detection self-test); ws: kCtrlBytes + 32 bytes, zeroed by the caller
 int selftest_lookback_timeout(unsigned char* ws, cudaStream_t st);
-// the same for the ring-slot reuse wait and a bulk copy's completion barrier
-// (ws: kCtrlBytes + 32 bytes, zeroed), and for the 16-bit pass's waits
+// the same for the ring-slot reuse wait, a bulk copy's completion barrier and the
+// arrivals of other CTAs (ws: kCtrlBytes + 32 bytes, zeroed), and for the 16-bit pass's waits
 // (which: 0 bucket prefix, 1 bucket look-back, 2 scheduler; ws:
 // selftest_wide_bytes(), zeroed)
 int selftest_ring_slot(unsigned char* ws, cudaStream_t st);
 int selftest_bulk_copy(unsigned char* ws, cudaStream_t st);
+int selftest_arrivals(unsigned char* ws, cudaStream_t st);
 size_t selftest_wide_bytes();
 int selftest_wide_wait(int which, unsigned char* ws, cudaStream_t st);
 uint32_t onesweep_grid(int bits, const DeviceInfo& dev, uint32_t n);

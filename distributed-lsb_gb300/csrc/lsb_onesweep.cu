@@ -1476,6 +1476,18 @@ __global__ void k_selftest_bulk_copy(Ctrl* ctrl) {
   if (threadIdx.x == 0) mbar_wait_bounded(bar, 0u);
 }
 
+// arrivals of other CTAs: one of two comes
+__global__ void k_selftest_arrivals(Ctrl* ctrl) {
+  if (threadIdx.x != 0) return;
+  atomicAdd(&ctrl->top.barrier, 1u);
+  (void)wait_arrivals(&ctrl->top.barrier, 2u, ctrl);
+}
+
+int selftest_arrivals(unsigned char* ws, cudaStream_t st) {
+  k_selftest_arrivals<<<1, 32, 0, st>>>(reinterpret_cast<Ctrl*>(ws));
+  return cudaPeekAtLastError() == cudaSuccess ? 0 : 5;
+}
+
 int selftest_ring_slot(unsigned char* ws, cudaStream_t st) {
   Ctrl* ctrl = reinterpret_cast<Ctrl*>(ws);
   k_selftest_ring_slot<<<1, 32, 0, st>>>(ctrl, reinterpret_cast<uint32_t*>(ws + kCtrlBytes));

@@ -457,8 +457,9 @@ def selftest_wait_timeout(stream=None) -> int:
 
 WAIT_LOOKBACK, WAIT_RING_SLOT, WAIT_BULK_COPY = 0, 1, 2
 WAIT_BUCKET_PREFIX, WAIT_BUCKET_LOOKBACK, WAIT_SCHEDULER = 3, 4, 5
+WAIT_ARRIVALS = 6
 WAITS = {"lookback": 0, "ring_slot": 1, "bulk_copy": 2, "bucket_prefix": 3, "bucket_lookback": 4,
-         "scheduler": 5}
+         "scheduler": 5, "arrivals": 6}
 
 
 def selftest_wait(which: int, stream=None) -> int:

@@ -372,8 +372,10 @@ enum lsb_wait {
   LSB_WAIT_BULK_COPY = 2,       /* a bulk copy's completion barrier that no copy completes */
   LSB_WAIT_BUCKET_PREFIX = 3,   /* 16-bit pass: a bucket's running prefix an earlier chunk never hands on */
   LSB_WAIT_BUCKET_LOOKBACK = 4, /* 16-bit pass: look-back among one bucket's tiles, predecessor silent */
-  LSB_WAIT_SCHEDULER = 5        /* 16-bit pass itself: no runnable work ever appears (a chunk plan
+  LSB_WAIT_SCHEDULER = 5,       /* 16-bit pass itself: no runnable work ever appears (a chunk plan
                                    nobody publishes) */
+  LSB_WAIT_ARRIVALS = 6         /* whole sorts: other CTAs' arrivals (a grid barrier, the work of a
+                                   step before) that stay below the count */
 };
 int lsb_selftest_wait(int which, void* stream, int* device_status);
 

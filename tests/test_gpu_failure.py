@@ -30,6 +30,16 @@ def test_lookback_wait_runs_out_and_reports(lsb, cuda, oracle):
     assert np.array_equal(to_np(A), oracle.stable_sort_by_key(a))
 
 
+def test_arrivals_wait_runs_out_and_reports(lsb, cuda, oracle):
+    """The grid barrier of the one-launch sort and the run merges' wait for the
+    work of a step before: one arrival of two comes."""
+    assert lsb.selftest_wait(lsb.WAIT_ARRIVALS) == lsb.LSB_ERR_DEVICE_TIMEOUT
+    a = oracle.generate(100003, oracle.DIST_ZIPF, 79)
+    A = to_dev(a, cuda)
+    lsb.sort_pairs(A, cuda.empty_like(A), 16)
+    assert np.array_equal(to_np(A), oracle.stable_sort_by_key(a))
+
+
 @pytest.mark.parametrize("which", ["ring_slot", "bulk_copy", "bucket_prefix", "bucket_lookback", "scheduler"])
 def test_every_bounded_wait_runs_out_and_reports(lsb, cuda, oracle, which):
     t0 = time.perf_counter()
