@@ -30,7 +30,8 @@ constexpr uint32_t kWhereScatter = 3;
 constexpr uint32_t kWhereBulkCopy = 6;   // a bulk copy's completion barrier
 constexpr uint32_t kWhereGridBarrier = 8;  // arrivals of other CTAs: a grid barrier, work items of a step before
 
-// Spin limit for every device-side wait: after this many polls (with a
+// Spin limit for every device-side wait but the barrier of a cluster of CTAs, which is
+// the hardware's: after this many polls (with a
 // nanosleep back-off of up to 256 ns each) the kernel records
 // kStatusTimeout, skips its stores and returns, so no wait can hang the GPU.
 constexpr uint32_t kSpinLimit = 1u << 22;
@@ -49,9 +50,10 @@ struct TopPlan {
   uint32_t run_mask;       // bit p: pass p runs (its digit is not constant)
   uint32_t par_mask;       // bit p: pass p reads Y, writes X
   uint32_t src_parity;     // 1: the passes leave the data in Y
-  uint32_t skewed;         // heavy keys: tiles of runs are mostly in order
+  uint32_t skewed;         // bit 0: heavy keys, tiles of runs are mostly in order; bit 1: most keys are duplicates
   uint32_t complete;       // the digits cover every bit in which keys differ
   uint32_t diff[2];        // bits in which some key differs from the first one
+  uint32_t apart[2];       // and from one key that agrees with it in the top window
   uint32_t hist_done;      // CTAs of the histogram that have finished
   uint32_t num_chunks;     // chunks of runs too long for a tile
   uint32_t num_runs;
@@ -60,10 +62,11 @@ struct TopPlan {
   uint32_t merge_ticket;   // the run merges' work items: handed out,
   uint32_t merge_done;     // and finished
   uint32_t merge_any;      // a run is not in order
+  uint32_t pass_done[8];   // tiles placed by the passes that share a launch
 };
 
-// Control block at the start of every workspace. Zeroed by
-// the host before each sort or pass; written only by the kernels after that.
+// Control block at the start of every workspace. Zeroed before each sort or pass, by
+// the host or by the first kernel; written only by the kernels after that.
 struct Ctrl {
   uint32_t error;                  // kStatusOk or kStatusTimeout (first error wins)
   uint32_t err_where;              // kWhere* of the first error
@@ -168,6 +171,12 @@ __device__ __forceinline__ Elem load_elem_stream(const Elem* p) {
   Elem e;
   e.key = v.x;
   e.val = v.y;
+  return e;
+}
+
+__device__ __forceinline__ Elem load_elem_l2(const Elem* p) {
+  Elem e;  // L2 only: another CTA has written it since this kernel began
+  asm volatile("ld.global.cg.v2.u64 {%0, %1}, [%2];" : "=l"(e.key), "=l"(e.val) : "l"(p) : "memory");
   return e;
 }
 

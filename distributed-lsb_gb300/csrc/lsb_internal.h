@@ -13,7 +13,8 @@
 //    is sorted there in one launch (lsb_top.cu); a larger one by its top digits
 //    only, as many passes as it takes until the runs of equal windows fit, and
 //    then run by run in shared memory: in one cooperative launch while every
-//    tile has a CTA of its own (lsb_mid.cu), else pass by pass (lsb_top.cu).
+//    tile has a CTA of its own on the stream's SMs (lsb_mid.cu), else pass by pass
+//    (lsb_top.cu).
 //  * "task" family (digit_bits >= 12, the reference's 16-bit digits): per pass
 //    a count kernel over contiguous tasks, a digit-major scan of the
 //    [digit][task] count table and a stable scatter -- the reference's own
@@ -109,11 +110,13 @@ int mid_run(Elem* X, Elem* Y, unsigned char* ws, const Layout& L, const DeviceIn
 // 0: 512 threads x 16, 1 CTA/SM; 2: 256 x 16, 2 CTAs/SM.
 uint32_t onesweep_top_tile(int variant);
 // Pass `pass` of the plan in ctrl->top, or of a batch's plans; gstart: that
-// pass's digit starts (one array); ctas: persistent CTAs, 0 = every resident slot. spare: one that even
-// keys do not need, under its own name in the launch times.
+// pass's digit starts (one array); ctas: persistent CTAs, 0 = every resident slot.
 int onesweep_top_pass(Elem* X, Elem* Y, uint32_t n, int pass, const uint32_t* gstart, uint64_t* ring,
-                      uint32_t tiles, Ctrl* ctrl, const SegDesc& seg, int variant, uint32_t ctas, bool spare,
+                      uint32_t tiles, Ctrl* ctrl, const SegDesc& seg, int variant, uint32_t ctas,
                       const DeviceInfo& dev, cudaStream_t st);
+// Every pass from `first` on that the plan has, in one launch; gstart: pass 0's.
+int onesweep_top_rest(Elem* X, Elem* Y, uint32_t n, int first, const uint32_t* gstart, uint64_t* ring, uint32_t tiles,
+                      Ctrl* ctrl, const SegDesc& seg, int variant, uint32_t ctas, const DeviceInfo& dev, cudaStream_t st);
 // The merges of runs longer than a tile (lsb_top.cu): list of chunks and marks
 // of their runs, at most top_list_bytes(n) together.
 struct RunChunk;

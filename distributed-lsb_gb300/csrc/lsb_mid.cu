@@ -14,81 +14,177 @@
 //   3. the totals are the exact lengths of the runs that one pass over the top
 //      digit leaves. If all fit in a tile, that one pass is made and the runs
 //      are sorted on chip. Otherwise a sample (the same in every CTA) says
-//      which digits to pass over, lowest first;
+//      which digits to pass over, lowest first: digits of bits that vary, and not
+//      those that the top digit tells (of signs, tags, sentinels), which is checked
+//      against every key (signed 8-bit numbers, 1.1 10^6: 152 us in eight passes,
+//      73 in two);
 //   4. runs longer than a tile that are not in order after that (the sample
 //      missed them) have the array passed over by every digit that differs.
 // Bound by latency: about four grid barriers and as many trips to L2. Measured
-// (GB300, sort alone, eight launched passes -> this): 10^4 uniform keys 131 ->
-// 25 us, 10^5 153 -> 28, 10^6 153 -> 42; Zipf keys (four digits) 10^5 153 -> 79,
-// 10^6 155 -> 139. The tile
+// (GB300, sort alone, eight launched passes -> this): 2 10^4 uniform keys 135 ->
+// 24 us, 2 10^5 152 -> 30, 1.1 10^6 157 -> 47; Zipf keys (four digits) 2 10^5 153 -> 88,
+// 1.1 10^6 155 -> 148. Above 622592 elements (152 SMs) a pass takes 18 us, and keys that
+// need seven or eight (exponents, many clusters) 175 in all where eight launched
+// passes took 154. The tile
 // stays in shared memory, not in registers: with 1024 threads its elements
 // spill, and beside 217 KB of shared memory there is no L1 to spill to (a
 // digit's count took 6.4 us).
 #include <algorithm>
+#include <cmath>
 
 #include "lsb_top.cuh"
 
 namespace lsb {
 
 using MidTile = TileSort<1024, 9>;
-constexpr int kMidSample = 1;  // keys per thread of the sample, which only skewed keys need: 1024
+constexpr uint32_t kMidFewPasses = 3;  // that leave nothing to sort: no sample is worth its time
 constexpr int kMidThreads = MidTile::kThreads;
 constexpr int kMidWarps = kMidThreads / 32;
 constexpr int kMidRow = kMidWarps + 1;  // padded row of a digit's per-warp counters
 constexpr size_t kMidStageBytes = (size_t)kMidThreads * 8u * sizeof(Elem);
 constexpr size_t kMidSmem = MidTile::kSmem;
-static_assert(kMidStageBytes + 256u * kMidRow * 2u + kMidThreads * 16u <= kMidSmem && kSampleSmem<kMidSample> <= kMidSmem, "shared memory is reused");
+constexpr size_t kMidSampleAt = kMidStageBytes + 256u * kMidRow * 2u + kMidThreads * 16u;  // beside the tile
+static_assert(kMidSampleAt + kSampleSmem<1> + 256u * 8u <= kMidSmem && kMidSampleAt % 16u == 0u, "shared memory is reused");
 static_assert(kSampleThreads == kMidThreads, "the sample is taken by the whole CTA");
 
 struct MidRun {
   uint32_t b, e;
 };
 
-// The keys' block, as in TopPlan, and the digit of the current pass.
-struct MidWindow {
-  uint64_t lo, hi;
-  uint32_t hb1, passes, right, left;
-  bool clamp;
-  __device__ __forceinline__ uint32_t digit(uint64_t key) const {
-    const uint32_t d = ((uint32_t)(key >> right) << left) & 255u;
-    return clamp ? (key < lo ? 0u : key > hi ? 255u : d) : d;
-  }
-  __device__ __forceinline__ void set_pass(uint32_t p) {
-    const uint32_t up = 8u * (passes - p);
-    right = hb1 > up ? hb1 - up : 0u;
-    left = hb1 < up ? up - hb1 : 0u;
-  }
+// A digit here is eight bits of the key that vary, wherever they are, and the
+// windows are counted from the top: bits that are the same in all keys take no pass.
+// (All bits are known exactly by then. 1.1 10^6 keys of 16 bits spread over 64: two
+// passes, not eight.) Digits keep the order of keys that differ in those bits only.
+struct MidDigit {  // its runs of neighbouring bits: ((key >> shift) & mask) << up
+  uint32_t runs, shift[8], mask[8], up[8];
 };
+__device__ __forceinline__ void set_digit(MidDigit& g, uint64_t bits) {  // one thread
+  uint32_t n = 0, up = 0;
+  while (bits) {
+    const uint32_t at = (uint32_t)__ffsll((long long)bits) - 1u;
+    const uint64_t rest = ~(bits >> at);
+    const uint32_t len = rest ? (uint32_t)__ffsll((long long)rest) - 1u : 64u;
+    g.shift[n] = at;
+    g.mask[n] = (1u << len) - 1u;
+    g.up[n++] = up;
+    up += len;
+    bits &= ~(((1ull << len) - 1ull) << at);
+  }
+  g.runs = n;
+}
+// The keys' block, as in TopPlan: keys outside it count as its ends.
+struct MidBlock {
+  uint64_t lo, hi;
+  bool clamp;
+};
+// The digits of K keys (every thread the same g and w).
+template <int K>
+__device__ __forceinline__ void mid_digits(const MidDigit& g, const MidBlock& w, const uint64_t (&key)[K], uint32_t (&d)[K]) {
+  const uint32_t runs = g.runs, shift = g.shift[0], mask = g.mask[0];
+#pragma unroll
+  for (int k = 0; k < K; k++) d[k] = (uint32_t)(key[k] >> shift) & mask;
+  for (uint32_t r = 1; r < runs; r++) {
+    const uint32_t s = g.shift[r], m = g.mask[r], up = g.up[r];
+#pragma unroll
+    for (int k = 0; k < K; k++) d[k] |= ((uint32_t)(key[k] >> s) & m) << up;
+  }
+  if (w.clamp) {
+#pragma unroll
+    for (int k = 0; k < K; k++) d[k] = key[k] < w.lo ? 0u : key[k] > w.hi ? 255u : d[k];
+  }
+}
+// The bits of `key` where `bits` has ones, next to each other.
+__device__ __forceinline__ uint64_t gather_bits(uint64_t key, uint64_t bits) {
+  uint64_t out = 0;
+  uint32_t up = 0;
+  while (bits) {
+    const uint32_t at = (uint32_t)__ffsll((long long)bits) - 1u;
+    const uint64_t rest = ~(bits >> at);
+    const uint32_t len = rest ? (uint32_t)__ffsll((long long)rest) - 1u : 64u;
+    const uint64_t ones = len < 64u ? (1ull << len) - 1ull : ~0ull;
+    out |= ((key >> at) & ones) << up;
+    up += len;
+    bits &= ~(ones << at);
+  }
+  return out;
+}
+
+// The runs that start in [g, limit) of src[0, n), into X.
+__device__ __forceinline__ void mid_finish(const Elem* src, Elem* X, uint32_t n, uint32_t g, uint32_t limit, bool known, const RunKey& w, bool clamped,
+                                           bool skewed, bool dups, uint32_t shift, unsigned char* smem, MidTile::Shared& sh, RunMarks& marks, MidRun* runs,
+                                        uint32_t max_runs, Ctrl* ctrl) {
+  Elem* in = reinterpret_cast<Elem*>(smem);
+  uint32_t* slot = reinterpret_cast<uint32_t*>(smem + MidTile::kElemBytes);
+  uint32_t* bins = reinterpret_cast<uint32_t*>(smem + MidTile::kElemBytes + MidTile::kSlotBytes);
+  auto load = [&](uint32_t from, uint32_t count) {
+    __syncthreads();  // in[] is no longer read
+    Elem e[MidTile::kItems];
+#pragma unroll
+    for (int k = 0; k < MidTile::kItems; k++) {
+      const uint32_t p = threadIdx.x + (uint32_t)k * kMidThreads;
+      if (p < count) e[k] = load_elem_l2(src + from + p);
+    }
+#pragma unroll
+    for (int k = 0; k < MidTile::kItems; k++) {
+      const uint32_t p = threadIdx.x + (uint32_t)k * kMidThreads;
+      if (p < count) in[p] = e[k];
+    }
+    __syncthreads();
+    return true;
+  };
+  auto long_run = [&](uint32_t b, uint32_t e) {
+    if (lane_id() == 0) {
+      const uint32_t i = atomicAdd(&ctrl->top.num_runs, 1u);
+      if (i < max_runs) runs[i] = MidRun{b, e};
+      else record_error(ctrl, kStatusInconsistent, kWhereScatter);
+    }
+  };
+  sort_runs<MidTile>(src, X, n, g, limit, known, w, clamped, skewed, dups, shift, in, slot, bins, sh, marks, load, long_run);
+}
 
 // K elements per thread: tiles of 1024 K. CLUSTER: the grid is one cluster, whose
 // barriers are in hardware, and clears the control block itself.
 template <int K, bool CLUSTER>
 __global__ void __launch_bounds__(kMidThreads, 1)
-    k_mid_sort(Elem* X, Elem* Y, uint32_t n, SampleRule rule, uint16_t* table, MidRun* runs, uint32_t max_runs,
+    k_mid_sort(Elem* X, Elem* Y, uint32_t n, SampleRule rule, uint16_t* table, MidRun* runs, uint32_t max_runs, uint64_t* keys_of,
                int bits, int num_digits, int api_bits, int sub, Ctrl* ctrl) {
   constexpr uint32_t E = (uint32_t)kMidThreads * K;
+  constexpr int R = K < 4 ? K : 4;  // rows at a time, where a thread would keep too much of all
   extern __shared__ __align__(128) unsigned char smem[];
-  __shared__ union {
-    typename MidTile::Shared tile;
-    SampleTile<kMidSample>::Shared sample;
-  } sh;
+  __shared__ typename MidTile::Shared sh;
+  __shared__ SampleStats s_stats;
   __shared__ uint32_t s_tot[256], s_pre[256];      // digit d at [(d & 7) 32 + (d >> 3)]
   __shared__ uint32_t s_start[256], s_delta[256], s_tstart[256];
-  __shared__ uint32_t s_near[8], s_far[9], s_scan[8], s_diff[2], s_max, s_one, s_part[2];
+  __shared__ uint32_t s_scan[8], s_diff[2], s_max, s_one, s_part[2];
+  __shared__ unsigned long long s_bits[8];  // the windows' bits, the highest first
+  __shared__ MidDigit s_digit[8];           // and how they are taken from a key
+  __shared__ uint32_t s_window;             // of the pass
+  __shared__ bool s_go;
+  // What is decided once, written by one thread with barriers around: with 1024
+  // threads a register kept for it is one that a pass has to take from local memory.
+  __shared__ struct {
+    uint64_t diff;         // bits in which keys differ
+    uint32_t all;          // passes over all of those, which leave nothing to sort
+    uint32_t passes, full;  // windows passed over, and those that there are
+    bool exact, skewed, dups;
+  } s_plan;
   __shared__ RunMarks s_marks;
   __shared__ RunKey s_w;
   Elem* in = reinterpret_cast<Elem*>(smem);
-  uint32_t* slot = reinterpret_cast<uint32_t*>(smem + MidTile::kElemBytes);
-  uint32_t* bins = reinterpret_cast<uint32_t*>(smem + MidTile::kElemBytes + MidTile::kSlotBytes);
   uint16_t* cnt = reinterpret_cast<uint16_t*>(smem + kMidStageBytes);  // [256][kMidRow]
   uint16_t* order = cnt + 256u * kMidRow;                              // [E] tile positions in digit order
   const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = lane_id(), lt = lanemask_lt();
   const uint32_t tiles = (n - 1u) / E + 1u, t = blockIdx.x;
-  const uint32_t begin = t * E;
-  const uint32_t m = t < tiles ? min(E, n - begin) : 0u;  // a CTA without a tile helps with the runs
-  const uint32_t p0 = warp * 32u * K + lane;              // this thread ranks positions p0 + 32 k
+  // The tile's place and length, reckoned anew at each use: kept, they are two more
+  // values that a pass has to fetch from local memory.
+  auto tile_begin = []() {
+    uint32_t cta;
+    asm volatile("mov.u32 %0, %%ctaid.x;" : "=r"(cta));
+    return cta * E;
+  };
+  auto tile_len = [&](uint32_t begin) { return begin < n ? min(E, n - begin) : 0u; };  // a CTA without a tile helps with the runs
   uint32_t barriers = 0, buf = 0;
-  MidWindow win;
+  __shared__ MidBlock win;  // written by one thread, with barriers around
 
   auto all_arrived = [&]() {
     if (!CLUSTER) return grid_barrier(ctrl, &barriers);
@@ -98,6 +194,7 @@ __global__ void __launch_bounds__(kMidThreads, 1)
   };
   auto load_tile = [&](const Elem* src) {
     __syncthreads();
+    const uint32_t begin = tile_begin(), m = tile_len(begin);
     Elem v[K];
 #pragma unroll
     for (int k = 0; k < K; k++)
@@ -109,13 +206,23 @@ __global__ void __launch_bounds__(kMidThreads, 1)
   };
   // ranks and counts of the digit in the tile: order[], and the counts to the table
   auto count_tile = [&]() {
+    const uint32_t m = tile_len(tile_begin());
+    const uint32_t p0 = warp * 32u * K + lane;  // this thread ranks positions p0 + 32 k
     for (uint32_t i = tid; i < 256u * kMidRow / 2u; i += kMidThreads) reinterpret_cast<uint32_t*>(cnt)[i] = 0u;
     if (tid < 256) s_tot[tid] = s_pre[tid] = 0u;
     if (tid == 0) s_max = s_one = 0u;
     __syncthreads();
     uint32_t rd[K];  // rank in the warp | digit << 16
 #pragma unroll
-    for (int k = 0; k < K; k++) rd[k] = win.digit(in[min(p0 + 32u * (uint32_t)k, E - 1u)].key) << 16;
+    for (int k = 0; k < K; k += R) {
+      uint64_t key[R];
+      uint32_t d[R];
+#pragma unroll
+      for (int i = 0; i < R; i++) key[i] = in[min(p0 + 32u * (uint32_t)(k + i), E - 1u)].key;
+      mid_digits<R>(s_digit[s_window], win, key, d);
+#pragma unroll
+      for (int i = 0; i < R; i++) rd[k + i] = d[i] << 16;
+    }
     if (m == E) {
 #pragma unroll
       for (int k = 0; k < K; k++) {
@@ -159,9 +266,9 @@ __global__ void __launch_bounds__(kMidThreads, 1)
     }
     uint32_t of_digit = sum + __shfl_xor_sync(0xffffffffu, sum, 1);
     of_digit += __shfl_xor_sync(0xffffffffu, of_digit, 2);
-    if (lane == 31) sh.tile.wtot[warp] = inc;
+    if (lane == 31) sh.wtot[warp] = inc;
     __syncthreads();
-    const uint32_t off = inc - sum + __reduce_add_sync(0xffffffffu, lane < warp ? sh.tile.wtot[lane] : 0u);
+    const uint32_t off = inc - sum + __reduce_add_sync(0xffffffffu, lane < warp ? sh.wtot[lane] : 0u);
 #pragma unroll
     for (int j = 0; j < 8; j++) c[j] = (uint16_t)(off + p8[j]);
     if (tid % 4u == 0u) {
@@ -219,21 +326,32 @@ __global__ void __launch_bounds__(kMidThreads, 1)
     __syncthreads();
   };
   auto scatter = [&](Elem* dst) {
+    const uint32_t m = tile_len(tile_begin());
+#pragma unroll 1
+    for (uint32_t row = tid; row < E; row += (uint32_t)(R * kMidThreads)) {
+      uint64_t key[R], val[R];
+      uint32_t d[R];
 #pragma unroll
-    for (int k = 0; k < K; k++) {
-      const uint32_t p = tid + (uint32_t)k * kMidThreads;
-      if (p < m) {
-        const Elem e = in[order[p]];
-        const uint32_t o = s_delta[win.digit(e.key)] + p;
-        if (o < n) store_elem(dst + o, e);
+      for (int k = 0; k < R; k++) {
+        const uint32_t p = row + (uint32_t)k * kMidThreads;
+        const Elem e = in[p < m ? order[p] : 0u];
+        key[k] = e.key;
+        val[k] = e.val;
+      }
+      mid_digits<R>(s_digit[s_window], win, key, d);
+#pragma unroll
+      for (int k = 0; k < R; k++) {
+        const uint32_t p = row + (uint32_t)k * kMidThreads;
+        const uint32_t o = s_delta[d[k]] + p;
+        if (p < m && o < n) store_elem(dst + o, Elem{key[k], val[k]});
       }
     }
   };
 
   // 1. the tile, and the bits in which keys differ
   if (tid < 2) s_diff[tid] = 0u;
-  if (tid < 8) s_near[tid] = 0u;
-  if (tid < 9) s_far[tid] = 0u;
+  clear_stats(s_stats);
+  if (tid == 0) s_bits[0] = 0ull;
   const uint64_t first_key = ld_relaxed_u64(&X[0].key);
   if (CLUSTER) {
     if (t == 0)
@@ -242,6 +360,7 @@ __global__ void __launch_bounds__(kMidThreads, 1)
   }
   load_tile(X);
   {
+    const uint32_t m = tile_len(tile_begin());
     uint64_t x = 0;
 #pragma unroll
     for (int k = 0; k < K; k++) {
@@ -262,37 +381,148 @@ __global__ void __launch_bounds__(kMidThreads, 1)
   const uint64_t diff = (uint64_t)__ldcg(&ctrl->top.diff[1]) << 32 | __ldcg(&ctrl->top.diff[0]);
   if (t == 0 && tid == 0) write_plan(ctrl, diff, n, bits, num_digits, api_bits, sub);
   if (diff == 0) return;
-  const uint32_t hb1 = 64u - (uint32_t)__clzll((long long)diff), full = (hb1 + 7u) / 8u;
+  // the windows of eight of the bits `of`, into s_bits and s_digit; a barrier behind it
+  auto set_windows = [&](uint64_t of) {
+    if (tid < 8) s_bits[tid] = 0ull;
+    __syncthreads();
+    if (tid < 64 && (of >> tid & 1ull)) atomicOr(&s_bits[(__popcll(of >> tid) - 1) >> 3], 1ull << tid);
+    __syncthreads();
+    if (lane == 0 && warp < 8u && s_bits[warp]) set_digit(s_digit[warp], s_bits[warp]);
+    __syncthreads();
+  };
+  auto passes_over = [](uint64_t of) { return ((uint32_t)__popcll(of) + 7u) / 8u; };
+  const uint32_t all = passes_over(diff);  // passes that leave nothing to sort
+  // v of all threads of the CTA, or'ed together
+  auto or_all = [&](uint64_t v) {
+    __syncthreads();
+    if (tid < 2) s_diff[tid] = 0u;
+    __syncthreads();
+    const uint32_t lo = __reduce_or_sync(0xffffffffu, (uint32_t)v), hi = __reduce_or_sync(0xffffffffu, (uint32_t)(v >> 32));
+    if (lane == 0) {
+      if (lo) atomicOr(&s_diff[0], lo);
+      if (hi) atomicOr(&s_diff[1], hi);
+    }
+    __syncthreads();
+    return (uint64_t)s_diff[1] << 32 | s_diff[0];
+  };
+  // The bits in which keys with the same digit in the top window differ: exactly,
+  // against one key of each digit that all CTAs agree on. s_go: no wait ran out.
+  auto told_apart = [&]() -> uint64_t {
+    uint64_t* one = reinterpret_cast<uint64_t*>(smem + kMidSampleAt + kSampleSmem<1>);
+    const uint32_t m = tile_len(tile_begin());
+    auto with_digit = [&](auto f) {
+#pragma unroll 1
+      for (uint32_t p = tid; p < m; p += (uint32_t)kMidThreads) {
+        const uint64_t key[1] = {in[p].key};
+        uint32_t d[1];
+        mid_digits<1>(s_digit[0], win, key, d);
+        f(key[0], d[0]);
+      }
+    };
+    __syncthreads();
+    with_digit([&](uint64_t key, uint32_t d) { one[d] = key; });  // any one of the tile's
+    __syncthreads();
+    if (tid < 256u && t < tiles && (tid < 255u ? s_tstart[tid + 1u] : m) > s_tstart[tid]) keys_of[tid] = one[tid];
+    bool go = all_arrived();
+    if (tid < 256u) one[tid] = __ldcg(&keys_of[tid]);
+    __syncthreads();
+    uint64_t x = 0;
+    with_digit([&](uint64_t key, uint32_t d) { x |= key ^ one[d]; });
+    x = or_all(x);
+    if (tid == 0) {
+      if ((uint32_t)x) atomicOr(&ctrl->top.apart[0], (uint32_t)x);
+      if (x >> 32) atomicOr(&ctrl->top.apart[1], (uint32_t)(x >> 32));
+    }
+    go = go && all_arrived();
+    if (tid == 0) s_go = go;
+    __syncthreads();
+    return (uint64_t)__ldcg(&ctrl->top.apart[1]) << 32 | __ldcg(&ctrl->top.apart[0]);
+  };
 
   // 2. the top digit alone, 3. or the digits that the sample says
-  win.lo = 0ull, win.hi = ~0ull, win.clamp = false;
-  win.hb1 = hb1, win.passes = 1u;
-  win.set_pass(0);
+  if (tid == 0) win.clamp = false;
+  if (tid == 0) s_plan = {diff, all, 1u, all, false, false, false};
+  auto low_bit = [&](uint32_t windows) { return (uint32_t)__ffsll((long long)s_bits[windows - 1u]) - 1u; };
+  uint64_t top_bits;  // the first window's
+  {
+    const uint32_t hb1 = 64u - (uint32_t)__clzll((long long)diff);
+    top_bits = diff & bits_below(hb1, 8u);
+    if (tid == 0 && __popcll(top_bits) == 8) {
+      s_digit[0].runs = 1u;
+      s_digit[0].shift[0] = hb1 - 8u;
+      s_digit[0].mask[0] = 255u;
+      s_bits[0] = top_bits;
+    }
+    while (__popcll(top_bits) < 8 && top_bits != diff) {
+      const uint64_t rest = diff & ~top_bits;
+      top_bits |= 1ull << (63u - (uint32_t)__clzll((long long)rest));
+    }
+  }
+  if (tid == 0) {
+    s_window = 0u;
+    if (s_bits[0] != top_bits) set_digit(s_digit[0], s_bits[0] = top_bits);
+  }
   count_tile();
   if (!all_arrived()) return;
   add_up();
-  const bool exact = full == 1u || s_max <= MidTile::kCap;
-  bool skewed = false;
-  if (!exact) {
+  if (all == 1u || s_max <= MidTile::kCap) {
+    // (a tile or two for each CTA: the ways of duplicates are the ones to try first
+    // unless there are bits that would make other keys uneven)
+    if (tid == 0) s_plan.exact = true, s_plan.dups = !ragged(low_bit(1u), 13u, 5u, diff);
     __syncthreads();
-    const uint64_t* s = sample_keys<kMidSample>(X, n, smem, sh.sample);
-    const uint64_t span = s[0] ^ s[SampleTile<kMidSample>::kCap - 1u];
-    if (span) win.hb1 = 64u - (uint32_t)__clzll((long long)span);
-    if (win.hb1 < hb1) {  // the few keys outside the sample's block are clamped to it
-      win.lo = s[0] >> win.hb1 << win.hb1;
-      win.hi = win.lo | ((1ull << win.hb1) - 1ull);
-      win.clamp = true;
-    } else {
-      rule.tmin = 2u;  // one pass over these bits has been ruled out
+  } else {
+    if (tid == 0) s_plan.passes = all;
+    set_windows(diff);
+    __syncthreads();
+    if (all > kMidFewPasses) {
+      uint64_t* buf = reinterpret_cast<uint64_t*>(smem + kMidSampleAt);
+      const uint64_t* s = sort_sample(sample_key(X, n, tid), buf);
+      const uint64_t lowest = s[0], span = lowest ^ s[kSampleThreads - 1];
+      uint64_t bits = diff;
+      MidBlock block{0ull, ~0ull, false};
+      if (span && (diff >> (63u - (uint32_t)__clzll((long long)span))) >> 1) {
+        // the few keys outside the sample's block are clamped to it
+        const uint32_t hb = 64u - (uint32_t)__clzll((long long)span);
+        bits &= (1ull << hb) - 1ull;
+        block.lo = lowest >> hb << hb;
+        block.hi = block.lo | ((1ull << hb) - 1ull);
+        block.clamp = true;
+      } else {
+        rule.tmin = 2u;  // one pass over these bits has been ruled out
+        // bits that the top window tells (of a sign, a tag, a sentinel) need no pass
+        const uint64_t step = tid + 1u < kSampleThreads ? s[tid] ^ s[tid + 1u] : 0ull;
+        if (passes_over(top_bits | or_all((step & top_bits) ? 0ull : step)) + 2u <= all) {
+          const uint64_t apart = told_apart();
+          if (!s_go) return;
+          bits = top_bits | apart;
+        }
+      }
+      const uint32_t count = (uint32_t)__popcll(bits);
+      const uint64_t mine = gather_bits(s[tid], bits);
+      set_windows(bits);
+      buf[tid] = mine;  // either half: every thread has read its key before the barrier
+      __syncthreads();
+      const uint32_t full = passes_over(bits);
+      const SampleChoice c = choose_passes<1>(buf, count, rule, block.clamp ? all : full, s_stats, bits, low_bit);
+      if (c.plain && block.clamp) {
+        __syncthreads();
+        set_windows(diff);
+      } else if (tid == 0) {
+        win = block;
+        s_plan.passes = c.plain ? full : c.passes;
+        s_plan.full = full;
+        s_plan.skewed = c.skewed;
+        s_plan.dups = c.dups || !ragged(low_bit(s_plan.passes), 13u, 5u, bits);
+      }
+      __syncthreads();
     }
-    win.passes = sample_passes<kMidSample>(s, win.hb1, rule, s_near, s_far, &skewed);
   }
   for (bool first = true;; first = false) {
     uint32_t par = 0;
-    for (uint32_t p = 0; p < win.passes; p++) {
-      win.set_pass(p);
-      if (p || !first || !exact) {
-        load_tile(par ? Y : X);
+    for (uint32_t p = 0; p < s_plan.passes; p++) {
+      if (p || !first || !s_plan.exact) {
+        if (p || !first) load_tile(par ? Y : X);  // else it is still there
+        if (tid == 0) s_window = s_plan.passes - 1u - p;
         buf ^= 1u;
         count_tile();
         if (!all_arrived()) return;
@@ -304,18 +534,20 @@ __global__ void __launch_bounds__(kMidThreads, 1)
       if (!all_arrived()) return;
     }
     const Elem* src = par ? Y : X;
-    if (win.passes == full && !win.clamp) {  // in order
+    if (s_plan.passes == s_plan.full && !win.clamp) {  // in order
+      const uint32_t begin = tile_begin(), m = tile_len(begin);
       if (par)
         for (uint32_t i = tid; i < m; i += kMidThreads) store_elem(X + begin + i, load_elem_l2(Y + begin + i));
       return;
     }
     // the runs that start in this CTA's part of the array
-    const uint32_t shift = win.hb1 > 8u * win.passes ? win.hb1 - 8u * win.passes : 0u;
+    const uint32_t shift = low_bit(s_plan.passes);
+    const bool exact = s_plan.exact;
     uint32_t g = (uint32_t)((uint64_t)n * blockIdx.x / gridDim.x);
     uint32_t limit = (uint32_t)((uint64_t)n * (blockIdx.x + 1u) / gridDim.x);
     bool known = blockIdx.x == 0;
     __syncthreads();
-    if (tid == 0) s_w = RunKey{win.lo, win.hi, shift};
+    if (tid == 0) s_w = RunKey{win.clamp ? win.lo : 0ull, win.clamp ? win.hi : ~0ull, shift};
     if (exact && first) {  // after one pass the runs are the digit's buckets
       if (tid < 2) s_part[tid] = n;
       __syncthreads();
@@ -328,31 +560,7 @@ __global__ void __launch_bounds__(kMidThreads, 1)
       limit = s_part[1];
       known = true;
     }
-    auto load = [&](uint32_t from, uint32_t count) {
-      __syncthreads();  // in[] is no longer read
-      Elem e[MidTile::kItems];
-#pragma unroll
-      for (int k = 0; k < MidTile::kItems; k++) {
-        const uint32_t p = tid + (uint32_t)k * kMidThreads;
-        if (p < count) e[k] = load_elem_l2(src + from + p);
-      }
-#pragma unroll
-      for (int k = 0; k < MidTile::kItems; k++) {
-        const uint32_t p = tid + (uint32_t)k * kMidThreads;
-        if (p < count) in[p] = e[k];
-      }
-      __syncthreads();
-      return true;
-    };
-    auto long_run = [&](uint32_t b, uint32_t e) {
-      if (lane == 0) {
-        const uint32_t i = atomicAdd(&ctrl->top.num_runs, 1u);
-        if (i < max_runs) runs[i] = MidRun{b, e};
-        else record_error(ctrl, kStatusInconsistent, kWhereScatter);
-      }
-    };
-    sort_runs<MidTile>(src, X, exact ? limit : n, g, limit, known, s_w, win.clamp, skewed, shift, in, slot, bins, sh.tile, s_marks,
-                       load, long_run);
+    mid_finish(src, X, exact ? limit : n, g, limit, known, s_w, win.clamp, s_plan.skewed, s_plan.dups, shift, smem, sh, s_marks, runs, max_runs, ctrl);
     if (exact) return;
     // 4. runs longer than a tile: copied into X, and whether they are in order
     if (!all_arrived()) return;
@@ -362,6 +570,7 @@ __global__ void __launch_bounds__(kMidThreads, 1)
     for (uint32_t i = tid; i < count; i += kMidThreads)
       list[i] = MidRun{ld_relaxed_u32(&runs[i].b), ld_relaxed_u32(&runs[i].e)};
     __syncthreads();
+    const uint32_t begin = tile_begin(), m = tile_len(begin);
     bool inversion = false;
     for (uint32_t i = 0; i < count; i++) {
       const uint32_t b = list[i].b, e = list[i].e;
@@ -374,8 +583,9 @@ __global__ void __launch_bounds__(kMidThreads, 1)
     if (__any_sync(0xffffffffu, inversion) && lane == 0) atomicOr(&ctrl->top.num_chunks, 1u);
     if (!all_arrived()) return;
     if (ld_relaxed_u32(&ctrl->top.num_chunks) == 0u) return;
-    win.lo = 0ull, win.hi = ~0ull, win.clamp = false;
-    win.hb1 = hb1, win.passes = full;
+    if (tid == 0) win.clamp = false, s_plan.passes = s_plan.full = s_plan.all;
+    set_windows(s_plan.diff);
+    __syncthreads();
   }
 }
 
@@ -392,13 +602,13 @@ static uint32_t mid_items(uint32_t n, const DeviceInfo& dev) {
 static uint32_t mid_tiles(uint32_t n, uint32_t items) { return (n - 1u) / (items * (uint32_t)kMidThreads) + 1u; }
 static uint32_t mid_max_runs(uint32_t n) { return n / MidTile::kCap + 1u; }
 
-// Two count tables and the list of long runs, after the control block: what any
+// Two count tables, the list of long runs and a key for each digit, after the control block: what any
 // size up to n needs, so that a workspace of the largest array serves the smaller
 // ones (the tiles double where they outnumber the SMs, and are then half as many).
 size_t mid_workspace_bytes(uint32_t n, const DeviceInfo& dev) {
   n = std::min(n, mid_limit(dev));
   const uint32_t tiles = std::min(mid_tiles(n, 2u), (uint32_t)dev.sm_count);
-  return kCtrlBytes + (size_t)tiles * 256u * 2u * 2u + (size_t)mid_max_runs(n) * sizeof(MidRun);
+  return kCtrlBytes + (size_t)tiles * 256u * 2u * 2u + (size_t)mid_max_runs(n) * sizeof(MidRun) + 256u * 8u;
 }
 
 // Up to 16 tiles of 2048 elements the grid is one cluster of 16 CTAs: no clear
@@ -449,9 +659,19 @@ int mid_run(Elem* X, Elem* Y, unsigned char* ws, const Layout& L, const DeviceIn
   uint32_t max_runs = mid_max_runs(n);
   // A key that overfills its bins makes a tile uneven, unless the tile is in
   // order: 2048 windows per element leave a tile without a mixed run.
-  SampleRule rule = sample_rule(n, SampleTile<kMidSample>::kCap, MidTile::kCap - 576u, MidTile::kMaxBin, 2048.0f);
+  SampleRule rule = sample_rule(n, kSampleThreads, MidTile::kCap, MidTile::kCap - 576u, MidTile::kMaxBin, 2048.0f);
+  rule.finish = 8u;
+  rule.copy = 2u;
+  rule.straddle = 25u;
+  // A run longer than a tile has the array passed over by every digit once more: a
+  // window with a tile's share of the sample, less half a deviation, is taken
+  // for one.
+  const float share = (float)MidTile::kCap * (float)kSampleThreads / (float)n;
+  rule.far = (uint32_t)std::max(4.0f, share - 0.5f * std::sqrt(share));
+  rule.far_limit = 2u;
   int bits = L.stat_bits, digits = L.stat_digits, api_bits = L.api_bits, sub = L.sub;
-  void* args[] = {&X, &Y, &n, &rule, &table, &runs, &max_runs, &bits, &digits, &api_bits, &sub, &ctrl};
+  uint64_t* keys_of = reinterpret_cast<uint64_t*>(runs + max_runs);
+  void* args[] = {&X, &Y, &n, &rule, &table, &runs, &max_runs, &keys_of, &bits, &digits, &api_bits, &sub, &ctrl};
   const uint32_t sms = stream_sms(st, dev);
   if (tiles > sms) return kMidRefused;
   if (n <= kMidCluster * kMidClusterItems * (uint32_t)kMidThreads && sms == (uint32_t)dev.sm_count) {

@@ -410,10 +410,12 @@ __device__ __forceinline__ void lookback_adjacent(const uint64_t* __restrict__ r
 // tile's stores from the next tile's ranking.
 // BITS > 0 fixes the digit width at compile time (8 and 11: the common widths);
 // BITS == 0 takes it from `bits_rt`. TOP: the digit's bits, whether the pass
-// runs and the buffers' parity come from ctrl->top (sorts by top digits).
-template <int THREADS, int K, int MINB, typename CNT, int BITS, bool TOP = false>
-__global__ void __launch_bounds__(THREADS, MINB)
-    k_onesweep(Elem* __restrict__ X, Elem* __restrict__ Y, uint32_t n, int bits_rt, int pass,
+// runs and the buffers' parity come from ctrl->top (sorts by top digits). REST:
+// the pass before ran in the same kernel, so the array is read from L2. Returns
+// the tiles that this CTA has placed.
+template <int THREADS, int K, typename CNT, int BITS, bool TOP, bool REST>
+__device__ __forceinline__ uint32_t
+    onesweep_tiles(Elem* __restrict__ X, Elem* __restrict__ Y, uint32_t n, int bits_rt, int pass,
                int digit, const uint32_t* __restrict__ gstart, uint64_t* __restrict__ ring,
                uint32_t* __restrict__ done, uint32_t ring_tiles, Ctrl* ctrl, SegDesc seg) {
   constexpr int W = THREADS / 32;
@@ -427,7 +429,7 @@ __global__ void __launch_bounds__(THREADS, MINB)
   __shared__ uint32_t s_wt[W];
 
   const bool segmented = TOP && seg.tile_seg != nullptr;
-  if (TOP ? !segmented && !((ctrl->top.run_mask >> pass) & 1u) : pass_skipped(ctrl, pass)) return;
+  if (TOP ? !segmented && !((ctrl->top.run_mask >> pass) & 1u) : pass_skipped(ctrl, pass)) return 0u;
   const int bits = BITS > 0 ? BITS : bits_rt;
   const uint32_t nbins = 1u << bits, mask = nbins - 1u;
   const int shift = bits * digit;  // `pass` indexes this call's passes, `digit` the key
@@ -490,11 +492,12 @@ __global__ void __launch_bounds__(THREADS, MINB)
     const Elem* p = src + ti.begin + warp * 32u * K + lane;
     if (ti.len == E) {
 #pragma unroll
-      for (int k = 0; k < K; k++) v[k] = load_elem_stream(p + k * 32);
+      for (int k = 0; k < K; k++) v[k] = REST ? load_elem_l2(p + k * 32) : load_elem_stream(p + k * 32);
     } else {
 #pragma unroll
       for (int k = 0; k < K; k++)
-        if (warp * 32u * K + (uint32_t)k * 32u + lane < ti.len) v[k] = load_elem_stream(p + k * 32);
+        if (warp * 32u * K + (uint32_t)k * 32u + lane < ti.len)
+          v[k] = REST ? load_elem_l2(p + k * 32) : load_elem_stream(p + k * 32);
     }
   };
   auto clear_counters = [&]() {
@@ -770,6 +773,53 @@ __global__ void __launch_bounds__(THREADS, MINB)
   bulk_wait_all();
   if (lb_steps) atomicAdd(&ctrl->lookback_steps, lb_steps);
   if (lb_polls) atomicAdd(&ctrl->lookback_polls, lb_polls);
+  return iter;
+}
+
+template <int THREADS, int K, int MINB, typename CNT, int BITS, bool TOP = false>
+__global__ void __launch_bounds__(THREADS, MINB)
+    k_onesweep(Elem* __restrict__ X, Elem* __restrict__ Y, uint32_t n, int bits_rt, int pass,
+               int digit, const uint32_t* __restrict__ gstart, uint64_t* __restrict__ ring,
+               uint32_t* __restrict__ done, uint32_t ring_tiles, Ctrl* ctrl, SegDesc seg) {
+  onesweep_tiles<THREADS, K, CNT, BITS, TOP, false>(X, Y, n, bits_rt, pass, digit, gstart, ring, done, ring_tiles, ctrl,
+                                                    seg);
+}
+
+// The plan's passes from `first` on, one after another in one launch: usual keys
+// need none, and a launch each would cost 2 us. A pass waits until the one before
+// has placed all its tiles. Tiles are handed out by tickets, so a pass's tiles are
+// with running CTAs, which wait for earlier tiles only: no CTA needs another one
+// to be resident.
+template <int THREADS, int K, int MINB>
+__global__ void __launch_bounds__(THREADS, MINB)
+    k_onesweep_rest(Elem* X, Elem* Y, uint32_t n, int first, const uint32_t* __restrict__ gstart,
+                    uint64_t* __restrict__ ring, uint32_t ring_tiles, Ctrl* ctrl, SegDesc seg) {
+  __shared__ bool s_go;
+  const bool segmented = seg.tile_seg != nullptr;
+  const int passes = segmented ? 8 : (int)ctrl->top.passes;
+  int before = -1;
+  uint32_t tiles_before = 0;
+  for (int pass = first; pass < passes; pass++) {
+    const uint32_t tiles = segmented ? seg.num_tiles[pass] : (n - 1u) / (uint32_t)(THREADS * K) + 1u;
+    if (segmented ? tiles == 0u : !((ctrl->top.run_mask >> pass) & 1u)) continue;
+    if (before >= 0) {
+      if (threadIdx.x == 0) {
+        s_go = wait_arrivals(&ctrl->top.pass_done[before], tiles_before, ctrl);
+        __threadfence();
+      }
+      __syncthreads();
+      if (!s_go) return;
+    }
+    const uint32_t placed = onesweep_tiles<THREADS, K, uint32_t, 8, true, true>(
+        X, Y, n, 8, pass, 0, segmented ? nullptr : gstart + (size_t)pass * 256u, ring, nullptr, ring_tiles, ctrl, seg);
+    __syncthreads();  // every thread's copies have been written
+    if (threadIdx.x == 0 && placed) {
+      __threadfence();
+      atomicAdd(&ctrl->top.pass_done[pass], placed);
+    }
+    before = pass;
+    tiles_before = tiles;
+  }
 }
 
 // One pass for 9- to 12-bit digits (512 to 4096 bins), the tile ranked in
@@ -1405,18 +1455,34 @@ uint32_t onesweep_tile_elems(int bits) { return onesweep_choice(bits).tile; }
 // batch's plans, in the shapes 0 and 2.
 uint32_t onesweep_top_tile(int variant) { return variant == 2 ? 4096u : 8192u; }
 
+static uint32_t top_grid(uint32_t tiles, int variant, uint32_t ctas, const DeviceInfo& dev) {
+  uint32_t grid = (uint32_t)dev.sm_count * (variant == 2 ? 2u : 1u);
+  if (ctas > 0) grid = std::min(grid, ctas);
+  return std::max<uint32_t>(1u, std::min(grid, tiles));
+}
+
+int onesweep_top_rest(Elem* X, Elem* Y, uint32_t n, int first, const uint32_t* gstart, uint64_t* ring, uint32_t tiles,
+                      Ctrl* ctrl, const SegDesc& seg, int variant, uint32_t ctas, const DeviceInfo& dev, cudaStream_t st) {
+  const int threads = variant == 2 ? 256 : 512;
+  auto kern = variant == 2 ? k_onesweep_rest<256, 16, 2> : k_onesweep_rest<512, 16, 1>;
+  const size_t smem = reg_kernel_smem(8, threads, 16);
+  static std::atomic<uint64_t> allowed[2];
+  if (!allow_smem((const void*)kern, smem, &allowed[variant == 2 ? 1 : 0])) return 5;
+  ProfScope prof("onesweep_rest", st);
+  kern<<<top_grid(tiles, variant, ctas, dev), threads, smem, st>>>(X, Y, n, first, gstart, ring, tiles, ctrl, seg);
+  return cudaPeekAtLastError() == cudaSuccess ? 0 : 5;
+}
+
 int onesweep_top_pass(Elem* X, Elem* Y, uint32_t n, int pass, const uint32_t* gstart, uint64_t* ring,
-                      uint32_t tiles, Ctrl* ctrl, const SegDesc& seg, int variant, uint32_t ctas, bool spare,
+                      uint32_t tiles, Ctrl* ctrl, const SegDesc& seg, int variant, uint32_t ctas,
                       const DeviceInfo& dev, cudaStream_t st) {
   const int threads = variant == 2 ? 256 : 512;
   auto kern = variant == 2 ? k_onesweep<256, 16, 2, uint32_t, 8, true> : k_onesweep<512, 16, 1, uint32_t, 8, true>;
   const size_t smem = reg_kernel_smem(8, threads, 16);
   static std::atomic<uint64_t> allowed[2];
   if (!allow_smem((const void*)kern, smem, &allowed[variant == 2 ? 1 : 0])) return 5;
-  uint32_t grid = (uint32_t)dev.sm_count * (variant == 2 ? 2u : 1u);
-  if (ctas > 0) grid = std::min(grid, ctas);
-  grid = std::max<uint32_t>(1u, std::min(grid, tiles));
-  ProfScope prof(spare ? "onesweep_spare" : "onesweep_scatter", st);
+  const uint32_t grid = top_grid(tiles, variant, ctas, dev);
+  ProfScope prof("onesweep_scatter", st);
   // one ring slot per tile: no slot is reused, so there are no completion tags
   kern<<<grid, threads, smem, st>>>(X, Y, n, 8, pass, 0, gstart, ring, nullptr, tiles, ctrl, seg);
   return cudaPeekAtLastError() == cudaSuccess ? 0 : 5;

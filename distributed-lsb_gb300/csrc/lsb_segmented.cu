@@ -35,11 +35,11 @@ constexpr int kSegSample = 1;  // keys per thread of an array's sample: 1024
 // a tile, else from a sample, as for one array (lsb_top.cu). Two CTAs per SM,
 // about 6 us per sampled array.
 __global__ void __launch_bounds__(kSampleThreads, 2)
-    k_seg_sample(const Elem* __restrict__ data, const int64_t* __restrict__ seg_off, uint32_t nseg, uint32_t max_passes,
+    k_seg_sample(const Elem* __restrict__ data, const int64_t* __restrict__ seg_off, uint32_t nseg, uint32_t straddle,
                  SegPlan* __restrict__ plans) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ typename SampleTile<kSegSample>::Shared sh;
-  __shared__ uint32_t s_near[8], s_far[9];
+  __shared__ SampleStats s_stats;
   for (uint32_t s = blockIdx.x; s < nseg; s += gridDim.x) {
     const uint32_t len = (uint32_t)(seg_off[s + 1] - seg_off[s]);
     SegPlan p{};
@@ -47,20 +47,20 @@ __global__ void __launch_bounds__(kSampleThreads, 2)
     p.hi = ~0ull;
     if (len > kCap) {
       __syncthreads();
-      if (threadIdx.x < 8) s_near[threadIdx.x] = 0u;
-      if (threadIdx.x < 9) s_far[threadIdx.x] = 0u;
+      clear_stats(s_stats);
       const uint64_t* k = sample_keys<kSegSample>(data + seg_off[s], len, smem, sh);
-      const uint64_t first = k[0], span = first ^ k[SampleTile<kSegSample>::kCap - 1u];
+      const uint64_t first = k[0], span = first ^ k[kSegSample * kSampleThreads - 1];
       if (span) p.hb1 = 64u - (uint32_t)__clzll((long long)span);
       // a key that overfills its bins is heavy (lsb_mid.cu); four passes leave
       // its runs pure up to 2^28 elements
       const float spread = fminf(2048.0f, fmaxf(16.0f, 4294967296.0f / (float)len));
-      SampleRule rule = sample_rule(len, SampleTile<kSegSample>::kCap, kMeanRun, Tile::kMaxBin, spread);
-      rule.tmax = max_passes;
-      rule.tmin = min(rule.tmin, max_passes);
-      bool skewed;
-      p.passes = sample_passes<kSegSample>(k, p.hb1, rule, s_near, s_far, &skewed);
-      p.skewed = skewed ? 1u : 0u;
+      SampleRule rule = sample_rule(len, kSegSample * kSampleThreads, Tile::kCap, kMeanRun, Tile::kMaxBin, spread);
+      rule.skips = false;
+      rule.straddle = straddle;
+      const SampleChoice c = choose_passes<kSegSample>(k, p.hb1, rule, 8u, s_stats, 0ull,
+                                                          [&](uint32_t t) { return p.hb1 > 8u * t ? p.hb1 - 8u * t : 0u; });
+      p.passes = c.passes;
+      p.skewed = (c.skewed ? 1u : 0u) | (c.dups ? 2u : 0u);
       if (p.hb1 < 64u) {
         p.clamp = 1u;
         p.lo = first >> p.hb1 << p.hb1;
@@ -306,15 +306,15 @@ __global__ void __launch_bounds__(Tile::kThreads, 2)
     if (passes == 0u) {
       if (len < 2u) continue;
       if (!load(0u, len)) return;
-      Tile::sort(in, 0u, len, 0ull, 0ull, slot, bins, sh, true,
+      Tile::sort(in, 0u, len, 0ull, 0ull, slot, bins, sh, true, Uneven::kDups,
                  [=](bool on, uint32_t r, const Elem& e) { store_elem_if(on, dst + r, e); });
       continue;
     }
     __syncthreads();
     if (threadIdx.x == 0) s_w = run_key(plan);
     auto long_run = [&](uint32_t b, uint32_t e) { push_run(ctrl, chunks, unsorted, n, at + b, at + e, par); };
-    if (!sort_runs<Tile>(src, dst, len, g, limit, g == 0, s_w, plan.clamp != 0u, plan.skewed != 0u, run_key(plan).shift,
-                         in, slot, bins, sh, s_marks, load, long_run))
+    if (!sort_runs<Tile>(src, dst, len, g, limit, g == 0, s_w, plan.clamp != 0u, (plan.skewed & 1u) != 0u, (plan.skewed & 2u) != 0u,
+                         run_key(plan).shift, in, slot, bins, sh, s_marks, load, long_run))
       return;
   }
 }
@@ -402,14 +402,10 @@ static int seg_run(Elem* A, Elem* B, const int64_t* seg_off, void* ws, const Seg
   if (!allow_smem((const void*)k_seg_sample, sample_smem, &allowed[0]) ||
       !allow_smem((const void*)k_seg_finish, Tile::kSmem, &allowed[1]))
     return LSB_ERR_CUDA;
-  // passes that the largest array there can be might need and two more, the
-  // four of heavy keys, or all eight when empty launches (2 us each) do not count
-  uint32_t passes = std::max(4u, passes_for((float)L.n, (float)kMeanRun) + 2u);
-  if (passes > 8u || L.n >= (1u << 26)) passes = 8u;
   {
     ProfScope prof("seg_sample", st);
     k_seg_sample<<<std::min<uint32_t>(L.nseg, (uint32_t)dev.sm_count * 2u), kSampleThreads, sample_smem, st>>>(
-        A, seg_off, L.nseg, passes, plans);
+        A, seg_off, L.nseg, straddle_time(L.n), plans);
   }
   {
     ProfScope prof("seg_tiles", st);
@@ -435,9 +431,14 @@ static int seg_run(Elem* A, Elem* B, const int64_t* seg_off, void* ws, const Seg
   seg.seg_gstart = counts;
   seg.num_tiles = ntiles;
   seg.plan = plans;
+  // a launch for each pass that an array of all the elements needs when its keys
+  // are even, and one for whatever passes follow
+  const uint32_t passes = passes_for((float)L.n, (float)kMeanRun);
   for (uint32_t p = 0; p < passes; p++)
-    if (onesweep_top_pass(A, B, L.n, (int)p, nullptr, ring, L.max_tiles, ctrl, seg, L.variant, L.ctas, false, dev, st))
+    if (onesweep_top_pass(A, B, L.n, (int)p, nullptr, ring, L.max_tiles, ctrl, seg, L.variant, L.ctas, dev, st))
       return LSB_ERR_CUDA;
+  if (onesweep_top_rest(A, B, L.n, (int)passes, nullptr, ring, L.max_tiles, ctrl, seg, L.variant, L.ctas, dev, st))
+    return LSB_ERR_CUDA;
   RunChunk* chunks = reinterpret_cast<RunChunk*>(ring);
   uint32_t* unsorted = reinterpret_cast<uint32_t*>(chunks + max_chunks(L.n));
   {

@@ -20,10 +20,11 @@
 // is checked before any element goes out (2^28 elements, every key thirty times:
 // 12.1 ms; 14.7 ms when every pair's whole keys are compared); a warp takes a
 // larger one key by key, and a bitmap of the key's positions gives the ranks
-// (heavy_bins). A tile with many different keys in a large bin (clusters) is
-// sorted by the bits in which its keys differ, eight at a time from the lowest
-// (stable ranks by ballots and per-warp counters).
-// 10^4 Zipf keys: 52 us bit by bit.
+// (heavy_bins). A tile with many different keys in a large bin (clusters, signs,
+// bits that never vary) gets bins that follow its keys (sort_spread); when that
+// fails too it is sorted by the bits in which its keys differ, eight at a time from
+// the lowest (stable ranks by ballots and per-warp counters; 10^4 Zipf keys took
+// 52 us so, 37 with heavy_bins).
 #pragma once
 
 #include "lsb_device.cuh"
@@ -50,6 +51,12 @@ __device__ __forceinline__ void store_elem_if(bool on, Elem* p, const Elem& e) {
                "l"(e.val), "r"((uint32_t)on)
                : "memory");
 }
+
+// What a tile whose keys are spread too unevenly for equal bins tries before it is
+// sorted bit by bit: nothing (where a kernel sorts a tile or two, code that has to
+// be fetched first costs as much as it saves), bins that follow the keys, or those
+// only after the ways of duplicates.
+enum class Uneven : uint32_t { kBits, kSpread, kDups };
 
 template <int THREADS, int K>
 struct TileSort {
@@ -129,16 +136,19 @@ struct TileSort {
   // before they are written again.
   template <typename Emit>
   static __device__ __forceinline__ void sort(const Elem* in, uint32_t lo, uint32_t hi, uint64_t base, uint64_t range,
-                                              uint32_t* slot, uint32_t* bins, Shared& sh, bool in_place, Emit emit) {
+                                              uint32_t* slot, uint32_t* bins, Shared& sh, bool in_place, Uneven uneven,
+                                              Emit emit) {
     if (range == 0 || !sort_even<false>(in, lo, hi, make_scale(base, range), slot, bins, sh, emit))
-      sort_any(in, lo, hi, slot, bins, sh, range == 0, in_place, emit);
+      sort_any(in, lo, hi, slot, bins, sh, range == 0, in_place, uneven, emit);
   }
 
   // Bins over the tile's own range of keys (unless other bins were tried and a
-  // few rounds of bits will do); bit by bit when that is uneven too.
+  // few rounds of bits will do), bins that follow the keys; bit by bit when those
+  // are uneven too.
   template <typename Emit>
   static __device__ __noinline__ void sort_any(const Elem* in, uint32_t lo, uint32_t hi, uint32_t* slot,
-                                               uint32_t* bins, Shared& sh, bool first_try, bool in_place, Emit emit) {
+                                               uint32_t* bins, Shared& sh, bool first_try, bool in_place,
+                                               Uneven uneven, Emit emit) {
     const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
     const uint64_t k0 = in[lo].key;
     uint64_t mn = ~0ull, mx = 0ull, diff = 0ull;
@@ -172,11 +182,175 @@ struct TileSort {
            __reduce_or_sync(0xffffffffu, (uint32_t)diff);
     uint32_t rounds = 0;
     for (uint64_t d = diff; d; d &= ~(255ull << (__ffsll((long long)d) - 1))) rounds++;
-    if ((first_try || rounds > kFewRounds) &&
-        sort_even<true>(in, lo, hi, make_scale(mn, mx - mn), slot, bins, sh, emit))
-      return;
+    constexpr bool kSpreads = kCuts * 8u + (kCuts + 1u) * sizeof(Part) <= kSlotBytes;  // cuts and parts in the slots' place
+    // bins that follow the keys at once, unless most of them are duplicates, which
+    // the sort by even bins has its own ways with, if it can; then they are better than bits
+    bool strict = kSpreads && uneven == Uneven::kSpread && !first_try && rounds > kFewRounds;
+    for (bool even = true;; strict = false, even = false) {
+      if constexpr (kSpreads)
+        if ((strict || !even) && sort_spread(in, lo, hi, mn, mx, strict, slot, bins, sh, emit)) return;
+      if (!even) break;
+      if ((first_try || rounds > kFewRounds) &&
+          sort_even<true>(in, lo, hi, make_scale(mn, mx - mn), slot, bins, sh, emit))
+        return;
+      if (!kSpreads || uneven == Uneven::kBits || rounds <= kFewRounds) break;
+    }
     __syncthreads();
     sort_bits(in + lo, hi - lo, diff, slot, bins, sh, emit);
+  }
+
+  // The rank of (v, key) among the slots q[0, cnt): whole keys where key bits agree, then positions.
+  static __device__ __forceinline__ uint32_t rank_exact(const Elem* in, const uint32_t* q, uint32_t cnt, uint32_t v,
+                                                        uint64_t key) {
+    uint32_t r = 0;
+    for (uint32_t j = 0; j < cnt; j += 4u) {
+      uint32_t u[4];
+      uint64_t ku[4];
+#pragma unroll
+      for (uint32_t x = 0; x < 4u; x++) u[x] = q[min(j + x, cnt - 1u)];
+#pragma unroll
+      for (uint32_t x = 0; x < 4u; x++) ku[x] = in[u[x] & kPosMask].key;
+#pragma unroll
+      for (uint32_t x = 0; x < 4u; x++) {
+        const bool tie = (u[x] ^ v) <= kPosMask && ku[x] != key;
+        r += j + x < cnt && (tie ? ku[x] < key : u[x] < v) ? 1u : 0u;
+      }
+    }
+    return r;
+  }
+
+  // The sort by bins that follow the keys: a key per thread, sorted, cut the tile's
+  // range into parts of some nine elements each, and every part has the same
+  // number of bins, equal cuts of its own range. Signs, clusters, exponents, text and
+  // keys with bits that never vary are spread by it like even ones, for a search
+  // among the cuts per element; false when a bin has too many elements, all the same
+  // (few different keys), or, when `strict`, an eighth of the cuts are equal to another. Ranks are found where an element lies, and an order list
+  // brings the elements out in theirs.
+  static constexpr uint32_t kCuts = (uint32_t)THREADS, kPartBins = kBins / (kCuts + 1u);
+  struct Part {
+    uint64_t base;
+    uint32_t up, f;
+  };
+  template <typename Emit>
+  static __device__ __noinline__ bool sort_spread(const Elem* in, uint32_t lo, uint32_t hi, uint64_t mn, uint64_t mx,
+                                                  bool strict, uint32_t* slot, uint32_t* bins, Shared& sh, Emit emit) {
+    const uint32_t tid = threadIdx.x, lane = lane_id(), warp = tid >> 5, m = hi - lo;
+    uint64_t* cut = reinterpret_cast<uint64_t*>(slot);
+    Part* part = reinterpret_cast<Part*>(cut + kCuts);
+    uint16_t* start = reinterpret_cast<uint16_t*>(bins);
+    __syncthreads();  // the arrays are no longer read
+    {
+      uint4* z = reinterpret_cast<uint4*>(bins) + tid * 2u;
+      z[0] = make_uint4(0, 0, 0, 0);
+      z[1] = make_uint4(0, 0, 0, 0);
+      if (tid == 0) start[kBins] = (uint16_t)m;
+    }
+    // the cuts, by bitonic exchanges
+    uint64_t v = in[lo + tid * m / kCuts].key;
+#pragma unroll
+    for (uint32_t k = 2; k <= kCuts; k <<= 1) {
+#pragma unroll
+      for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+        uint64_t o;
+        if (j >= 32u) {
+          __syncthreads();
+          cut[tid] = v;
+          __syncthreads();
+          o = cut[tid ^ j];
+        } else {
+          o = __shfl_xor_sync(0xffffffffu, v, (int)j);
+        }
+        const bool lower = ((tid & k) == 0u) == ((tid & j) == 0u);
+        v = lower == (o < v) ? o : v;
+      }
+    }
+    __syncthreads();
+    cut[tid] = v;
+    __syncthreads();
+    if (__syncthreads_count(tid > 0u && cut[tid - 1u] == v) > (int)(kCuts / 8u) && strict) return false;
+    for (uint32_t i = tid; i <= kCuts; i += THREADS) {  // part i: keys from cut i - 1 up to below cut i
+      const uint64_t a = i ? cut[i - 1u] : mn, b = i < kCuts ? cut[i] : mx;
+      const uint64_t range = b > a ? b - a : 1ull;
+      const uint32_t up = (uint32_t)__clzll((long long)range);
+      const uint32_t xr = (uint32_t)((range << up) >> 32);
+      part[i] = Part{a, up, (uint32_t)(__fdividef((float)kPartBins * 4294967296.0f, (float)xr + 1.0f) * (1.0f - 1.0f / 524288.0f))};
+    }
+    __syncthreads();
+    uint32_t place[K], frac[K];
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      const uint32_t p = tid + (uint32_t)k * THREADS;
+      const bool on = p - lo < m;
+      const uint64_t key = in[on ? p : lo].key;
+      uint32_t i = 0;  // cuts not above the key
+#pragma unroll
+      for (uint32_t s = kCuts / 2u; s > 0; s >>= 1) i += cut[i + s - 1u] <= key ? s : 0u;
+      i += cut[i] <= key ? 1u : 0u;
+      const Part c = part[i];
+      const uint64_t x = (uint64_t)(uint32_t)(((key - c.base) << c.up) >> 32) * c.f;
+      frac[k] = (uint32_t)x;
+      const uint32_t b = i * kPartBins + (uint32_t)(x >> 32);
+      const uint32_t s16 = (b & 1u) << 4;
+      const uint32_t old = atom_add_if(on, bins + (b >> 1), 1u << s16);
+      place[k] = b << 16 | ((old >> s16) & 0xffffu);
+    }
+    __syncthreads();
+    {
+      uint32_t w8[8], maxc = 0, sum = 0;
+      uint4* q = reinterpret_cast<uint4*>(bins) + tid * 2u;
+      {
+        const uint4 a = q[0], b = q[1];
+        w8[0] = a.x, w8[1] = a.y, w8[2] = a.z, w8[3] = a.w;
+        w8[4] = b.x, w8[5] = b.y, w8[6] = b.z, w8[7] = b.w;
+      }
+#pragma unroll
+      for (int i = 0; i < 8; i++) {
+        maxc = __vmaxu2(maxc, w8[i]);
+        const uint32_t c0 = w8[i] & 0xffffu, c1 = w8[i] >> 16;
+        w8[i] = sum | (sum + c0) << 16;
+        sum += c0 + c1;
+      }
+      uint32_t inc = sum;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= (uint32_t)o) inc += y;
+      }
+      if (lane == 31) sh.wtot[warp] = inc;
+      maxc = max(maxc & 0xffffu, maxc >> 16);
+      if (__syncthreads_or(maxc > kSlotsBin)) return false;
+      uint32_t off = inc - sum;
+      const uint32_t wt = lane < (uint32_t)kWarps ? sh.wtot[lane] : 0u;
+      off += __reduce_add_sync(0xffffffffu, lane < warp ? wt : 0u);
+      const uint32_t both = off | off << 16;
+      q[0] = make_uint4(w8[0] + both, w8[1] + both, w8[2] + both, w8[3] + both);
+      q[1] = make_uint4(w8[4] + both, w8[5] + both, w8[6] + both, w8[7] + both);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      const uint32_t p = tid + (uint32_t)k * THREADS;
+      st_shared_if(p - lo < m, slot + start[place[k] >> 16] + (place[k] & 0xffffu), (frac[k] & ~kPosMask) | p);
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int k = 0; k < K; k++) {
+      const uint32_t p = tid + (uint32_t)k * THREADS;
+      if (p - lo < m) {
+        const uint32_t b = place[k] >> 16, s = start[b];
+        place[k] = s + rank_exact(in, slot + s, start[b + 1u] - s, (frac[k] & ~kPosMask) | p, in[p].key);
+      }
+    }
+    __syncthreads();
+    uint16_t* order = reinterpret_cast<uint16_t*>(slot);
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      const uint32_t p = tid + (uint32_t)k * THREADS;
+      if (p - lo < m) order[place[k]] = (uint16_t)p;
+    }
+    __syncthreads();
+    for (uint32_t i = tid; i < m; i += THREADS) emit(true, i, in[order[i]]);
+    return true;
   }
 
   // The sort by bins; false when a bin has too many elements (HEAVY: too many
@@ -273,24 +447,7 @@ struct TileSort {
     // their loads in flight together; the first four slots of the bin without
     // a branch (slots past the tile's last are read but not counted)
     constexpr int R = K % 3 == 0 ? 3 : K % 2 == 0 ? 2 : 1;
-    // the rank of (v, key) among the slots q[0, cnt): whole keys where key bits agree, then positions
-    auto exact = [&](const uint32_t* q, uint32_t cnt, uint32_t v, uint64_t key) {
-      uint32_t r = 0;
-      for (uint32_t j = 0; j < cnt; j += 4u) {
-        uint32_t u[4];
-        uint64_t ku[4];
-#pragma unroll
-        for (uint32_t x = 0; x < 4u; x++) u[x] = q[min(j + x, cnt - 1u)];
-#pragma unroll
-        for (uint32_t x = 0; x < 4u; x++) ku[x] = in[u[x] & kPosMask].key;
-#pragma unroll
-        for (uint32_t x = 0; x < 4u; x++) {
-          const bool tie = (u[x] ^ v) <= kPosMask && ku[x] != key;
-          r += j + x < cnt && (tie ? ku[x] < key : u[x] < v) ? 1u : 0u;
-        }
-      }
-      return r;
-    };
+    auto exact = [&](const uint32_t* q, uint32_t cnt, uint32_t v, uint64_t key) { return rank_exact(in, q, cnt, v, key); };
     bool lost = false;
     auto load_rows = [&](uint32_t row, uint32_t (&v)[R], Elem (&e)[R]) {
 #pragma unroll

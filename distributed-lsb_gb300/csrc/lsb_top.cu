@@ -17,7 +17,7 @@ namespace lsb {
 // ---------------------------------------------------------------------------
 // one CTA, one launch
 
-// Bound by latency: one read of the tile, seven barriers, one write. Twelve
+// Bound by latency: one read of the tile, nine barriers, one write. Twelve
 // launches (clears, the histogram, the plan, eight passes and the copy back)
 // took 112 us for 1000 elements with the array's own copy; this takes 11.3 us.
 template <int THREADS, int K>
@@ -61,7 +61,7 @@ __global__ void __launch_bounds__(THREADS, 1)
       atomicOr(&s_diff[1], hi);
     }
   }
-  TS::sort(in, 0, n, 0, 0, slot, bins, sh, true, [&](bool on, uint32_t r, const Elem& e) { store_elem_if(on, a + r, e); });
+  TS::sort(in, 0, n, 0, 0, slot, bins, sh, true, Uneven::kBits, [&](bool on, uint32_t r, const Elem& e) { store_elem_if(on, a + r, e); });
   // s_diff: the sort's barriers lie between
   if (threadIdx.x == 0)
     write_plan(ctrl, (uint64_t)s_diff[1] << 32 | s_diff[0], n, bits, num_digits, api_bits, sub);
@@ -89,12 +89,15 @@ static int small_sort(Elem* X, const Layout& L, Ctrl* ctrl, cudaStream_t st) {
 //   k_top_sample  one CTA: a sorted sample of the keys chooses the digits
 //   k_top_hist    one read of the keys: counts of those digits; its last CTA
 //                 writes the pass plan
-//   k_onesweep    one stable pass per digit, lowest first
+//   k_onesweep    one stable pass per digit, lowest first, as many as even keys need,
+//   k_onesweep_rest  and any further ones in one launch
 //   k_top_finish  the array is now in the order of the digits' windows; each
 //                 CTA takes whole runs of equal windows, up to a tile of them
 //                 at a time, and sorts them by the whole key
 //   k_top_merge   runs longer than a tile (the sample missed them): checked,
 //                 and sorted by chunks and merges unless they are in order
+// Keys of which so many digits would be needed, or that the last step would take
+// long for, are passed over by every byte in which they differ (choose_passes).
 // The result does not depend on the sample: it only decides how short the
 // runs are, and so the time. Measured (GB300, sort alone): 2^24 uniform 1.10 ->
 // 0.47 ms, 2^28 15.0 -> 6.5 ms, 2^29 29.4 -> 13.7 ms (two passes), 2^30 58.6 ->
@@ -108,34 +111,33 @@ constexpr int kTopSample = 4;  // keys per thread of the sample: 4096
 constexpr int kTopHistThreads = 512;
 constexpr int kTopHistUnroll = 4;
 
-// Bound by latency (one CTA: scattered reads, a tile sort, two counts: 11 us with
-// 1024 keys, 17 to 20 with 4096); it also clears what the later kernels count in,
+// Bound by latency (one CTA: scattered reads, a sort of the keys, two counts: with
+// 1024 keys 13 us under events, whatever the keys are, with 4096 up to 55); it also clears what the later kernels count in,
 // in place of three memsets.
 template <int S>
 __global__ void __launch_bounds__(kSampleThreads, 1)
     k_top_sample(const Elem* __restrict__ data, uint32_t n, SampleRule rule, uint32_t* __restrict__ hist, Ctrl* ctrl) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ typename SampleTile<S>::Shared sh;
-  __shared__ uint32_t s_near[8], s_far[11];
+  __shared__ SampleStats s_stats;
   const uint32_t tid = threadIdx.x;
   for (uint32_t i = tid; i < kCtrlBytes / 4u; i += kSampleThreads) reinterpret_cast<uint32_t*>(ctrl)[i] = 0u;
   for (uint32_t i = tid; i < 8u * 256u; i += kSampleThreads) hist[i] = 0u;
-  if (tid < 8) s_near[tid] = 0u;
-  if (tid < 11) s_far[tid] = 0u;
+  clear_stats(s_stats);
   const uint64_t* s = sample_keys<S>(data, n, smem, sh);
-  const uint64_t first = s[0], span = first ^ s[SampleTile<S>::kCap - 1u];
+  const uint64_t first = s[0], span = first ^ s[S * kSampleThreads - 1];
   const uint32_t hb1 = span ? 64u - (uint32_t)__clzll((long long)span) : 64u;
-  bool skewed, big;
-  const uint32_t t = sample_passes<S>(s, hb1, rule, s_near, s_far, &skewed, &big);
+  const SampleChoice c = choose_passes<S>(s, hb1, rule, 0u, s_stats, 0ull, [=](uint32_t t) { return hb1 > 8u * t ? hb1 - 8u * t : 0u; });
   if (tid == 0) {
     TopPlan& p = ctrl->top;
-    p.passes = t;
-    p.skewed = skewed ? 1u : 0u;
-    p.big = big ? 1u : 0u;
-    p.hb1 = hb1;
-    p.clamp = hb1 < 64u ? 1u : 0u;
-    p.lo = hb1 < 64u ? first >> hb1 << hb1 : 0ull;
-    p.hi = hb1 < 64u ? p.lo | ((1ull << hb1) - 1ull) : ~0ull;
+    const bool block = hb1 < 64u && !c.plain;
+    p.passes = c.plain ? 8u : c.passes;
+    p.skewed = (c.skewed ? 1u : 0u) | (c.dups ? 2u : 0u);
+    p.big = c.big ? 1u : 0u;
+    p.hb1 = c.plain ? 64u : hb1;
+    p.clamp = block ? 1u : 0u;
+    p.lo = block ? first >> hb1 << hb1 : 0ull;
+    p.hi = block ? p.lo | ((1ull << hb1) - 1ull) : ~0ull;
   }
 }
 
@@ -187,27 +189,51 @@ __device__ __forceinline__ void count_windows(const Elem* __restrict__ data, uin
   *diff = acc;
 }
 
-// The same for five to eight digits, which only unusual keys need.
+// The same for five to eight digits: bytes of two words. (2^26 keys, five digits:
+// 590 us a key and a digit at a time, 178 so.)
+template <bool CLAMP>
 __device__ __noinline__ void count_many_windows(const Elem* __restrict__ data, uint32_t n, const TopPlan& p,
                                                 uint32_t* h, uint64_t first, uint64_t* diff) {
+  const uint32_t lane = lane_id();
   const uint64_t warps_total = (uint64_t)gridDim.x * (kTopHistThreads / 32);
   const uint64_t gw = (uint64_t)blockIdx.x * (kTopHistThreads / 32) + (threadIdx.x >> 5);
-  const int T = (int)p.passes;
+  constexpr uint32_t chunk = 32u * kTopHistUnroll;
+  const uint64_t block_lo = p.lo, block_hi = p.hi;
+  const uint32_t left = 64u - p.hb1;
+  const int low = 8 - (int)p.passes;  // lowest byte that is a digit
   uint64_t acc = 0;
-  for (uint64_t base = gw * 32u; base < n; base += warps_total * 32u) {
-    const bool valid = base + lane_id() < n;
-    const uint64_t key = valid ? load_elem_stream(data + base + lane_id()).key : first;
-    acc |= key ^ first;
-    const bool whole = base + 32u <= n;
-    for (int t = 0; t < T; t++) {
-      const TopWindow w = top_window(p, t);
-      const uint32_t d = w.clamp ? top_digit_clamped(w, key) : top_digit(w, key);
-      if (whole && __all_sync(0xffffffffu, d == __shfl_sync(0xffffffffu, d, 0))) {
-        if (lane_id() == 0) atomicAdd(&h[t * 256 + d], 32u);
-      } else if (valid) {
-        atomicAdd(&h[t * 256 + d], 1u);
+  auto digits_of = [&](uint64_t key) {
+    return CLAMP ? (key < block_lo ? 0ull : key > block_hi ? ~0ull : key << left) : key << left;
+  };
+  const uint64_t full_end = (uint64_t)n / chunk * chunk;
+  for (uint64_t base = gw * chunk; base < full_end; base += warps_total * chunk) {
+    uint64_t key[kTopHistUnroll];
+#pragma unroll
+    for (int u = 0; u < kTopHistUnroll; u++) key[u] = load_elem_stream(data + base + (uint64_t)u * 32u + lane).key;
+#pragma unroll
+    for (int u = 0; u < kTopHistUnroll; u++) {
+      acc |= key[u] ^ first;
+      const uint64_t d = digits_of(key[u]);
+#pragma unroll
+      for (int half = 1; half >= 0; half--) {
+        const uint32_t w = (uint32_t)(d >> (32 * half));
+        const uint32_t x = __reduce_or_sync(0xffffffffu, w ^ __shfl_sync(0xffffffffu, w, 0));
+#pragma unroll
+        for (int t = 3; t >= 0; t--) {
+          if (half == 0 && t < low) break;
+          uint32_t* c = &h[(4 * half + t - low) * 256 + ((w >> (8 * t)) & 255u)];
+          if ((x >> (8 * t)) & 255u) atomicAdd(c, 1u);
+          else if (lane == 0) atomicAdd(c, 32u);
+        }
       }
     }
+  }
+  for (uint64_t i = full_end + (uint64_t)blockIdx.x * kTopHistThreads + threadIdx.x; i < n;
+       i += (uint64_t)gridDim.x * kTopHistThreads) {
+    const uint64_t key = load_elem_stream(data + i).key;
+    acc |= key ^ first;
+    const uint64_t d = digits_of(key);
+    for (int t = low; t < 8; t++) atomicAdd(&h[(t - low) * 256 + ((d >> (8 * t)) & 255u)], 1u);
   }
   *diff = acc;
 }
@@ -237,7 +263,7 @@ __global__ void __launch_bounds__(kTopHistThreads, 4)
       case 2: count_windows<2, true>(data, n, p, h, first, &diff); break;
       case 3: count_windows<3, true>(data, n, p, h, first, &diff); break;
       case 4: count_windows<4, true>(data, n, p, h, first, &diff); break;
-      default: count_many_windows(data, n, p, h, first, &diff); break;
+      default: count_many_windows<true>(data, n, p, h, first, &diff); break;
     }
   } else {
     switch (T) {
@@ -245,7 +271,7 @@ __global__ void __launch_bounds__(kTopHistThreads, 4)
       case 2: count_windows<2, false>(data, n, p, h, first, &diff); break;
       case 3: count_windows<3, false>(data, n, p, h, first, &diff); break;
       case 4: count_windows<4, false>(data, n, p, h, first, &diff); break;
-      default: count_many_windows(data, n, p, h, first, &diff); break;
+      default: count_many_windows<false>(data, n, p, h, first, &diff); break;
     }
   }
   {
@@ -269,42 +295,11 @@ __global__ void __launch_bounds__(kTopHistThreads, 4)
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  const uint32_t warp = threadIdx.x >> 5, lane = lane_id();
-  if (warp < T) {  // warp t scans digit t: exclusive starts, and whether one value holds every key
-    uint32_t c[8], sum = 0;
-    bool one = false;
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-      c[i] = __ldcg(&hist[warp * 256u + lane * 8u + i]);
-      one |= c[i] == n;
-      sum += c[i];
-    }
-    uint32_t inc = sum;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
-      if (lane >= (uint32_t)o) inc += y;
-    }
-    uint32_t off = inc - sum;
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-      gstart[warp * 256u + lane * 8u + i] = off;
-      off += c[i];
-    }
-    if (__any_sync(0xffffffffu, one) && lane == 0) atomicOr(&s_const, 1u << warp);
-  }
+  scan_digits(hist, gstart, n, T, &s_const);
   __syncthreads();
   if (threadIdx.x == 0) {
     TopPlan& q = ctrl->top;
     const uint64_t d = (uint64_t)__ldcg(&q.diff[1]) << 32 | __ldcg(&q.diff[0]);
-    uint32_t par = 0, pars = 0, run = 0;
-    for (uint32_t t = 0; t < T; t++) {
-      pars |= par << t;
-      if (!((s_const >> t) & 1u)) {
-        run |= 1u << t;
-        par ^= 1u;
-      }
-    }
     if (single) {  // every pass runs, so that the result lands in its place whatever the digits
       const uint32_t constant = single == 1u ? s_const & 1u : 0u;
       q.run_mask = (1u << T) - 1u;
@@ -318,9 +313,7 @@ __global__ void __launch_bounds__(kTopHistThreads, 4)
       ctrl->n = n;
       return;
     }
-    q.run_mask = run;
-    q.par_mask = pars;
-    q.src_parity = par;
+    chain_passes(q, T, s_const);
     // keys in the block, as usual: no pass need look
     const bool inside = q.hb1 >= 64u || ((d | (first ^ q.lo)) >> q.hb1) == 0;
     q.clamp = inside ? 0u : 1u;
@@ -373,7 +366,7 @@ __global__ void __launch_bounds__(TS::kThreads, CTAS)
     mbar_init(bar, 1);
     fence_mbar_init();
   }
-  const bool clamped = plan.clamp != 0u, skewed = plan.skewed != 0u;
+  const bool clamped = plan.clamp != 0u, skewed = (plan.skewed & 1u) != 0u, dups = (plan.skewed & 2u) != 0u;
   const uint32_t shift = run_key(plan).shift;
   const uint32_t parts = (uint32_t)(((uint64_t)n + stride - 1u) / stride);
   uint32_t phase = 0;
@@ -382,7 +375,7 @@ __global__ void __launch_bounds__(TS::kThreads, CTAS)
   for (uint32_t part = blockIdx.x; part < parts; part += gridDim.x) {
     const uint32_t g = (uint32_t)((uint64_t)part * stride);
     const uint32_t limit = (uint32_t)min((uint64_t)g + stride, (uint64_t)n);
-    if (!sort_runs<TS>(src, X, n, g, limit, part == 0, s_w, clamped, skewed, shift, in, slot, bins, sh, s_marks, load,
+    if (!sort_runs<TS>(src, X, n, g, limit, part == 0, s_w, clamped, skewed, dups, shift, in, slot, bins, sh, s_marks, load,
                          long_run))
       return;
   }
@@ -490,7 +483,7 @@ __global__ void __launch_bounds__(Tile::kThreads, 2)
           }
           __syncthreads();
           Elem* out = ((rounds_of(t) & 1u) ? Y : X) + t.b + pos;
-          Tile::sort(in, 0, cnt, 0, 0, slot, bins, sh, out == src,
+          Tile::sort(in, 0, cnt, 0, 0, slot, bins, sh, out == src, Uneven::kSpread,
                      [&](bool on, uint32_t r, const Elem& e) { store_elem_if(on, out + r, e); });
         } else if (const uint32_t r = step - 2u, mine = rounds_of(t); r < mine) {
           const Elem* from = (((mine - r) & 1u) ? Y : X) + t.b;
@@ -594,10 +587,10 @@ int top_pass_run(const Elem* src, Elem* mid, Elem* dst, int first_digit, unsigne
   }
   if (int rc = top_hist(src, ws, L, passes, dev, st)) return rc;
   Elem* in = const_cast<Elem*>(src);  // read only: pass 0 reads X
-  if (int rc = onesweep_top_pass(in, passes == 1u ? dst : mid, L.n, 0, gstart, ring, L.ring_tiles, ctrl, SegDesc{}, 0, 0u, false, dev, st))
+  if (int rc = onesweep_top_pass(in, passes == 1u ? dst : mid, L.n, 0, gstart, ring, L.ring_tiles, ctrl, SegDesc{}, 0, 0u, dev, st))
     return rc;
   if (passes == 1u) return 0;
-  return onesweep_top_pass(dst, mid, L.n, 1, gstart + 256u, ring, L.ring_tiles, ctrl, SegDesc{}, 0, 0u, false, dev, st);
+  return onesweep_top_pass(dst, mid, L.n, 1, gstart + 256u, ring, L.ring_tiles, ctrl, SegDesc{}, 0, 0u, dev, st);
 }
 
 // ---------------------------------------------------------------------------
@@ -622,7 +615,8 @@ int top_run(Elem* X, Elem* Y, unsigned char* ws, const Layout& L, cudaStream_t s
   // elements: 89 against 104 us). Where it can save the third, it is launched
   // beside the other one and the sample decides, which may find keys denser than
   // even ones: 2^29 uniform keys 15.5 -> 13.7 ms, 2^28 of a 29-bit range 8.2 -> 6.7
-  // ms. Else even runs up to kSmallRun leave the small one half full or better,
+  // ms. (After two windows only: behind more of them are clusters, whose runs it
+  // cannot tell from longer ones.) Else even runs up to kSmallRun leave the small one half full or better,
   // with six standard deviations of room.
   const uint32_t least = passes_for((float)n, (float)kMeanRun);
   const bool only_big = least == 2u && n <= 256u * 7600u;  // runs of repeated keys vary more
@@ -632,22 +626,11 @@ int top_run(Elem* X, Elem* Y, unsigned char* ws, const Layout& L, cudaStream_t s
   // a smaller sample decides as well for fewer elements, and 5 us sooner
   const bool short_sample = n < (1u << 26);
   const uint32_t mean_run = only_big ? kBigRun : small_tile ? kSmallRun : kMeanRun;
-  SampleRule rule = sample_rule(n, short_sample ? SampleTile<1>::kCap : SampleTile<kTopSample>::kCap, mean_run, mean_run,
+  const uint32_t tile = only_big ? BigTile::kCap : small_tile ? SmallTile::kCap : Tile::kCap;
+  SampleRule rule = sample_rule(n, kSampleThreads * (short_sample ? 1u : (uint32_t)kTopSample), tile, mean_run, mean_run,
                                 n <= (1u << 28) ? 16.0f : 4.0f);  // four passes for heavy keys up to 2^30 elements
-  // With so few windows most neighbours share one, and hardly more do when runs
-  // are twice as long, all for the merges (1.6 10^6 nearly sorted keys: 167 us, with
-  // a pass more 115): the limit is that of even runs, and three standard deviations.
-  if (only_big) {
-    const double lam = (double)kBigRun * SampleTile<1>::kCap / n, f = 1.0 - (1.0 - std::exp(-lam)) / lam;
-    rule.near_limit = (uint32_t)(SampleTile<1>::kCap * f + 3.0 * std::sqrt(SampleTile<1>::kCap * f * (1.0 - f)));
-  }
-  // Unused launches cost about 2 us each: below 2^26 elements only the four
-  // passes of heavy keys, or two more than even keys need, are kept ready, and
-  // the merges, whose rounds then stay nearly in L2, take what those leave.
-  if (n < (1u << 26)) rule.tmax = std::max(4u, std::min(8u, rule.tmin + 2u));
   if (may_big) {
-    const SampleRule wide = sample_rule(n, SampleTile<kTopSample>::kCap, (uint32_t)(kBigRun / 1.25f), kBigRun, 16.0f);
-    rule.big_tmin = 2u;
+    const SampleRule wide = sample_rule(n, kSampleThreads * (uint32_t)kTopSample, BigTile::kCap, kBigRun, kBigRun, 16.0f);
     rule.big_near = wide.near_limit;
   }
   static std::atomic<uint64_t> allowed[5];
@@ -659,11 +642,11 @@ int top_run(Elem* X, Elem* Y, unsigned char* ws, const Layout& L, cudaStream_t s
     sample<<<1, kSampleThreads, sample_smem, st>>>(X, n, rule, hist, ctrl);
   }
   if (int rc = top_hist(X, ws, L, 0u, dev, st)) return rc;
-  for (uint32_t p = 0; p < rule.tmax; p++) {
-    const bool spare = p >= rule.tmin - (may_big ? 1u : 0u);  // one that even keys do not need: most return at once
-    if (int rc = onesweep_top_pass(X, Y, n, (int)p, gstart + p * 256u, ring, L.ring_tiles, ctrl, SegDesc{}, 0, 0u, spare, dev, st))
+  for (uint32_t p = 0; p < rule.tmin; p++)  // (one may not be in the plan: the big tile's)
+    if (int rc = onesweep_top_pass(X, Y, n, (int)p, gstart + p * 256u, ring, L.ring_tiles, ctrl, SegDesc{}, 0, 0u, dev, st))
       return rc;
-  }
+  if (int rc = onesweep_top_rest(X, Y, n, (int)rule.tmin, gstart, ring, L.ring_tiles, ctrl, SegDesc{}, 0, 0u, dev, st))
+    return rc;
   RunChunk* chunks = reinterpret_cast<RunChunk*>(ring);
   uint32_t* unsorted = reinterpret_cast<uint32_t*>(chunks + max_chunks(n));
   // A tile is left a run short on average (its last run is not whole), so a
