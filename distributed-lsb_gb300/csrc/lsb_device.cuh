@@ -53,6 +53,7 @@ struct TopPlan {
   uint32_t skewed;         // bit 0: heavy keys, tiles of runs are mostly in order; bit 1: most keys are duplicates
   uint32_t complete;       // the digits cover every bit in which keys differ
   uint32_t diff[2];        // bits in which some key differs from the first one
+  uint32_t copy;           // a single pass whose digit is constant: the array is copied
   uint32_t apart[2];       // and from one key that agrees with it in the top window
   uint32_t hist_done;      // CTAs of the histogram that have finished
   uint32_t num_chunks;     // chunks of runs too long for a tile

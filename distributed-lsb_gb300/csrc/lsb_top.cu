@@ -302,6 +302,7 @@ __global__ void __launch_bounds__(kTopHistThreads, 4)
     const uint64_t d = (uint64_t)__ldcg(&q.diff[1]) << 32 | __ldcg(&q.diff[0]);
     if (single) {  // every pass runs, so that the result lands in its place whatever the digits
       const uint32_t constant = single == 1u ? s_const & 1u : 0u;
+      q.copy = constant;
       q.run_mask = (1u << T) - 1u;
       q.par_mask = 2u;
       ctrl->skip_mask_lo = constant;

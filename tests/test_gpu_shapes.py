@@ -143,3 +143,17 @@ def test_passes_not_merges(lsb, cuda, n):
         lsb.profile_enable(False)
         ms = {k: v[1] for k, v in lsb.profile_read().items()}
         assert ms["top_merge"] < 0.2 * sum(ms.values()), (name, ms)
+
+
+@pytest.mark.parametrize("n", [1, 8193, 8192 * 152 + 77, 3000001])
+def test_pass_over_a_constant_digit(lsb, cuda, n):
+    """A single pass whose digit is the same in all keys copies the array, over more
+    than one round of every CTA too; the source stays as it was."""
+    torch = cuda
+    a = _array(torch, torch.randint(0, 1 << 32, (n,), dtype=torch.int64, device="cuda"))
+    src, dst = a.clone(), torch.zeros_like(a)
+    ws = torch.empty(lsb.pass_workspace_bytes(n, 8), dtype=torch.uint8, device="cuda")
+    lsb.global_shuffle(src, dst, 5, 8, workspace=ws)
+    st = lsb.query(ws)
+    assert (st.device_status, st.skipped_mask, st.passes_run) == (0, 1, 0)
+    assert torch.equal(dst, a) and torch.equal(src, a)
