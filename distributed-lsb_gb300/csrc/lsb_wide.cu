@@ -209,7 +209,10 @@ __device__ __forceinline__ void byte_flush(const uint32_t* words, uint32_t* g) {
 // ---------------------------------------------------------------------------
 // histogram of ND 16-bit digits, one read of the keys
 
-constexpr int kH16Threads = 1024;
+// One digit per CTA: three CTAs of 512 threads per SM (in two of 1024 the counters
+// of LSB_HIST16=quads spill: 2^30 keys 9.7 ms, so 5.1); else one of 1024.
+constexpr int h16_threads(int nd) { return nd == 1 ? 512 : 1024; }
+constexpr uint32_t h16_ctas(int nd) { return nd == 1 ? 3u : 1u; }
 constexpr int kH16Unroll = 8;
 
 // group == 1: the CTAs share the whole array (grid-stride) and count digits
@@ -225,7 +228,7 @@ constexpr int kH16Unroll = 8;
 // them up; without it they go to the counts by one global atomic for each bin
 // that is not empty, which for 2^26 even keys took a third of the time.
 template <int ND>
-__global__ void __launch_bounds__(kH16Threads, ND == 1 ? 2 : 1)
+__global__ void __launch_bounds__(h16_threads(ND), h16_ctas(ND))
     k_hist16(const Elem* __restrict__ data, uint32_t n, int first_digit,
              uint32_t* __restrict__ ghist, uint32_t group, uint32_t* __restrict__ dump) {
   extern __shared__ __align__(16) uint32_t cw[];  // [ND][16384]
@@ -376,7 +379,7 @@ __global__ void __launch_bounds__(256)
 // d_counts[num_digits][65536] (uint32; zeroed here). Four digits: one HBM read
 // by groups of CTAs over the same range (L2 serves the group's other reads),
 // "pairs" of CTAs with two digits each (128 KiB, one CTA per SM) by default;
-// LSB_HIST16 selects "quads" (one digit each, 64 KiB, two CTAs per SM) or
+// LSB_HIST16 selects "quads" (one digit each, 64 KiB, three CTAs per SM) or
 // "split" (a read per three digits). All give the same counts. Where a CTA
 // counts 2^14 keys or more its counters are stored and summed up by a second
 // kernel (scratch: they may come from the library's pool): 4 10^6 keys 74 -> 41
@@ -398,15 +401,15 @@ static int hist16_launch(const Elem* data, uint32_t n, int first_digit, uint32_t
   if (!allow_smem((const void*)k_hist16<ND>, smem, &allowed)) return 5;
   // enough groups to fill every resident slot, none with less than a round of
   // work (65537 keys 29 -> 19 us against groups of four rounds)
-  const uint64_t least = (uint64_t)kH16Threads * kH16Unroll;
+  const uint64_t least = (uint64_t)h16_threads(ND) * kH16Unroll;
   const uint64_t want = ((uint64_t)n + least - 1) / least;
-  const uint64_t slots = std::max<uint64_t>(1, (uint64_t)dev.sm_count * (ND == 1 ? 2u : 1u) / group);
+  const uint64_t slots = std::max<uint64_t>(1, (uint64_t)dev.sm_count * h16_ctas(ND) / group);
   const uint32_t groups = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(want, slots));
   void* dump = nullptr;
   if (scratch && n / groups >= (1u << 14) && pool_alloc(&dump, (size_t)group * groups * smem, st) != 0) dump = nullptr;
   {
     ProfScope prof("hist16", st);
-    k_hist16<ND><<<group * groups, kH16Threads, smem, st>>>(data, n, first_digit, d_counts, group,
+    k_hist16<ND><<<group * groups, h16_threads(ND), smem, st>>>(data, n, first_digit, d_counts, group,
                                                             static_cast<uint32_t*>(dump));
   }
   if (dump) {
