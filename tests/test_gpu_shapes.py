@@ -89,20 +89,25 @@ def test_batches_sorted_stably(lsb, cuda, variant):
         assert torch.equal(got[:, 0], keys[order]) and torch.equal(got[:, 1] - int(off[s]), order), s
 
 
-@pytest.mark.parametrize("far", [False, True])
+@pytest.mark.parametrize("far", [False, True, "five", "clamped"])
 def test_many_digits_of_a_large_array(lsb, cuda, far):
     """Above 2^26 elements (a larger sample): half of the keys even, half in a cluster
-    of 2^20 neighbours, so that every digit is passed over; a dense block with a gap
-    in it, and the same with keys far outside the block, which are clamped to it. Also
-    as one array of a batch."""
+    of 2^20 neighbours, so that every digit is passed over; a block with a gap in it
+    and keys far outside; a cluster of 2^32, which five or six digits part, in the
+    whole range and in a block with keys outside, which are clamped to it. Also as one
+    array of a batch."""
     torch = cuda
     n = (1 << 26) + 12345
     g = torch.Generator(device="cuda")
-    g.manual_seed(n + far)
+    g.manual_seed(n + len(str(far)))
     u = torch.randint(SIGN, (1 << 63) - 1, (n,), dtype=torch.int64, device="cuda", generator=g)
     even = torch.rand(n, device="cuda", generator=g) < 0.5
     near = (5 << 40) + (u & 0xFFFFF)
-    if far:  # 47 bits, five to six digits of a block that three keys are outside of
+    if far in ("five", "clamped"):
+        keys = torch.where(even, u if far == "five" else u & 0xFFFFFFFFFFFFFF, (5 << 40) + (u & 0xFFFFFFFF))
+        if far == "clamped":
+            keys[[5, n // 2, n - 7]] = torch.tensor([-1, -2, 1 << 62], dtype=torch.int64, device="cuda")
+    elif far:  # a block of 47 bits that three keys are outside of
         keys = torch.where(even, (u & 0x7F) << 40, near & 0x7FFFFFFFFFF)
         keys[[5, n // 2, n - 7]] = torch.tensor([-1, -2, 1 << 62], dtype=torch.int64, device="cuda")
     else:
