@@ -136,7 +136,10 @@ int lsb_pass(const lsb_elem_t* d_src, lsb_elem_t* d_dst, int64_t n, int digit_bi
  * d_counts[p * 2^b + d] (int64, lsb_num_passes(b) * 2^b entries, device memory)
  * = number of elements whose digit p equals d. This is the count loop of
  * localShuffle (mpi/mpi_lsbsort.cpp:237-241) for all digits at once, summed
- * over ranks like GlobalCounts (mpi/mpi_lsbsort.cpp:339-395). Asynchronous. */
+ * over ranks like GlobalCounts (mpi/mpi_lsbsort.cpp:339-395). Asynchronous. Scratch
+ * comes from the library's pool, which keeps it for later calls: at 16 bits and from
+ * about 10^6 elements 128 KiB for each SM (20 MB), and where that is not to be had
+ * the counts are taken without it. */
 int lsb_histogram(const lsb_elem_t* d_data, int64_t n, int digit_bits, int64_t* d_counts,
                   void* stream);
 
