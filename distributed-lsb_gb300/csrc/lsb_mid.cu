@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(kMidThreads, 1)
     uint64_t diff;         // bits in which keys differ
     uint32_t all;          // passes over all of those, which leave nothing to sort
     uint32_t passes, full;  // windows passed over, and those that there are
-    bool exact, skewed, dups;
+    bool skewed, dups;
   } s_plan;
   __shared__ RunMarks s_marks;
   __shared__ RunKey s_w;
@@ -327,6 +327,20 @@ __global__ void __launch_bounds__(kMidThreads, 1)
   };
   auto scatter = [&](Elem* dst) {
     const uint32_t m = tile_len(tile_begin());
+    const MidDigit& g = s_digit[s_window];
+    if (g.runs == 1u && !win.clamp) {  // as most digits are
+      const uint32_t shift = g.shift[0], mask = g.mask[0];
+#pragma unroll
+      for (int k = 0; k < K; k++) {
+        const uint32_t p = tid + (uint32_t)k * kMidThreads;
+        if (p < m) {
+          const Elem e = in[order[p]];
+          const uint32_t o = s_delta[(uint32_t)(e.key >> shift) & mask] + p;
+          if (o < n) store_elem(dst + o, e);
+        }
+      }
+      return;
+    }
 #pragma unroll 1
     for (uint32_t row = tid; row < E; row += (uint32_t)(R * kMidThreads)) {
       uint64_t key[R], val[R];
@@ -338,7 +352,7 @@ __global__ void __launch_bounds__(kMidThreads, 1)
         key[k] = e.key;
         val[k] = e.val;
       }
-      mid_digits<R>(s_digit[s_window], win, key, d);
+      mid_digits<R>(g, win, key, d);
 #pragma unroll
       for (int k = 0; k < R; k++) {
         const uint32_t p = row + (uint32_t)k * kMidThreads;
@@ -351,7 +365,6 @@ __global__ void __launch_bounds__(kMidThreads, 1)
   // 1. the tile, and the bits in which keys differ
   if (tid < 2) s_diff[tid] = 0u;
   clear_stats(s_stats);
-  if (tid == 0) s_bits[0] = 0ull;
   const uint64_t first_key = ld_relaxed_u64(&X[0].key);
   if (CLUSTER) {
     if (t == 0)
@@ -441,39 +454,35 @@ __global__ void __launch_bounds__(kMidThreads, 1)
 
   // 2. the top digit alone, 3. or the digits that the sample says
   if (tid == 0) win.clamp = false;
-  if (tid == 0) s_plan = {diff, all, 1u, all, false, false, false};
+  if (tid == 0) s_plan = {diff, all, 1u, all, false, false};
   auto low_bit = [&](uint32_t windows) { return (uint32_t)__ffsll((long long)s_bits[windows - 1u]) - 1u; };
-  uint64_t top_bits;  // the first window's
-  {
+  if (tid == 0) {  // the first window: the eight highest bits that vary, mostly neighbours
     const uint32_t hb1 = 64u - (uint32_t)__clzll((long long)diff);
-    top_bits = diff & bits_below(hb1, 8u);
-    if (tid == 0 && __popcll(top_bits) == 8) {
+    s_window = 0u;
+    if (hb1 >= 8u && diff >> (hb1 - 8u) == 255u) {
       s_digit[0].runs = 1u;
       s_digit[0].shift[0] = hb1 - 8u;
       s_digit[0].mask[0] = 255u;
-      s_bits[0] = top_bits;
+      s_bits[0] = 255ull << (hb1 - 8u);
+    } else {
+      uint64_t top = 0;
+      for (uint64_t rest = diff; rest && __popcll(top) < 8; rest = diff & ~top) top |= 1ull << (63u - (uint32_t)__clzll((long long)rest));
+      s_bits[0] = top;
+      set_digit(s_digit[0], top);
     }
-    while (__popcll(top_bits) < 8 && top_bits != diff) {
-      const uint64_t rest = diff & ~top_bits;
-      top_bits |= 1ull << (63u - (uint32_t)__clzll((long long)rest));
-    }
-  }
-  if (tid == 0) {
-    s_window = 0u;
-    if (s_bits[0] != top_bits) set_digit(s_digit[0], s_bits[0] = top_bits);
   }
   count_tile();
+  // a tile or two for each CTA: the ways of duplicates are the ones to try first
+  // unless there are bits that would make other keys uneven
+  if (tid == 32u) s_plan.dups = !ragged(low_bit(1u), 13u, 5u, diff);
   if (!all_arrived()) return;
   add_up();
-  if (all == 1u || s_max <= MidTile::kCap) {
-    // (a tile or two for each CTA: the ways of duplicates are the ones to try first
-    // unless there are bits that would make other keys uneven)
-    if (tid == 0) s_plan.exact = true, s_plan.dups = !ragged(low_bit(1u), 13u, 5u, diff);
-    __syncthreads();
-  } else {
+  const bool exact = all == 1u || s_max <= MidTile::kCap;
+  if (!exact) {
+    const uint64_t top_bits = s_bits[0];
     if (tid == 0) s_plan.passes = all;
-    set_windows(diff);
     __syncthreads();
+    set_windows(diff);
     if (all > kMidFewPasses) {
       uint64_t* buf = reinterpret_cast<uint64_t*>(smem + kMidSampleAt);
       const uint64_t* s = sort_sample(sample_key(X, n, tid), buf);
@@ -520,7 +529,7 @@ __global__ void __launch_bounds__(kMidThreads, 1)
   for (bool first = true;; first = false) {
     uint32_t par = 0;
     for (uint32_t p = 0; p < s_plan.passes; p++) {
-      if (p || !first || !s_plan.exact) {
+      if (p || !first || !exact) {
         if (p || !first) load_tile(par ? Y : X);  // else it is still there
         if (tid == 0) s_window = s_plan.passes - 1u - p;
         buf ^= 1u;
@@ -542,7 +551,6 @@ __global__ void __launch_bounds__(kMidThreads, 1)
     }
     // the runs that start in this CTA's part of the array
     const uint32_t shift = low_bit(s_plan.passes);
-    const bool exact = s_plan.exact;
     uint32_t g = (uint32_t)((uint64_t)n * blockIdx.x / gridDim.x);
     uint32_t limit = (uint32_t)((uint64_t)n * (blockIdx.x + 1u) / gridDim.x);
     bool known = blockIdx.x == 0;
