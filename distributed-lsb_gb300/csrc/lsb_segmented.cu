@@ -564,14 +564,10 @@ int lsb_tune_segmented(const int64_t* h_seg_offsets, int64_t nseg, lsb_tuning_t*
   const int64_t sseg = (int64_t)off.size() - 1;
   if (sn <= 1) return LSB_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  const int cand_bits[] = {8};  // the kernels choose their own digits: the width changes nothing
+  const int width = 8;  // the kernels choose their own digits: another width changes nothing
   const int cand_var[] = {0, 2};
   size_t wsb = 0;
-  for (int cb : cand_bits) {
-    size_t x = 0;
-    if (int rc = lsb_segmented_workspace_bytes(sn, sseg, cb, &x)) return rc;
-    wsb = std::max(wsb, x);
-  }
+  if (int rc = lsb_segmented_workspace_bytes(sn, sseg, width, &wsb)) return rc;
   DeviceInfo dev;
   if (int rc = current_device_info(&dev)) return rc;
   // CTA counts: every resident slot, or one CTA per SM with two-CTA shapes, or half the SMs
@@ -594,14 +590,13 @@ int lsb_tune_segmented(const int64_t* h_seg_offsets, int64_t nseg, lsb_tuning_t*
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (rc == LSB_OK && (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess))
     rc = LSB_ERR_CUDA;
-  for (int cb : cand_bits) {
-    for (int cv : cand_var) {
-     for (int cc : cand_ctas) {
+  for (int cv : cand_var) {
+    for (int cc : cand_ctas) {
       if (rc != LSB_OK) break;
       if (cv == 0 && cc == dev.sm_count) continue;  // the variant-0 default is already one CTA per SM
       lsb_tuning_t t;
       std::memset(&t, 0, sizeof t);
-      t.digit_bits = cb;
+      t.digit_bits = width;
       t.variant = cv;
       t.ctas = cc;
       float total = 0.f;
@@ -621,7 +616,6 @@ int lsb_tune_segmented(const int64_t* h_seg_offsets, int64_t nseg, lsb_tuning_t*
         best_ms = total;
         best = t;
       }
-     }
     }
   }
   if (e0) cudaEventDestroy(e0);
