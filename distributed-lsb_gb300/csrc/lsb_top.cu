@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(kSampleThreads, 1)
   const uint64_t* s = sample_keys<S>(data, n, smem, sh);
   const uint64_t first = s[0], span = first ^ s[S * kSampleThreads - 1];
   const uint32_t hb1 = span ? 64u - (uint32_t)__clzll((long long)span) : 64u;
-  const SampleChoice c = choose_passes<S>(s, hb1, rule, 0u, s_stats, 0ull, [=](uint32_t t) { return hb1 > 8u * t ? hb1 - 8u * t : 0u; });
+  const SampleChoice c = choose_passes<S, true>(s, hb1, rule, 0u, s_stats, 0ull, [=](uint32_t t) { return hb1 > 8u * t ? hb1 - 8u * t : 0u; });
   if (tid == 0) {
     TopPlan& p = ctrl->top;
     const bool block = hb1 < 64u && !c.plain;
@@ -612,28 +612,32 @@ int top_run(Elem* X, Elem* Y, unsigned char* ws, const Layout& L, cudaStream_t s
   uint32_t* gstart = reinterpret_cast<uint32_t*>(ws + L.off_gstart);
   uint64_t* ring = reinterpret_cast<uint64_t*>(ws + L.off_ring);
   // The tile of the last step. The big one is slower (one CTA per SM) but holds
-  // runs twice as long. It is the only one where it leaves one pass (1.5M
-  // elements: 89 against 104 us). Where it can save the third, it is launched
+  // runs twice as long. Where it can save the second or third pass, it is launched
   // beside the other one and the sample decides, which may find keys denser than
   // even ones: 2^29 uniform keys 15.5 -> 13.7 ms, 2^28 of a 29-bit range 8.2 -> 6.7
-  // ms. (After two windows only: behind more of them are clusters, whose runs it
-  // cannot tell from longer ones.) Else even runs up to kSmallRun leave the small one half full or better,
+  // ms, 1.5 10^6 neighbours 101 -> 86 us (uniform keys 96 -> 95; as the only tile there it
+  // took 221 instead of 111 us for keys that occur a thousand times). Up to 7600 elements in a
+  // run of one pass: 2.05 10^6 uniform keys 103 -> 93 us, but with a thousandth of
+  // sentinels 132 -> 179. (After the one or two top windows only: behind more of them are clusters,
+  // whose runs it cannot tell from longer ones.) Else even runs up to kSmallRun leave the small one half full or better,
   // with six standard deviations of room.
   const uint32_t least = passes_for((float)n, (float)kMeanRun);
-  const bool only_big = least == 2u && n <= 256u * 7600u;  // runs of repeated keys vary more
-  const bool may_big = n > (1u << 27) && n <= 65536u * kBigRun;
-  const double even_run = (double)n / std::pow(256.0, (double)(only_big ? 1u : least));
+  const uint32_t big_passes = least == 2u && n <= 256u * 7600u ? 1u : n > (1u << 27) && n <= 65536u * kBigRun ? 2u : 0u;
+  const double even_run = (double)n / std::pow(256.0, (double)least);
   const bool small_tile = even_run <= (double)kSmallRun;
   // a smaller sample decides as well for fewer elements, and 5 us sooner
   const bool short_sample = n < (1u << 26);
-  const uint32_t mean_run = only_big ? kBigRun : small_tile ? kSmallRun : kMeanRun;
-  const uint32_t tile = only_big ? BigTile::kCap : small_tile ? SmallTile::kCap : Tile::kCap;
+  const uint32_t mean_run = small_tile ? kSmallRun : kMeanRun;
+  const uint32_t tile = small_tile ? SmallTile::kCap : Tile::kCap;
   SampleRule rule = sample_rule(n, kSampleThreads * (short_sample ? 1u : (uint32_t)kTopSample), tile, mean_run, mean_run,
                                 n <= (1u << 28) ? 16.0f : 4.0f);  // four passes for heavy keys up to 2^30 elements
-  if (may_big) {
-    const SampleRule wide = sample_rule(n, kSampleThreads * (uint32_t)kTopSample, BigTile::kCap, kBigRun, kBigRun, 16.0f);
+  if (big_passes) {
+    const SampleRule wide = sample_rule(n, kSampleThreads * (short_sample ? 1u : (uint32_t)kTopSample), BigTile::kCap, kBigRun, kBigRun, 16.0f);
+    rule.big_passes = big_passes;
     rule.big_near = wide.near_limit;
+    rule.big_far = big_passes == 1u ? wide.far : rule.far;
   }
+  const uint32_t lead = big_passes == 1u ? 1u : rule.tmin;  // passes with a launch each
   static std::atomic<uint64_t> allowed[5];
   const auto sample = short_sample ? k_top_sample<1> : k_top_sample<kTopSample>;
   const size_t sample_smem = short_sample ? kSampleSmem<1> : kSampleSmem<kTopSample>;
@@ -643,10 +647,10 @@ int top_run(Elem* X, Elem* Y, unsigned char* ws, const Layout& L, cudaStream_t s
     sample<<<1, kSampleThreads, sample_smem, st>>>(X, n, rule, hist, ctrl);
   }
   if (int rc = top_hist(X, ws, L, 0u, dev, st)) return rc;
-  for (uint32_t p = 0; p < rule.tmin; p++)  // (one may not be in the plan: the big tile's)
+  for (uint32_t p = 0; p < lead; p++)  // (one may not be in the plan: the big tile's)
     if (int rc = onesweep_top_pass(X, Y, n, (int)p, gstart + p * 256u, ring, L.ring_tiles, ctrl, SegDesc{}, 0, 0u, dev, st))
       return rc;
-  if (int rc = onesweep_top_rest(X, Y, n, (int)rule.tmin, gstart, ring, L.ring_tiles, ctrl, SegDesc{}, 0, 0u, dev, st))
+  if (int rc = onesweep_top_rest(X, Y, n, (int)lead, gstart, ring, L.ring_tiles, ctrl, SegDesc{}, 0, 0u, dev, st))
     return rc;
   RunChunk* chunks = reinterpret_cast<RunChunk*>(ring);
   uint32_t* unsorted = reinterpret_cast<uint32_t*>(chunks + max_chunks(n));
@@ -668,11 +672,9 @@ int top_run(Elem* X, Elem* Y, unsigned char* ws, const Layout& L, cudaStream_t s
     kernel<<<grid, TS::kThreads, TS::kSmem, st>>>(X, Y, n, stride, chunks, unsorted, big, ctrl);
     return cudaPeekAtLastError() == cudaSuccess;
   };
-  const auto big_kernel = k_top_finish<BigTile, 1>;
-  if (!(only_big     ? finish(big_kernel, BigTile{}, 1u, even_run, 0u, &allowed[2])
-        : small_tile ? finish(k_top_finish<SmallTile, 4>, SmallTile{}, 4u, even_run, 0u, &allowed[1])
-                     : finish(k_top_finish<Tile, 2>, Tile{}, 2u, even_run, 0u, &allowed[0])) ||
-      (may_big && !finish(big_kernel, BigTile{}, 1u, (double)n / 65536.0, 1u, &allowed[2])))
+  if (!(small_tile ? finish(k_top_finish<SmallTile, 4>, SmallTile{}, 4u, even_run, 0u, &allowed[1])
+                   : finish(k_top_finish<Tile, 2>, Tile{}, 2u, even_run, 0u, &allowed[0])) ||
+      (big_passes && !finish(k_top_finish<BigTile, 1>, BigTile{}, 1u, (double)n / (big_passes == 1u ? 256.0 : 65536.0), 1u, &allowed[2])))
     return 5;
   if (cudaPeekAtLastError() != cudaSuccess) return 5;
   return top_merge(X, Y, n, chunks, unsorted, ctrl, dev, st);

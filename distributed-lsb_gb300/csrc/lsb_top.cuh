@@ -92,7 +92,9 @@ struct SampleRule {
   uint32_t near_limit;  // neighbours that may share a window before the mean run is too long
   uint32_t dups;        // equal neighbours from which most keys occur eight times or more
   uint32_t far_limit;   // keys in runs longer than a tile that are put up with
-  uint32_t big_near;    // near_limit for the big tile; 0: it is not to be had
+  uint32_t big_passes;  // passes that leave runs for the big tile, one less than tmin; 0: it is not to be had
+  uint32_t big_near;    // near_limit and far for it
+  uint32_t big_far;
   uint32_t finish;      // time of the last step
   uint32_t uneven;      // more of it where keys are too unevenly spread
   uint32_t straddle;    // and where only the tiles between clusters of keys are
@@ -117,7 +119,7 @@ __host__ __device__ inline SampleRule sample_rule(uint32_t n, uint32_t sample, u
   SampleRule r;
   const float per = (float)sample / (float)n;
   r.tmin = passes_for((float)n, (float)mean_run);
-  r.big_near = 0u;
+  r.big_passes = r.big_near = r.big_far = 0u;
   // the last step over a pass, 2^24 to 2^30 elements: 1.0 to 1.16; of uneven tiles,
   // sort_spread or bits: 2^24 pairs of 20 bits in 52, 504 us and a pass 127; 2^24
   // elements in a batch, nibbles, 2160 and 380
@@ -248,6 +250,7 @@ struct SampleChoice {
 // Counts over the sorted sample; zeroed by its owner before the sample is sorted.
 struct SampleStats {
   uint32_t near[8], far[8];  // keys that share T windows with the next one, with the one rule.far - 1 places on
+  uint32_t big_far;          // keys that share rule.big_passes windows with the one rule.big_far - 1 places on
   uint32_t equal, diff[2];   // equal neighbours, bits in which keys differ
   SampleChoice choice;
 };
@@ -262,14 +265,15 @@ __device__ __forceinline__ void clear_stats(SampleStats& st) {
 // tell: tags, sentinels, signs, text, exponents) that step takes several times as
 // long, and more windows are passed over, up to all of them. plain_passes: passes of
 // a sort by every byte, 0: those in which the sample differs. low_bit(t): the lowest
-// bit of the key in t windows; key_bits: those that vary (0: the sample's).
-template <int S, class LowBit>
+// bit of the key in t windows; key_bits: those that vary (0: the sample's). BIG: there
+// is a kernel for the big tile.
+template <int S, bool BIG = false, class LowBit>
 __device__ __forceinline__ SampleChoice choose_passes(const uint64_t* s, uint32_t hb1, const SampleRule& rule,
                                                       uint32_t plain_passes, SampleStats& st, uint64_t key_bits, LowBit low_bit) {
   // nibble T-1 of near / far: this thread's keys that share T windows (but
   // not all 64 bits) with the next key / with the key `far` places on
   constexpr uint32_t kSample = (uint32_t)(S * kSampleThreads);
-  uint32_t near = 0, farm = 0, equal = 0;
+  uint32_t near = 0, farm = 0, equal = 0, big_far = 0;
   uint64_t diff = 0;
   bool heavy = false;
 #pragma unroll
@@ -286,6 +290,8 @@ __device__ __forceinline__ SampleChoice choose_passes(const uint64_t* s, uint32_
       else equal++;
     }
     if (i + rule.far - 1u < kSample && s[i + rule.far - 1u] != ki) farm += shared_windows(i + rule.far - 1u);
+    if (BIG && rule.big_passes && i + rule.big_far - 1u < kSample && s[i + rule.big_far - 1u] != ki)
+      big_far += shared_windows(i + rule.big_far - 1u) >> (4u * (rule.big_passes - 1u)) & 1u;
     heavy |= i + rule.heavy - 1u < kSample && s[i + rule.heavy - 1u] == ki;
   }
   {
@@ -295,6 +301,7 @@ __device__ __forceinline__ SampleChoice choose_passes(const uint64_t* s, uint32_
     const uint32_t f1 = __reduce_add_sync(0xffffffffu, (farm >> 4) & 0x0F0F0F0Fu);
     const uint32_t d0 = __reduce_or_sync(0xffffffffu, (uint32_t)diff), d1 = __reduce_or_sync(0xffffffffu, (uint32_t)(diff >> 32));
     equal = __reduce_add_sync(0xffffffffu, equal);
+    if (BIG) big_far = __reduce_add_sync(0xffffffffu, big_far);
     const uint32_t l = lane_id();
     if (l < 8) {
       atomicAdd(&st.near[l], ((l & 1u ? n1 : n0) >> (8u * (l >> 1))) & 0xFFu);
@@ -302,6 +309,7 @@ __device__ __forceinline__ SampleChoice choose_passes(const uint64_t* s, uint32_
     }
     if (l == 0) {
       if (equal) atomicAdd(&st.equal, equal);
+      if (BIG && big_far) atomicAdd(&st.big_far, big_far);
       atomicOr(&st.diff[0], d0);
       atomicOr(&st.diff[1], d1);
     }
@@ -343,10 +351,11 @@ __device__ __forceinline__ SampleChoice choose_passes(const uint64_t* s, uint32_
     const uint32_t ok = __ballot_sync(0xffffffffu, at_all && (t == full || enough(rule.near_limit)));
     const uint32_t first = (uint32_t)__ffs((int)ok) - 1u;
     const uint32_t best = __reduce_min_sync(0xffffffffu, at_all && t >= first && (t == first || even) ? time << 8 | t : ~0u);
-    const bool fits_big = t == 2u && full > 3u && even && rule.big_near && enough(rule.big_near) && !many_dups && varies == bits_below(hb1, 64u);
-    // a pass less for the big tile, whose runs are the two top windows' and even
-    const bool big = first == 3u && __any_sync(0xffffffffu, fits_big);
-    const uint32_t passes = big ? 2u : varies == 0ull ? min(rule.tmin, full) : best & 255u;
+    // a pass less for the big tile, whose runs are even and of the one or two top windows
+    const bool fits_big = BIG && counts && t == rule.big_passes && full > t + 1u && even && near_t <= rule.big_near && st.big_far <= rule.far_limit &&
+                          !heavy && !many_dups && varies == bits_below(hb1, 64u);
+    const bool big = BIG && first == rule.big_passes + 1u && __any_sync(0xffffffffu, fits_big);
+    const uint32_t passes = big ? rule.big_passes : varies == 0ull ? min(rule.tmin, full) : best & 255u;
     const uint32_t every = plain_passes ? plain_passes : (uint32_t)__popc(bytes);
     const uint32_t plain = 10u * every + (every > 4u || full <= 4u ? 3u : 0u) + ((every & 1u) ? rule.copy : 0u);
     const uint32_t near_of = __shfl_sync(0xffffffffu, near_t, (int)passes);
