@@ -186,6 +186,11 @@ struct TileSort {
     // bins that follow the keys at once, unless most of them are duplicates, which
     // the sort by even bins has its own ways with, if it can; then they are better than bits
     bool strict = kSpreads && uneven == Uneven::kSpread && !first_try && rounds > kFewRounds;
+    if (strict) {  // of keys that occur five times and more in the tile, eight of the CTA's have an equal in their warp
+      const uint64_t key = in[lo + threadIdx.x * (hi - lo) / (uint32_t)THREADS].key;
+      const uint32_t same = __match_any_sync(0xffffffffu, (unsigned long long)key);
+      strict = __syncthreads_count(__ffs((int)same) - 1 != (int)lane) < (int)(THREADS / 64);
+    }
     for (bool even = true;; strict = false, even = false) {
       if constexpr (kSpreads)
         if ((strict || !even) && sort_spread(in, lo, hi, mn, mx, strict, slot, bins, sh, emit)) return;
