@@ -424,9 +424,11 @@ __global__ void __launch_bounds__(Tile::kThreads, 2)
   uint32_t* bins = reinterpret_cast<uint32_t*>(smem + Tile::kElemBytes + Tile::kSlotBytes);
   const uint32_t tid = threadIdx.x, warp = tid >> 5;
   const uint32_t steps = 2u + ctrl->top.max_rounds;
-  // eight items for each CTA: an item costs a trip to the ticket and two barriers
-  // (2^28 Zipf keys, 58000 chunks in order: 11.2 ms the sort with an item per chunk, 10.0 so)
-  const uint32_t per = total / (gridDim.x * 8u) + 1u, items = (total - 1u) / per + 1u;
+  // sixteen items for each CTA: an item costs a trip to the ticket and two barriers, and
+  // few of them leave CTAs idle at a step's end (2^28 Zipf keys, 58000 chunks in order:
+  // 11.2 ms the sort with an item per chunk, 10.2 so, 10.1 with eight for each; keys
+  // that occur a thousand times: 16.1 with one for each, 15.4 with eight, 15.05 so)
+  const uint32_t items = min(total, gridDim.x * 16u);
   auto rounds_of = [](const RunChunk& t) { return 32u - (uint32_t)__clz((int)((t.e - t.b - 1u) / kCap)); };
   uint32_t step_now = 0;
   if (tid == 0) s_item = atomicAdd(&ctrl->top.merge_ticket, 1u);
@@ -447,7 +449,7 @@ __global__ void __launch_bounds__(Tile::kThreads, 2)
       if (!s_go) return;
       step_now = step;
     }
-    for (uint32_t c = item % items * per; c < min(total, (item % items + 1u) * per); c++) {
+    for (uint32_t c = item % items; c < total; c += items) {  // (neighbours are chunks of one run: all to be merged, or none)
       const RunChunk t = chunks[c];
       const uint32_t len = t.e - t.b, pos = t.k * kCap, cnt = min(kCap, len - pos);
       if (step == 0u) {
