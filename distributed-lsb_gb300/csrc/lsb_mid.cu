@@ -110,8 +110,8 @@ __device__ __forceinline__ uint64_t gather_bits(uint64_t key, uint64_t bits) {
 }
 
 // The runs that start in [g, limit) of src[0, n), into X.
-__device__ __forceinline__ void mid_finish(const Elem* src, Elem* X, uint32_t n, uint32_t g, uint32_t limit, bool known, const RunKey& w, bool clamped,
-                                           bool skewed, bool dups, uint32_t shift, unsigned char* smem, MidTile::Shared& sh, RunMarks& marks, MidRun* runs,
+__device__ __forceinline__ void mid_finish(const Elem* src, Elem* X, uint32_t n, uint32_t g, uint32_t limit, bool known, const RunKey& w, const bool& clamped,
+                                           const bool& skewed, const bool& dups, uint32_t shift, unsigned char* smem, MidTile::Shared& sh, RunMarks& marks, MidRun* runs,
                                         uint32_t max_runs, Ctrl* ctrl) {
   Elem* in = reinterpret_cast<Elem*>(smem);
   uint32_t* slot = reinterpret_cast<uint32_t*>(smem + MidTile::kElemBytes);

@@ -449,7 +449,7 @@ struct RunMarks {
 };
 template <class TS, class Load, class Long>
 __device__ __forceinline__ bool sort_runs(const Elem* src, Elem* X, uint32_t n, uint32_t g, uint32_t limit, bool known,
-                                          const RunKey& w, bool clamped, bool skewed, bool dups, uint32_t shift, const Elem* in, uint32_t* slot,
+                                          const RunKey& w, const bool& clamped, const bool& skewed, const bool& dups, uint32_t shift, const Elem* in, uint32_t* slot,
                                           uint32_t* bins, typename TS::Shared& sh, RunMarks& marks, Load load,
                                           Long long_run) {
   constexpr uint32_t kNone = 0xffffffffu;
@@ -541,8 +541,9 @@ __device__ __forceinline__ bool sort_runs(const Elem* src, Elem* X, uint32_t n, 
         range = (r1 << shift | ((1ull << shift) - 1ull)) - base;
       }
       Elem* out = X + w0 + from;
-      TS::sort(in, from, end, base, range, slot, bins, sh, in_place, dups ? Uneven::kDups : Uneven::kSpread,
-               [=](bool on, uint32_t r, const Elem& e) { store_elem_if(on, out + r, e); });
+      auto emit = [=](bool on, uint32_t r, const Elem& e) { store_elem_if(on, out + r, e); };
+      if (range == 0 || !TS::template sort_even<false>(in, from, end, TS::make_scale(base, range), slot, bins, sh, emit))
+        TS::sort_any(in, from, end, slot, bins, sh, range == 0, in_place, dups ? Uneven::kDups : Uneven::kSpread, emit);
     } else if (first > 0u) {  // one run from `first`, not whole in the tile yet
       g = w0 + first;
     } else {  // a run of at least a tile
