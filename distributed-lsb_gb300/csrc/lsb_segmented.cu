@@ -52,7 +52,9 @@ __global__ void __launch_bounds__(kSampleThreads, 2)
       const uint64_t first = k[0], span = first ^ k[kSegSample * kSampleThreads - 1];
       if (span) p.hb1 = 64u - (uint32_t)__clzll((long long)span);
       // a key that overfills its bins is heavy (lsb_mid.cu); four passes leave
-      // its runs pure up to 2^28 elements
+      // its runs pure up to 2^28 elements. Zipf keys in arrays of 2^10 to 2^20 take
+      // 2690 us in all; with 16 windows per element for all lengths 3658. Of 2^20 to 2^23:
+      // 2031; with 2048 for all 2433.
       const float spread = fminf(2048.0f, fmaxf(16.0f, 4294967296.0f / (float)len));
       SampleRule rule = sample_rule(len, kSegSample * kSampleThreads, Tile::kCap, kMeanRun, Tile::kMaxBin, spread);
       rule.skips = false;

@@ -627,12 +627,17 @@ int top_run(Elem* X, Elem* Y, unsigned char* ws, const Layout& L, cudaStream_t s
   const uint32_t big_passes = least == 2u && n <= 256u * 7600u ? 1u : n > (1u << 27) && n <= 65536u * kBigRun ? 2u : 0u;
   const double even_run = (double)n / std::pow(256.0, (double)least);
   const bool small_tile = even_run <= (double)kSmallRun;
+  // Windows per element after which a heavy key is alone in its run: 16 ask for three
+  // passes up to 2^20 elements and for four up to 2^28, and 4 for four up to 2^30. With 2,
+  // a pass less, 2 to 5 10^6 Zipf keys take 234 and 350 us, not 150 and 266; with 16 above 2^28,
+  // a pass more, 3 10^8 of them 13.6 ms, not 11.7. (Half zeros and half even keys take
+  // less with 2: 151 -> 125, 268 -> 258 us.)
   // a smaller sample decides as well for fewer elements, and 5 us sooner
   const bool short_sample = n < (1u << 26);
   const uint32_t mean_run = small_tile ? kSmallRun : kMeanRun;
   const uint32_t tile = small_tile ? SmallTile::kCap : Tile::kCap;
   SampleRule rule = sample_rule(n, kSampleThreads * (short_sample ? 1u : (uint32_t)kTopSample), tile, mean_run, mean_run,
-                                n <= (1u << 28) ? 16.0f : 4.0f);  // four passes for heavy keys up to 2^30 elements
+                                n <= (1u << 28) ? 16.0f : 4.0f);
   if (big_passes) {
     const SampleRule wide = sample_rule(n, kSampleThreads * (short_sample ? 1u : (uint32_t)kTopSample), BigTile::kCap, kBigRun, kBigRun, 16.0f);
     rule.big_passes = big_passes;
