@@ -110,10 +110,11 @@ int mid_run(Elem* X, Elem* Y, unsigned char* ws, const Layout& L, const DeviceIn
 // 0: 512 threads x 16, 1 CTA/SM; 2: 256 x 16, 2 CTAs/SM.
 uint32_t onesweep_top_tile(int variant);
 // Pass `pass` of the plan in ctrl->top, or of a batch's plans; gstart: that
-// pass's digit starts (one array); ctas: persistent CTAs, 0 = every resident slot.
+// pass's digit starts (one array); ctas: persistent CTAs, 0 = every resident slot;
+// spare: a launch that finds nothing to do for even keys, in the profile by itself.
 int onesweep_top_pass(Elem* X, Elem* Y, uint32_t n, int pass, const uint32_t* gstart, uint64_t* ring,
                       uint32_t tiles, Ctrl* ctrl, const SegDesc& seg, int variant, uint32_t ctas,
-                      const DeviceInfo& dev, cudaStream_t st);
+                      const DeviceInfo& dev, cudaStream_t st, bool spare = false);
 // Every pass from `first` on that the plan has, in one launch; gstart: pass 0's.
 int onesweep_top_rest(Elem* X, Elem* Y, uint32_t n, int first, const uint32_t* gstart, uint64_t* ring, uint32_t tiles,
                       Ctrl* ctrl, const SegDesc& seg, int variant, uint32_t ctas, const DeviceInfo& dev, cudaStream_t st);

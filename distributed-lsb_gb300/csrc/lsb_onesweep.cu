@@ -1493,14 +1493,14 @@ int onesweep_top_rest(Elem* X, Elem* Y, uint32_t n, int first, const uint32_t* g
 
 int onesweep_top_pass(Elem* X, Elem* Y, uint32_t n, int pass, const uint32_t* gstart, uint64_t* ring,
                       uint32_t tiles, Ctrl* ctrl, const SegDesc& seg, int variant, uint32_t ctas,
-                      const DeviceInfo& dev, cudaStream_t st) {
+                      const DeviceInfo& dev, cudaStream_t st, bool spare) {
   const int threads = variant == 2 ? 256 : 512;
   auto kern = variant == 2 ? k_onesweep<256, 16, 2, uint32_t, 8, true> : k_onesweep<512, 16, 1, uint32_t, 8, true>;
   const size_t smem = reg_kernel_smem(8, threads, 16);
   static std::atomic<uint64_t> allowed[2];
   if (!allow_smem((const void*)kern, smem, &allowed[variant == 2 ? 1 : 0])) return 5;
   const uint32_t grid = top_grid(tiles, variant, ctas, dev);
-  ProfScope prof("onesweep_scatter", st);
+  ProfScope prof(spare ? "onesweep_spare" : "onesweep_scatter", st);
   // one ring slot per tile: no slot is reused, so there are no completion tags
   kern<<<grid, threads, smem, st>>>(X, Y, n, 8, pass, 0, gstart, ring, nullptr, tiles, ctrl, seg);
   return cudaPeekAtLastError() == cudaSuccess ? 0 : 5;

@@ -657,7 +657,7 @@ int top_run(Elem* X, Elem* Y, unsigned char* ws, const Layout& L, cudaStream_t s
   }
   if (int rc = top_hist(X, ws, L, 0u, dev, st)) return rc;
   for (uint32_t p = 0; p < lead; p++)  // (one may not be in the plan: the big tile's)
-    if (int rc = onesweep_top_pass(X, Y, n, (int)p, gstart + p * 256u, ring, L.ring_tiles, ctrl, SegDesc{}, 0, 0u, dev, st))
+    if (int rc = onesweep_top_pass(X, Y, n, (int)p, gstart + p * 256u, ring, L.ring_tiles, ctrl, SegDesc{}, 0, 0u, dev, st, p >= rule.tmin))
       return rc;
   if (int rc = onesweep_top_rest(X, Y, n, (int)lead, gstart, ring, L.ring_tiles, ctrl, SegDesc{}, 0, 0u, dev, st))
     return rc;

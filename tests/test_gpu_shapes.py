@@ -150,6 +150,21 @@ def test_passes_not_merges(lsb, cuda, n):
         assert ms["top_merge"] < 0.2 * sum(ms.values()), (name, ms)
 
 
+@pytest.mark.parametrize("n,passes", [(1500001, 1), (2000003, 2), ((1 << 27) + 1, 2)])
+def test_profile_counts_passes(lsb, cuda, n, passes):
+    """Launches that find nothing to do are not among the pass launches whose mean
+    time a profile gives: even keys make all of those."""
+    torch = cuda
+    a = _array(torch, torch.randint(SIGN, (1 << 63) - 1, (n,), dtype=torch.int64, device="cuda"))
+    A, B = a.clone(), torch.empty_like(a)
+    lsb.profile_enable(True)
+    lsb.sort_pairs(A, B, 16)
+    torch.cuda.synchronize()
+    lsb.profile_enable(False)
+    assert lsb.profile_read()["onesweep_scatter"][0] == passes
+    assert lsb.verify(a, A) == 0
+
+
 @pytest.mark.parametrize("n", [1, 8193, 8192 * 152 + 77, 3000001])
 def test_pass_over_a_constant_digit(lsb, cuda, n):
     """A single pass whose digit is the same in all keys copies the array, over more
