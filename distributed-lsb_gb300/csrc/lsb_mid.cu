@@ -22,9 +22,9 @@
 //      missed them) have the array passed over by every digit that differs.
 // Bound by latency: about four grid barriers and as many trips to L2. Measured
 // (GB300, sort alone, eight launched passes -> this): 2 10^4 uniform keys 135 ->
-// 24 us, 2 10^5 152 -> 30, 1.1 10^6 157 -> 47; Zipf keys (four digits) 2 10^5 153 -> 88,
-// 1.1 10^6 155 -> 148. Above 622592 elements (152 SMs) a pass takes 18 us, and keys that
-// need seven or eight (exponents, many clusters) 175 in all where eight launched
+// 23 us, 2 10^5 152 -> 30, 1.1 10^6 157 -> 44; Zipf keys (four digits) 2 10^5 153 -> 82,
+// 1.1 10^6 155 -> 137. Above 622592 elements (152 SMs) a pass takes 18 us, and keys that
+// need seven or eight (exponents, many clusters) 170 in all where eight launched
 // passes took 154. The tile
 // stays in shared memory, not in registers: with 1024 threads its elements
 // spill, and beside 217 KB of shared memory there is no L1 to spill to (a
