@@ -150,6 +150,34 @@ def test_passes_not_merges(lsb, cuda, n):
         assert ms["top_merge"] < 0.2 * sum(ms.values()), (name, ms)
 
 
+@pytest.mark.parametrize("kind", ["thousandfold", "clusters"])
+def test_big_tile_only_where_it_fits(lsb, cuda, kind):
+    """1.5 million keys of a thousand equals each, or in a hundred clusters: one pass
+    leaves many of their runs longer than any tile, so that the sample has to say no
+    to the tile that takes the runs of even keys after one pass."""
+    torch = cuda
+    n = 1500001
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n)
+    few = torch.randint(SIGN, (1 << 63) - 1, (n // 1000 if kind == "thousandfold" else 100,), dtype=torch.int64, device="cuda", generator=g)
+    keys = few[torch.randint(0, few.shape[0], (n,), device="cuda", generator=g)]
+    if kind == "clusters":
+        keys = keys + torch.randint(0, 1 << 32, (n,), dtype=torch.int64, device="cuda", generator=g)
+    a = _array(torch, keys)
+    A, B = a.clone(), torch.empty_like(a)
+    ws = lsb.alloc_workspace(n, 16)
+    for timed in (False, True):
+        A.copy_(a)
+        torch.cuda.synchronize()
+        lsb.profile_enable(timed)
+        lsb.sort_pairs(A, B, 16, workspace=ws)
+        torch.cuda.synchronize()
+    lsb.profile_enable(False)
+    ms = {k: v[1] for k, v in lsb.profile_read().items()}
+    assert lsb.query(ws).device_status == 0 and lsb.verify(a, A) == 0
+    assert ms["top_merge"] < 0.2 * sum(ms.values()), ms
+
+
 @pytest.mark.parametrize("n,passes", [(1500001, 1), (2000003, 2), ((1 << 27) + 1, 2)])
 def test_profile_counts_passes(lsb, cuda, n, passes):
     """Launches that find nothing to do are not among the pass launches whose mean
